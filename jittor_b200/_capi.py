@@ -4,12 +4,15 @@ The library is the only compute path of this package: if it is missing the impor
 instructions to build it, and a call without a CUDA device raises -- there is no CPU fallback.
 """
 import ctypes
+import importlib.util
 import os
+import threading
 
 import torch
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "csrc", "libb200jt.so")
+HOST_PATH = os.path.join(_HERE, "csrc", "_b200jt_host.so")
 
 MAX_DIMS = 10
 
@@ -36,7 +39,17 @@ def _load():
     return ctypes.CDLL(LIB_PATH)
 
 
+def _load_host():
+    if not os.path.exists(HOST_PATH):
+        raise ImportError(f"{HOST_PATH} not found: build it with `make -C {os.path.join(_HERE, 'csrc')}`")
+    spec = importlib.util.spec_from_file_location("_b200jt_host", HOST_PATH)
+    mod = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(mod)
+    return mod
+
+
 lib = _load()
+host = _load_host()
 
 _TP = ctypes.POINTER(Tensor)
 _SP = ctypes.POINTER(ctypes.c_char_p)
@@ -160,3 +173,140 @@ def descs(tensors):
 
 def stream_ptr():
     return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+
+
+# ---- allocations and launches of a plan -----------------------------------------------------------------------------
+# Plans allocate and launch through the functions below. While a graph is run for the first time, `recorder` writes each of
+# them down with its pointers as (buffer number, offset); csrc/host.cpp replays that tape when a graph of the same structure
+# is synced again.
+ARGTYPES = {name: args for name, _, args in SIGNATURES}
+recorder = None
+SCALAR_TYPES = {torch.uint8: 0, torch.int8: 1, torch.int16: 2, torch.int32: 3, torch.int64: 4, torch.float16: 5,
+                torch.float32: 6, torch.float64: 7, torch.bool: 11, torch.bfloat16: 15}
+
+
+class _NotReplayable(Exception):
+    pass
+
+
+def recording():
+    return recorder is not None and recorder.thread == threading.get_ident()
+
+
+class Recorder:
+    def __init__(self, leaves):
+        self.ok = True
+        self.thread = threading.get_ident()   # what other threads launch meanwhile is not part of this graph
+        self.steps = []
+        self.spans = []                       # (base, bytes) per buffer
+        self.keep = []                        # nothing is freed while recording, so an address names one buffer
+        for t in leaves:
+            self._add(t)
+
+    def _add(self, t):
+        self.spans.append((t.data_ptr(), t.numel() * t.element_size()))
+        self.keep.append(t)
+        return len(self.spans) - 1
+
+    def locate(self, ptr):
+        for k in range(len(self.spans) - 1, -1, -1):
+            base, n = self.spans[k]
+            if n and base <= ptr < base + n:
+                return k, ptr - base
+        raise _NotReplayable(f"pointer {ptr:#x} belongs to no buffer of the plan")
+
+    def alloc(self, t):
+        k = self._add(t)
+        self.steps.append(("alloc", k, tuple(t.shape), SCALAR_TYPES[t.dtype]))
+        return k
+
+    def _tensor(self, d):
+        buf, off = self.locate(d.ptr) if d.ptr else (-1, 0)
+        return (d.dtype, tuple(d.shape[:d.ndim]), buf, off)
+
+    def _args(self, name, args):
+        out, last = [], -1
+        for a, ty in zip(args, ARGTYPES[name]):
+            if isinstance(a, Tensor):
+                out.append(("T", [self._tensor(a)]))
+            elif isinstance(a, ctypes.Array) and a._type_ is Tensor:
+                out.append(("T", [self._tensor(d) for d in a]))
+            elif isinstance(a, ctypes.Array) and a._type_ is ctypes.c_char_p:
+                out.append(("S", [s for s in a if s is not None]))
+            elif isinstance(a, ctypes.Array) and a._type_ in (ctypes.c_int64, ctypes.c_int32):
+                out.append(("q" if a._type_ is ctypes.c_int64 else "w", list(a)))
+            elif isinstance(a, bytes):
+                out.append(("b", a))
+            elif ty in (ctypes.c_double,):
+                out.append(("d", float(a)))
+            elif ty is ctypes.c_size_t:
+                out.append(("n", last) if last >= 0 else ("i", int(a)))       # the size of the workspace passed before it
+            elif ty is ctypes.c_void_p or a is None:
+                v = a.value if isinstance(a, ctypes.c_void_p) else a
+                if v:
+                    last, off = self.locate(v)
+                    out.append(("p", last, off))
+                else:
+                    last = -1
+                    out.append(("0",))
+            else:
+                out.append(("i", int(a)))
+        return out
+
+    def note(self, fn, *args):
+        if self.ok:
+            try:
+                fn(*args)
+            except _NotReplayable:
+                self.ok = False
+
+    def call(self, name, args):
+        self.note(lambda: self.steps.append(("call", -1, name, self._args(name, args) + [("z",)])))
+
+    def workspace(self, name, args, t):
+        k = self._add(t)
+        self.note(lambda: self.steps.append(("workspace", k, name, self._args(name, args))))
+
+    def fill(self, t, value):
+        def write():
+            if isinstance(value, int) and abs(value) >= 1 << 53:
+                raise _NotReplayable("an integer a double does not hold")
+            self.steps.append(("fill", self.locate(t.data_ptr())[0], float(value)))
+        if t.numel():
+            self.note(write)
+
+
+def alloc(shape, dtype):
+    """An uninitialised CUDA tensor of a plan; `dtype` is a torch dtype."""
+    t = torch.empty(shape, dtype=dtype, device="cuda")
+    if recording():
+        recorder.alloc(t)
+    return t
+
+
+def full(shape, value, dtype):
+    t = torch.full(shape, value, dtype=dtype, device="cuda")
+    if recording():
+        recorder.alloc(t)
+        recorder.fill(t, value)
+    return t
+
+
+def workspace(name, *args):
+    """(bytes, pointer, tensor that owns it) of the scratch memory `name` asks for."""
+    n = getattr(lib, name)(*args)
+    if n == 0:
+        return 0, None, None
+    t = torch.empty(int(n), dtype=torch.uint8, device="cuda")
+    if recording():
+        recorder.workspace(name, args, t)
+    return n, t.data_ptr(), t
+
+
+def call(name, *args, what=None):
+    """Launches entry point `name` on the current stream (its last argument)."""
+    rc = getattr(lib, name)(*args, stream_ptr())
+    if rc:
+        check(rc, what() if callable(what) else what or name)
+    if recording():
+        recorder.call(name, args)

@@ -80,6 +80,7 @@ class overlap_collectives:
     def _reserve(self):
         from . import _capi as C
         C.check(C.lib.b200jt_set_sm_reserve(self.sms), "set_sm_reserve")
+        C.host.set_context(self.sms)                # plans made for a smaller grid are kept apart
         C.check(C.lib.b200jt_peer_comm_set_max_blocks(_PEER._h, self.blocks), "peer max blocks")
 
     def __enter__(self):
@@ -118,6 +119,7 @@ class overlap_collectives:
             _OVERLAP["active"] = False
             _OVERLAP["scope"] = None
             C.lib.b200jt_set_sm_reserve(0)
+            C.host.set_context(0)
             C.lib.b200jt_peer_comm_set_max_blocks(_PEER._h, 0)
         return False
 

@@ -23,7 +23,19 @@ from . import dtypes as dt
 from .var import Var
 
 _MATERIALIZE_LIMIT = 1 << 33       # elements; beyond this an unfused intermediate is refused
-counters = {"plans": 0}            # plans run so far: one per kernel group, the analogue of the reference's fused-op count
+
+
+class _Counters(dict):
+    """"plans": plans run so far, one per kernel group (the analogue of the reference's fused-op count); replayed plans are
+    counted natively and added when somebody looks."""
+
+    def __getitem__(self, k):
+        if k == "plans":
+            dict.__setitem__(self, k, dict.__getitem__(self, k) + C.host.take_plans())
+        return dict.__getitem__(self, k)
+
+
+counters = _Counters(plans=0)
 
 
 class Plan:
@@ -35,6 +47,47 @@ class Plan:
 
 
 def realize(roots):
+    """Computes the roots. A graph of a structure that ran before is replayed natively (csrc/host.cpp); others are planned
+    here, and the first run of a structure is written to a tape for the next."""
+    if C.host.realize(roots):
+        return
+    _realize(roots)
+
+
+def _realize(roots):
+    if C.recording():
+        C.recorder.ok = False                       # a plan that syncs other graphs (running statistics moved op by op)
+    _run_plans(roots)
+
+
+def _record(roots, nodes, leaves):
+    """Runs the planner over `roots` with its allocations and launches recorded. Returns what host.cpp makes a tape of, or
+    None if the run did something a tape does not hold."""
+    before = counters["plans"]
+    bn = [v for v in nodes if v._bn_running is not None]
+    C.recorder = rec = C.Recorder([v._data for v in leaves])
+    try:
+        _run_plans(roots)
+        results = []
+        for i, v in enumerate(nodes):
+            if v._data is None:
+                continue
+            if v._data.numel() == 0 or not v._data.is_contiguous():
+                return None
+            try:
+                buf, off = rec.locate(v._data.data_ptr())
+            except C._NotReplayable:
+                return None
+            results.append((i, buf, off, tuple(v._data.shape)))
+    finally:
+        C.recorder = None
+    if not rec.ok:
+        return None
+    done = [i for i, v in enumerate(nodes) if v._bn_running is None and any(v is b for b in bn)]
+    return len(rec.spans), rec.steps, results, done, counters["plans"] - before
+
+
+def _run_plans(roots):
     for root in roots:
         stack = [root]
         plans = {}
@@ -58,7 +111,7 @@ def realize(roots):
             v._data = out.reshape(list(v.shape))
             plans.pop(id(v), None)
             stack.pop()
-            pending_update = getattr(v, "_bn_running", None)
+            pending_update = v._bn_running
             if pending_update is not None:          # a BatchNorm output computed op by op: move its running statistics now
                 v._bn_running = None
                 module, xmean, xvar = pending_update
@@ -66,7 +119,7 @@ def realize(roots):
 
 
 def _make_plan(v):
-    relay = getattr(v, "_relay", None)
+    relay = v._relay
     if relay is not None:                       # a convolution built by nn with its relay record (its graph may not be written yet)
         kind, x, w, geo, groups = relay
         if x.dtype in ("float32", "bfloat16") and w.dtype in ("float32", "bfloat16"):
@@ -90,14 +143,7 @@ def _make_plan(v):
 # --------------------------------------------------------------------------------- helpers
 def _empty(shape, dtype):
     C.require_cuda()
-    return torch.empty(list(shape), dtype=C.TORCH_DTYPES[str(dtype)], device="cuda")
-
-
-def _workspace(nbytes):
-    if nbytes == 0:
-        return None, ctypes.c_void_p(0)
-    ws = torch.empty(int(nbytes), dtype=torch.uint8, device="cuda")
-    return ws, ctypes.c_void_p(ws.data_ptr())
+    return C.alloc(list(shape), C.TORCH_DTYPES[str(dtype)])
 
 
 def _cast(t, dtype):
@@ -105,7 +151,7 @@ def _cast(t, dtype):
     if C.DTYPE_NAMES[t.dtype] == str(dtype):
         return t
     out = _empty(t.shape, dtype)
-    C.check(C.lib.b200jt_unary(C.desc(t), C.desc(out), str(dtype).encode(), C.stream_ptr()), f"cast({dtype})")
+    C.call("b200jt_unary", C.desc(t), C.desc(out), str(dtype).encode(), what=lambda: f"cast({dtype})")
     return out
 
 
@@ -121,7 +167,7 @@ def _node(v, kind, **attrs):
 
 
 def _const(v):
-    return getattr(v, "_const", None)
+    return v._const
 
 
 def _strip_cast(v, to):
@@ -137,10 +183,9 @@ def _run_reindex(v, op):
     out = _empty(v.shape, v.dtype)
     a = op.attrs
     keep = [e._data for e in extras]
-    C.check(C.lib.b200jt_reindex(C.desc(x._data), C.desc(out), C.strings(a["indexes"]), len(a["indexes"]),
-                                 a["overflow_value"], C.strings(a["overflow_conditions"]),
-                                 len(a["overflow_conditions"]), C.descs(keep), len(keep), C.stream_ptr()),
-            f"reindex {list(x.shape)}->{list(v.shape)} {a['indexes']}")
+    C.call("b200jt_reindex", C.desc(x._data), C.desc(out), C.strings(a["indexes"]), len(a["indexes"]), a["overflow_value"],
+           C.strings(a["overflow_conditions"]), len(a["overflow_conditions"]), C.descs(keep), len(keep),
+           what=lambda: f"reindex {list(x.shape)}->{list(v.shape)} {a['indexes']}")
     return out
 
 
@@ -151,10 +196,9 @@ def _run_reindex_reduce(v, op):
     keep = [e._data for e in extras]
     args = (C.desc(y._data), C.desc(out), a["op"].encode(), C.strings(a["indexes"]), len(a["indexes"]),
             C.strings(a["overflow_conditions"]), len(a["overflow_conditions"]), C.descs(keep), len(keep))
-    nbytes = C.lib.b200jt_reindex_reduce_workspace(*args)
-    ws, wsp = _workspace(nbytes)
-    C.check(C.lib.b200jt_reindex_reduce(*args, wsp, nbytes, C.stream_ptr()),
-            f"reindex_reduce({a['op']}) {list(y.shape)}->{list(v.shape)} {a['indexes']}")
+    nbytes, wsp, ws = C.workspace("b200jt_reindex_reduce_workspace", *args)
+    C.call("b200jt_reindex_reduce", *args, wsp, nbytes,
+           what=lambda: f"reindex_reduce({a['op']}) {list(y.shape)}->{list(v.shape)} {a['indexes']}")
     return out
 
 
@@ -183,7 +227,7 @@ def _run_broadcast(v, op):
             eff |= 1 << i
         elif view[i] != v.shape[i]:
             raise C.B200Error(f"broadcast: cannot stretch {list(x.shape)} to {list(v.shape)}")
-    C.check(C.lib.b200jt_broadcast_to(C.desc(x._data, view), C.desc(out), eff, C.stream_ptr()), "broadcast_to")
+    C.call("b200jt_broadcast_to", C.desc(x._data, view), C.desc(out), eff, what="broadcast_to")
     return out
 
 
@@ -194,10 +238,8 @@ def _run_reduce(v, op):
     out = _empty(v.shape, v.dtype)
     name = op.attrs["op"].encode()
     xd, yd = C.desc(x._data), C.desc(out, yfull)
-    nbytes = C.lib.b200jt_reduce_workspace(xd, yd, name, mask)
-    ws, wsp = _workspace(nbytes)
-    C.check(C.lib.b200jt_reduce(xd, yd, name, mask, wsp, nbytes, C.stream_ptr()),
-            f"reduce({op.attrs['op']}) {list(x.shape)} mask {mask:b}")
+    nbytes, wsp, ws = C.workspace("b200jt_reduce_workspace", xd, yd, name, mask)
+    C.call("b200jt_reduce", xd, yd, name, mask, wsp, nbytes, what=lambda: f"reduce({op.attrs['op']}) {list(x.shape)} mask {mask:b}")
     return out
 
 
@@ -205,17 +247,15 @@ def _run_binary(v, op):
     x, y = op.inputs
     out = _empty(v.shape, v.dtype)
     r = v.ndim
-    C.check(C.lib.b200jt_binary(C.desc(x._data, _pad_shape(x.shape, r)), C.desc(y._data, _pad_shape(y.shape, r)),
-                                C.desc(out), op.attrs["op"].encode(), C.stream_ptr()),
-            f"binary({op.attrs['op']}) {list(x.shape)} {list(y.shape)}")
+    C.call("b200jt_binary", C.desc(x._data, _pad_shape(x.shape, r)), C.desc(y._data, _pad_shape(y.shape, r)), C.desc(out),
+           op.attrs["op"].encode(), what=lambda: f"binary({op.attrs['op']}) {list(x.shape)} {list(y.shape)}")
     return out
 
 
 def _run_unary(v, op):
     x = op.inputs[0]
     out = _empty(v.shape, v.dtype)
-    C.check(C.lib.b200jt_unary(C.desc(x._data), C.desc(out), op.attrs["op"].encode(), C.stream_ptr()),
-            f"unary({op.attrs['op']})")
+    C.call("b200jt_unary", C.desc(x._data), C.desc(out), op.attrs["op"].encode(), what=lambda: f"unary({op.attrs['op']})")
     return out
 
 
@@ -224,8 +264,8 @@ def _run_ternary(v, op):
     out = _empty(v.shape, v.dtype)
     r = v.ndim
     xd, yd = x._data, y._data
-    C.check(C.lib.b200jt_ternary(C.desc(c._data, _pad_shape(c.shape, r)), C.desc(xd, _pad_shape(x.shape, r)),
-                                 C.desc(yd, _pad_shape(y.shape, r)), C.desc(out), C.stream_ptr()), "ternary")
+    C.call("b200jt_ternary", C.desc(c._data, _pad_shape(c.shape, r)), C.desc(xd, _pad_shape(x.shape, r)),
+           C.desc(yd, _pad_shape(y.shape, r)), C.desc(out), what="ternary")
     return out
 
 
@@ -247,7 +287,7 @@ def _run_all_reduce(v, op):
 
 def _run_fill(v, op):
     C.require_cuda()
-    return torch.full(list(v.shape), op.attrs["value"], dtype=C.TORCH_DTYPES[str(v.dtype)], device="cuda")
+    return C.full(list(v.shape), op.attrs["value"], C.TORCH_DTYPES[str(v.dtype)])
 
 
 def _run_custom(v, op):
@@ -432,8 +472,8 @@ def _swap01(t):
     a, b, c, d = t.shape
     out = _empty([b, a, c, d], C.DTYPE_NAMES[t.dtype])
     idx = ["i1", "i0", "i2", "i3"]
-    C.check(C.lib.b200jt_reindex(C.desc(t), C.desc(out), C.strings(idx), 4, 0.0, C.strings([]), 0, None, 0, C.stream_ptr()),
-            "reindex (swap of the two leading axes)")
+    C.call("b200jt_reindex", C.desc(t), C.desc(out), C.strings(idx), 4, 0.0, C.strings([]), 0, None, 0,
+           what="reindex (swap of the two leading axes)")
     return out
 
 
@@ -458,11 +498,10 @@ def _wgrad_as_conv(xd, dyd, geo, w_shape):
     xt, dyt = _swap01(xd), _swap01(dyd)                   # [C, N, H, W], [Co, N, OH, OW]
     out = _empty([Ci, Co, KH, KW], "bfloat16")
     args = (C.desc(xt), C.desc(dyt), C.desc(out), dh, dw, ph, pw, sh, sw, 1)
-    nbytes = C.lib.b200jt_conv2d_workspace(*args)
+    nbytes, wsp, ws = C.workspace("b200jt_conv2d_workspace", *args)
     if nbytes == 0:
         return None                                       # not a tensor-core shape after all
-    ws, wsp = _workspace(nbytes)
-    C.check(C.lib.b200jt_conv2d(*args, ctypes.c_void_p(0), wsp, nbytes, C.stream_ptr()), "conv2d (weight gradient form)")
+    C.call("b200jt_conv2d", *args, None, wsp, nbytes, what="conv2d (weight gradient form)")
     return _swap01(out)
 
 
@@ -476,18 +515,16 @@ def run_conv2d_backward_w(x, dy, geo, w_shape, out_dtype):
     out = _empty(w_shape, x.dtype)
     args = (C.desc(xd), C.desc(dyd), C.desc(out), *geo)
     if mode == 1:
-        nbytes = C.lib.b200jt_conv2d_backward_w_workspace(*args)
+        nbytes, wsp, ws = C.workspace("b200jt_conv2d_backward_w_workspace", *args)
         if nbytes:
-            ws, wsp = _workspace(nbytes)
-            C.check(C.lib.b200jt_conv2d_backward_w_tc(*args, wsp, nbytes, C.stream_ptr()),
-                    f"conv2d_backward_w (tensor cores) x{list(x.shape)} dy{list(dy.shape)} geo{geo}")
+            C.call("b200jt_conv2d_backward_w_tc", *args, wsp, nbytes,
+                   what=lambda: f"conv2d_backward_w (tensor cores) x{list(x.shape)} dy{list(dy.shape)} geo{geo}")
             return _cast(out, out_dtype)
     if mode:
         got = _wgrad_as_conv(xd, dyd, geo, w_shape)
         if got is not None:
             return _cast(got, out_dtype)
-    C.check(C.lib.b200jt_conv2d_backward_w(*args, C.stream_ptr()),
-            f"conv2d_backward_w x{list(x.shape)} dy{list(dy.shape)} geo{geo}")
+    C.call("b200jt_conv2d_backward_w", *args, what=lambda: f"conv2d_backward_w x{list(x.shape)} dy{list(dy.shape)} geo{geo}")
     return _cast(out, out_dtype)
 
 
@@ -500,10 +537,9 @@ def run_conv2d_backward_w_formats(x, dy, geo, kh, kw, xformat, wformat, yformat,
     dyd = _cast(dy._data.view(list(dy.shape)), x.dtype)
     out = _empty([Co, Ci, kh, kw] if wformat == "oihw" else [Co, kh, kw, Ci], x.dtype)
     args = (C.desc(xd), C.desc(dyd), C.desc(out), *geo, xformat.encode(), wformat.encode(), yformat.encode())
-    nbytes = C.lib.b200jt_conv2d_backward_w_formats_workspace(*args)
-    ws, wsp = _workspace(nbytes)
-    C.check(C.lib.b200jt_conv2d_backward_w_formats(*args, wsp, nbytes, C.stream_ptr()),
-            f"conv2d_backward_w x{list(x.shape)} ({xformat}) dy{list(dy.shape)} ({yformat}) -> {wformat} geo{geo}")
+    nbytes, wsp, ws = C.workspace("b200jt_conv2d_backward_w_formats_workspace", *args)
+    C.call("b200jt_conv2d_backward_w_formats", *args, wsp, nbytes,
+           what=lambda: f"conv2d_backward_w x{list(x.shape)} ({xformat}) dy{list(dy.shape)} ({yformat}) -> {wformat} geo{geo}")
     return _cast(out, out_dtype)
 
 
@@ -512,8 +548,8 @@ def run_conv2d_transpose(x, w, geo, groups, out_shape, out_dtype):
     xd = x._data
     wd = _cast(w._data, x.dtype)
     out = _empty(out_shape, x.dtype)
-    C.check(C.lib.b200jt_conv2d_transpose(C.desc(xd), C.desc(wd), C.desc(out), sh, sw, ph, pw, dh, dw, groups, C.stream_ptr()),
-            f"conv2d_transpose x{list(x.shape)} w{list(w.shape)} geo{geo} groups {groups}")
+    C.call("b200jt_conv2d_transpose", C.desc(xd), C.desc(wd), C.desc(out), sh, sw, ph, pw, dh, dw, groups,
+           what=lambda: f"conv2d_transpose x{list(x.shape)} w{list(w.shape)} geo{geo} groups {groups}")
     return _cast(out, out_dtype)
 
 
@@ -527,12 +563,9 @@ def run_conv2d(x, w, geo, out_dtype, stats=None, groups=1):
     wd = _cast(wd, x.dtype)
     out = _empty([N, Co, OH, OW], x.dtype)
     args = (C.desc(xd), C.desc(wd), C.desc(out), sh, sw, ph, pw, dh, dw, groups)
-    nbytes = C.lib.b200jt_conv2d_workspace(*args)
-    ws, wsp = _workspace(nbytes)
-    sp = ctypes.c_void_p(stats.data_ptr()) if stats is not None else ctypes.c_void_p(0)
-    rc = C.lib.b200jt_conv2d(*args, sp, wsp, nbytes, C.stream_ptr())
-    if rc:                                       # the message is only put together when there is one to show
-        C.check(rc, f"conv2d x{list(x.shape)} w{list(w.shape)} geo{geo}")
+    nbytes, wsp, ws = C.workspace("b200jt_conv2d_workspace", *args)
+    C.call("b200jt_conv2d", *args, stats.data_ptr() if stats is not None else None, wsp, nbytes,
+           what=lambda: f"conv2d x{list(x.shape)} w{list(w.shape)} geo{geo}")
     return _cast(out, out_dtype)
 
 
@@ -547,10 +580,9 @@ def run_conv2d_formats(x, w, geo, xformat, wformat, yformat, out_dtype):
     xd, wd = x._data, _cast(w._data, x.dtype)
     out = _empty([N, Co, OH, OW] if yformat == "abcd" else [N, OH, OW, Co], x.dtype)
     args = (C.desc(xd), C.desc(wd), C.desc(out), sh, sw, ph, pw, dh, dw, xformat.encode(), wformat.encode(), yformat.encode())
-    nbytes = C.lib.b200jt_conv2d_formats_workspace(*args)
-    ws, wsp = _workspace(nbytes)
-    C.check(C.lib.b200jt_conv2d_formats(*args, None, wsp, nbytes, C.stream_ptr()),
-            f"conv2d x{list(x.shape)} ({xformat}) w{list(w.shape)} ({wformat}) -> {yformat} geo{geo}")
+    nbytes, wsp, ws = C.workspace("b200jt_conv2d_formats_workspace", *args)
+    C.call("b200jt_conv2d_formats", *args, None, wsp, nbytes,
+           what=lambda: f"conv2d x{list(x.shape)} ({xformat}) w{list(w.shape)} ({wformat}) -> {yformat} geo{geo}")
     return _cast(out, out_dtype)
 
 
@@ -577,10 +609,8 @@ def run_matmul(a, b, trans_a, trans_b, out_dtype):
     N = b.shape[0] if trans_b else b.shape[1]
     out = _empty([M, N], a.dtype)
     args = (C.desc(ad), C.desc(bd), C.desc(out), int(trans_a), int(trans_b))
-    nbytes = C.lib.b200jt_matmul_workspace(*args)
-    ws, wsp = _workspace(nbytes)
-    C.check(C.lib.b200jt_matmul(*args, wsp, nbytes, C.stream_ptr()),
-            f"matmul a{list(a.shape)} b{list(b.shape)} t{int(trans_a)}{int(trans_b)}")
+    nbytes, wsp, ws = C.workspace("b200jt_matmul_workspace", *args)
+    C.call("b200jt_matmul", *args, wsp, nbytes, what=lambda: f"matmul a{list(a.shape)} b{list(b.shape)} t{int(trans_a)}{int(trans_b)}")
     return _cast(out, out_dtype)
 
 
@@ -671,8 +701,8 @@ def _match_batched_matmul(v):
         for idx in itertools.product(*[range(s) for s in batch[:k0]]):
             ai = tuple(i if s != 1 else 0 for i, s in zip(idx, ab))
             bi = tuple(i if s != 1 else 0 for i, s in zip(idx, bb))
-            C.check(C.lib.b200jt_batched_matmul(C.desc(a3[ai]), C.desc(b3[bi]), C.desc(o3[idx]), 0, 0, C.stream_ptr()),
-                    f"batched matmul a{list(a.shape)} b{list(b.shape)}")
+            C.call("b200jt_batched_matmul", C.desc(a3[ai]), C.desc(b3[bi]), C.desc(o3[idx]), 0, 0,
+                   what=lambda: f"batched matmul a{list(a.shape)} b{list(b.shape)}")
         return _cast(out, v.dtype)
 
     return Plan([a, b], run)
@@ -755,8 +785,8 @@ def _match_pool(v):
     def run():
         xd = x._data.view(list(x.shape))
         out = _empty([N, Cn, h, w], x.dtype)
-        C.check(C.lib.b200jt_pool2d(C.desc(xd), C.desc(out), ctypes.c_void_p(0), op.encode(), kh, kw, sh, sw, ph, pw, 1,
-                                    C.stream_ptr()), f"pool2d x{list(x.shape)} k{(kh, kw)} s{(sh, sw)} p{(ph, pw)}")
+        C.call("b200jt_pool2d", C.desc(xd), C.desc(out), None, op.encode(), kh, kw, sh, sw, ph, pw, 1,
+               what=lambda: f"pool2d x{list(x.shape)} k{(kh, kw)} s{(sh, sw)} p{(ph, pw)}")
         return _cast(out, v.dtype)
 
     return Plan([x], run)
@@ -803,7 +833,7 @@ def _match_softmax(v):
 
     def run():
         out = _empty([rows, cols], x.dtype)
-        C.check(C.lib.b200jt_softmax(C.desc(x._data, [rows, cols]), C.desc(out), int(log), C.stream_ptr()), "softmax")
+        C.call("b200jt_softmax", C.desc(x._data, [rows, cols]), C.desc(out), int(log), what="softmax")
         return out
 
     return Plan([x], run)
@@ -929,8 +959,7 @@ def _match_layernorm(v):
         out = _empty([rows, cols], xin.dtype)
         gd = C.desc(g[1]._data, [cols]) if g[0] == "var" else None
         bd = C.desc(b[1]._data, [cols]) if b[0] == "var" else None
-        C.check(C.lib.b200jt_layer_norm(C.desc(xin._data, [rows, cols]), gd, bd, C.desc(out), m["eps"],
-                                        C.stream_ptr()), "layer_norm")
+        C.call("b200jt_layer_norm", C.desc(xin._data, [rows, cols]), gd, bd, C.desc(out), m["eps"], what="layer_norm")
         return out
 
     return Plan(leaves, run)
@@ -997,7 +1026,7 @@ def _match_batchnorm(v):
             geo = conv_geometry(got[1], got[2]) or conv_geometry(got[2], got[1])
             conv = geo
     leaves = ([conv[0], conv[1]] if conv else [x]) + [p[1] for p in (g, b) if p[0] == "var"]
-    running = getattr(root, "_bn_running", None)
+    running = root._bn_running
     if running is not None:
         rm, rv = running[0].running_mean, running[0].running_var
         if rm.dtype == "float32" and rv.dtype == "float32" and rm.numel() == Cn and rv.numel() == Cn:
@@ -1006,13 +1035,13 @@ def _match_batchnorm(v):
             running = None
 
     def run():
-        stats = torch.empty(2 * Cn, dtype=torch.float32, device="cuda")
+        stats = C.alloc([2 * Cn], torch.float32)
         if conv:
             xd = run_conv2d(conv[0], conv[1], conv[2], x.dtype, stats=stats)
             x._data = xd                       # the conv output is a by-product other consumers may want
         else:
             xd = x._data
-            C.check(C.lib.b200jt_bn_stats(C.desc(xd), ctypes.c_void_p(stats.data_ptr()), C.stream_ptr()), "bn_stats")
+            C.call("b200jt_bn_stats", C.desc(xd), stats.data_ptr(), what="bn_stats")
         count = float(x.numel() // Cn)
         if synced and tdist.is_initialized() and tdist.get_world_size() > 1:
             from . import dist
@@ -1022,20 +1051,17 @@ def _match_batchnorm(v):
         def param(p, fill):
             if p[0] == "var":
                 return p[1]._data
-            return torch.full((Cn,), p[1], dtype=torch.float32, device="cuda") if p[1] != fill else None
+            return C.full([Cn], p[1], torch.float32) if p[1] != fill else None
 
         gt, bt = param(g, 1.0), param(b, 0.0)
         out = _empty(x.shape, v.dtype)
-        rmp = rvp = 0
+        rmp = rvp = None
         momentum = 0.0
-        if running is not None and getattr(root, "_bn_running", None) is not None:
+        if running is not None and root._bn_running is not None:
             root._bn_running = None                # consumed here: the kernel updates the running statistics in place
             rmp, rvp, momentum = running[0].running_mean._data.data_ptr(), running[0].running_var._data.data_ptr(), running[0].momentum
-        C.check(C.lib.b200jt_bn_apply(C.desc(xd), ctypes.c_void_p(stats.data_ptr()), count,
-                                      ctypes.c_void_p(gt.data_ptr() if gt is not None else 0),
-                                      ctypes.c_void_p(bt.data_ptr() if bt is not None else 0),
-                                      m["eps"], int(relu), C.desc(out), ctypes.c_void_p(rmp), ctypes.c_void_p(rvp),
-                                      float(momentum), C.stream_ptr()), "bn_apply")
+        C.call("b200jt_bn_apply", C.desc(xd), stats.data_ptr(), count, gt.data_ptr() if gt is not None else None,
+               bt.data_ptr() if bt is not None else None, m["eps"], int(relu), C.desc(out), rmp, rvp, float(momentum), what="bn_apply")
         return out
 
     return Plan(leaves, run)
@@ -1064,3 +1090,13 @@ def _match_fused_chain(v):
 
 _MATCHERS = [_match_conv, _match_conv_dgrad, _match_conv_wgrad, _match_pool, _match_matmul, _match_batched_matmul, _match_softmax, _match_layernorm, _match_batchnorm,
              _match_fused_chain]
+
+
+def _setup_host():
+    from . import var as V
+    from .flags import flags
+    addresses = {n: ctypes.cast(getattr(C.lib, n), ctypes.c_void_p).value for n, _, _ in C.SIGNATURES}
+    C.host.setup(V.Shape, V._make_shape, dt.DType, dt.canon, _record, C.B200Error, flags._v, addresses)
+
+
+_setup_host()

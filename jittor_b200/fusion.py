@@ -436,8 +436,8 @@ def run_program(words, inputs, full, k, out):
         descs[i] = C.desc(var._data, view)
     shp = (ctypes.c_int64 * len(full))(*full)
     code = (ctypes.c_int32 * len(words))(*words)
-    C.check(C.lib.b200jt_fused_chain(descs, n, shp, len(full), k, code, len(words), C.desc(out), C.stream_ptr()),
-            f"fused chain over {full} ({len(words)} words, {n} inputs)")
+    C.call("b200jt_fused_chain", descs, n, shp, len(full), k, code, len(words), C.desc(out),
+           what=lambda: f"fused chain over {full} ({len(words)} words, {n} inputs)")
     return out
 
 

@@ -77,7 +77,7 @@ class Function(Module):
             if not isinstance(o, Var):
                 wrapped.append(o)
                 continue
-            node = V.Op("custom", [o] + var_args, fn=lambda first, *rest: first, grad=rule_for(k_out), name="function")
+            node = V.Op("custom", [o] + var_args, fn=lambda first, *rest: first, grad=rule_for(k_out), name="function", sig=("first",))
             wrapped.append(Var(o.shape, o.dtype, node))
         return wrapped[0] if single else tuple(wrapped)
 
@@ -156,13 +156,12 @@ def _softmax_backward(y, dout, log, cols):
     rows = y.numel() // cols if cols else 0
 
     def run(yt, dyt):
-        import torch
-        dx = torch.empty_like(yt)
-        C.check(C.lib.b200jt_softmax_backward(C.desc(yt, [rows, cols]), C.desc(dyt.contiguous(), [rows, cols]), C.desc(dx, [rows, cols]),
-                                              int(log), C.stream_ptr()), "softmax_backward")
+        dx = C.alloc(yt.shape, yt.dtype)
+        C.call("b200jt_softmax_backward", C.desc(yt, [rows, cols]), C.desc(dyt.contiguous(), [rows, cols]), C.desc(dx, [rows, cols]),
+               int(log), what="softmax_backward")
         return dx
 
-    return Var(y.shape, y.dtype, V.Op("custom", [y, dout], fn=run, name="softmax_backward"))
+    return Var(y.shape, y.dtype, V.Op("custom", [y, dout], fn=run, name="softmax_backward", sig=("softmax_backward", bool(log), cols)))
 
 
 def softmax(x, dim=None, log=False):

@@ -102,11 +102,12 @@ def _register_builtins():
         ow = (wd_ + 2 * paddingw - kw * dilationw + dilationw - 1) // stridew + 1
         shape = [n, co, oh, ow] if yf == "abcd" else [n, oh, ow, co]
         geo = (strideh, stridew, paddingh, paddingw, dilationh, dilationw)
-        return _relayed(x, w, shape, lambda xd, wd: executor.run_conv2d_formats(x, w, geo, xformat, wformat, yf, x.dtype))
+        return _relayed(x, w, shape, lambda xd, wd: executor.run_conv2d_formats(x, w, geo, xformat, wformat, yf, x.dtype),
+                        ("conv", geo, xformat, wformat, yf))
 
-    def _relayed(x, w_or_dy, shape, run):
+    def _relayed(x, w_or_dy, shape, run, sig):
         """A Var produced by one relay launch (inputs synced by the executor first)."""
-        node = V.Op("custom", [V.to_var(x), V.to_var(w_or_dy)], fn=run, name="relay")
+        node = V.Op("custom", [V.to_var(x), V.to_var(w_or_dy)], fn=run, name="relay", sig=sig)
         return V.Var(shape, V.to_var(x).dtype, node)
 
     def cudnn_conv_backward_x(w, dy, height, width, strideh, stridew, paddingh, paddingw, dilationh=1, dilationw=1, groups=1,
@@ -118,7 +119,8 @@ def _register_builtins():
         w, dy = V.to_var(w), V.to_var(dy)
         shape = [dy.shape[0], w.shape[1], height, width]
         geo = (strideh, stridew, paddingh, paddingw, dilationh, dilationw)
-        return _relayed(dy, w, shape, lambda dyd, wd: executor.run_conv2d_transpose(dy, w, geo, 1, shape, dy.dtype))
+        return _relayed(dy, w, shape, lambda dyd, wd: executor.run_conv2d_transpose(dy, w, geo, 1, shape, dy.dtype),
+                        ("conv_x", geo))
 
     def cudnn_conv_backward_w(x, dy, kh, kw, strideh, stridew, paddingh, paddingw, dilationh=1, dilationw=1, groups=1,
                               xformat="abcd", wformat="oihw", yformat="abcd"):
@@ -133,12 +135,13 @@ def _register_builtins():
         geo = (strideh, stridew, paddingh, paddingw, dilationh, dilationw)
         if xformat == "abcd" and wformat == "oihw" and yformat == "abcd":
             shape = [dy.shape[1], x.shape[1], kh, kw]
-            return _relayed(x, dy, shape, lambda xd, dyd: executor.run_conv2d_backward_w(x, dy, geo, shape, x.dtype))
+            return _relayed(x, dy, shape, lambda xd, dyd: executor.run_conv2d_backward_w(x, dy, geo, shape, x.dtype),
+                            ("conv_w", geo))
         ci = x.shape[1] if xformat == "abcd" else x.shape[3]
         co = dy.shape[1] if yformat == "abcd" else dy.shape[3]
         shape = [co, ci, kh, kw] if wformat == "oihw" else [co, kh, kw, ci]
         return _relayed(x, dy, shape, lambda xd, dyd: executor.run_conv2d_backward_w_formats(
-            x, dy, geo, kh, kw, xformat, wformat, yformat, x.dtype))
+            x, dy, geo, kh, kw, xformat, wformat, yformat, x.dtype), ("conv_w", geo, xformat, wformat, yformat))
 
     register_op("cublas_matmul", cublas_matmul)
     register_op("cudnn_conv", cudnn_conv)

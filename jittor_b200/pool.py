@@ -6,8 +6,6 @@ minimum (and for mean in ceil mode) and falls back to reindex + reduce otherwise
     the jt.code bodies: clipped windows, first-match gradient for maximum / minimum;
   * otherwise, and for mean in floor mode exactly as in the reference (pool.py:46-50,187-197): the meta-operator lowering
     x.reindex([N,C,h,w,kh,kw], ...).reduce(op, [4,5]), whose overflow value 0 stands for the padding."""
-import ctypes
-
 import torch
 
 from . import _capi as C
@@ -21,35 +19,35 @@ def _pair(v):
     return tuple(v) if isinstance(v, (tuple, list)) else (v, v)
 
 
-def _run_pool(op, k, s, p, cip, oshape, want_indices, keep=None):
-    """Forward relay. For maximum / minimum the index map is always written (one extra int32 per output); `keep`, a dict
-    shared with the backward relay, holds on to it so that the backward needs neither x nor a scan."""
+def _run_pool(op, k, s, p, cip, oshape, indices=None, want_indices=False):
+    """Forward relay. For maximum / minimum the index map is always written (one extra int32 per output) and becomes the
+    value of the Var `indices`, so that the backward needs neither x nor a scan."""
     with_idx = op != "mean"
 
     def run(xd):
         xd = xd.contiguous()
-        y = torch.empty(oshape, dtype=xd.dtype, device=xd.device)
-        idx = torch.empty(oshape, dtype=torch.int32, device=xd.device) if with_idx else None
-        C.check(C.lib.b200jt_pool2d(C.desc(xd), C.desc(y), ctypes.c_void_p(idx.data_ptr() if with_idx else 0),
-                                    op.encode(), k[0], k[1], s[0], s[1], p[0], p[1], int(cip), C.stream_ptr()), "pool2d")
-        if keep is not None and with_idx:
-            keep["idx"] = idx
+        y = C.alloc(oshape, xd.dtype)
+        idx = C.alloc(oshape, torch.int32) if with_idx else None
+        C.call("b200jt_pool2d", C.desc(xd), C.desc(y), idx.data_ptr() if with_idx else None, op.encode(), k[0], k[1], s[0], s[1],
+               p[0], p[1], int(cip), what="pool2d")
+        if indices is not None and indices._data is None:
+            indices._data = idx
         return idx if want_indices else y
     return run
 
 
-def _run_pool_bwd(op, k, s, p, cip, xshape, oshape, keep):
-    def run(xd, yd, dyd):
+def _run_pool_bwd(op, k, s, p, cip, xshape, oshape, with_idx):
+    def run(*tensors):
+        idx = tensors[0] if with_idx else None
+        xd, yd, dyd = tensors[-3:]
         xd, yd, dyd = xd.view(xshape).contiguous(), yd.view(oshape).contiguous(), dyd.view(oshape).contiguous()
-        dx = torch.empty_like(xd)
-        idx = keep.get("idx")
-        if idx is not None:
-            C.check(C.lib.b200jt_pool2d_backward_indices(C.desc(xd), C.desc(yd), ctypes.c_void_p(idx.data_ptr()), C.desc(dyd),
-                                                         C.desc(dx), k[0], k[1], s[0], s[1], p[0], p[1], C.stream_ptr()),
-                    "pool2d_backward_indices")
-            return dx
-        C.check(C.lib.b200jt_pool2d_backward(C.desc(xd), C.desc(yd), C.desc(dyd), C.desc(dx), op.encode(),
-                                             k[0], k[1], s[0], s[1], p[0], p[1], int(cip), C.stream_ptr()), "pool2d_backward")
+        dx = C.alloc(xshape, xd.dtype)
+        if with_idx:
+            C.call("b200jt_pool2d_backward_indices", C.desc(xd), C.desc(yd), idx.data_ptr(), C.desc(dyd), C.desc(dx),
+                   k[0], k[1], s[0], s[1], p[0], p[1], what="pool2d_backward_indices")
+        else:
+            C.call("b200jt_pool2d_backward", C.desc(xd), C.desc(yd), C.desc(dyd), C.desc(dx), op.encode(),
+                   k[0], k[1], s[0], s[1], p[0], p[1], int(cip), what="pool2d_backward")
         return dx
     return run
 
@@ -95,18 +93,22 @@ class Pool(Module):
                            ["i0", "i1", f"i2*{s[0]}-{p[0]}+i4", f"i3*{s[1]}-{p[1]}+i5"])
             return xx.reduce(self.op, [4, 5])
         oshape, xshape, op, cip = [N, Cn, h, w], list(x.shape), self.op, self.count_include_pad
-        keep = {}
+        sig = (op, k, s, p, int(cip))
+        idx = None
+        if op != "mean":
+            idx = V.Var(oshape, "int32", V.Op("custom", [x], fn=_run_pool(op, k, s, p, cip, oshape, want_indices=True),
+                                              name="pool2d_indices", sig=("pool2d_indices",) + sig))
 
         def grad_rule(out, dout, which):
-            node = V.Op("custom", [x, out, dout], fn=_run_pool_bwd(op, k, s, p, cip, xshape, oshape, keep), name="pool2d_backward")
+            # the index map comes last off the planner's stack: y, whose launch writes it, is asked for first
+            node = V.Op("custom", ([idx] if idx is not None else []) + [x, out, dout],
+                        fn=_run_pool_bwd(op, k, s, p, cip, xshape, oshape, idx is not None), name="pool2d_backward",
+                        sig=("pool2d_backward",) + sig)
             return V.Var(xshape, x.dtype, node)
 
-        y = V.Var(oshape, x.dtype, V.Op("custom", [x], fn=_run_pool(op, k, s, p, cip, oshape, False, keep), name="pool2d",
-                                         grad=grad_rule))
-        if not self.return_indices:
-            return y
-        idx = V.Var(oshape, "int32", V.Op("custom", [x], fn=_run_pool(op, k, s, p, cip, oshape, True), name="pool2d_indices"))
-        return y, idx
+        y = V.Var(oshape, x.dtype, V.Op("custom", [x], fn=_run_pool(op, k, s, p, cip, oshape, idx), name="pool2d",
+                                         grad=grad_rule, sig=("pool2d",) + sig, **({"also": [idx]} if idx is not None else {})))
+        return (y, idx) if self.return_indices else y
 
 
 def pool(x, kernel_size, op, padding=0, stride=None):

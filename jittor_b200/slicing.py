@@ -11,11 +11,9 @@ A tuple of slices is first resolved against the input shape exactly as GetitemOp
               Var stands (this is the reference's rule; numpy moves them to the front when they are separated),
 and `None` adds an output axis of size 1. getitem then is ONE reindex (gather), setitem ONE b200jt_setitem launch
 (copy + scatter with the reduce op), both on the CUDA kernels of the path."""
-import ctypes
 import re
 
 import numpy as np
-import torch
 
 from . import _capi as C
 from . import var as V
@@ -175,10 +173,10 @@ def _setitem_run(op, xshape, yshape, eshapes):
     def run(xd, yd, *extra_data, indexes=None):
         xd, yd = xd.view(xshape), yd.view(yshape)
         extra_data = [e.view(s) for e, s in zip(extra_data, eshapes)]
-        out = torch.empty_like(xd)
+        out = C.alloc(xshape, xd.dtype)
         ex = C.descs(list(extra_data)) if extra_data else None
-        C.check(C.lib.b200jt_setitem(C.desc(xd), C.desc(yd), C.desc(out), op.encode(), C.strings(indexes), len(indexes),
-                                     ex, len(extra_data), C.stream_ptr()), "setitem")
+        C.call("b200jt_setitem", C.desc(xd), C.desc(yd), C.desc(out), op.encode(), C.strings(indexes), len(indexes), ex,
+               len(extra_data), what="setitem")
         return out
     return run
 
@@ -207,7 +205,7 @@ def setitem(x, slices, value, op="void"):
     extras = [e if e.ndim else e.reshape([1]) for e in extras]
     run = _setitem_run(op, list(x.shape), list(out_shape), [list(e.shape) for e in extras])
     node = V.Op("custom", [x, value] + extras, fn=lambda xd, yd, *ed: run(xd, yd, *ed, indexes=exprs),
-                name="setitem", indexes=exprs, region=list(out_shape), reduce=op)
+                name="setitem", indexes=exprs, region=list(out_shape), reduce=op, sig=("setitem", op, exprs))
     return V.Var(list(x.shape), x.dtype, node)
 
 

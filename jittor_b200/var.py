@@ -12,7 +12,7 @@ import numpy as np
 import torch
 
 from . import dtypes as dt
-from ._capi import TORCH_DTYPES, DTYPE_NAMES, B200Error, require_cuda
+from ._capi import TORCH_DTYPES, DTYPE_NAMES, B200Error, host, require_cuda
 from .flags import flags
 
 MAX_DIMS = 10
@@ -31,13 +31,7 @@ class Shape(list):
     __hash__ = None
 
 
-class Op:
-    __slots__ = ("kind", "inputs", "attrs")
-
-    def __init__(self, kind, inputs, **attrs):
-        self.kind = kind
-        self.inputs = list(inputs)
-        self.attrs = attrs
+Op = host.Op                     # kind, inputs (list), attrs (dict): csrc/host.cpp
 
 
 def _check_shape(shape):
@@ -47,29 +41,18 @@ def _check_shape(shape):
     return shape
 
 
-class Var:
+def _make_shape(shape):
+    return Shape(_check_shape(shape))
+
+
+class Var(host.VarBase):
+    """The state lives in the native base class: `_shape` / `shape`, `_dtype` / `dtype`, `_op` (the producer; written down on
+    first access when `_builder` is set), `_data` (contiguous torch tensor on the CUDA device once computed), `is_scalar`,
+    `_const` (the Python number this Var was made from, if any), `_pending` (handle of a collective still in flight on
+    another stream), `_relay`, `_vjp`, `_bn_running`, `_stop_grad`, `_stop_fuse`, `compile_options`."""
     __array_priority__ = 100
 
-    def __init__(self, shape, dtype, op=None, data=None, is_scalar=False):
-        self._shape = shape if type(shape) is Shape else Shape(_check_shape(shape))
-        self._dtype = dtype if type(dtype) is dt.DType else dt.canon(dtype)
-        self._op = op
-        self._data = data            # contiguous torch tensor on the CUDA device once computed
-        self.is_scalar = is_scalar
-        self._name = None
-        self._const = None           # the Python number this Var was made from, if any
-        self._pending = None         # handle of a collective still in flight on another stream
-        self.compile_options = {}
-
     # ---- metadata -----------------------------------------------------------------------------
-    @property
-    def shape(self):
-        return self._shape
-
-    @property
-    def dtype(self):
-        return self._dtype
-
     @property
     def ndim(self):
         return len(self._shape)
@@ -79,8 +62,6 @@ class Var:
         for s in self._shape:
             n *= s
         return n
-
-    size = property(lambda self: self._shape)
 
     def name(self, n=None):
         if n is None:
@@ -97,7 +78,7 @@ class Var:
         return self
 
     def is_stop_grad(self):
-        return getattr(self, "_stop_grad", False)
+        return self._stop_grad
 
     def stop_fuse(self):
         """This Var is computed on its own and stored: no fused chain reaches through it
@@ -106,7 +87,7 @@ class Var:
         return self
 
     def is_stop_fuse(self):
-        return getattr(self, "_stop_fuse", False)
+        return self._stop_fuse
 
     def __len__(self):
         return self._shape[0]
@@ -132,9 +113,11 @@ class Var:
 
     def torch(self):
         """The computed value as a torch CUDA tensor (no copy)."""
-        self.sync()
-        self.wait()
-        return self._data.view(list(self._shape))
+        if self._data is None:
+            self.sync()
+        if self._pending is not None:
+            self.wait()
+        return self._data.view(self._shape)
 
     @property
     def data(self):
@@ -567,17 +550,8 @@ class LazyVar(Var):
     matchers of consumers read `_op` and find the same meta-operator graph the eager construction would have made."""
 
     def __init__(self, shape, dtype, builder):
-        Var.__init__(self, shape, dtype, None)
-        del self.__dict__["_op"]
-        self.__dict__["_op_builder"] = builder
-
-    def __getattr__(self, name):               # only reached for attributes the instance does not have
-        if name == "_op":
-            builder = self.__dict__.pop("_op_builder", None)
-            op = builder() if builder is not None else None
-            self.__dict__["_op"] = op
-            return op
-        raise AttributeError(name)
+        Var.__init__(self, shape, dtype)
+        self._builder = builder
 
 
 # ------------------------------------------------------------------------------------ element-wise

@@ -1,0 +1,95 @@
+"""Replayed graphs (csrc/host.cpp): a graph synced for the second and third time, with other inputs, gives the bits the
+planner's own run of it gives -- across shared sub-expressions, by-products, constants, in-place running statistics,
+unaligned leaves, streams and threads."""
+import threading
+
+import pytest
+import torch
+
+import jittor_b200 as jt
+from jittor_b200 import _capi as C, nn, pool
+
+pytestmark = pytest.mark.gpu
+
+
+def data(seed, *shape, dtype=torch.float32, skew=0):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    n = 1
+    for s in shape:
+        n *= s
+    return jt.array(torch.randn(n + skew, generator=g, device="cuda").to(dtype)[skew:].view(*shape))
+
+
+def chain(s, skew):
+    x, w = data(s, 33, 65, skew=skew), data(s + 1, 65)
+    u = nn.relu(x * w + 0.5)
+    return [u, (u * u).sum(1), u + u, x.reshape([65, 33])]
+
+
+def softmax(s, skew):
+    x, dy = data(s, 20, 300, skew=skew), data(s + 1, 20, 300)
+    y = nn.softmax(x, -1)
+    return [y, jt.grad((y * dy).sum(), x)]
+
+
+def block(s, skew):
+    x, w = data(s, 4, 64, 14, 14, dtype=torch.bfloat16, skew=skew), data(s + 1, 64, 64, 3, 3, dtype=torch.bfloat16)
+    bn = nn.BatchNorm(64)
+    with jt.flag_scope(amp_reg=2):
+        y = nn.relu(bn(nn.conv2d(x, w, None, 1, 1)))
+        return [y] + jt.grad((y * data(s + 2, 4, 64, 14, 14, dtype=torch.bfloat16)).sum(), [x, w, bn.weight, bn.bias]) + [bn.running_mean, bn.running_var]
+
+
+def pooled(s, skew):
+    x = data(s, 2, 3, 17, 18, skew=skew)
+    y = pool.max_pool2d(x, 3, 2, 1)
+    return [y, jt.grad((y * data(s + 1, 2, 3, 9, 9)).sum(), x)]
+
+
+def rows(s, skew):
+    t = data(s, 50, 24, skew=skew)
+    r = t[jt.array(torch.arange(7, device="cuda", dtype=torch.int32) * 5)]
+    return [r, jt.grad((r * data(s + 1, 7, 24)).sum(), t), t.setitem((slice(2, 9),), 1.5)]
+
+
+def values(outs):
+    jt.sync(outs)
+    return [v.torch().clone() for v in outs]
+
+
+@pytest.mark.parametrize("skew", [0, 1])
+@pytest.mark.parametrize("graph", [chain, softmax, block, pooled, rows])
+def test_replay_gives_the_planners_bits(graph, skew):
+    want = []
+    for s in (1, 5, 9):
+        C.host.clear()                                        # planned
+        want.append(values(graph(s, skew)))
+    before = C.host.stats()["replayed"]
+    C.host.clear()
+    got = [values(graph(s, skew)) for s in (1, 5, 9)]         # planned once, replayed twice
+    assert C.host.stats()["replayed"] >= before + 2
+    for a, b in zip(want, got):
+        for x, y in zip(a, b):
+            if graph is block:                                # its statistics are summed with atomics
+                assert (x.float() - y.float()).norm() <= 1e-3 * x.float().norm()
+            else:
+                assert torch.equal(x, y)
+
+
+def test_threads_and_streams_share_the_tapes():
+    want = {s: values(softmax(s, 0)) for s in range(4)}
+    bad = []
+
+    def work(s):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for _ in range(20):
+                got = values(softmax(s, 0))
+                torch.cuda.current_stream().synchronize()
+                if not all(torch.equal(a, b) for a, b in zip(want[s], got)):
+                    bad.append(s)
+
+    C.host.clear()
+    ts = [threading.Thread(target=work, args=(s,)) for s in range(4)]
+    [t.start() for t in ts]
+    [t.join() for t in ts]
+    assert not bad
