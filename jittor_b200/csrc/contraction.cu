@@ -17,6 +17,7 @@ extern "C" size_t b200jt_matmul_workspace(const b200jt_tensor* a, const b200jt_t
     if (!matmul_dims(a, b, trans_a, trans_b, &M, &N, &K) || !valid_tensor(c)) return 0;
     if (a->dtype == B200JT_BFLOAT16 && matmul_tc_supported(M, N, K, a->ptr, b->ptr, c->ptr))
         return matmul_tc_workspace(M, N, K, trans_a != 0, trans_b != 0);
+    if (a->dtype == B200JT_FLOAT32) return matmul_f32_workspace(M, N, K);
     return 0;
 }
 
@@ -45,6 +46,8 @@ extern "C" int b200jt_matmul(const b200jt_tensor* a, const b200jt_tensor* b, con
         B200JT_CHECK_ARG(workspace_bytes >= need && (need == 0 || workspace), "workspace too small: need " + std::to_string(need) + " bytes");
         return matmul_tc(a->ptr, b->ptr, c->ptr, M, N, K, trans_a != 0, trans_b != 0, workspace, st);
     }
+    if (a->dtype == B200JT_FLOAT32 && matmul_f32_supported(1, M, N, K))
+        return matmul_f32(a->ptr, b->ptr, c->ptr, 1, 1, 1, M, N, K, trans_a != 0, trans_b != 0, workspace, workspace_bytes, st);
     return matmul_simt(a->ptr, b->ptr, c->ptr, a->dtype, M, N, K, trans_a != 0, trans_b != 0, st);
 }
 
@@ -68,6 +71,8 @@ extern "C" int b200jt_batched_matmul(const b200jt_tensor* a, const b200jt_tensor
     cudaStream_t st = (cudaStream_t)stream;
     if (a->dtype == B200JT_BFLOAT16 && batched_matmul_tc_supported(batch, M, N, K, trans_a != 0, trans_b != 0, a->ptr, b->ptr, c->ptr))
         return batched_matmul_tc(a->ptr, b->ptr, c->ptr, batch, a->shape[0], b->shape[0], M, N, K, trans_b != 0, st);
+    if (a->dtype == B200JT_FLOAT32 && matmul_f32_supported(batch, M, N, K))
+        return matmul_f32(a->ptr, b->ptr, c->ptr, batch, a->shape[0], b->shape[0], M, N, K, trans_a != 0, trans_b != 0, nullptr, 0, st);
     return batched_matmul_simt(a->ptr, b->ptr, c->ptr, a->dtype, batch, a->shape[0], b->shape[0], M, N, K,
                                trans_a != 0, trans_b != 0, st);
 }
@@ -207,7 +212,8 @@ extern "C" int b200jt_conv2d(const b200jt_tensor* x, const b200jt_tensor* w, con
             if (rc == 1) return 0;             // statistics came out of the conv epilogue
             if (rc) return rc;
         } else {
-            rc = conv2d_simt(x->ptr, w->ptr, y->ptr, x->dtype, s, st);
+            rc = x->dtype == B200JT_FLOAT32 && conv2d_f32_supported(s) ? conv2d_f32(x->ptr, w->ptr, y->ptr, s, st)
+                                                                       : conv2d_simt(x->ptr, w->ptr, y->ptr, x->dtype, s, st);
             if (rc) return rc;
         }
     }
@@ -235,6 +241,8 @@ extern "C" int b200jt_conv2d_transpose(const b200jt_tensor* x, const b200jt_tens
                      s.OW >= ow0 && s.OW < ow0 + std::max(sw, dw), "y has the wrong shape " + shape_str(y));
     s.sh = sh; s.sw = sw; s.ph = ph; s.pw = pw; s.dh = dh; s.dw = dw; s.groups = groups;
     if (numel(y) == 0) return 0;
+    if (x->dtype == B200JT_FLOAT32 && conv2d_transpose_f32_supported(s))
+        return conv2d_transpose_f32(x->ptr, w->ptr, y->ptr, s, (cudaStream_t)stream);
     return conv2d_transpose_simt(x->ptr, w->ptr, y->ptr, x->dtype, s, (cudaStream_t)stream);
 }
 
@@ -245,6 +253,8 @@ extern "C" int b200jt_conv2d_backward_w(const b200jt_tensor* x, const b200jt_ten
     if (rc) return rc;
     if (numel(dw) == 0) return 0;
     if (numel(dy) == 0) return fail(-1, "b200jt_conv2d_backward_w: empty dy");
+    if (x->dtype == B200JT_FLOAT32 && conv2d_f32_supported(s))
+        return conv2d_wgrad_f32(x->ptr, dy->ptr, dw->ptr, s, nullptr, 0, (cudaStream_t)stream);
     return conv2d_backward_w_simt(x->ptr, dy->ptr, dw->ptr, x->dtype, s, (cudaStream_t)stream);
 }
 
@@ -253,6 +263,7 @@ extern "C" size_t b200jt_conv2d_backward_w_workspace(const b200jt_tensor* x, con
     ConvShape s;
     if (conv_shape(x, dw, dy, sh, sw, ph, pw, dh, dw_, 1, &s)) return 0;
     if (x->dtype == B200JT_BFLOAT16 && conv2d_wgrad_tc_supported(s, x->ptr, dy->ptr, dw->ptr)) return conv2d_wgrad_tc_workspace(s);
+    if (x->dtype == B200JT_FLOAT32) return conv2d_wgrad_f32_workspace(s);
     return 0;
 }
 
@@ -269,5 +280,7 @@ extern "C" int b200jt_conv2d_backward_w_tc(const b200jt_tensor* x, const b200jt_
         B200JT_CHECK_ARG(workspace_bytes >= need && workspace, "workspace too small: need " + std::to_string(need) + " bytes");
         return conv2d_wgrad_tc(x->ptr, dy->ptr, dw->ptr, s, workspace, (cudaStream_t)stream);
     }
+    if (x->dtype == B200JT_FLOAT32 && conv2d_f32_supported(s))
+        return conv2d_wgrad_f32(x->ptr, dy->ptr, dw->ptr, s, workspace, workspace ? workspace_bytes : 0, (cudaStream_t)stream);
     return conv2d_backward_w_simt(x->ptr, dy->ptr, dw->ptr, x->dtype, s, (cudaStream_t)stream);
 }

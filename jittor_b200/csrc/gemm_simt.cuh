@@ -40,6 +40,18 @@ int conv2d_wgrad_tc(const void* x, const void* dy, void* dw, const ConvShape& s,
 int tcconv_status_fetch_and_clear();
 int peer_status_fetch_and_clear();          // peer_allreduce.cu
 
+// float32 contractions (gemm_f32.cu): tiled fp32x2 FMAs, k split over clusters; sizes beyond its 32-bit offsets stay below
+bool matmul_f32_supported(int64_t batch, int64_t M, int64_t N, int64_t K);
+size_t matmul_f32_workspace(int64_t M, int64_t N, int64_t K);
+int matmul_f32(const void* a, const void* b, void* c, int64_t batch, int64_t a_batch, int64_t b_batch, int64_t M, int64_t N, int64_t K,
+               bool trans_a, bool trans_b, void* workspace, size_t workspace_bytes, cudaStream_t st);
+bool conv2d_f32_supported(const ConvShape& s);
+int conv2d_f32(const void* x, const void* w, void* y, const ConvShape& s, cudaStream_t st);
+bool conv2d_transpose_f32_supported(const ConvShape& s);
+int conv2d_transpose_f32(const void* x, const void* w, void* y, const ConvShape& s, cudaStream_t st);
+size_t conv2d_wgrad_f32_workspace(const ConvShape& s);
+int conv2d_wgrad_f32(const void* x, const void* dy, void* dw, const ConvShape& s, void* workspace, size_t workspace_bytes, cudaStream_t st);
+
 int conv2d_simt(const void* x, const void* w, void* y, int dtype, const ConvShape& s, cudaStream_t st);
 int conv2d_backward_w_simt(const void* x, const void* dy, void* dw, int dtype, const ConvShape& s, cudaStream_t st);
 int conv2d_transpose_simt(const void* x, const void* w, void* y, int dtype, const ConvShape& s, cudaStream_t st);
