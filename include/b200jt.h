@@ -207,6 +207,22 @@ int b200jt_softmax_backward(const b200jt_tensor* y, const b200jt_tensor* dy, con
 int b200jt_layer_norm(const b200jt_tensor* x, const b200jt_tensor* gamma, const b200jt_tensor* beta,
                       const b200jt_tensor* y, double eps, void* stream);
 
+/* Gradient of the row LayerNorm of x [rows, cols] (cols <= 8192, gamma may be NULL): dx and / or params = float[2 * cols]
+ * (dgamma, then dbeta), either NULL when it is not wanted. */
+size_t b200jt_layer_norm_backward_workspace(const b200jt_tensor* x, int want_params);
+int b200jt_layer_norm_backward(const b200jt_tensor* x, const b200jt_tensor* gamma, const b200jt_tensor* dy, const b200jt_tensor* dx,
+                               float* params, double eps, void* workspace, size_t workspace_bytes, void* stream);
+
+/* Gradient of b200jt_bn_apply (relu included) from x, dy and the batch sums `stats`: first sums (sum of the
+ * gradient that reaches the normalised value = dbeta, its product with the normalised value = dgamma, the mean
+ * square), then dx.
+ * sums here is float[4 * C], the last row the gradient of the scale. relu: bit 0 says that a ReLU follows; adding 2 or 4 rounds
+ * the steps the meta-op graph of a bfloat16 x keeps in bfloat16 (2: with a float32 activation, 4: with a bfloat16 one). */
+int b200jt_bn_backward_sums(const b200jt_tensor* x, const b200jt_tensor* dy, const float* stats, double count, const float* gamma,
+                            const float* beta, double eps, int relu, float* sums, void* stream);
+int b200jt_bn_backward_dx(const b200jt_tensor* x, const b200jt_tensor* dy, const float* stats, double count, const float* gamma,
+                          const float* beta, double eps, int relu, const float* sums, const b200jt_tensor* dx, void* stream);
+
 /* c = op_a(a) . op_b(b), fp32 accumulation. Replaces the relay
  * CublasMatmulOp(Var* a, Var* b, bool trans_a, bool trans_b), python/jittor/extern/cuda/cublas/ops/cublas_matmul_op.h:18,
  * chosen by MatmulTuner for reduce.add(multiply(broadcast_to(a), broadcast_to(b))), python/jittor/src/opt/tuner/matmul_tuner.cc:21-102.

@@ -347,7 +347,8 @@ Entry g_entries[] = {
     E(b200jt_batched_matmul), E(b200jt_conv2d_workspace), E(b200jt_conv2d), E(b200jt_conv2d_formats_workspace), E(b200jt_conv2d_formats),
     E(b200jt_conv2d_transpose), E(b200jt_conv2d_backward_w), E(b200jt_conv2d_backward_w_workspace), E(b200jt_conv2d_backward_w_tc),
     E(b200jt_conv2d_backward_w_formats_workspace), E(b200jt_conv2d_backward_w_formats), E(b200jt_bn_stats), E(b200jt_bn_apply),
-    E(b200jt_pool2d), E(b200jt_pool2d_backward), E(b200jt_pool2d_backward_indices),
+    E(b200jt_layer_norm_backward_workspace), E(b200jt_layer_norm_backward), E(b200jt_bn_backward_sums),
+    E(b200jt_bn_backward_dx), E(b200jt_pool2d), E(b200jt_pool2d_backward), E(b200jt_pool2d_backward_indices),
 };
 #undef E
 Entry* entry_of(const char* name) {
@@ -572,8 +573,9 @@ bool replay(Tape& t, const Walk& w) {
     for (const Result& r : t.results) {
         at::Tensor out = t.bufs[r.buf];
         if (!r.same) {
-            if (r.off == 0 && r.buf < t.n_leaves) out = out.view(r.shape);
-            else if (r.off == 0) out = out.view({-1}).view(r.shape);
+            int64_t n = 1;
+            for (int64_t d : r.shape) n *= d;
+            if (r.off == 0 && n == out.numel()) out = out.view(r.shape);
             else {
                 std::vector<int64_t> stride(r.shape.size(), 1);
                 for (int i = (int)r.shape.size() - 2; i >= 0; i--) stride[i] = stride[i + 1] * r.shape[i + 1];

@@ -6,7 +6,9 @@
 //   cluster kernel -- rows too long for one CTA's registers (above 8192 float32 / 16384 bfloat16 columns, up to 8x
 //                  that): a thread-block cluster of 2, 4 or 8 CTAs holds the row, every CTA reduces its slice and the
 //                  slices' partial results are exchanged through distributed shared memory. Still 1R + 1W.
-//   pass kernel -- any cols / alignment: three sweeps by one CTA per row (re-reads hit L2).
+//                  Rows whose length or address is no multiple of 16 bytes take the same kernel one element per access (a
+//                  [5000, 1001] float32 LayerNorm: 27 us in three sweeps, 9 us held in registers).
+//   pass kernel -- longer ragged rows: three sweeps by one CTA per row (re-reads hit L2).
 // IO dtype float32 or bfloat16; all math in float32.
 #include "common.cuh"
 #include <algorithm>
@@ -50,6 +52,13 @@ template <typename T> __device__ __forceinline__ void st1(T* p, float v);
 template <> __device__ __forceinline__ void st1<float>(float* p, float v) { *p = v; }
 template <> __device__ __forceinline__ void st1<__nv_bfloat16>(__nv_bfloat16* p, float v) { *p = __float2bfloat16(v); }
 
+// One element per access, for rows that 16-byte vectors do not fit.
+template <typename T> struct Single {
+    static constexpr int N = 1;
+    static __device__ __forceinline__ void load(const T* p, float* out) { out[0] = ld1<T>(p); }
+    static __device__ __forceinline__ void store(T* p, const float* in) { st1<T>(p, in[0]); }
+};
+
 __device__ __forceinline__ float ex2_approx(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -84,6 +93,10 @@ __device__ __forceinline__ float group_reduce(float v, float* sm) {
 
 template <int N>
 __device__ __forceinline__ void load_gb(const float* __restrict__ gamma, const float* __restrict__ beta, int c, float* g, float* b) {
+    if constexpr (N == 1) {
+        g[0] = gamma ? __ldg(gamma + c) : 1.f;
+        b[0] = beta ? __ldg(beta + c) : 0.f;
+    }
 #pragma unroll
     for (int q = 0; q < N / 4; q++) {
         const float4 g4 = gamma ? __ldg(reinterpret_cast<const float4*>(gamma + c + q * 4)) : make_float4(1.f, 1.f, 1.f, 1.f);
@@ -116,13 +129,13 @@ __device__ __forceinline__ void group_reduce_n(float (&v)[NV], float* sm) {
     }
 }
 
-// GROUP threads per row, VPT 16-byte vectors per thread; requires cols % Vec16<T>::N == 0 and
+// GROUP threads per row, VPT vectors per thread (V: 16 bytes, or one element); requires cols % V::N == 0 and
 // cols <= GROUP * VPT * N. RPI rows are taken per round (their reductions share the shared-memory exchanges).
-template <typename T, int GROUP, int VPT, int OP>
+template <typename T, typename V, int GROUP, int VPT, int OP>
 __global__ void __launch_bounds__(256)
 row_reg_kernel(const T* __restrict__ x, T* __restrict__ y, const float* __restrict__ gamma,
                const float* __restrict__ beta, int64_t rows, int cols, float eps) {
-    constexpr int N = Vec16<T>::N;
+    constexpr int N = V::N;
     constexpr int ROWS_PER_CTA = 256 / GROUP;
     constexpr int RPI = 1;          // two rows per round were measured slower (fewer CTAs in flight outweigh the shared exchange)
     __shared__ float sm[32];
@@ -149,7 +162,7 @@ row_reg_kernel(const T* __restrict__ x, T* __restrict__ y, const float* __restri
 #pragma unroll
             for (int k = 0; k < VPT; k++) {
                 const int vi = t + k * GROUP;
-                if (vi < nvec && live[r]) Vec16<T>::load(xr + (int64_t)vi * N, v[r][k]);
+                if (vi < nvec && live[r]) V::load(xr + (int64_t)vi * N, v[r][k]);
                 else {
 #pragma unroll
                     for (int e = 0; e < N; e++) v[r][k][e] = (OP == ROW_LAYERNORM) ? 0.f : -FLT_MAX;
@@ -190,7 +203,7 @@ row_reg_kernel(const T* __restrict__ x, T* __restrict__ y, const float* __restri
 #pragma unroll
                             for (int e = 0; e < N; e++) { const float w = g1[e] * rstd; o[e] = v[r][k][e] * w + (b1[e] - mean * w); }
                         }
-                        Vec16<T>::store(yr + (int64_t)vi * N, o);
+                        V::store(yr + (int64_t)vi * N, o);
                     }
                 }
             }
@@ -239,7 +252,7 @@ row_reg_kernel(const T* __restrict__ x, T* __restrict__ y, const float* __restri
                         float o[N];
 #pragma unroll
                         for (int e = 0; e < N; e++) o[e] = (OP == ROW_SOFTMAX) ? v[r][k][e] * inv : v[r][k][e] - ls;
-                        Vec16<T>::store(yr + (int64_t)vi * N, o);
+                        V::store(yr + (int64_t)vi * N, o);
                     }
                 }
             }
@@ -435,7 +448,18 @@ static int launch_rows(const T* x, T* y, const float* gamma, const float* beta, 
     do { const int rpc = 256 / GROUP;                                                               \
          int64_t ctas = (rows + rpc - 1) / rpc;                                                     \
          unsigned grid = (unsigned)(ctas < (int64_t)kNumSMs * 16 ? ctas : (int64_t)kNumSMs * 16);   \
-         row_reg_kernel<T, GROUP, VPT, OP><<<grid, 256, 0, st>>>(x, y, gamma, beta, rows, (int)cols, eps); } while (0)
+         row_reg_kernel<T, V, GROUP, VPT, OP><<<grid, 256, 0, st>>>(x, y, gamma, beta, rows, (int)cols, eps); } while (0)
+    if (!vec_ok && cols <= 256 * 32) {
+        using V = Single<T>;
+        if (cols <= 32 * 8) B200JT_ROW(32, 8);
+        else if (cols <= 256 * 4) B200JT_ROW(256, 4);
+        else if (cols <= 256 * 8) B200JT_ROW(256, 8);
+        else if (cols <= 256 * 16) B200JT_ROW(256, 16);
+        else B200JT_ROW(256, 32);
+        B200JT_LAUNCH_CHECK();
+        return 0;
+    }
+    using V = Vec16<T>;
     if (vec_ok && nvec <= 32 * 8) {
         if (nvec <= 32) B200JT_ROW(32, 1);
         else if (nvec <= 64) B200JT_ROW(32, 2);
@@ -467,10 +491,10 @@ static int launch_rows(const T* x, T* y, const float* gamma, const float* beta, 
 // dx = y * (dy - sum(y * dy))   for y = softmax(x),      dx = dy - exp(y) * sum(dy)   for y = log_softmax(x),
 // the two reductions of the reference's hand-written backward (python/jittor/other/code_softmax.py:109-147). The row of y
 // and of dy live in registers: one read of each, one write of dx.
-template <typename T, int GROUP, int VPT, bool LOG>
+template <typename T, typename V, int GROUP, int VPT, bool LOG>
 __global__ void __launch_bounds__(256)
 softmax_bwd_reg_kernel(const T* __restrict__ y, const T* __restrict__ dy, T* __restrict__ dx, int64_t rows, int cols) {
-    constexpr int N = Vec16<T>::N;
+    constexpr int N = V::N;
     constexpr int ROWS_PER_CTA = 256 / GROUP;
     __shared__ float sm[32];
     const int g = threadIdx.x / GROUP, t = threadIdx.x % GROUP;
@@ -486,8 +510,8 @@ softmax_bwd_reg_kernel(const T* __restrict__ y, const T* __restrict__ dy, T* __r
         for (int k = 0; k < VPT; k++) {
             const int vi = t + k * GROUP;
             if (live && vi < nvec) {
-                Vec16<T>::load(y + row * cols + (int64_t)vi * N, a[k]);
-                Vec16<T>::load(dy + row * cols + (int64_t)vi * N, b[k]);
+                V::load(y + row * cols + (int64_t)vi * N, a[k]);
+                V::load(dy + row * cols + (int64_t)vi * N, b[k]);
 #pragma unroll
                 for (int e = 0; e < N; e++) s += LOG ? b[k][e] : a[k][e] * b[k][e];
             }
@@ -500,7 +524,7 @@ softmax_bwd_reg_kernel(const T* __restrict__ y, const T* __restrict__ dy, T* __r
                 float o[N];
 #pragma unroll
                 for (int e = 0; e < N; e++) o[e] = LOG ? b[k][e] - expf(a[k][e]) * s : a[k][e] * (b[k][e] - s);
-                Vec16<T>::store(dx + row * cols + (int64_t)vi * N, o);
+                V::store(dx + row * cols + (int64_t)vi * N, o);
             }
         }
     }
@@ -532,7 +556,18 @@ static int launch_softmax_bwd(const T* y, const T* dy, T* dx, int64_t rows, int6
     do { const int rpc = 256 / GROUP;                                                               \
          int64_t ctas = (rows + rpc - 1) / rpc;                                                     \
          unsigned grid = (unsigned)(ctas < (int64_t)kNumSMs * 16 ? ctas : (int64_t)kNumSMs * 16);   \
-         softmax_bwd_reg_kernel<T, GROUP, VPT, LOG><<<grid, 256, 0, st>>>(y, dy, dx, rows, (int)cols); } while (0)
+         softmax_bwd_reg_kernel<T, V, GROUP, VPT, LOG><<<grid, 256, 0, st>>>(y, dy, dx, rows, (int)cols); } while (0)
+    if (!vec_ok && cols <= 256 * 32) {
+        using V = Single<T>;
+        if (cols <= 32 * 8) B200JT_SB(32, 8);
+        else if (cols <= 256 * 4) B200JT_SB(256, 4);
+        else if (cols <= 256 * 8) B200JT_SB(256, 8);
+        else if (cols <= 256 * 16) B200JT_SB(256, 16);
+        else B200JT_SB(256, 32);
+        B200JT_LAUNCH_CHECK();
+        return 0;
+    }
+    using V = Vec16<T>;
     if (vec_ok && nvec <= 32 * 4) {
         if (nvec <= 32) B200JT_SB(32, 1);
         else if (nvec <= 64) B200JT_SB(32, 2);
@@ -541,6 +576,8 @@ static int launch_softmax_bwd(const T* y, const T* dy, T* dx, int64_t rows, int6
         if (nvec <= 256) B200JT_SB(256, 1);
         else if (nvec <= 512) B200JT_SB(256, 2);
         else B200JT_SB(256, 4);
+    } else if (vec_ok && nvec <= 256 * 8 && V::N == 4) {
+        B200JT_SB(256, 8);
     } else {
         unsigned grid = (unsigned)(rows < (int64_t)kNumSMs * 16 ? rows : (int64_t)kNumSMs * 16);
         softmax_bwd_pass_kernel<T, LOG><<<grid, 256, 0, st>>>(y, dy, dx, rows, cols);

@@ -20,6 +20,7 @@ import torch.distributed as tdist
 
 from . import _capi as C
 from . import dtypes as dt
+from . import relay
 from .var import Var
 
 _MATERIALIZE_LIMIT = 1 << 33       # elements; beyond this an unfused intermediate is refused
@@ -88,7 +89,7 @@ def _record(roots, nodes, leaves):
 
 
 def _run_plans(roots):
-    for root in roots:
+    for root in relay.ahead(roots) + list(roots):
         stack = [root]
         plans = {}
         while stack:
@@ -119,13 +120,10 @@ def _run_plans(roots):
 
 
 def _make_plan(v):
-    relay = v._relay
-    if relay is not None:                       # a convolution built by nn with its relay record (its graph may not be written yet)
-        kind, x, w, geo, groups = relay
-        if x.dtype in ("float32", "bfloat16") and w.dtype in ("float32", "bfloat16"):
-            if kind == "conv2d":
-                return Plan([x, w], lambda: run_conv2d(x, w, geo, v.dtype, groups=groups))
-            return Plan([x, w], lambda: run_conv2d_transpose(x, w, geo, groups, list(v.shape), v.dtype))
+    if v._relay is not None:                    # a layer with its record (its graph may not be written yet)
+        p = relay.plan(v)
+        if p is not None:
+            return p
     if v._op is None:
         raise C.B200Error("Var has neither data nor a producer")
     for matcher in _MATCHERS:
@@ -429,6 +427,11 @@ def _match_conv_dgrad(v):
     geo = _conv_index_geometry(list(m.shape), list(v.shape), a["indexes"])
     if geo is None:
         return None
+    return conv_dgrad_plan(v, dy, w, geo)
+
+
+def conv_dgrad_plan(v, dy, w, geo):
+    Co, Ci, KH, KW = w.shape
     sh, sw, ph, pw, dh, dw = geo
     fp, fq = dh * (KH - 1) - ph, dw * (KW - 1) - pw
     if sh == 1 and sw == 1 and fp >= 0 and fq >= 0 and dy.dtype == "bfloat16":
@@ -1017,14 +1020,20 @@ def _match_batchnorm(v):
     g, b = _affine_param(m["weight"], Cn), _affine_param(m["bias"], Cn)
     if g is None or b is None:
         return None
-    synced = r1[1]
+    return batch_norm_plan(v, x, g, b, m["eps"], relu, r1[1], root, None)
+
+
+def batch_norm_plan(v, x, g, b, eps, relu, synced, root, stats_var):
+    """Statistics (from the epilogue of an unrealised convolution when x is one), then normalise (+ ReLU) with the running
+    statistics of `root`'s module moved in place. stats_var: where the batch sums are kept for the gradient."""
+    Cn = x.shape[1]
     conv = None
-    if x._data is None:
-        cplan = _match_conv(x)
-        if cplan is not None:
-            got = _mul_operands(x, 7)
-            geo = conv_geometry(got[1], got[2]) or conv_geometry(got[2], got[1])
-            conv = geo
+    if x._data is None and x._relay is not None and x._relay[0] == "conv2d":
+        if x._relay[4] == 1 and x._relay[1].dtype in ("float32", "bfloat16") and x._relay[2].dtype in ("float32", "bfloat16"):
+            conv = x._relay[1:4]
+    elif x._data is None and _match_conv(x) is not None:
+        got = _mul_operands(x, 7)
+        conv = conv_geometry(got[1], got[2]) or conv_geometry(got[2], got[1])
     leaves = ([conv[0], conv[1]] if conv else [x]) + [p[1] for p in (g, b) if p[0] == "var"]
     running = root._bn_running
     if running is not None:
@@ -1036,12 +1045,14 @@ def _match_batchnorm(v):
 
     def run():
         stats = C.alloc([2 * Cn], torch.float32)
-        if conv:
+        if conv and x._data is None:
             xd = run_conv2d(conv[0], conv[1], conv[2], x.dtype, stats=stats)
             x._data = xd                       # the conv output is a by-product other consumers may want
         else:
             xd = x._data
             C.call("b200jt_bn_stats", C.desc(xd), stats.data_ptr(), what="bn_stats")
+        if stats_var is not None and stats_var._data is None:
+            stats_var._data = stats
         count = float(x.numel() // Cn)
         if synced and tdist.is_initialized() and tdist.get_world_size() > 1:
             from . import dist
@@ -1061,7 +1072,7 @@ def _match_batchnorm(v):
             root._bn_running = None                # consumed here: the kernel updates the running statistics in place
             rmp, rvp, momentum = running[0].running_mean._data.data_ptr(), running[0].running_var._data.data_ptr(), running[0].momentum
         C.call("b200jt_bn_apply", C.desc(xd), stats.data_ptr(), count, gt.data_ptr() if gt is not None else None,
-               bt.data_ptr() if bt is not None else None, m["eps"], int(relu), C.desc(out), rmp, rvp, float(momentum), what="bn_apply")
+               bt.data_ptr() if bt is not None else None, eps, int(relu), C.desc(out), rmp, rvp, float(momentum), what="bn_apply")
         return out
 
     return Plan(leaves, run)

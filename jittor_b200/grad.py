@@ -171,17 +171,18 @@ def _op_grad(out, dout, k):
     return None
 
 
-def _grad_inputs(v):
-    """The Vars a gradient flows to from v: its op's inputs, or the single input of a Var with its own backward rule."""
-    vjp = getattr(v, "_vjp", None)
-    return [vjp[0]] if vjp is not None else v._op.inputs
+def _grad_inputs(v, through_graph):
+    """The Vars a gradient flows to from v: the inputs of its own backward rule if it brings one, else its op's inputs."""
+    if v._vjp is not None and v is not through_graph:
+        return v._vjp[0]
+    op = v._op
+    return op.inputs if op is not None else ()
 
 
-def grad(loss, targets, retain_graph=True):
-    """d(sum(loss)) / d(target) for every target; a list of Vars (a single Var if `targets` is one)."""
-    single = isinstance(targets, V.Var)
-    tlist = [targets] if single else list(targets)
-    tids = {id(t) for t in tlist}
+def backprop(loss, dout, targets, through_graph=None):
+    """The gradients that reach `targets` when `dout` is the gradient at `loss`. `through_graph`: a Var whose own rule is
+    passed over in favour of its graph's."""
+    tids = {id(t) for t in targets}
     # nodes from which a target is reachable, in topological order
     order, needs, seen = [], {}, set()
     stack = [(loss, False)]
@@ -189,8 +190,11 @@ def grad(loss, targets, retain_graph=True):
         v, done = stack.pop()
         if done:
             need = id(v) in tids
-            if v._op is not None and not v.is_stop_grad():
-                need = need or any(needs.get(id(i), False) for i in _grad_inputs(v))
+            if not need and not v._stop_grad:
+                for i in _grad_inputs(v, through_graph):
+                    if needs.get(id(i), False):
+                        need = True
+                        break
             needs[id(v)] = need
             order.append(v)
             continue
@@ -198,33 +202,34 @@ def grad(loss, targets, retain_graph=True):
             continue
         seen.add(id(v))
         stack.append((v, True))
-        if v._op is not None and id(v) not in tids and not v.is_stop_grad():     # no gradient flows through stop_grad Vars
-            for i in _grad_inputs(v):
+        if id(v) not in tids and not v._stop_grad:     # no gradient flows through stop_grad Vars
+            for i in _grad_inputs(v, through_graph):
                 if id(i) not in seen:
                     stack.append((i, False))
-    dmap = {id(loss): V.full(list(loss.shape), 1, loss.dtype if loss.dtype.is_float() else "float32")}
+    dmap = {id(loss): dout}
     for v in reversed(order):
-        if not needs.get(id(v)) or id(v) not in dmap or v._op is None or id(v) in tids:
+        if not needs[id(v)] or id(v) in tids:
             continue
-        dout = dmap[id(v)]
-        vjp = getattr(v, "_vjp", None)
-        if vjp is not None:                 # a fused op that brings its own backward: one step from v to its input
-            inp, rule = vjp
-            if needs.get(id(inp)):
-                g = rule(v, dout)
-                if g.dtype != inp.dtype and inp.dtype.is_float():
-                    g = g.cast(inp.dtype)
-                dmap[id(inp)] = dmap[id(inp)] + g if id(inp) in dmap else g
+        d = dmap.get(id(v))
+        if d is None:
             continue
-        for k, inp in enumerate(v._op.inputs):
-            if not needs.get(id(inp)):
-                continue
-            g = _op_grad(v, dout, k)
-            if g is None:
+        inputs = _grad_inputs(v, through_graph)
+        if v._vjp is not None and v is not through_graph:      # a layer that brings its own backward
+            grads = v._vjp[1](v, d, [needs.get(id(i), False) for i in inputs])
+        else:
+            grads = [_op_grad(v, d, k) if needs.get(id(i), False) else None for k, i in enumerate(inputs)]
+        for inp, g in zip(inputs, grads):
+            if g is None or not needs.get(id(inp), False):
                 continue
             if g.dtype != inp.dtype and inp.dtype.is_float():
                 g = g.cast(inp.dtype)
             dmap[id(inp)] = dmap[id(inp)] + g if id(inp) in dmap else g
-    out = [dmap.get(id(t), None) for t in tlist]
-    out = [g if g is not None else _zeros_like(t) for g, t in zip(out, tlist)]
+    out = [dmap.get(id(t)) for t in targets]
+    return [g if g is not None else _zeros_like(t) for g, t in zip(out, targets)]
+
+
+def grad(loss, targets, retain_graph=True):
+    """d(sum(loss)) / d(target) for every target; a list of Vars (a single Var if `targets` is one)."""
+    single = isinstance(targets, V.Var)
+    out = backprop(loss, V.full(list(loss.shape), 1, loss.dtype if loss.dtype.is_float() else "float32"), [targets] if single else list(targets))
     return out[0] if single else out

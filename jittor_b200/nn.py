@@ -5,6 +5,7 @@ import numpy as np
 
 from . import var as V
 from . import dtypes
+from . import relay
 from .flags import flags, flag_scope
 from .var import Var, to_var
 
@@ -99,15 +100,36 @@ def matmul_transpose(a, b):
         return cc.reshape(list(a.shape[:-1]) + [-1])
     assert a.ndim == 2 and b.ndim == 2
     shape = list(a.shape)[:-1] + list(b.shape)
-    with flag_scope(amp_reg=flags.amp_reg | 36):
-        a = a.broadcast(shape, [len(shape) - 2])
-        b = b.broadcast(shape)
-        return (a * b).sum(len(shape) - 1)
+    amp = flags.amp_reg | 36
+
+    def graph():
+        with flag_scope(amp_reg=amp):
+            return (a.broadcast(shape, [len(shape) - 2]) * b.broadcast(shape)).sum(len(shape) - 1)
+    return _matmul_record(a, b, True, amp, graph)
+
+
+def _matmul_record(a, b, trans_b, amp, graph):
+    """A 2-D product as a record where the contraction kernels take it (float32 / bfloat16 on both sides), else its graph."""
+    if a.dtype != b.dtype or a.dtype not in ("float32", "bfloat16") or amp & dtypes.AMP_PREFER32 or a.is_scalar or b.is_scalar:
+        return graph()
+    with flag_scope(amp_reg=amp):
+        dtype = dtypes.reduce_dtype_infer("add", dtypes.binary_dtype_infer("multiply", a.dtype, b.dtype))
+    return relay.matmul(a, b, False, trans_b, dtype, graph)
 
 
 def matmul(a, b):
     """Broadcast-multiply-sum matrix product, every branch of python/jittor/nn.py:118-159."""
     a, b = to_var(a), to_var(b)
+    if a.ndim == 2 and b.ndim == 2:
+        n, m = a.shape
+        m_, k = b.shape
+        assert m == m_, f"dimension not match, a.shape:{a.shape}, b.shape:{b.shape}"
+        amp = flags.amp_reg | 36
+
+        def graph():
+            with flag_scope(amp_reg=amp):
+                return (a.broadcast([n, m, k], [-1]) * b.broadcast([n, m, k], [-3])).sum(-2)
+        return _matmul_record(a, b, False, amp, graph)
     with flag_scope(amp_reg=flags.amp_reg | 36):
         len_a, len_b = a.ndim, b.ndim
         if len_b == 1:
@@ -141,7 +163,8 @@ bmm = matmul
 
 def relu(x):
     x = to_var(x)
-    return V.ternary(x > 0.0, x, 0.0)
+    y = relay.relu_of(x, lambda: V.ternary(x > 0.0, x, 0.0))
+    return y if y is not None else V.ternary(x > 0.0, x, 0.0)
 
 
 def _softmax_backward(y, dout, log, cols):
@@ -165,23 +188,31 @@ def _softmax_backward(y, dout, log, cols):
 
 
 def softmax(x, dim=None, log=False):
-    x0 = x = to_var(x)
+    x = to_var(x)
     if dim is None:
         dim = ()
-    dtype, x = x.dtype, x._to_float()
-    if log:
-        a = x - x.max(dim, keepdims=True)
-        ret = a - a.exp().sum(dim, keepdims=True).log()
-    else:
-        e = (x - x.max(dim, keepdims=True)).exp()
-        ret = e / e.sum(dim, keepdims=True)
-    ret = ret.cast(dtype)
-    # over the last axis (or over everything) the backward is one fused kernel, as the forward is
+    dtype = x.dtype
+
+    def graph():
+        f = x._to_float()
+        if log:
+            a = f - f.max(dim, keepdims=True)
+            ret = a - a.exp().sum(dim, keepdims=True).log()
+        else:
+            e = (f - f.max(dim, keepdims=True)).exp()
+            ret = e / e.sum(dim, keepdims=True)
+        return ret.cast(dtype)
+    # over the last axis (or over everything) the forward and the backward are one fused kernel each
     whole = dim == () or dim == []
-    last = isinstance(dim, int) and dim % max(x0.ndim, 1) == x0.ndim - 1
-    if (whole or last) and str(dtype) in ("float32", "bfloat16") and x0.numel() > 0 and ret is not x0:
-        cols = x0.numel() if whole else x0.shape[-1]
-        ret._vjp = (x0, lambda y, dout: _softmax_backward(y, dout, log, cols))
+    last = isinstance(dim, int) and dim % max(x.ndim, 1) == x.ndim - 1
+    if whole or last:
+        cols = x.numel() if whole else x.shape[-1]
+        y = relay.softmax(x, bool(log), x.numel() // cols if cols else 0, cols, graph, lambda y, dout: _softmax_backward(y, dout, log, cols))
+        if y is not None:
+            return y
+    ret = graph()
+    if (whole or last) and str(dtype) in ("float32", "bfloat16") and x.numel() > 0 and ret is not x:
+        ret._vjp = ((x,), lambda y, dout, wanted: (_softmax_backward(y, dout, log, cols),))
     return ret
 
 
@@ -241,6 +272,8 @@ def conv2d(x, weight, bias=None, stride=1, padding=0, dilation=1, groups=1):
         ydt = dtypes.reduce_dtype_infer("add", dtypes.binary_dtype_infer("multiply", x.dtype, weight.dtype, x.is_scalar, weight.is_scalar))
     y = V.LazyVar([N, out_channels, oh, ow], ydt, lambda: graph()._op)
     y._relay = ("conv2d", x, weight, stride + padding + dilation, 1)
+    if x.dtype in ("float32", "bfloat16") and weight.dtype == x.dtype:
+        relay.conv_vjp(y, x, weight, stride + padding + dilation)
     if bias is not None:
         y = y + to_var(bias).broadcast(y.shape, [0, 2, 3])
     return y
@@ -369,6 +402,15 @@ class LayerNorm(Module):
 
     def execute(self, x):
         x = to_var(x)
+        k = len(self.normalized_shape)
+        if k <= x.ndim and list(x.shape[x.ndim - k:]) == list(self.normalized_shape):
+            w, b = self.weight, self.bias
+            y = relay.layer_norm(x, w, b, self.eps, k, lambda: self._graph(x, w, b))
+            if y is not None:
+                return y
+        return self._graph(x, self.weight, self.bias)
+
+    def _graph(self, x, weight, bias):
         dtype = x.dtype
         # fp32_guard (python/jittor/nn.py:731-750): half inputs are normalised in float32
         guard = dtype in ("float16", "bfloat16")
@@ -378,8 +420,8 @@ class LayerNorm(Module):
         xmean = x.mean(dims=dims, keepdims=True)
         x2mean = (x * x).mean(dims=dims, keepdims=True)
         xvar = (x2mean - xmean * xmean).maximum(0.0)
-        w = self.weight / (xvar + self.eps).sqrt()
-        b = self.bias - xmean * w
+        w = weight / (xvar + self.eps).sqrt()
+        b = bias - xmean * w
         y = x * w + b
         return y.cast(dtype) if guard else y
 
@@ -413,17 +455,26 @@ class BatchNorm(Module):
         x = to_var(x)
         dims = [0] + list(range(2, x.ndim))
         if self.is_train:
-            xmean = x.mean(dims=dims)
-            x2mean = (x * x).mean(dims=dims)
-            if self.sync and dist.in_mpi():
-                xmean = xmean.mpi_all_reduce("mean")
-                x2mean = x2mean.mpi_all_reduce("mean")
-            xvar = (x2mean - xmean * xmean).maximum(0.0)
-            w = self.weight / (xvar + self.eps).sqrt()
-            b = self.bias - xmean * w
-            norm_x = x * w.broadcast(x, dims) + b.broadcast(x, dims)
-            # the running statistics move when norm_x is computed: the executor either folds the update into the fused
+            weight, bias = self.weight, self.bias
+            synced = self.sync and dist.in_mpi()
+
+            def graph():
+                xmean = x.mean(dims=dims)
+                x2mean = (x * x).mean(dims=dims)
+                if synced:
+                    xmean = xmean.mpi_all_reduce("mean")
+                    x2mean = x2mean.mpi_all_reduce("mean")
+                xvar = (x2mean - xmean * xmean).maximum(0.0)
+                w = weight / (xvar + self.eps).sqrt()
+                b = bias - xmean * w
+                return x * w.broadcast(x, dims) + b.broadcast(x, dims), xmean, xvar
+            # the running statistics move when the result is computed: the executor either folds the update into the fused
             # normalise kernel or calls _update_running once the batch statistics exist
+            if not synced:
+                y = relay.batch_norm(self, x, weight, bias, self.eps, graph)
+                if y is not None:
+                    return y
+            norm_x, xmean, xvar = graph()
             norm_x._bn_running = (self, xmean, xvar)
             return norm_x
         w = self.weight / (self.running_var + self.eps).sqrt()

@@ -1,0 +1,70 @@
+"""Gradient kernels of LayerNorm and training BatchNorm (csrc/norm_bwd.cu) and the one-element row kernels (csrc/rownorm.cu) at
+the edges of their register tiles, against float64 and, for bfloat16 BatchNorm, against the meta-op graph they stand for."""
+import pytest
+import torch
+
+import jittor_b200 as jt
+from jittor_b200 import nn
+from jittor_b200.grad import backprop
+
+pytestmark = pytest.mark.gpu
+
+
+def near(got, want, tol):
+    assert (got.double() - want.double()).norm() <= tol * want.double().norm() + 1e-12
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rows,cols", [(1, 1), (3, 7), (40, 255), (33, 256), (2000, 264), (7, 513), (100, 1001), (9, 1024), (5, 1025), (64, 2049),
+                                       (300, 4096), (3, 4100), (2, 8191), (2, 8192)])
+def test_layer_norm_and_softmax(rows, cols, dtype):
+    x, dy = (torch.randn(rows, cols, device="cuda").to(dtype) for _ in range(2))
+    g, b = 1 + 0.1 * torch.randn(cols, device="cuda"), torch.randn(cols, device="cuda")
+    vx, vg, vb, vdy = jt.array(x), jt.array(g), jt.array(b), jt.array(dy)
+    y = nn.layer_norm(vx, (cols,), vg, vb)
+    dx, dg, db = jt.grad((y * vdy).sum(), [vx, vg, vb])
+    jt.sync([y, dx, dg, db])
+    xd, gd, bd = (t.double().requires_grad_() for t in (x, g, b))
+    ref = torch.nn.functional.layer_norm(xd, (cols,), gd, bd)
+    ref.backward(dy.double())
+    tol = 1e-5 if dtype == torch.float32 else 6e-3
+    if cols > 1:
+        near(y.torch(), ref.detach(), tol)
+        near(dx.torch(), xd.grad, tol)
+        near(dg.torch(), gd.grad, 1e-5)
+    near(db.torch(), bd.grad, 1e-5)
+    only = jt.grad((nn.layer_norm(vx, (cols,), vg, vb) * vdy).sum(), vx)             # without the parameters' sums
+    assert torch.equal(only.torch(), dx.torch())
+    for log in (False, True):
+        s = nn.softmax(vx, -1, log)
+        ds = jt.grad((s * vdy).sum(), vx)
+        jt.sync([s, ds])
+        xs = x.double().requires_grad_()
+        ref = torch.log_softmax(xs, -1) if log else torch.softmax(xs, -1)
+        ref.backward(dy.double())
+        near(s.torch(), ref.detach(), tol)
+        if cols > 1 and dtype == torch.float32:
+            near(ds.torch(), xs.grad, 2e-5)
+
+
+@pytest.mark.parametrize("dtype,amp", [(torch.float32, 0), (torch.bfloat16, 0), (torch.bfloat16, 2)])
+@pytest.mark.parametrize("relu", [False, True])
+@pytest.mark.parametrize("n,c,h,w", [(2, 1, 3, 5), (2, 3, 5, 7), (33, 5, 7, 7), (4, 16, 16, 16), (64, 130, 4, 4), (3, 700, 9, 8)])
+def test_batch_norm(n, c, h, w, relu, dtype, amp):
+    with jt.flag_scope(amp_reg=amp):
+        bn = nn.BatchNorm(c)
+        bn.weight, bn.bias = jt.array(1 + 0.1 * torch.randn(c, device="cuda")), jt.array(0.3 * torch.randn(c, device="cuda"))
+        vx = jt.array((torch.randn(n, c, h, w, device="cuda") + 0.2).to(dtype))
+        y = nn.relu(bn(vx)) if relu else bn(vx)
+        vdy = jt.array(torch.randn(n, c, h, w, device="cuda").to(torch.bfloat16 if y.dtype == "bfloat16" else torch.float32))
+        targets = [vx, bn.weight, bn.bias]
+        got = jt.grad((y * vdy).sum(), targets)
+        jt.sync([y] + got)
+        root = y._relay[1] if relu else y
+        node = jt.Var(root.shape, root.dtype, root._op)                               # the graph itself, op by op
+        want = backprop(jt.ternary(node > 0.0, node, 0.0) if relu else node, vdy, targets)
+        for a, b in zip(got, want):
+            if dtype == torch.float32:
+                near(a.torch(), b.torch(), 1e-4)
+            else:
+                near(a.torch(), b.torch(), 4e-3 if amp == 0 else 1e-5)
