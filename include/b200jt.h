@@ -223,6 +223,13 @@ int b200jt_bn_backward_sums(const b200jt_tensor* x, const b200jt_tensor* dy, con
 int b200jt_bn_backward_dx(const b200jt_tensor* x, const b200jt_tensor* dy, const float* stats, double count, const float* gamma,
                           const float* beta, double eps, int relu, const float* sums, const b200jt_tensor* dx, void* stream);
 
+/* One optimiser step over `count` float32 parameters: kind "sgd" (hyper: lr, momentum, weight decay, 1 - dampening; s0 = velocity),
+ * "adam" / "adamw" (b0, 1 - b0, b1, 1 - b1, step size, eps, weight decay or 1 - lr * weight decay, sqrt(1 - b1^n); s0 = second
+ * moment, s1 = first) or "rmsprop" (lr, alpha, 1 - alpha, eps; s0 = mean square). Outputs may be the inputs. */
+int b200jt_optim_step(const char* kind, int count, const int64_t* sizes, const float* const* p, const float* const* g,
+                      const float* const* s0, const float* const* s1, float* const* p_out, float* const* s0_out,
+                      float* const* s1_out, const double* hyper, int n_hyper, int nesterov, void* stream);
+
 /* c = op_a(a) . op_b(b), fp32 accumulation. Replaces the relay
  * CublasMatmulOp(Var* a, Var* b, bool trans_a, bool trans_b), python/jittor/extern/cuda/cublas/ops/cublas_matmul_op.h:18,
  * chosen by MatmulTuner for reduce.add(multiply(broadcast_to(a), broadcast_to(b))), python/jittor/src/opt/tuner/matmul_tuner.cc:21-102.

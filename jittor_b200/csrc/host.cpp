@@ -592,6 +592,504 @@ bool replay(Tape& t, const Walk& w) {
     return true;
 }
 
+// ------------------------------------------------------------------------------------------------ building the graph
+// What an expression costs before anything runs: shape and dtype inference and a node per op. The rules are the Python
+// ones (var.py, dtypes.py), which are asked once per (op, dtypes, flags) and remembered.
+PyObject *h_var_type, *h_infer_binary, *h_infer_unary, *h_infer_reduce, *h_to_var, *h_op_grad;
+PyObject* h_dtypes[10];                         // DType objects by code
+PyObject *k_binary, *k_unary, *k_ternary, *k_reduce, *k_fill, *k_broadcast, *k_reshape, *k_reindex, *k_op, *k_value, *k_mask, *k_keep, *k_rmask,
+    *s_amp, *o_add, *o_subtract, *o_multiply, *o_divide, *o_maximum, *o_minimum, *o_equal, *o_negative, *o_mean, *o_log, *o_exp, *i_zero;
+enum { BOOL, INT8, INT16, INT32, INT64, UINT8, F16, BF16, F32, F64 };
+
+int dtype_code(PyObject* s) {
+    for (int i = 0; i < 10; i++) if (h_dtypes[i] == s) return i;
+    for (int i = 0; i < 10; i++) if (PyUnicode_Compare(h_dtypes[i], s) == 0) return i;
+    return -1;
+}
+inline bool is_float(int d) { return d >= F16; }
+inline bool is_half(int d) { return d == F16 || d == BF16; }
+inline long amp() {
+    PyObject* a = PyDict_GetItem(h_flags, s_amp);
+    return a ? PyLong_AsLong(a) : 0;
+}
+struct Ref {                                     // owned reference
+    PyObject* p;
+    Ref(PyObject* o = nullptr) : p(o) {}
+    Ref(Ref&& r) : p(r.p) { r.p = nullptr; }
+    Ref& operator=(Ref&& r) { PyObject* o = r.p; r.p = nullptr; Py_XSETREF(p, o); return *this; }
+    Ref(const Ref&) = delete;
+    ~Ref() { Py_XDECREF(p); }
+    PyObject* give() { PyObject* o = p; p = nullptr; return o; }
+    explicit operator bool() const { return p != nullptr; }
+};
+inline VarObj* V(PyObject* o) { return (VarObj*)o; }
+inline Py_ssize_t rank_of(PyObject* v) { return PyList_GET_SIZE(V(v)->shape); }
+inline int64_t dim_of(PyObject* v, Py_ssize_t i) { return PyLong_AsLongLong(PyList_GET_ITEM(V(v)->shape, i)); }
+int64_t numel_of(PyObject* v) {
+    int64_t n = 1;
+    for (Py_ssize_t i = 0; i < rank_of(v); i++) n *= dim_of(v, i);
+    return n;
+}
+bool same_shape(PyObject* a, PyObject* b) {
+    if (V(a)->shape == V(b)->shape) return true;
+    if (rank_of(a) != rank_of(b)) return false;
+    for (Py_ssize_t i = 0; i < rank_of(a); i++) if (dim_of(a, i) != dim_of(b, i)) return false;
+    return true;
+}
+PyObject* make_shape(const int64_t* d, size_t n) {
+    PyTypeObject* t = (PyTypeObject*)h_shape_type;
+    PyObject* s = t->tp_alloc(t, 0);
+    if (!s) return nullptr;
+    for (size_t i = 0; i < n; i++) {
+        Ref v(PyLong_FromLongLong(d[i]));
+        if (!v || PyList_Append(s, v.p) < 0) { Py_DECREF(s); return nullptr; }
+    }
+    return s;
+}
+// shape and op are taken over
+PyObject* new_var(PyObject* shape, int dtype, PyObject* op, bool scalar = false) {
+    PyTypeObject* t = (PyTypeObject*)h_var_type;
+    VarObj* v = shape && op ? (VarObj*)t->tp_alloc(t, 0) : nullptr;
+    if (!v) { Py_XDECREF(shape); Py_XDECREF(op); return nullptr; }
+    v->shape = shape;
+    v->dtype = Py_NewRef(h_dtypes[dtype]);
+    v->op = op;
+    v->data = Py_NewRef(Py_None);
+    v->is_scalar = scalar;
+    return (PyObject*)v;
+}
+PyObject* new_op(PyObject* kind, std::initializer_list<PyObject*> inputs, std::initializer_list<std::pair<PyObject*, PyObject*>> attrs) {
+    OpObj* o = (OpObj*)OpType.tp_alloc(&OpType, 0);
+    if (!o) return nullptr;
+    o->kind = Py_NewRef(kind);
+    o->inputs = PyList_New((Py_ssize_t)inputs.size());
+    o->attrs = PyDict_New();
+    if (!o->inputs || !o->attrs) { Py_DECREF(o); return nullptr; }
+    Py_ssize_t i = 0;
+    for (PyObject* v : inputs) PyList_SET_ITEM(o->inputs, i++, Py_NewRef(v));
+    for (auto& a : attrs) if (!a.second || PyDict_SetItem(o->attrs, a.first, a.second) < 0) { Py_DECREF(o); return nullptr; }
+    return (PyObject*)o;
+}
+PyObject* number_var(PyObject* value, int dtype) {               // a scalar made from a Python number
+    const int64_t one = 1;
+    PyObject* v = new_var(make_shape(&one, 1), dtype, new_op(k_fill, {}, {{k_value, value}}), true);
+    if (v) V(v)->konst = Py_NewRef(value);
+    return v;
+}
+PyObject* to_var(PyObject* x) {
+    if (is_var(x)) return Py_NewRef(x);
+    if (PyFloat_CheckExact(x)) return number_var(x, F32);
+    if (PyBool_Check(x)) return number_var(x, BOOL);
+    if (PyLong_CheckExact(x)) return number_var(x, INT32);
+    return PyObject_CallOneArg(h_to_var, x);
+}
+PyObject* fill_like(PyObject* v, PyObject* value, int dtype) { return new_var(Py_NewRef(V(v)->shape), dtype, new_op(k_fill, {}, {{k_value, value}})); }
+
+struct InferKey {
+    const void* op;
+    uint32_t rest;
+    bool operator==(const InferKey& k) const { return op == k.op && rest == k.rest; }
+};
+struct InferHash { size_t operator()(const InferKey& k) const { return (size_t)(uintptr_t)k.op * 0x9e3779b97f4a7c15ull ^ (size_t)k.rest * 0x85ebca6bull; } };
+std::unordered_map<InferKey, int, InferHash> g_infer;
+int infer(PyObject* fn, PyObject* op, int x, int y, bool xs, bool ys) {
+    if (x < 0 || y < 0) { PyErr_SetString(PyExc_ValueError, "unsupported dtype"); return -1; }
+    PyObject* name = Py_NewRef(op);
+    if (PyUnicode_CheckExact(name)) PyUnicode_InternInPlace(&name);
+    Ref hold(name);
+    const InferKey key{name, (uint32_t)((amp() & 63) << 16 | x << 12 | y << 8 | xs << 7 | ys << 6 | (fn == h_infer_binary ? 1 : fn == h_infer_unary ? 2 : 3))};
+    auto it = g_infer.find(key);
+    if (it != g_infer.end()) return it->second;
+    Ref r(fn == h_infer_binary ? PyObject_CallFunction(fn, "OOOOO", op, h_dtypes[x], h_dtypes[y], xs ? Py_True : Py_False, ys ? Py_True : Py_False)
+                               : PyObject_CallFunction(fn, "OO", op, h_dtypes[x]));
+    if (!r) return -1;
+    const int d = dtype_code(r.p);
+    if (PyUnicode_CheckExact(name)) { Py_INCREF(name); g_infer.emplace(key, d); }       // the address stays this name's
+    return d;
+}
+
+// the stretched shape of two operands (right-aligned, size-1 axes stretch); new reference, shared where it equals one of theirs
+PyObject* stretched(PyObject* xs, PyObject* ys) {
+    const Py_ssize_t nx = PyList_GET_SIZE(xs), ny = PyList_GET_SIZE(ys), n = nx > ny ? nx : ny;
+    int64_t z[32];
+    bool is_x = nx == n, is_y = ny == n;
+    if (n > 32) { PyErr_SetString(PyExc_ValueError, "too many dims"); return nullptr; }
+    for (Py_ssize_t i = 0; i < n; i++) {
+        const int64_t a = i < n - nx ? 1 : PyLong_AsLongLong(PyList_GET_ITEM(xs, i - (n - nx))), b = i < n - ny ? 1 : PyLong_AsLongLong(PyList_GET_ITEM(ys, i - (n - ny)));
+        if (a == b || b == 1) z[i] = a;
+        else if (a == 1) z[i] = b;
+        else { PyErr_Format(PyExc_ValueError, "Shape not match, x:%R y:%R", xs, ys); return nullptr; }
+        is_x = is_x && z[i] == a;
+        is_y = is_y && z[i] == b;
+    }
+    return is_x ? Py_NewRef(xs) : is_y ? Py_NewRef(ys) : make_shape(z, (size_t)n);
+}
+
+PyObject* binary(PyObject* a, PyObject* b, PyObject* op) {
+    Ref x(to_var(a)), y(x ? to_var(b) : nullptr);
+    if (!x || !y) return nullptr;
+    const int d = infer(h_infer_binary, op, dtype_code(V(x.p)->dtype), dtype_code(V(y.p)->dtype), V(x.p)->is_scalar, V(y.p)->is_scalar);
+    if (d < 0) return nullptr;
+    PyObject* s = stretched(V(x.p)->shape, V(y.p)->shape);
+    return s ? new_var(s, d, new_op(k_binary, {x.p, y.p}, {{k_op, op}})) : nullptr;
+}
+PyObject* unary(PyObject* a, PyObject* op) {
+    Ref x(to_var(a));
+    if (!x) return nullptr;
+    const int dx = dtype_code(V(x.p)->dtype), to = dtype_code(op);
+    if (to >= 0 && to == dx) return x.give();
+    const int d = to >= 0 ? to : infer(h_infer_unary, op, dx, 0, false, false);
+    if (d < 0) return nullptr;
+    return new_var(Py_NewRef(V(x.p)->shape), d, new_op(k_unary, {x.p}, {{k_op, to >= 0 ? h_dtypes[to] : op}}), V(x.p)->is_scalar);
+}
+PyObject* ternary(PyObject* c0, PyObject* a, PyObject* b) {
+    Ref c(to_var(c0)), x(c ? to_var(a) : nullptr), y(x ? to_var(b) : nullptr);
+    if (!c || !x || !y) return nullptr;
+    Ref z(stretched(V(c.p)->shape, V(x.p)->shape));
+    if (!z) return nullptr;
+    PyObject* s = stretched(z.p, V(y.p)->shape);
+    if (!s) return nullptr;
+    const int d = infer(h_infer_binary, o_add, dtype_code(V(x.p)->dtype), dtype_code(V(y.p)->dtype), V(x.p)->is_scalar, V(y.p)->is_scalar);
+    if (d < 0) { Py_DECREF(s); return nullptr; }
+    return new_var(s, d, new_op(k_ternary, {c.p, x.p, y.p}, {}));
+}
+PyObject* cast_to(PyObject* x, int d) { return unary(x, h_dtypes[d]); }
+PyObject* reduce_masks(PyObject* x, PyObject* op, long mask, long keep) {
+    int64_t z[32];
+    size_t n = 0;
+    for (Py_ssize_t i = 0; i < rank_of(x); i++) {
+        if (!(mask >> i & 1)) z[n++] = dim_of(x, i);
+        else if (keep >> i & 1) z[n++] = 1;
+    }
+    if (!n) z[n++] = 1;
+    const int d = infer(h_infer_reduce, op, dtype_code(V(x)->dtype), 0, false, false);
+    if (d < 0) return nullptr;
+    Ref m(PyLong_FromLong(mask)), k(PyLong_FromLong(keep));
+    return new_var(make_shape(z, n), d, new_op(k_reduce, {x}, {{k_op, op}, {k_rmask, m.p}, {k_keep, k.p}}));
+}
+PyObject* reshape_like(PyObject* g, PyObject* x) {
+    if (same_shape(g, x)) return Py_NewRef(g);
+    return new_var(Py_NewRef(V(x)->shape), dtype_code(V(g)->dtype), new_op(k_reshape, {g}, {}));
+}
+PyObject* bcast_like(PyObject* x, PyObject* ref, long mask, long keep) {
+    Ref m(PyLong_FromLong(mask)), k(PyLong_FromLong(keep));
+    return new_var(Py_NewRef(V(ref)->shape), dtype_code(V(x)->dtype), new_op(k_broadcast, {x}, {{k_mask, m.p}, {k_keep, k.p}}));
+}
+// jt.reduce: half inputs are summed in float32 unless amp_reg bit 32 is set
+PyObject* reduce(PyObject* x0, PyObject* op, long mask, long keep) {
+    Ref x(Py_NewRef(x0));
+    const int d = dtype_code(V(x0)->dtype);
+    const bool up = is_half(d) && !(amp() & 32) && (PyUnicode_Compare(op, o_add) == 0 || PyUnicode_Compare(op, o_mean) == 0);
+    if (up) x = Ref(cast_to(x0, F32));
+    if (!x) return nullptr;
+    Ref r(reduce_masks(x.p, op, mask, keep));
+    if (!r || !up) return r.give();
+    return cast_to(r.p, d);
+}
+
+// ------------------------------------------------------------------------------------------------ reverse mode
+// The per-op rules on the node constructors above; kinds that are rare stay in Python (grad.py, h_op_grad).
+bool op_is(PyObject* name, PyObject* what) { return name == what || PyUnicode_Compare(name, what) == 0; }
+
+// v is the constant 1 stretched to its shape (the seed of a gradient pushed through sums and casts)
+bool is_ones(PyObject* v) {
+    for (int i = 0; i < 8; i++) {
+        VarObj* o = V(v);
+        if (!none(o->data) || !none(o->builder) || none(o->op) || Py_TYPE(o->op) != &OpType) return false;
+        OpObj* op = (OpObj*)o->op;
+        if (op_is(op->kind, k_fill)) {
+            PyObject* x = PyDict_GetItem(op->attrs, k_value);
+            return x && !PyBool_Check(x) && ((PyLong_Check(x) && PyLong_AsLong(x) == 1) || (PyFloat_Check(x) && PyFloat_AS_DOUBLE(x) == 1.0));
+        }
+        if (!op_is(op->kind, k_broadcast)) {
+            PyObject* name = op_is(op->kind, k_unary) ? PyDict_GetItem(op->attrs, k_op) : nullptr;
+            if (!name || !is_float(dtype_code(name))) return false;
+        }
+        v = PyList_GET_ITEM(op->inputs, 0);
+    }
+    return false;
+}
+
+// sums g over the axes along which an operand of x's shape was stretched by a binary op
+PyObject* unbroadcast(PyObject* g, PyObject* x) {
+    if (same_shape(g, x)) return Py_NewRef(g);
+    const Py_ssize_t pad = rank_of(g) - rank_of(x);
+    long mask = 0;
+    for (Py_ssize_t i = 0; i < rank_of(g); i++)
+        if (i < pad || (dim_of(x, i - pad) == 1 && dim_of(g, i) != 1)) mask |= 1l << i;
+    if (!mask) return reshape_like(g, x);
+    Ref r(reduce(g, o_add, mask, (1l << rank_of(g)) - 1));
+    return r ? reshape_like(r.p, x) : nullptr;
+}
+
+// gradient with respect to input k of the op that produced out; None where none flows
+PyObject* op_grad(PyObject* out, PyObject* dout, Py_ssize_t k) {
+    OpObj* o = (OpObj*)V(out)->op;
+    PyObject* x = PyList_GET_ITEM(o->inputs, k);
+    auto attr = [&](PyObject* name) { return PyDict_GetItem(o->attrs, name); };
+    auto mask_of = [&](PyObject* name) { PyObject* m = attr(name); return m ? PyLong_AsLong(m) : 0l; };
+    auto zeros = [&](PyObject* v) { return fill_like(v, i_zero, dtype_code(V(v)->dtype)); };
+    if (op_is(o->kind, k_binary)) {
+        PyObject *p = PyList_GET_ITEM(o->inputs, 0), *q = PyList_GET_ITEM(o->inputs, 1), *name = attr(k_op);
+        Ref g;
+        if (op_is(name, o_add)) g = Ref(Py_NewRef(dout));
+        else if (op_is(name, o_subtract)) g = Ref(k == 0 ? Py_NewRef(dout) : unary(dout, o_negative));
+        else if (op_is(name, o_multiply)) {
+            // 1 * y is y bit for bit: the gradient of (p * q).sum() is the other factor itself, not a pass over it (not when the
+            // factor is the reindex / broadcast operand of a convolution: its gradient graphs are recognised with the product)
+            PyObject* other = k == 0 ? q : p;
+            bool same = same_shape(other, dout) && op_is(V(other)->dtype, V(dout)->dtype) && is_float(dtype_code(V(other)->dtype)) && is_ones(dout);
+            if (same && none(V(other)->builder) && !none(V(other)->op)) {
+                PyObject* kind = ((OpObj*)V(other)->op)->kind;
+                same = !op_is(kind, k_broadcast) && !op_is(kind, k_reindex);
+            }
+            g = Ref(same ? Py_NewRef(other) : binary(other, dout, o_multiply));
+        } else if (op_is(name, o_divide)) {
+            if (k == 0) g = Ref(binary(dout, q, o_divide));
+            else {
+                Ref n(unary(dout, o_negative)), np(n ? binary(n.p, p, o_multiply) : nullptr), qq(np ? binary(q, q, o_multiply) : nullptr);
+                g = Ref(qq ? binary(np.p, qq.p, o_divide) : nullptr);
+            }
+        } else if (op_is(name, o_maximum) || op_is(name, o_minimum)) {
+            Ref cond(binary(q, out, o_equal)), z(cond ? zeros(dout) : nullptr);
+            g = Ref(z ? (k == 1 ? ternary(cond.p, dout, z.p) : ternary(cond.p, z.p, dout)) : nullptr);
+        } else return PyObject_CallFunction(h_op_grad, "OOn", out, dout, k);
+        return g ? unbroadcast(g.p, x) : nullptr;
+    }
+    if (op_is(o->kind, k_unary)) {
+        PyObject* name = attr(k_op);
+        const int dx = dtype_code(V(x)->dtype);
+        if (!is_float(dx)) Py_RETURN_NONE;
+        if (dtype_code(name) >= 0) return cast_to(dout, dx);
+        if (op_is(name, o_negative)) return unary(dout, o_negative);
+        if (op_is(name, o_log)) return binary(dout, x, o_divide);
+        if (op_is(name, o_exp)) return binary(dout, out, o_multiply);
+        return PyObject_CallFunction(h_op_grad, "OOn", out, dout, k);
+    }
+    if (op_is(o->kind, k_ternary)) {
+        if (k == 0) Py_RETURN_NONE;
+        PyObject* cond = PyList_GET_ITEM(o->inputs, 0);
+        Ref z(zeros(dout)), g(z ? (k == 1 ? ternary(cond, dout, z.p) : ternary(cond, z.p, dout)) : nullptr);
+        return g ? unbroadcast(g.p, x) : nullptr;
+    }
+    if (op_is(o->kind, k_reshape)) return reshape_like(dout, x);
+    if (op_is(o->kind, k_broadcast)) {
+        const long mask = mask_of(k_mask), keep = mask_of(k_keep);
+        if (!mask) return Py_NewRef(dout);
+        Ref g(reduce_masks(dout, o_add, mask, keep));
+        return g ? reshape_like(g.p, x) : nullptr;
+    }
+    if (op_is(o->kind, k_reduce)) {
+        const long mask = mask_of(k_rmask), keep = mask_of(k_keep);
+        PyObject* name = attr(k_op);
+        if (op_is(name, o_add)) return bcast_like(dout, x, mask, keep);
+        if (op_is(name, o_mean)) {
+            Ref b(bcast_like(dout, x, mask, keep)), f(PyFloat_FromDouble((double)numel_of(out) / (double)numel_of(x)));
+            return b && f ? binary(b.p, f.p, o_multiply) : nullptr;
+        }
+    }
+    return PyObject_CallFunction(h_op_grad, "OOn", out, dout, k);
+}
+
+// backprop(loss, dout, targets, through_graph) -> list of gradients, None where none arrives
+PyObject* m_backprop(PyObject*, PyObject* args) {
+    PyObject *loss, *dout0, *targets, *through;
+    if (!PyArg_ParseTuple(args, "O!OO!O", &VarType, &loss, &dout0, &PyList_Type, &targets, &through)) return nullptr;
+    struct Node { PyObject *v, *inputs; bool rule, need, target; };                    // inputs: a list or tuple the Var holds
+    std::vector<Node> order;
+    std::unordered_map<PyObject*, int> index;                                          // Var -> place in `order` (-1: on the stack)
+    std::unordered_map<PyObject*, bool> wanted;
+    for (Py_ssize_t i = 0; i < PyList_GET_SIZE(targets); i++) {
+        if (!is_var(PyList_GET_ITEM(targets, i))) { PyErr_SetString(PyExc_TypeError, "grad: targets must be Vars"); return nullptr; }
+        wanted[PyList_GET_ITEM(targets, i)] = true;
+    }
+    struct Frame { PyObject *v, *inputs; bool rule; Py_ssize_t next; };
+    std::vector<Frame> stack;
+    auto push = [&](PyObject* v) -> bool {
+        Frame f{v, nullptr, false, 0};
+        if (!wanted.count(v) && !V(v)->stop_grad) {                                    // no gradient flows through stop_grad Vars
+            if (!none(V(v)->vjp) && v != through) { f.inputs = PyTuple_GET_ITEM(V(v)->vjp, 0); f.rule = true; }
+            else {
+                PyObject* op = var_get_op(V(v), nullptr);
+                if (!op) return false;
+                Py_DECREF(op);                                                         // v keeps it
+                if (!none(op)) f.inputs = ((OpObj*)op)->inputs;
+            }
+        }
+        index[v] = -1;
+        stack.push_back(f);
+        return true;
+    };
+    auto count = [](PyObject* in) { return !in ? 0 : PyTuple_Check(in) ? PyTuple_GET_SIZE(in) : PyList_GET_SIZE(in); };
+    auto item = [](PyObject* in, Py_ssize_t i) { return PyTuple_Check(in) ? PyTuple_GET_ITEM(in, i) : PyList_GET_ITEM(in, i); };
+    if (!push(loss)) return nullptr;
+    while (!stack.empty()) {
+        const size_t top = stack.size() - 1;
+        const Py_ssize_t n = count(stack[top].inputs);
+        if (stack[top].next < n) {
+            PyObject* i = item(stack[top].inputs, n - 1 - stack[top].next++);
+            if (!index.count(i) && !push(i)) return nullptr;
+            continue;
+        }
+        const Frame f = stack[top];
+        const bool target = wanted.count(f.v) > 0;
+        bool need = target;
+        for (Py_ssize_t i = 0; !need && i < n; i++) need = order[index[item(f.inputs, i)]].need;
+        index[f.v] = (int)order.size();
+        order.push_back({f.v, f.inputs, f.rule, need, target});
+        stack.pop_back();
+    }
+    std::vector<Ref> d(order.size());
+    d[index[loss]] = Ref(Py_NewRef(dout0));
+    auto add = [&](PyObject* inp, Ref g) -> bool {
+        if (!g) return false;
+        if (g.p == Py_None) return true;
+        const int di = dtype_code(V(inp)->dtype);
+        if (is_float(di) && dtype_code(V(g.p)->dtype) != di) g = Ref(cast_to(g.p, di));
+        if (!g) return false;
+        Ref& slot = d[index[inp]];
+        if (slot) g = Ref(binary(slot.p, g.p, o_add));
+        if (!g) return false;
+        slot = std::move(g);
+        return true;
+    };
+    for (size_t at = order.size(); at-- > 0;) {
+        const Node& n = order[at];
+        if (!n.need || n.target || !d[at] || !n.inputs) continue;
+        const Py_ssize_t k = count(n.inputs);
+        if (n.rule) {
+            Ref want(PyList_New(k));
+            if (!want) return nullptr;
+            for (Py_ssize_t i = 0; i < k; i++) PyList_SET_ITEM(want.p, i, Py_NewRef(order[index[item(n.inputs, i)]].need ? Py_True : Py_False));
+            Ref gs(PyObject_CallFunctionObjArgs(PyTuple_GET_ITEM(V(n.v)->vjp, 1), n.v, d[at].p, want.p, nullptr));
+            if (!gs) return nullptr;
+            Ref seq(PySequence_Fast(gs.p, "a gradient rule returns a sequence"));
+            if (!seq) return nullptr;
+            for (Py_ssize_t i = 0; i < k && i < PySequence_Fast_GET_SIZE(seq.p); i++)
+                if (order[index[item(n.inputs, i)]].need && !add(item(n.inputs, i), Ref(Py_NewRef(PySequence_Fast_GET_ITEM(seq.p, i))))) return nullptr;
+        } else
+            for (Py_ssize_t i = 0; i < k; i++)
+                if (order[index[item(n.inputs, i)]].need && !add(item(n.inputs, i), Ref(op_grad(n.v, d[at].p, i)))) return nullptr;
+    }
+    PyObject* out = PyList_New(PyList_GET_SIZE(targets));
+    for (Py_ssize_t i = 0; out && i < PyList_GET_SIZE(targets); i++) {
+        auto it = index.find(PyList_GET_ITEM(targets, i));
+        PyList_SET_ITEM(out, i, Py_NewRef(it != index.end() && d[it->second] ? d[it->second].p : Py_None));
+    }
+    return out;
+}
+PyObject* m_binary(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    if (n != 3) { PyErr_SetString(PyExc_TypeError, "binary(x, y, op)"); return nullptr; }
+    return binary(a[0], a[1], a[2]);
+}
+PyObject* m_unary(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    if (n != 2) { PyErr_SetString(PyExc_TypeError, "unary(x, op)"); return nullptr; }
+    Ref op(PyUnicode_Check(a[1]) ? Py_NewRef(a[1]) : PyObject_Str(a[1]));
+    return op ? unary(a[0], op.p) : nullptr;
+}
+PyObject* m_ternary(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    if (n != 3) { PyErr_SetString(PyExc_TypeError, "ternary(cond, x, y)"); return nullptr; }
+    return ternary(a[0], a[1], a[2]);
+}
+// reduce(x, op, dims, keepdims): a whole number or a sequence of them; () or None folds every axis
+PyObject* m_reduce(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    if (n != 4) { PyErr_SetString(PyExc_TypeError, "reduce(x, op, dims, keepdims)"); return nullptr; }
+    Ref x(to_var(a[0]));
+    if (!x) return nullptr;
+    const Py_ssize_t nd = rank_of(x.p);
+    long mask = 0;
+    auto axis = [&](PyObject* d) {
+        Ref i(PyNumber_Long(d));
+        long v = i ? PyLong_AsLong(i.p) : -1;
+        if (v == -1 && PyErr_Occurred()) return false;
+        if (v < 0) v += nd;
+        if (v < 0 || v >= nd) { PyErr_Format(PyExc_ValueError, "Wrong dims number: %R", a[2]); return false; }
+        mask |= 1l << v;
+        return true;
+    };
+    if (PyLong_Check(a[2])) { if (!axis(a[2])) return nullptr; }
+    else if (a[2] != Py_None) {
+        Ref seq(PySequence_Fast(a[2], "dims: a whole number or a sequence of them"));
+        if (!seq) return nullptr;
+        for (Py_ssize_t i = 0; i < PySequence_Fast_GET_SIZE(seq.p); i++) if (!axis(PySequence_Fast_GET_ITEM(seq.p, i))) return nullptr;
+    }
+    if (!mask) mask = (1l << nd) - 1;
+    const int keep = PyObject_IsTrue(a[3]);
+    return keep < 0 ? nullptr : reduce(x.p, a[1], mask, keep ? (1l << nd) - 1 : 0);
+}
+PyObject* m_to_var(PyObject*, PyObject* x) { return to_var(x); }
+// setup_graph(Var, dtypes, infer_binary, infer_unary, infer_reduce, to_var, op_grad)
+PyObject* m_setup_graph(PyObject*, PyObject* args) {
+    PyObject *var, *dtypes, *b, *u, *r, *tv, *og;
+    if (!PyArg_ParseTuple(args, "OO!OOOOO", &var, &PyTuple_Type, &dtypes, &b, &u, &r, &tv, &og)) return nullptr;
+    h_var_type = Py_NewRef(var);
+    for (int i = 0; i < 10; i++) h_dtypes[i] = Py_NewRef(PyTuple_GET_ITEM(dtypes, i));
+    h_infer_binary = Py_NewRef(b); h_infer_unary = Py_NewRef(u); h_infer_reduce = Py_NewRef(r); h_to_var = Py_NewRef(tv); h_op_grad = Py_NewRef(og);
+    Py_RETURN_NONE;
+}
+
+// optim_step(kind, params, grads, states0, states1 or None, hyper, nesterov) -> False where a tensor is not float32 on the GPU.
+// The new values of one step live in one flat buffer per slot; the Vars are rebound to views of it.
+decltype(&b200jt_optim_step) g_optim = nullptr;
+PyObject* m_optim_step(PyObject*, PyObject* args) {
+    const char* kind;
+    PyObject *lists[4], *hyper;
+    int nesterov;
+    if (!PyArg_ParseTuple(args, "sO!O!O!OO!i", &kind, &PyList_Type, &lists[0], &PyList_Type, &lists[1], &PyList_Type, &lists[2], &lists[3], &PyTuple_Type,
+                          &hyper, &nesterov)) return nullptr;
+    const bool two = lists[3] != Py_None;
+    const Py_ssize_t n = PyList_GET_SIZE(lists[0]);
+    if (!g_optim || n == 0) Py_RETURN_FALSE;
+    std::vector<const float*> in[4];
+    std::vector<int64_t> sizes;
+    int64_t total = 0;
+    for (int l = 0; l < (two ? 4 : 3); l++) {
+        if (!PyList_Check(lists[l]) || PyList_GET_SIZE(lists[l]) != n) { PyErr_SetString(PyExc_ValueError, "optim_step: lists differ in length"); return nullptr; }
+        for (Py_ssize_t i = 0; i < n; i++) {
+            PyObject* v = PyList_GET_ITEM(lists[l], i);
+            if (!is_var(v) || none(V(v)->data) || !THPVariable_Check(V(v)->data)) Py_RETURN_FALSE;
+            const at::Tensor& t = THPVariable_Unpack(V(v)->data);
+            if (!t.is_cuda() || !t.is_contiguous() || t.scalar_type() != at::kFloat || (l && t.numel() != sizes[i])) Py_RETURN_FALSE;
+            if (l == 0) { sizes.push_back(t.numel()); total += (t.numel() + 3) / 4 * 4; }
+            in[l].push_back((const float*)t.const_data_ptr());
+        }
+    }
+    std::vector<double> h;
+    for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(hyper); i++) h.push_back(PyFloat_AsDouble(PyTuple_GET_ITEM(hyper, i)));
+    if (PyErr_Occurred()) return nullptr;
+    try {
+        const auto device = c10::Device(c10::kCUDA, c10::cuda::current_device());
+        static const int slot[3] = {0, 2, 3};
+        at::Tensor flat[3];
+        std::vector<float*> out[3];
+        for (int o = 0; o < (two ? 3 : 2); o++) {
+            flat[o] = at::Tensor(at::detail::empty_cuda({total}, at::kFloat, device, std::nullopt));
+            float* base = (float*)flat[o].data_ptr();
+            for (int64_t s : sizes) { out[o].push_back(base); base += (s + 3) / 4 * 4; }
+        }
+        const int rc = g_optim(kind, (int)n, sizes.data(), in[0].data(), in[1].data(), in[2].data(), two ? in[3].data() : nullptr, out[0].data(), out[1].data(),
+                               two ? out[2].data() : nullptr, h.data(), (int)h.size(), nesterov, (void*)c10::cuda::getCurrentCUDAStream().stream());
+        if (rc) { PyErr_Format(h_error, "optim_step: %s (status %d)", g_last_error ? g_last_error() : "", rc); return nullptr; }
+        for (int o = 0; o < (two ? 3 : 2); o++) {
+            int64_t at = 0;
+            for (Py_ssize_t i = 0; i < n; i++) {
+                VarObj* v = V(PyList_GET_ITEM(lists[slot[o]], i));
+                const at::Tensor& old = THPVariable_Unpack(v->data);
+                PyObject* py = THPVariable_Wrap(flat[o].as_strided(old.sizes(), old.strides(), at));
+                if (!py) return nullptr;
+                at += (sizes[i] + 3) / 4 * 4;
+                Py_XSETREF(v->data, py);
+                Py_CLEAR(v->builder);
+                Py_XSETREF(v->op, Py_NewRef(Py_None));
+            }
+        }
+    } catch (const std::exception& e) {
+        PyErr_SetString(h_error, e.what());
+        return nullptr;
+    }
+    Py_RETURN_TRUE;
+}
+
 // ------------------------------------------------------------------------------------------------ module functions
 // realize(roots) -> True when every root is computed; False: the caller has to run the Python planner.
 PyObject* m_realize(PyObject*, PyObject* arg) {
@@ -654,6 +1152,7 @@ PyObject* m_setup(PyObject*, PyObject* args) {
     for (Entry& e : g_entries)
         if (PyObject* a = PyDict_GetItemString(symbols, e.name)) e.fn = PyLong_AsVoidPtr(a);
     if (PyObject* a = PyDict_GetItemString(symbols, "b200jt_last_error")) g_last_error = (const char* (*)())PyLong_AsVoidPtr(a);
+    if (PyObject* a = PyDict_GetItemString(symbols, "b200jt_optim_step")) g_optim = (decltype(g_optim))PyLong_AsVoidPtr(a);
     if (PyErr_Occurred()) return nullptr;
     Py_RETURN_NONE;
 }
@@ -676,6 +1175,10 @@ PyObject* m_take_plans(PyObject*, PyObject*) {
     return PyLong_FromLongLong(n);
 }
 PyMethodDef methods[] = {
+    {"binary", (PyCFunction)(void*)m_binary, METH_FASTCALL, nullptr}, {"unary", (PyCFunction)(void*)m_unary, METH_FASTCALL, nullptr},
+    {"ternary", (PyCFunction)(void*)m_ternary, METH_FASTCALL, nullptr}, {"reduce", (PyCFunction)(void*)m_reduce, METH_FASTCALL, nullptr},
+    {"to_var", m_to_var, METH_O, nullptr}, {"backprop", m_backprop, METH_VARARGS, nullptr}, {"setup_graph", m_setup_graph, METH_VARARGS, nullptr},
+    {"optim_step", m_optim_step, METH_VARARGS, nullptr},
     {"realize", m_realize, METH_O, nullptr}, {"setup", m_setup, METH_VARARGS, nullptr}, {"set_record", m_set_record, METH_O, nullptr},
     {"set_context", m_context, METH_O, nullptr}, {"clear", m_clear, METH_NOARGS, nullptr}, {"stats", m_stats, METH_NOARGS, nullptr},
     {"take_plans", m_take_plans, METH_NOARGS, nullptr}, {nullptr}};
@@ -710,6 +1213,13 @@ PyMODINIT_FUNC PyInit__b200jt_host(void) {
     s_momentum = PyUnicode_InternFromString("momentum"); s_wait = PyUnicode_InternFromString("wait");
     s_sig = PyUnicode_InternFromString("sig"); s_also = PyUnicode_InternFromString("also");
     s_custom = PyUnicode_InternFromString("custom"); s_fuse = PyUnicode_InternFromString("b200_fuse_chains");
+    struct { PyObject** at; const char* text; } names[] = {
+        {&k_binary, "binary"}, {&k_unary, "unary"}, {&k_ternary, "ternary"}, {&k_reduce, "reduce"}, {&k_fill, "fill"}, {&k_broadcast, "broadcast_to"},
+        {&k_reshape, "reshape"}, {&k_reindex, "reindex"}, {&k_op, "op"}, {&k_value, "value"}, {&k_mask, "bcast_mask"}, {&k_keep, "keepdims_mask"},
+        {&k_rmask, "reduce_mask"}, {&s_amp, "amp_reg"}, {&o_add, "add"}, {&o_subtract, "subtract"}, {&o_multiply, "multiply"}, {&o_divide, "divide"},
+        {&o_maximum, "maximum"}, {&o_minimum, "minimum"}, {&o_equal, "equal"}, {&o_negative, "negative"}, {&o_mean, "mean"}, {&o_log, "log"}, {&o_exp, "exp"}};
+    for (auto& n : names) *n.at = PyUnicode_InternFromString(n.text);
+    i_zero = PyLong_FromLong(0);
     s_collective = PyUnicode_InternFromString("mpi_all_reduce");
     s_wgrad = PyUnicode_InternFromString("b200_wgrad_tc");
     if (PyModule_AddObjectRef(m, "Op", (PyObject*)&OpType) < 0 || PyModule_AddObjectRef(m, "VarBase", (PyObject*)&VarType) < 0) return nullptr;

@@ -345,8 +345,7 @@ def array(data, dtype=None):
     return Var(shape, DTYPE_NAMES[t.dtype], data=t.reshape(shape))
 
 
-def to_var(x):
-    return x if isinstance(x, Var) else array(x)
+to_var = host.to_var             # Vars pass through; Python numbers become lazily filled scalars, the rest goes to array()
 
 
 def full(shape, value, dtype="float32"):
@@ -507,41 +506,15 @@ broadcast_var = broadcast
 
 
 def reduce(x, op, dims=(), keepdims=False):
-    """jt.reduce(x, op, dim | dims, keepdims) (python/jittor/src/ops/reduce_op.cc:257-337)."""
-    x = to_var(x)
+    """jt.reduce(x, op, dim | dims, keepdims) (python/jittor/src/ops/reduce_op.cc:257-337). Half inputs are summed in float32
+    unless amp_reg bit 32 is set (reduce_op.cc:260-266)."""
+    return host.reduce(x, op, int(dims) if isinstance(dims, numbers.Integral) else dims, keepdims)
+
+
+def _infer_reduce(op, x):
     if op not in dt.REDUCE_OPS:
         raise ValueError(f"unknown reduce op {op!r}")
-    if isinstance(dims, numbers.Integral):
-        dims = (int(dims),)
-    if dims is None:
-        dims = ()
-    # half inputs are summed in float32 unless amp_reg bit 32 is set (reduce_op.cc:260-266)
-    if not (flags.amp_reg & dt.AMP_NO_REDUCE_UPCAST) and x.dtype in ("float16", "bfloat16") and op in ("mean", "add"):
-        return reduce(x.float32(), op, dims, keepdims).cast(x.dtype)
-    nd = x.ndim
-    if len(dims) == 0:
-        mask = (1 << nd) - 1
-    else:
-        mask = 0
-        for d in dims:
-            d = int(d)
-            if d < 0:
-                d += nd
-            if not 0 <= d < nd:
-                raise ValueError(f"Wrong dims number: {list(dims)}")
-            mask |= 1 << d
-    keep_mask = (1 << nd) - 1 if keepdims else 0
-    yshape = []
-    for i in range(nd):
-        if mask >> i & 1:
-            if keep_mask >> i & 1:
-                yshape.append(1)
-        else:
-            yshape.append(x.shape[i])
-    if not yshape:
-        yshape = [1]
-    ydt = dt.reduce_dtype_infer(op, x.dtype)
-    return Var(yshape, ydt, Op("reduce", [x], op=op, reduce_mask=mask, keepdims_mask=keep_mask))
+    return dt.reduce_dtype_infer(op, x)
 
 
 class LazyVar(Var):
@@ -555,49 +528,21 @@ class LazyVar(Var):
 
 
 # ------------------------------------------------------------------------------------ element-wise
-def _bshape(a, b):
-    """Result shape of a binary op on shapes a, b: right-aligned, size-1 axes stretch
-    (python/jittor/src/ops/binary_op.cc:421-441)."""
-    n = max(len(a), len(b))
-    pa, pb = [1] * (n - len(a)) + list(a), [1] * (n - len(b)) + list(b)
-    z = []
-    for x, y in zip(pa, pb):
-        if x == y or y == 1:
-            z.append(x)
-        elif x == 1:
-            z.append(y)
-        else:
-            raise ValueError(f"Shape not match, x:{list(a)} y:{list(b)}")
-    return z
-
-
-def binary(x, y, op):
+def _infer_binary(op, x, y, xscalar, yscalar):
     if op not in dt.BINARY_OPS or op == "mean":
         raise ValueError(f"unknown binary op {op!r}")
-    x, y = to_var(x), to_var(y)
-    z = _bshape(x.shape, y.shape)
-    zdt = dt.binary_dtype_infer(op, x.dtype, y.dtype, x.is_scalar, y.is_scalar)
-    return Var(z, zdt, Op("binary", [x, y], op=op))
+    return dt.binary_dtype_infer(op, x, y, xscalar, yscalar)
 
 
-def unary(x, op):
-    x = to_var(x)
-    op = str(op)
+def _infer_unary(op, x):
     if op not in dt.UNARY_OPS and op not in dt.DTYPES:
         raise ValueError(f"unknown unary op {op!r}")
-    ydt = dt.unary_dtype_infer(op, x.dtype)
-    if op in dt.DTYPES and ydt == x.dtype:
-        return x
-    return Var(x.shape, ydt, Op("unary", [x], op=op), is_scalar=x.is_scalar)
+    return dt.unary_dtype_infer(op, x)
 
 
-def ternary(cond, x, y):
-    cond, x, y = to_var(cond), to_var(x), to_var(y)
-    z = _bshape(_bshape(cond.shape, x.shape), y.shape)
-    zdt = dt.binary_dtype_infer("add", x.dtype, y.dtype, x.is_scalar, y.is_scalar)
-    return Var(z, zdt, Op("ternary", [cond, x, y]))
-
-
+# Node constructors of csrc/host.cpp: shapes stretch from the right over size-1 axes (python/jittor/src/ops/binary_op.cc:421-441),
+# dtypes follow the rules above.
+binary, unary, ternary = host.binary, host.unary, host.ternary
 ternary_out_hint = ternary
 
 
@@ -643,3 +588,11 @@ def index(shape, dim, dtype="int32"):
 
 
 _install_operators()
+
+
+def _python_op_grad(out, dout, k):
+    from .grad import _op_grad
+    return _op_grad(out, dout, k)
+
+
+host.setup_graph(Var, tuple(dt.DType(n) for n in dt.DTYPES), _infer_binary, _infer_unary, _infer_reduce, array, _python_op_grad)

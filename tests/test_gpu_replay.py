@@ -93,3 +93,27 @@ def test_threads_and_streams_share_the_tapes():
     [t.start() for t in ts]
     [t.join() for t in ts]
     assert not bad
+
+
+@pytest.mark.parametrize("kind", ["sgd", "nesterov", "adam", "adamw", "rmsprop"])
+def test_many_tensor_update_has_the_bits_of_the_op_by_op_rule(kind):
+    from jittor_b200 import optim
+
+    def steps(together):
+        make = {"sgd": lambda p: optim.SGD(p, 0.1, momentum=0.9, weight_decay=1e-3, dampening=0.2), "nesterov": lambda p: optim.SGD(p, 0.1, 0.9, nesterov=True),
+                "adam": lambda p: optim.Adam(p, 1e-2, weight_decay=1e-3), "adamw": lambda p: optim.AdamW(p, 1e-2, weight_decay=1e-2),
+                "rmsprop": lambda p: optim.RMSprop(p)}[kind]
+        shapes = [(1,), (3,), (7, 5), (2048,), (2049,), (64, 100)] + [(k + 1,) for k in range(60)]         # more than one launch takes
+        params = [data(k, *s) for k, s in enumerate(shapes)]
+        opt = make(params)
+        if not together:
+            opt._step_together = lambda *a: False
+        for k in range(3):
+            loss = None
+            for p in params:
+                term = (p * p * p).sum()
+                loss = term if loss is None else loss + term
+            opt.step(loss)
+        return [p.torch().clone() for p in params]
+    for a, b in zip(steps(True), steps(False)):
+        assert torch.equal(a, b)
