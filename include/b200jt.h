@@ -348,6 +348,13 @@ int b200jt_pool2d(const b200jt_tensor* x, const b200jt_tensor* y, int32_t* indic
                   int kh, int kw, int sh, int sw, int ph, int pw, int count_include_pad, void* stream);
 int b200jt_pool2d_backward(const b200jt_tensor* x, const b200jt_tensor* y, const b200jt_tensor* dy, const b200jt_tensor* dx,
                            const char* op, int kh, int kw, int sh, int sw, int ph, int pw, int count_include_pad, void* stream);
+/* Maximum / minimum with the place of the first extreme element in its window as one byte per output (row * kw + column, 255:
+ * none), and the gradient from that map: what a layer keeps between its two passes, a quarter of the index map's traffic. */
+int b200jt_pool2d_taps(const b200jt_tensor* x, const b200jt_tensor* y, uint8_t* taps, const char* op,
+                       int kh, int kw, int sh, int sw, int ph, int pw, void* stream);
+int b200jt_pool2d_backward_taps(const uint8_t* taps, const b200jt_tensor* dy, const b200jt_tensor* dx,
+                                int kh, int kw, int sh, int sw, int ph, int pw, void* stream);
+
 /* The same gradient for maximum / minimum from the index map the forward produced (x and y only give the geometry, they
  * are not read): element (p, q) receives dy of every window whose index is p*W+q. Identical results, less traffic. */
 int b200jt_pool2d_backward_indices(const b200jt_tensor* x, const b200jt_tensor* y, const int32_t* indices,

@@ -9,6 +9,8 @@
 // The output write stream dominates traffic (the gather source is usually much smaller and L2
 // resident), so both kernels are organised around coalesced output stores.
 #include "index_program.cuh"
+
+#include <algorithm>
 #include "reindex_jit.cuh"
 
 namespace b200jt {
@@ -170,13 +172,45 @@ reindex_generic_kernel(const T* __restrict__ x, T* __restrict__ y, const __grid_
 }
 
 // ---- row gather: the index program is evaluated once per run of `inner` consecutive elements ----------------------
-// (x[idx[i], :] style gathers: embedding look-ups, getitem with an index Var on a leading axis). A warp takes 32 runs
-// at a time: every lane interprets the program for ONE of them, then the offsets are passed around with shuffles and
-// the whole warp copies each run, 16 bytes per lane when aligned.
+// (x[idx[i], :] style gathers: embedding look-ups, getitem with an index Var on a leading axis). A warp takes `runs` <= 32 runs
+// at a time: every lane interprets the program for ONE of them, then the runs are copied as one list of vectors (16 bytes, or
+// one element for ragged runs) with eight accesses in flight, the offsets going round by shuffle. The host picks `runs` so that
+// few rows still make enough warps: 8192 rows of 1 KB 18.8 -> 8 us (32 runs a warp kept 256 warps waiting for one load each).
+template <typename T, typename V>
+__device__ __forceinline__ void copy_runs(const T* __restrict__ x, T* __restrict__ y, int64_t inner, long long off, int active, V fill) {
+    constexpr int N = sizeof(V) / sizeof(T), U = 8;
+    const int lane = threadIdx.x & 31;
+    const unsigned nv = (unsigned)(inner / N);
+    const int64_t total = (int64_t)active * nv;
+    V* out = reinterpret_cast<V*>(y);
+    for (int64_t f0 = 0; f0 < total; f0 += 32 * U) {
+        V v[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int64_t f = f0 + u * 32 + lane;
+            const unsigned k = total < 0x7fffffff ? (unsigned)f / nv : (unsigned)(f / nv), i = (unsigned)(f - (int64_t)k * nv);
+            const long long o = __shfl_sync(0xffffffffu, off, (int)(k & 31));
+            if (f >= total) continue;
+            if (o < 0) v[u] = fill;
+            else if (N == 1 || o % N == 0) v[u] = reinterpret_cast<const V*>(x + o)[i];
+            else {                                          // a run that starts off a 16-byte boundary: element by element
+                T* t = reinterpret_cast<T*>(&v[u]);
+#pragma unroll
+                for (int e = 0; e < N; e++) t[e] = x[o + (long long)i * N + e];
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int64_t f = f0 + u * 32 + lane;
+            if (f < total) out[f] = v[u];
+        }
+    }
+}
+
 template <typename T, typename I>
 __global__ void __launch_bounds__(256)
 reindex_rows_kernel(const T* __restrict__ x, T* __restrict__ y, const __grid_constant__ IndexProgram P,
-                    int64_t rows, int64_t inner, T fill) {
+                    int64_t rows, int64_t inner, int runs, T fill) {
     const int nl = P.ndim_loop - P.inner_dims, nx = P.ndim_x;
     const int lane = threadIdx.x & 31;
     const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5, nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -188,12 +222,12 @@ reindex_rows_kernel(const T* __restrict__ x, T* __restrict__ y, const __grid_con
 #pragma unroll
         for (int e = 0; e < V; e++) fp[e] = fill;
     }
-    for (int64_t row0 = warp * 32; row0 < rows; row0 += nwarps * 32) {
-        const int64_t row = row0 + lane;
+    for (int64_t row0 = warp * runs; row0 < rows; row0 += nwarps * runs) {
+        const int active = (int)min((int64_t)runs, rows - row0);
         long long off = -1;                                   // -1: overflow (fill), else element offset of the run in x
-        if (row < rows) {
+        if (lane < active) {
             I iv[kMaxDims];
-            int64_t r = row;
+            int64_t r = row0 + lane;
             for (int d = P.ndim_loop - 1; d >= nl; d--) iv[d] = 0;
 #pragma unroll 1
             for (int d = nl - 1; d >= 0; d--) { int64_t s = P.loop_shape[d]; iv[d] = (I)(r % s); r /= s; }
@@ -203,48 +237,9 @@ reindex_rows_kernel(const T* __restrict__ x, T* __restrict__ y, const __grid_con
                 for (int d = 0; d < nx; d++) off = off * P.x_shape[d] + (long long)xid[d];
             }
         }
-        const int active = (int)min((int64_t)32, rows - row0);
-        const int64_t nv = inner / V;                       // 16-byte vectors per run
-        if (vec_shape && nv <= 32 && (32 % nv) == 0) {
-            // short runs (an embedding row of 64 floats is 16 vectors): the warp copies 32 / nv runs per access and keeps eight
-            // accesses in flight, instead of one run per access with half of the lanes idle
-            const int per = 32 / (int)nv, sub = lane / (int)nv, li = lane % (int)nv;
-            constexpr int U = 8;
-            for (int k0 = 0; k0 < active; k0 += per * U) {
-                uint4 v[U];
-                long long o[U];
-#pragma unroll
-                for (int u = 0; u < U; u++) {
-                    const int k = k0 + u * per + sub;
-                    o[u] = __shfl_sync(0xffffffffu, off, k & 31);
-                    if (k < active) {
-                        if (o[u] >= 0 && o[u] % V == 0) v[u] = reinterpret_cast<const uint4*>(x + o[u])[li];
-                        else if (o[u] < 0) v[u] = f;
-                        else {                              // a run that starts off a 16-byte boundary: element by element
-                            T* t = reinterpret_cast<T*>(&v[u]);
-#pragma unroll
-                            for (int e = 0; e < V; e++) t[e] = x[o[u] + (long long)li * V + e];
-                        }
-                    }
-                }
-#pragma unroll
-                for (int u = 0; u < U; u++) {
-                    const int k = k0 + u * per + sub;
-                    if (k < active) reinterpret_cast<uint4*>(y + (row0 + k) * inner)[li] = v[u];
-                }
-            }
-            continue;
-        }
-        for (int k = 0; k < active; k++) {
-            const long long o = __shfl_sync(0xffffffffu, off, k);
-            T* dst = y + (row0 + k) * inner;
-            if (vec_shape && (o < 0 || o % V == 0)) {
-                const uint4* src = reinterpret_cast<const uint4*>(x + (o < 0 ? 0 : o));
-                for (int64_t i = lane; i < inner / V; i += 32) reinterpret_cast<uint4*>(dst)[i] = o < 0 ? f : src[i];
-            } else {
-                for (int64_t i = lane; i < inner; i += 32) dst[i] = o < 0 ? fill : x[o + i];
-            }
-        }
+        __syncwarp();
+        if (vec_shape) copy_runs<T, uint4>(x, y + row0 * inner, inner, off, active, f);
+        else copy_runs<T, T>(x, y + row0 * inner, inner, off, active, fill);
     }
 }
 
@@ -443,11 +438,14 @@ static int launch_reindex(const b200jt_tensor* x, const b200jt_tensor* y, const 
             const uint32_t nv = (uint32_t)(n / VMAX);
             reindex_affine_flat_kernel<T, VMAX, 8, 4><<<grid_for(nv, 256), 256, 0, st>>>(xp, yp, A, nv, fill);
         } else launch_affine<T, 1>(xp, yp, A, n, fill, small, st);
-    } else if (P.inner_dims > 0 && P.inner_elems * (int64_t)sizeof(T) >= 64 && numel(x) > 0) {
+    } else if (P.inner_dims > 0 && P.inner_elems * (int64_t)sizeof(T) >= 64 && P.inner_elems < (1LL << 31) && numel(x) > 0) {
         const int64_t rows = n / P.inner_elems;
-        const unsigned grid = grid_for(rows, 256);
-        if (small) reindex_rows_kernel<T, int32_t><<<grid, 256, 0, st>>>(xp, yp, P, rows, P.inner_elems, fill);
-        else       reindex_rows_kernel<T, int64_t><<<grid, 256, 0, st>>>(xp, yp, P, rows, P.inner_elems, fill);
+        // 32 runs a warp once there are 14 warps per SM, fewer before (the program costs a warp the same for one run as for 32);
+        // at most 4096 vectors a warp
+        const int runs = (int)std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(32, rows / (kNumSMs * 14)), (int64_t)65536 / (P.inner_elems * (int64_t)sizeof(T))));
+        const unsigned grid = grid_for((rows + runs - 1) / runs * 32, 256);
+        if (small) reindex_rows_kernel<T, int32_t><<<grid, 256, 0, st>>>(xp, yp, P, rows, P.inner_elems, runs, fill);
+        else       reindex_rows_kernel<T, int64_t><<<grid, 256, 0, st>>>(xp, yp, P, rows, P.inner_elems, runs, fill);
     } else {
         unsigned grid = grid_for(n, 256);
         if (small) reindex_generic_kernel<T, int32_t><<<grid, 256, 0, st>>>(xp, yp, P, n, fill);

@@ -113,6 +113,130 @@ rr_rows_kernel(const T* __restrict__ y, T* __restrict__ x, const __grid_constant
     }
 }
 
+// Float row scatter-add with duplicates folded before memory sees them (the gradient of an embedding table: word frequencies
+// are skewed, and same-address vector reductions in L2 take 75 ns each, one after the other -- the hottest of 8192 Zipf rows
+// was 89 us by itself; now 10 us). A CTA takes `chunk` <= 1024 runs, sorts them by destination in shared memory, and groups of
+// LPG lanes walk the sorted list with the current destination's sum in registers; sums that continue into the next group meet
+// in shared memory, so a CTA issues ONE reduction per destination and column. V: floats per lane and access. gridDim.y: column
+// slices.
+template <typename I, int V, int LPG>
+__global__ void __launch_bounds__(256)
+rr_rows_folded_kernel(const float* __restrict__ y, float* __restrict__ x, const __grid_constant__ IndexProgram P,
+                      int64_t rows, int64_t inner, int chunk) {
+    constexpr int G = 256 / LPG, U = 8;
+    __shared__ unsigned long long key[1024];                  // one per run: destination << 10 | place in the chunk
+    __shared__ float cont[G][LPG * V];                        // the part of a group's first sum that belongs to an earlier group's row
+    const int nl = P.ndim_loop - P.inner_dims, nx = P.ndim_x, tid = threadIdx.x;
+    const int64_t row0 = (int64_t)blockIdx.x * chunk;
+    const unsigned long long kNone = ~0ull;
+    for (int k = tid; k < chunk; k += 256) {
+        unsigned long long v = kNone;
+        if (row0 + k < rows) {
+            I iv[kMaxDims];
+            int64_t r = row0 + k;
+            for (int d = P.ndim_loop - 1; d >= nl; d--) iv[d] = 0;
+#pragma unroll 1
+            for (int d = nl - 1; d >= 0; d--) { int64_t s = P.loop_shape[d]; iv[d] = (I)(r % s); r /= s; }
+            I xid[kMaxDims];
+            if (!eval_index_program<I>(P, iv, xid)) {
+                long long off = 0;
+                for (int d = 0; d < nx; d++) off = off * P.x_shape[d] + (long long)xid[d];
+                v = (unsigned long long)off << 10 | (unsigned)k;
+            }
+        }
+        key[k] = v;
+    }
+    __syncthreads();
+    for (int k = 2; k <= chunk; k <<= 1)                      // bitonic
+        for (int j = k >> 1; j > 0; j >>= 1) {
+            for (int i = tid; i < chunk / 2; i += 256) {
+                const int lo = (i / j) * 2 * j + i % j, hi = lo + j;
+                const unsigned long long a = key[lo], b = key[hi];
+                if ((a > b) == ((lo & k) == 0)) { key[lo] = b; key[hi] = a; }
+            }
+            __syncthreads();
+        }
+    const int g = tid / LPG, l = tid % LPG, per = chunk / G, begin = g * per, end = begin + per;
+    const int64_t col = ((int64_t)blockIdx.y * LPG + l) * V;
+    const bool live = col < inner;                            // V divides inner
+    auto dest = [&](int i) { return key[i] >> 10; };
+    const unsigned long long kEnd = kNone >> 10;
+    auto flush = [&](unsigned long long d, const float (&s)[V]) {
+        if (!live || d == kEnd) return;
+        float* p = x + d + col;
+        if constexpr (V == 4) {
+            if (((uintptr_t)p & 15) == 0) {
+                asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(s[0]), "f"(s[1]), "f"(s[2]), "f"(s[3]) : "memory");
+                return;
+            }
+        }
+#pragma unroll
+        for (int e = 0; e < V; e++) atomicAdd(p + e, s[e]);
+    };
+    const bool joins = begin > 0 && dest(begin) == dest(begin - 1);       // the first sum belongs to a row of an earlier group
+    bool first = joins;
+    unsigned long long cur = dest(begin);
+    float sum[V] = {};
+    for (int i0 = begin; i0 < end && dest(i0) != kEnd; i0 += U) {
+        float v[U][V];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const unsigned long long k = i0 + u < end ? key[i0 + u] : kNone;
+#pragma unroll
+            for (int e = 0; e < V; e++) v[u][e] = 0.f;
+            if (live && k != kNone) {
+                const float* src = y + (row0 + (int)(k & 1023)) * inner + col;
+                if constexpr (V == 4) { const float4 q = *reinterpret_cast<const float4*>(src); v[u][0] = q.x; v[u][1] = q.y; v[u][2] = q.z; v[u][3] = q.w; }
+                else v[u][0] = *src;
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            if (i0 + u >= end) break;
+            const unsigned long long d = dest(i0 + u);
+            if (d != cur) {
+                if (first) {
+#pragma unroll
+                    for (int e = 0; e < V; e++) cont[g][l * V + e] = sum[e];
+                    first = false;
+                } else flush(cur, sum);
+                cur = d;
+#pragma unroll
+                for (int e = 0; e < V; e++) sum[e] = 0.f;
+            }
+#pragma unroll
+            for (int e = 0; e < V; e++) sum[e] += v[u][e];
+        }
+    }
+    if (first)                                                // one row from end to end, and not this group's to write
+#pragma unroll
+        for (int e = 0; e < V; e++) cont[g][l * V + e] = sum[e];
+    __syncthreads();
+    if (first || cur == kEnd) return;
+    for (int h = g + 1; h < G && dest(h * per) == cur; h++) {
+#pragma unroll
+        for (int e = 0; e < V; e++) sum[e] += cont[h][l * V + e];
+        if (dest(h * per + per - 1) != cur) break;
+    }
+    flush(cur, sum);
+}
+
+// chunk: as many runs as still leave two CTAs for every SM, and a group at least four sorted places
+template <typename I>
+static void launch_rows_folded(const float* y, float* x, const IndexProgram& P, int64_t rows, int64_t inner, cudaStream_t st) {
+    const bool vec = inner % 4 == 0 && (((uintptr_t)x | (uintptr_t)y) & 15) == 0;
+    const int64_t lanes = vec ? inner / 4 : inner;
+    const int lpg = lanes > 16 ? 32 : lanes > 8 ? 16 : 8;
+    const int64_t slices = (lanes + lpg - 1) / lpg;
+    int chunk = 128;
+    while (chunk < 1024 && (rows + chunk * 2 - 1) / (chunk * 2) * slices >= 2 * kNumSMs) chunk *= 2;
+    const dim3 grid((unsigned)((rows + chunk - 1) / chunk), (unsigned)slices);
+#define B200JT_ROWS(V, L) rr_rows_folded_kernel<I, V, L><<<grid, 256, 0, st>>>(y, x, P, rows, inner, chunk)
+    if (vec) { if (lpg == 32) B200JT_ROWS(4, 32); else if (lpg == 16) B200JT_ROWS(4, 16); else B200JT_ROWS(4, 8); }
+    else { if (lpg == 32) B200JT_ROWS(1, 32); else if (lpg == 16) B200JT_ROWS(1, 16); else B200JT_ROWS(1, 8); }
+#undef B200JT_ROWS
+}
+
 // ---- injective affine map: x[A.i + c] = op(init, y[i]) with plain stores -----------------------------
 // One thread takes 4 consecutive y elements (one 128-bit load for 4-byte types), advances the loop
 // coordinates like an odometer and pairs neighbouring x offsets into 8/16-byte stores.
@@ -669,6 +793,15 @@ static int run_typed(const b200jt_tensor* y, const b200jt_tensor* x, int op, con
     const bool small = n < (1LL << 31) && bins < (1LL << 31);
     if (P.inner_dims > 0 && P.inner_elems * (int64_t)sizeof(T) >= 64) {
         const int64_t rows = n / P.inner_elems;
+        if constexpr (std::is_same<T, float>::value) {
+            // destinations fit 54 bits beside the place in the chunk; column slices fit grid y
+            if (op == OP_ADD && bins < (1LL << 53) && P.inner_elems <= 32 * 65535 && rows < (1LL << 37)) {
+                if (small) launch_rows_folded<int32_t>(yp, xp, P, rows, P.inner_elems, st);
+                else launch_rows_folded<int64_t>(yp, xp, P, rows, P.inner_elems, st);
+                B200JT_LAUNCH_CHECK();
+                return 0;
+            }
+        }
         const unsigned rgrid = grid_for(rows, 256);
         if (small) rr_rows_kernel<T, int32_t><<<rgrid, 256, 0, st>>>(yp, xp, P, rows, P.inner_elems, op);
         else       rr_rows_kernel<T, int64_t><<<rgrid, 256, 0, st>>>(yp, xp, P, rows, P.inner_elems, op);

@@ -9,6 +9,7 @@ minimum (and for mean in ceil mode) and falls back to reindex + reduce otherwise
 import torch
 
 from . import _capi as C
+from . import relay
 from . import var as V
 from .nn import Module
 
@@ -19,35 +20,40 @@ def _pair(v):
     return tuple(v) if isinstance(v, (tuple, list)) else (v, v)
 
 
-def _run_pool(op, k, s, p, cip, oshape, indices=None, want_indices=False):
-    """Forward relay. For maximum / minimum the index map is always written (one extra int32 per output) and becomes the
-    value of the Var `indices`, so that the backward needs neither x nor a scan."""
-    with_idx = op != "mean"
-
+def _run_pool(op, k, s, p, cip, oshape, kept=None, want=None):
+    """Forward relay. For maximum / minimum the place of the extreme element is always written (`kept`, a Var, receives it), so
+    that the backward needs neither x nor a scan: one byte per output, or an int32 index map when the caller asked for
+    indices. `want` "indices" / "taps": return that map instead of the values."""
     def run(xd):
         xd = xd.contiguous()
         y = C.alloc(oshape, xd.dtype)
-        idx = C.alloc(oshape, torch.int32) if with_idx else None
-        C.call("b200jt_pool2d", C.desc(xd), C.desc(y), idx.data_ptr() if with_idx else None, op.encode(), k[0], k[1], s[0], s[1],
-               p[0], p[1], int(cip), what="pool2d")
-        if indices is not None and indices._data is None:
-            indices._data = idx
-        return idx if want_indices else y
+        found = None
+        if op != "mean":
+            found = C.alloc(oshape, torch.int32 if want == "indices" or (kept is not None and kept.dtype == "int32") else torch.uint8)
+        if found is not None and found.dtype == torch.uint8:
+            C.call("b200jt_pool2d_taps", C.desc(xd), C.desc(y), found.data_ptr(), op.encode(), *k, *s, *p, what="pool2d")
+        else:
+            C.call("b200jt_pool2d", C.desc(xd), C.desc(y), found.data_ptr() if found is not None else None, op.encode(), *k, *s, *p, int(cip),
+                   what="pool2d")
+        if kept is not None and kept._data is None:
+            kept._data = found
+        return y if want is None else found
     return run
 
 
-def _run_pool_bwd(op, k, s, p, cip, xshape, oshape, with_idx):
+def _run_pool_bwd(op, k, s, p, cip, xshape, oshape):
     def run(*tensors):
-        idx = tensors[0] if with_idx else None
-        xd, yd, dyd = tensors[-3:]
+        found, xd, yd, dyd = tensors if op != "mean" else (None,) + tensors
         xd, yd, dyd = xd.view(xshape).contiguous(), yd.view(oshape).contiguous(), dyd.view(oshape).contiguous()
         dx = C.alloc(xshape, xd.dtype)
-        if with_idx:
-            C.call("b200jt_pool2d_backward_indices", C.desc(xd), C.desc(yd), idx.data_ptr(), C.desc(dyd), C.desc(dx),
-                   k[0], k[1], s[0], s[1], p[0], p[1], what="pool2d_backward_indices")
+        if op == "mean":
+            C.call("b200jt_pool2d_backward", C.desc(xd), C.desc(yd), C.desc(dyd), C.desc(dx), op.encode(), *k, *s, *p, int(cip),
+                   what="pool2d_backward")
+        elif found.dtype == torch.uint8:
+            C.call("b200jt_pool2d_backward_taps", found.data_ptr(), C.desc(dyd), C.desc(dx), *k, *s, *p, what="pool2d_backward")
         else:
-            C.call("b200jt_pool2d_backward", C.desc(xd), C.desc(yd), C.desc(dyd), C.desc(dx), op.encode(),
-                   k[0], k[1], s[0], s[1], p[0], p[1], int(cip), what="pool2d_backward")
+            C.call("b200jt_pool2d_backward_indices", C.desc(xd), C.desc(yd), found.data_ptr(), C.desc(dyd), C.desc(dx), *k, *s, *p,
+                   what="pool2d_backward_indices")
         return dx
     return run
 
@@ -91,24 +97,34 @@ class Pool(Module):
         if not (use_code_op and pool_use_code_op):
             xx = x.reindex([N, Cn, h, w, k[0], k[1]],
                            ["i0", "i1", f"i2*{s[0]}-{p[0]}+i4", f"i3*{s[1]}-{p[1]}+i5"])
-            return xx.reduce(self.op, [4, 5])
+            y = xx.reduce(self.op, [4, 5])
+            if self.op == "mean" and pool_use_code_op and y.dtype == x.dtype and str(x.dtype) in ("float32", "bfloat16", "float16"):
+                # padding counts in this lowering; its gradient is one gather per input element instead of a scatter of the windows
+                def mean_rule(y, dout, wanted):
+                    if dout.dtype != x.dtype:
+                        dout = dout.cast(x.dtype)
+                    if list(dout.shape) != [N, Cn, h, w]:
+                        dout = dout.broadcast([N, Cn, h, w])
+                    return (relay.mean_pool_dx(x, y, dout, k, s, p),)
+                y._vjp = ((x,), mean_rule)
+            return y
         oshape, xshape, op, cip = [N, Cn, h, w], list(x.shape), self.op, self.count_include_pad
         sig = (op, k, s, p, int(cip))
-        idx = None
+        kept = None
         if op != "mean":
-            idx = V.Var(oshape, "int32", V.Op("custom", [x], fn=_run_pool(op, k, s, p, cip, oshape, want_indices=True),
-                                              name="pool2d_indices", sig=("pool2d_indices",) + sig))
+            kind = "indices" if self.return_indices or k[0] * k[1] > 255 else "taps"
+            kept = V.Var(oshape, "int32" if kind == "indices" else "uint8",
+                         V.Op("custom", [x], fn=_run_pool(op, k, s, p, cip, oshape, want=kind), name="pool2d_" + kind, sig=("pool2d_" + kind,) + sig))
 
         def grad_rule(out, dout, which):
-            # the index map comes last off the planner's stack: y, whose launch writes it, is asked for first
-            node = V.Op("custom", ([idx] if idx is not None else []) + [x, out, dout],
-                        fn=_run_pool_bwd(op, k, s, p, cip, xshape, oshape, idx is not None), name="pool2d_backward",
-                        sig=("pool2d_backward",) + sig)
+            # the map comes last off the planner's stack: y, whose launch writes it, is asked for first
+            node = V.Op("custom", ([kept] if kept is not None else []) + [x, out, dout],
+                        fn=_run_pool_bwd(op, k, s, p, cip, xshape, oshape), name="pool2d_backward", sig=("pool2d_backward",) + sig)
             return V.Var(xshape, x.dtype, node)
 
-        y = V.Var(oshape, x.dtype, V.Op("custom", [x], fn=_run_pool(op, k, s, p, cip, oshape, idx), name="pool2d",
-                                         grad=grad_rule, sig=("pool2d",) + sig, **({"also": [idx]} if idx is not None else {})))
-        return (y, idx) if self.return_indices else y
+        y = V.Var(oshape, x.dtype, V.Op("custom", [x], fn=_run_pool(op, k, s, p, cip, oshape, kept), name="pool2d",
+                                         grad=grad_rule, sig=("pool2d",) + sig, **({"also": [kept]} if kept is not None else {})))
+        return (y, kept) if self.return_indices else y
 
 
 def pool(x, kernel_size, op, padding=0, stride=None):

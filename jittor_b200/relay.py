@@ -143,6 +143,22 @@ def _plan_softmax(v, r):
     return _plan([x], run)
 
 
+# ------------------------------------------------------------------------------------------------ mean pooling
+def mean_pool_dx(x, y, dout, k, s, p):
+    return lazy(x.shape, x.dtype, ("mean_pool_dx", dout, tuple(x.shape), tuple(k), tuple(s), tuple(p)), lambda: _graph_grad(y, dout, x))
+
+
+def _plan_mean_pool_dx(v, r):
+    _, dy, xshape, k, s, p = r
+
+    def run():
+        dx = C.alloc(list(xshape), C.TORCH_DTYPES[v.dtype])
+        d = C.desc(dy._data, list(dy.shape))
+        C.call("b200jt_pool2d_backward", C.desc(dx), d, d, C.desc(dx), b"mean", *k, *s, *p, 1, what="pool2d_backward")
+        return dx
+    return _plan([dy], run)
+
+
 # ------------------------------------------------------------------------------------------------ parameters of the norms
 def _param(p, n):
     """A float32 Var of n elements, "const" for the neutral Python number, or None for what the kernels do not take."""
@@ -376,6 +392,6 @@ def _plan_bn_dx(v, r):
 
 
 _PLANS = {"matmul": _plan_matmul, "conv2d": _plan_conv, "conv2d_transpose": _plan_conv, "conv2d_dx": _plan_conv_dx, "conv2d_dw": _plan_conv_dw,
-          "softmax": _plan_softmax, "layer_norm": _plan_layer_norm, "layer_norm_dx": _plan_layer_norm_dx,
+          "softmax": _plan_softmax, "mean_pool_dx": _plan_mean_pool_dx, "layer_norm": _plan_layer_norm, "layer_norm_dx": _plan_layer_norm_dx,
           "layer_norm_params": _plan_layer_norm_params, "part": _plan_part, "batch_norm": _plan_batch_norm,
           "batch_norm_relu": _plan_batch_norm, "batch_norm_sums": _plan_bn_sums, "batch_norm_dx": _plan_bn_dx}

@@ -117,3 +117,38 @@ def test_many_tensor_update_has_the_bits_of_the_op_by_op_rule(kind):
         return [p.torch().clone() for p in params]
     for a, b in zip(steps(True), steps(False)):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("rows,dim,vocab,skew", [(1, 16, 5, 0), (3, 17, 2, 0), (127, 16, 3, 1), (129, 36, 40, 0), (1000, 64, 7, 0), (2500, 132, 900, 0), (40000, 20, 11, 0),
+                                                 (90000, 128, 3000, 0)])
+def test_row_gather_and_folded_row_scatter(rows, dim, vocab, skew):
+    table, dy = data(1, vocab, dim, skew=skew), data(2, rows, dim, skew=skew)
+    idx = jt.array(torch.randint(0, vocab, (rows,), device="cuda", dtype=torch.int32))
+    r = table[idx]
+    g = jt.grad((r * dy).sum(), table)
+    jt.sync([r, g])
+    at = idx.torch().long()
+    assert torch.equal(r.torch(), table.torch()[at])
+    want = torch.zeros(vocab, dim, device="cuda", dtype=torch.float64)
+    want.index_add_(0, at, dy.torch().double())
+    assert (g.torch().double() - want).norm() <= 1e-5 * want.norm()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("k,s,p", [(2, 2, 0), (3, 2, 1), (3, 2, 0), (3, 1, 1), (3, 1, 0), (5, 3, 2)])
+@pytest.mark.parametrize("h,w", [(6, 7), (8, 8), (9, 16), (17, 12), (33, 20)])
+def test_pool_tiles_against_torch(h, w, k, s, p, dtype):
+    x = (torch.randint(-9, 9, (2, 3, h, w), device="cuda").float() / 4).to(dtype)              # ties: the first element wins
+    vx = jt.array(x)
+    for op, ref in (("maximum", torch.nn.functional.max_pool2d), ("minimum", lambda t, *a: -torch.nn.functional.max_pool2d(-t, *a)),
+                    ("mean", torch.nn.functional.avg_pool2d)):
+        y = pool.Pool(k, s, p, op=op)(vx)
+        xt = x.double().requires_grad_()
+        yt = ref(xt, k, s, p)
+        dy = torch.randn(yt.shape, device="cuda").to(dtype)
+        dx = jt.grad((y * jt.array(dy)).sum(), vx)
+        jt.sync([y, dx])
+        yt.backward(dy.double())
+        tol = 1e-6 if dtype == torch.float32 else 1e-2
+        assert (y.torch().double() - yt.detach()).abs().max() <= tol * (1 + yt.detach().abs().max())
+        assert (dx.torch().double() - xt.grad).abs().max() <= tol * (1 + xt.grad.abs().max())
