@@ -121,13 +121,18 @@ static int conv_formats(const b200jt_tensor* x, const b200jt_tensor* w, const b2
     return 0;
 }
 
+// the default layouts go to the plain entry point, which takes more shapes than the channels-last ones
+static bool formats_run_here(const ConvLayout& lay, bool layout_ok) {
+    return layout_ok || (!lay.x_nhwc && !lay.w_ohwi && !lay.y_nhwc);
+}
+
 extern "C" size_t b200jt_conv2d_formats_workspace(const b200jt_tensor* x, const b200jt_tensor* w, const b200jt_tensor* y,
                                                   int sh, int sw, int ph, int pw, int dh, int dw,
                                                   const char* xformat, const char* wformat, const char* yformat) {
     b200jt_tensor xl, wl, yl; ConvLayout lay; ConvShape s;
     if (conv_formats(x, w, y, xformat, wformat, yformat, &xl, &wl, &yl, &lay)) return 0;
     if (conv_shape(&xl, &wl, &yl, sh, sw, ph, pw, dh, dw, 1, &s)) return 0;
-    if (x->dtype == B200JT_BFLOAT16 && conv2d_tc_supported(s, x->ptr, w->ptr, y->ptr)) return conv2d_tc_workspace(s);
+    if (x->dtype == B200JT_BFLOAT16 && conv2d_tc_supported(s, x->ptr, w->ptr, y->ptr) && formats_run_here(lay, conv2d_tc_layout_supported(s))) return conv2d_tc_workspace(s);
     return 0;
 }
 
@@ -143,7 +148,8 @@ extern "C" int b200jt_conv2d_formats(const b200jt_tensor* x, const b200jt_tensor
     rc = conv_shape(&xl, &wl, &yl, sh, sw, ph, pw, dh, dw, 1, &s);
     if (rc) return rc;
     if (numel(y) == 0) return 0;
-    if (!(x->dtype == B200JT_BFLOAT16 && conv2d_tc_supported(s, x->ptr, w->ptr, y->ptr) && ((uintptr_t)y->ptr % 16 == 0)))
+    if (!(x->dtype == B200JT_BFLOAT16 && conv2d_tc_supported(s, x->ptr, w->ptr, y->ptr) && conv2d_tc_layout_supported(s) &&
+          ((uintptr_t)y->ptr % 16 == 0)))
         return fail(-5, "b200jt_conv2d_formats: acdb / ohwi layouts run on the tensor-core kernel only (bfloat16, in channels a "
                         "multiple of 8 and >= 64, out channels >= 64, at least 1024 output pixels, 16-byte aligned tensors)");
     const size_t need = conv2d_tc_workspace(s);
@@ -164,7 +170,8 @@ extern "C" size_t b200jt_conv2d_backward_w_formats_workspace(const b200jt_tensor
     b200jt_tensor xl, wl, yl; ConvLayout lay; ConvShape s;
     if (conv_formats(x, dw, dy, xformat, wformat, yformat, &xl, &wl, &yl, &lay)) return 0;
     if (conv_shape(&xl, &wl, &yl, sh, sw, ph, pw, dh, dw_, 1, &s)) return 0;
-    if (x->dtype == B200JT_BFLOAT16 && conv2d_wgrad_tc_supported(s, x->ptr, dy->ptr, dw->ptr)) return conv2d_wgrad_tc_workspace(s);
+    if (x->dtype == B200JT_BFLOAT16 && conv2d_wgrad_tc_supported(s, x->ptr, dy->ptr, dw->ptr) &&
+        formats_run_here(lay, conv2d_wgrad_tc_layout_supported(s))) return conv2d_wgrad_tc_workspace(s);
     return 0;
 }
 
@@ -180,7 +187,8 @@ extern "C" int b200jt_conv2d_backward_w_formats(const b200jt_tensor* x, const b2
     rc = conv_shape(&xl, &wl, &yl, sh, sw, ph, pw, dh, dw_, 1, &s);
     if (rc) return rc;
     if (numel(dw) == 0) return 0;
-    if (!(x->dtype == B200JT_BFLOAT16 && conv2d_wgrad_tc_supported(s, x->ptr, dy->ptr, dw->ptr)))
+    if (!(x->dtype == B200JT_BFLOAT16 && conv2d_wgrad_tc_supported(s, x->ptr, dy->ptr, dw->ptr) &&
+          conv2d_wgrad_tc_layout_supported(s)))
         return fail(-5, "b200jt_conv2d_backward_w_formats: acdb / ohwi layouts run on the tensor-core kernel only (bfloat16, in and "
                         "out channels multiples of 8 and >= 64, outputs of at least 8 x 8 per image and 4096 pixels in all, "
                         "16-byte aligned x and dy)");

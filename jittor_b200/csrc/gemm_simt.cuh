@@ -27,6 +27,8 @@ int batched_matmul_tc(const void* a, const void* b, void* c, int64_t batch, int6
 int tc_status_fetch_and_clear();
 
 bool conv2d_tc_supported(const ConvShape& s, const void* x, const void* w, const void* y);
+bool conv2d_tc_layout_supported(const ConvShape& s);
+bool conv2d_wgrad_tc_layout_supported(const ConvShape& s);
 size_t conv2d_tc_workspace(const ConvShape& s);
 // returns < 0 / > 1 on error, 0 on success, 1 on success with `stats` filled by the epilogue
 int conv2d_tc(const void* x, const void* w, void* y, float* stats, const ConvShape& s, void* workspace, cudaStream_t st,
