@@ -70,7 +70,7 @@ extern "C" int b200jt_batched_matmul(const b200jt_tensor* a, const b200jt_tensor
     if (batch == 0 || M == 0 || N == 0) return 0;
     cudaStream_t st = (cudaStream_t)stream;
     if (a->dtype == B200JT_BFLOAT16 && batched_matmul_tc_supported(batch, M, N, K, trans_a != 0, trans_b != 0, a->ptr, b->ptr, c->ptr))
-        return batched_matmul_tc(a->ptr, b->ptr, c->ptr, batch, a->shape[0], b->shape[0], M, N, K, trans_b != 0, st);
+        return batched_matmul_tc(a->ptr, b->ptr, c->ptr, batch, a->shape[0], b->shape[0], M, N, K, trans_a != 0, trans_b != 0, st);
     if (a->dtype == B200JT_FLOAT32 && matmul_f32_supported(batch, M, N, K))
         return matmul_f32(a->ptr, b->ptr, c->ptr, batch, a->shape[0], b->shape[0], M, N, K, trans_a != 0, trans_b != 0, nullptr, 0, st);
     return batched_matmul_simt(a->ptr, b->ptr, c->ptr, a->dtype, batch, a->shape[0], b->shape[0], M, N, K,

@@ -3,14 +3,14 @@
 // The broadcast-multiply-sum matmul of the reference (python/jittor/nn.py:157-159) is a dense contraction; its
 // relay is cublasGemmEx (python/jittor/extern/cuda/cublas/ops/cublas_matmul_op.cc:117-123). Here it is one
 // persistent, warp-specialised kernel:
-//   warp 0     TMA producer: cp.async.bulk.tensor 2-D loads of 128x64 (A) and 256x64 (Bt) bf16 tiles, 128-byte
-//              swizzle, into a 4-stage shared-memory ring (192 KB), completion on mbarriers;
-//   warp 1     MMA issuer: one lane issues tcgen05.mma.cta_group::1.kind::f16 (M=128, N=256, K=16) on shared-memory
-//              descriptors; accumulators live in TMEM, 2 x 256 columns so the next tile starts while the previous
-//              one is drained; tcgen05.commit releases ring slots / publishes accumulators;
+//   warp 0     TMA producer: cp.async.bulk.tensor loads of 64-deep bf16 tiles, 128-byte swizzle, into a 192 KB
+//              shared-memory ring, completion on mbarriers;
+//   warp 1     MMA issuer: one lane issues tcgen05.mma.kind::f16 (M = 128 per CTA, N <= 256, K = 16) on shared-memory
+//              descriptors, for one CTA or for a pair of CTAs; accumulators live in TMEM; tcgen05.commit releases ring
+//              slots / publishes accumulators;
 //   warps 2-5  epilogue: tcgen05.ld (32 lanes x 32 columns), fp32 -> bf16, 16-byte global stores.
-// Tiles are scheduled statically (tile = blockIdx.x + i*gridDim.x) in groups of 8 tile-rows for L2 reuse; one CTA
-// per SM. Ragged M/N/K edges rely on TMA zero fill and masked stores. No cluster launch and no multicast.
+// Work items are scheduled statically in groups of tile-rows for L2 reuse; one CTA per SM. Ragged M/N/K edges rely on TMA
+// zero fill and masked stores. No load is multicast.
 // Every mbarrier wait is bounded: on expiry the CTA records a status word, stops issuing, drains and frees TMEM.
 #include "gemm_simt.cuh"
 #include "tc_common.cuh"
@@ -22,104 +22,124 @@ namespace b200jt {
 
 namespace tc {
 
-constexpr int BM = 128, BN = 256, BK = 64;          // one MMA tile; BK * 2 B = 128 B = swizzle width
-constexpr int A_BYTES = BM * BK * 2, B_BYTES = BN * BK * 2;
+constexpr int BM = 128, BK = 64;                    // rows of one CTA's MMA tile; BK * 2 B = 128 B = swizzle width
+constexpr int MAX_BN = 256;
+constexpr int A_BYTES = BM * BK * 2;
+constexpr int BOX_BYTES = 64 * BK * 2;              // one MN-major box: 64 elements of the operand's own axis x 64 of K
 constexpr int THREADS = 192;                        // 6 warps
+constexpr int EPI_PITCH = 34;                       // bf16 per staged row of a ragged store
 
-// MT = number of 128-row MMA tiles a CTA stacks per output tile. MT = 2 re-uses every Bt stage for two MMAs
-// (64 KB of operands per 8.4 MFLOP instead of 48 KB per 4.2 MFLOP), so the same 192 KB ring covers 1.5x more time
-// of tensor work -- enough to hide an HBM miss -- at the price of a single TMEM accumulator set (512 columns).
-template <int MT> struct Cfg {
-    static constexpr int STAGES = MT == 1 ? 4 : 3;
+// What bounds a large product is the tensor pipe as long as the operands' way from L2 into shared memory stays below it: a
+// 128 x 256 tile per SM takes 48 KB per 4.2 MFLOP, a 256 x 256 tile per CTA pair 32 KB per SM, a 512 x 256 tile per pair 48 KB
+// per 8.4 MFLOP. 16384 x 4096 x 4096: 375, 342 and 356 us (1467, 1607 and 1542 TFLOP/s; 256 x 256 per single CTA was 465);
+// 4096 x 4096 x 16384 with both operands MN-major: 550, 429 and 390 us (and 560 with A transposed by a pass of its own).
+//   PAIR  two CTAs of a cluster share one accumulator of 256 rows (tcgen05 cta_group::2): each loads its 128 rows of A and
+//         HALF of the Bt tile, the leader's MMA reads both. No load is multicast.
+//   MT    accumulators per CTA: 2 re-uses each Bt stage for two MMAs and takes all 512 TMEM columns; with 1 there are two
+//         accumulator sets and the epilogue of a tile overlaps the next tile's MMAs.
+template <bool PAIR, int MT> struct Cfg {
+    static constexpr int CTAS = PAIR ? 2 : 1;
+    static constexpr int B_BYTES = MAX_BN / CTAS * BK * 2;
     static constexpr int STAGE_BYTES = MT * A_BYTES + B_BYTES;
-    static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*alignment slack*/ + 256 /*barriers*/;
+    static constexpr int STAGES = (192 * 1024) / STAGE_BYTES;
+    static constexpr int EPI_BYTES = 4 * 32 * EPI_PITCH * 2;
+    static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*alignment slack*/ + 256 /*barriers*/ + EPI_BYTES;
     static constexpr int NBUF = 2 / MT;             // accumulator sets in the 512 TMEM columns
+    static constexpr int TILE_M = CTAS * MT * BM;
 };
 
-struct Tiles {
-    int tiles_m, tiles_n, total, G;                          // G: tile-rows per group (L2 reuse of the Bt tiles)
-    __device__ __forceinline__ void coords(int t, int& m, int& n) const {
-        const int per_group = G * tiles_n;
-        const int g = t / per_group, r = t - g * per_group;
-        const int rows = min(G, tiles_m - g * G);
-        m = g * G + r % rows;
-        n = r / rows;
-    }
+struct GemmArgs {
+    int M, N, K;
+    int tiles_m, tiles_n, bn, k_blocks;
+    int units;                     // splits x batch x tiles_m x tiles_n work items
+    int batch, splits, group;      // group: tile-rows that are walked together (L2 reuse of the Bt tiles)
+    int a_batched, b_batched;      // an operand whose batch extent is 1 is shared by all products
+    int pitch;                     // of a row of partial sums (splits > 1)
 };
 
-// BMN: B is given as [K, N] (N contiguous) and used as an MN-major operand -- four 64 x 64 TMA boxes per stage -- instead
-// of being transposed into K-major form by a separate pass.
-// BATCH: the maps are 3-D ([batch][rows][cols]) and the tile index runs over batch x tiles; an operand whose batch
-// extent is 1 is shared by all products (its batch coordinate stays 0). This is the strided-batched product the
-// reference relays to cublasGemmStridedBatchedEx (python/jittor/extern/cuda/cublas/ops/cublas_batched_matmul_op.cc:160).
-template <int MT, bool BMN, bool BATCH = false>
+struct Unit { int split, batch, tm, tn, kb0, kb1; };
+__device__ __forceinline__ Unit unit_at(const GemmArgs& A, int u) {
+    Unit w;
+    const int tiles = A.tiles_m * A.tiles_n;
+    int i = u / tiles;
+    const int t = u - i * tiles;
+    w.split = i / A.batch; w.batch = i - w.split * A.batch;
+    const int per_group = A.group * A.tiles_n, g = t / per_group, r = t - g * per_group;
+    const int rows = min(A.group, A.tiles_m - g * A.group);
+    w.tm = g * A.group + r % rows; w.tn = r / rows;
+    w.kb0 = (int)((int64_t)A.k_blocks * w.split / A.splits);
+    w.kb1 = (int)((int64_t)A.k_blocks * (w.split + 1) / A.splits);
+    return w;
+}
+
+// AMN / BMN: the operand's own axis (M / N) is the contiguous one in memory; it is then loaded in 64 x 64 boxes and used
+// as an MN-major operand, so no operand is ever transposed by a pass of its own.
+// Accumulators leave as bf16 in c, or -- when K is split -- as fp32 partial sums in part[split][M][pitch], which
+// fold_kernel adds in split order. The tensor maps are 3-D ([batch][rows][cols]).
+template <bool PAIR, int MT, bool AMN, bool BMN>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                 __nv_bfloat16* __restrict__ c, int M, int N, int K, int group, uint32_t b_lbo, uint32_t b_sbo,
-                 int batch = 1, int a_batched = 0, int b_batched = 0) {
-    constexpr int STAGES = Cfg<MT>::STAGES, STAGE_BYTES = Cfg<MT>::STAGE_BYTES, NBUF = Cfg<MT>::NBUF;
+                 __nv_bfloat16* __restrict__ c, float* __restrict__ part, const __grid_constant__ GemmArgs A) {
+    using F = Cfg<PAIR, MT>;
+    constexpr int STAGES = F::STAGES, STAGE_BYTES = F::STAGE_BYTES, NBUF = F::NBUF, CTAS = F::CTAS;
     extern __shared__ unsigned char smem_raw[];
     // operand tiles need 1024-byte alignment for the 128-byte swizzle
     unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint64_t* bars = (uint64_t*)(smem + STAGES * STAGE_BYTES);
-    uint64_t* full = bars;                 // [STAGES] TMA -> MMA
-    uint64_t* empty = bars + STAGES;       // [STAGES] MMA -> TMA
+    uint64_t* full = bars;                       // [STAGES] TMA -> MMA (a pair uses the leader's)
+    uint64_t* empty = bars + STAGES;             // [STAGES] MMA -> TMA
     uint64_t* acc_full = bars + 2 * STAGES;      // [2] MMA -> epilogue
-    uint64_t* acc_empty = bars + 2 * STAGES + 2; // [2] epilogue -> MMA
+    uint64_t* acc_empty = bars + 2 * STAGES + 2; // [2] epilogue -> MMA (a pair uses the leader's)
     uint32_t* tmem_slot = (uint32_t*)(bars + 2 * STAGES + 4);
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
+    unsigned char* epi = smem + STAGES * STAGE_BYTES + 256;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    Tiles T;
-    T.tiles_m = (M + MT * BM - 1) / (MT * BM); T.tiles_n = (N + BN - 1) / BN; T.total = T.tiles_m * T.tiles_n; T.G = group;
-    const int k_blocks = (K + BK - 1) / BK;
-    const int per_batch = T.total;
-    const int all_tiles = BATCH ? per_batch * batch : per_batch;
+    const int rank = PAIR ? (int)cluster_rank() : 0;
+    const int first = blockIdx.x / CTAS, step = gridDim.x / CTAS;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; s++) { mbar_init(full + s, 1); mbar_init(empty + s, 1); }
-        for (int b = 0; b < NBUF; b++) { mbar_init(acc_full + b, 1); mbar_init(acc_empty + b, 4); }
+        for (int b = 0; b < NBUF; b++) { mbar_init(acc_full + b, 1); mbar_init(acc_empty + b, 4 * CTAS); }
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 1) {
-        // all 512 TMEM columns: two 128 x 256 fp32 accumulators
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(tmem_slot)) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
+    if (warp == 1) tmem_alloc<CTAS>(tmem_slot);             // all 512 columns
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if (PAIR) cluster_sync();                               // the peer's barriers exist before anything signals them
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = *tmem_slot;
 
     if (warp == 0) {
         // ---------------- TMA producer ----------------
         if (lane == 0) {
+            const int half = A.bn / CTAS;                   // this CTA's columns of the Bt tile
+            const int boxes = (half + 63) / 64;
+            const uint32_t bytes = CTAS * (uint32_t)(MT * A_BYTES + (BMN ? boxes * BOX_BYTES : half * BK * 2));
             int stage = 0; uint32_t phase = 0;
             bool ok = true;
-            for (int t = blockIdx.x; t < all_tiles && ok; t += gridDim.x) {
-                const int bi = BATCH ? t / per_batch : 0;
-                int tm, tn; T.coords(BATCH ? t - bi * per_batch : t, tm, tn);
-                const int ba = a_batched ? bi : 0, bb = b_batched ? bi : 0;
-                for (int kb = 0; kb < k_blocks; kb++) {
+            for (int u = first; u < A.units && ok; u += step) {
+                const Unit w = unit_at(A, u);
+                const int ba = A.a_batched ? w.batch : 0, bb = A.b_batched ? w.batch : 0;
+                const int col0 = w.tn * A.bn + rank * half;
+                for (int kb = w.kb0; kb < w.kb1; kb++) {
                     if (!(ok = mbar_wait(empty + stage, phase ^ 1, abort_flag, 1))) break;
                     unsigned char* sa = smem + stage * STAGE_BYTES;
-                    mbar_expect_tx(full + stage, STAGE_BYTES);
+                    if (rank == 0) mbar_expect_tx(full + stage, bytes);      // both CTAs' bytes
+                    const uint32_t bar = PAIR ? leader_addr(full + stage) : smem_u32(full + stage);
 #pragma unroll
                     for (int j = 0; j < MT; j++) {
-                        if (BATCH) tma_load_3d(sa + j * A_BYTES, &map_a, full + stage, kb * BK, (tm * MT + j) * BM, ba);
-                        else tma_load_2d(sa + j * A_BYTES, &map_a, full + stage, kb * BK, (tm * MT + j) * BM);
+                        const int row0 = w.tm * F::TILE_M + (j * CTAS + rank) * BM;
+                        if (AMN) {
+                            tma_load_tile<CTAS>(sa + j * A_BYTES, &map_a, bar, row0, kb * BK, ba);
+                            tma_load_tile<CTAS>(sa + j * A_BYTES + BOX_BYTES, &map_a, bar, row0 + 64, kb * BK, ba);
+                        } else tma_load_tile<CTAS>(sa + j * A_BYTES, &map_a, bar, kb * BK, row0, ba);
                     }
+                    unsigned char* sb = sa + MT * A_BYTES;
                     if (BMN) {
-#pragma unroll
-                        for (int cch = 0; cch < BN / 64; cch++) {
-                            if (BATCH) tma_load_3d(sa + MT * A_BYTES + cch * (64 * BK * 2), &map_b, full + stage, tn * BN + cch * 64, kb * BK, bb);
-                            else tma_load_2d(sa + MT * A_BYTES + cch * (64 * BK * 2), &map_b, full + stage, tn * BN + cch * 64, kb * BK);
-                        }
-                    } else {
-                        if (BATCH) tma_load_3d(sa + MT * A_BYTES, &map_b, full + stage, kb * BK, tn * BN, bb);
-                        else tma_load_2d(sa + MT * A_BYTES, &map_b, full + stage, kb * BK, tn * BN);
-                    }
+                        for (int q = 0; q < boxes; q++) tma_load_tile<CTAS>(sb + q * BOX_BYTES, &map_b, bar, col0 + q * 64, kb * BK, bb);
+                    } else tma_load_tile<CTAS>(sb, &map_b, bar, kb * BK, col0, bb);
                     if (++stage == STAGES) { stage = 0; phase ^= 1; }
                 }
             }
@@ -130,36 +150,37 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             }
         }
     } else if (warp == 1) {
-        // ---------------- MMA issuer ----------------
-        if (lane == 0) {
-            constexpr uint32_t idesc = make_idesc(BM, BN, BMN);
+        // ---------------- MMA issuer (of a pair: the leader's) ----------------
+        if (lane == 0 && rank == 0) {
+            const uint32_t idesc = make_idesc(BM * CTAS, A.bn, BMN) | ((AMN ? 1u : 0u) << 15);
+            // advancing K by 16: K-major +32 B inside the swizzled row (+2 units of 16 B); MN-major 16 rows of 128 B
+            constexpr int A_KSTEP = AMN ? (UMMA_K * 128) / 16 : 2, B_KSTEP = BMN ? (UMMA_K * 128) / 16 : 2;
             int stage = 0; uint32_t phase = 0;
             int it = 0;
             bool ok = true;
-            for (int t = blockIdx.x; t < all_tiles && ok; t += gridDim.x, it++) {
+            for (int u = first; u < A.units && ok; u += step, it++) {
+                const Unit w = unit_at(A, u);
                 const int buf = it % NBUF;
                 const uint32_t acc_phase = (it / NBUF) & 1;
-                if (!(ok = mbar_wait(acc_empty + buf, acc_phase ^ 1, abort_flag, 2))) break;
+                if (!(ok = mbar_wait<PAIR>(acc_empty + buf, acc_phase ^ 1, abort_flag, 2))) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t tmem_d = tmem_base + buf * (MT * BN);
-                for (int kb = 0; kb < k_blocks; kb++) {
+                const uint32_t tmem_d = tmem_base + buf * (MT * MAX_BN);
+                for (int kb = w.kb0; kb < w.kb1; kb++) {
                     if (!(ok = mbar_wait(full + stage, phase, abort_flag, 3))) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint32_t sa = smem_u32(smem + stage * STAGE_BYTES);
-                    const uint64_t db = BMN ? make_smem_desc_mn(sa + MT * A_BYTES, b_lbo, b_sbo) : make_smem_desc(sa + MT * A_BYTES);
-                    // advancing K by 16: K-major +32 B inside the swizzled row (+2 units of 16 B); MN-major 16 rows of 128 B
-                    constexpr int B_KSTEP = BMN ? (UMMA_K * 128) / 16 : 2;
+                    const uint64_t db = BMN ? make_smem_desc_mn(sa + MT * A_BYTES, BOX_BYTES, 1024) : make_smem_desc(sa + MT * A_BYTES);
 #pragma unroll
                     for (int j = 0; j < MT; j++) {
-                        const uint64_t da = make_smem_desc(sa + j * A_BYTES);
+                        const uint64_t da = AMN ? make_smem_desc_mn(sa + j * A_BYTES, BOX_BYTES, 1024) : make_smem_desc(sa + j * A_BYTES);
 #pragma unroll
                         for (int k = 0; k < BK / UMMA_K; k++)
-                            umma_f16(tmem_d + j * BN, da + 2 * k, db + B_KSTEP * k, idesc, (kb | k) != 0);
+                            umma_f16<CTAS>(tmem_d + j * MAX_BN, da + A_KSTEP * k, db + B_KSTEP * k, idesc, kb > w.kb0 || k != 0);
                     }
-                    umma_commit(empty + stage);                 // slot reusable once these MMAs have read it
+                    umma_commit<CTAS>(empty + stage);            // slot reusable (in both CTAs) once these MMAs have read it
                     if (++stage == STAGES) { stage = 0; phase ^= 1; }
                 }
-                if (ok) umma_commit(acc_full + buf);             // accumulator complete
+                if (ok) umma_commit<CTAS>(acc_full + buf);       // accumulator complete
             }
         }
     } else {
@@ -167,10 +188,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         const int quad = warp & 3;
         int it = 0;
         bool ok = true;
-        const bool vec_ok = (N % 8 == 0) && (((uintptr_t)c & 15) == 0);
-        for (int t = blockIdx.x; t < all_tiles && ok; t += gridDim.x, it++) {
-            const int bi = BATCH ? t / per_batch : 0;
-            int tm, tn; T.coords(BATCH ? t - bi * per_batch : t, tm, tn);
+        const bool vec_ok = (A.N % 8 == 0) && (((uintptr_t)c & 15) == 0);
+        __nv_bfloat16* rows = reinterpret_cast<__nv_bfloat16*>(epi) + quad * (32 * EPI_PITCH);
+        for (int u = first; u < A.units && ok; u += step, it++) {
+            const Unit w = unit_at(A, u);
             const int buf = it % NBUF;
             const uint32_t acc_phase = (it / NBUF) & 1;
             ok = mbar_wait(acc_full + buf, acc_phase, abort_flag, 4);
@@ -179,68 +200,106 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll 1
             for (int j = 0; j < MT; j++) {
-            const int row = (tm * MT + j) * BM + quad * 32 + lane;
-            const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + buf * (MT * BN) + j * BN;
-            __nv_bfloat16* crow = c + ((int64_t)bi * M + row) * N + (int64_t)tn * BN;
+                const int row0 = w.tm * F::TILE_M + (j * CTAS + rank) * BM + quad * 32, row = row0 + lane;
+                const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + buf * (MT * MAX_BN) + j * MAX_BN;
+                __nv_bfloat16* crow = c + ((int64_t)w.batch * A.M + row) * A.N;
 #pragma unroll 1
-            for (int ch = 0; ch < BN / 32; ch++) {
-                uint32_t r[32];
-                tmem_ld32(taddr + ch * 32, r);
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                const int col0 = tn * BN + ch * 32;
-                if (row < M && col0 < N) {
-                    if (vec_ok && col0 + 32 <= N) {
+                for (int ch = 0; ch < A.bn; ch += 32) {
+                    const int col0 = w.tn * A.bn + ch;
+                    if (row0 >= A.M || col0 >= A.N) break;       // uniform over the warp
+                    uint32_t r[32];
+                    tmem_ld32(taddr + ch, r);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    if (A.splits > 1) {
+                        float* prow = part + ((int64_t)w.split * A.M + row) * A.pitch + col0;
+                        if (row < A.M) {
 #pragma unroll
-                        for (int q = 0; q < 4; q++) {
-                            uint4 v;
-                            __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&v);
+                            for (int q = 0; q < 8; q++)
+                                if (col0 + q * 4 < A.pitch)
+                                    *reinterpret_cast<uint4*>(prow + q * 4) = make_uint4(r[q * 4], r[q * 4 + 1], r[q * 4 + 2], r[q * 4 + 3]);
+                        }
+                        continue;
+                    }
+                    __align__(16) __nv_bfloat162 h[16];
 #pragma unroll
-                            for (int e = 0; e < 4; e++)
-                                h[e] = __floats2bfloat162_rn(__uint_as_float(r[q * 8 + 2 * e]), __uint_as_float(r[q * 8 + 2 * e + 1]));
-                            *reinterpret_cast<uint4*>(crow + ch * 32 + q * 8) = v;
+                    for (int e = 0; e < 16; e++) h[e] = __floats2bfloat162_rn(__uint_as_float(r[2 * e]), __uint_as_float(r[2 * e + 1]));
+                    if (vec_ok) {
+                        if (row < A.M) {
+#pragma unroll
+                            for (int q = 0; q < 4; q++)
+                                if (col0 + q * 8 < A.N)
+                                    *reinterpret_cast<uint4*>(crow + col0 + q * 8) = reinterpret_cast<const uint4*>(h)[q];
                         }
                     } else {
-                        for (int e = 0; e < 32 && col0 + e < N; e++) crow[ch * 32 + e] = __float2bfloat16(__uint_as_float(r[e]));
+                        // rows start at any multiple of 2 bytes: turned around in shared memory, a warp then writes 64 B of a row at a time
+                        __syncwarp();
+#pragma unroll
+                        for (int e = 0; e < 16; e++) *reinterpret_cast<__nv_bfloat162*>(rows + lane * EPI_PITCH + 2 * e) = h[e];
+                        __syncwarp();
+                        if (col0 + lane < A.N) {
+                            __nv_bfloat16* q = c + ((int64_t)w.batch * A.M + row0) * A.N + col0 + lane;
+#pragma unroll 8
+                            for (int i = 0; i < 32; i++)
+                                if (row0 + i < A.M) q[(int64_t)i * A.N] = rows[i * EPI_PITCH + lane];
+                        }
                     }
                 }
             }
-            }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
-            if (lane == 0) mbar_arrive(acc_empty + buf);
+            if (lane == 0) { if (PAIR) mbar_arrive_leader(acc_empty + buf); else mbar_arrive(acc_empty + buf); }
         }
     }
     // ---------------- teardown ----------------
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if (PAIR) cluster_sync();          // neither CTA leaves while the other may still signal it or read its tiles
     if (warp == 1) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem_base) : "memory");
+        tmem_dealloc<CTAS>(tmem_base);
     }
 }
 
-// ---- bf16 transpose: out[c, r] = in[r, c] (used to bring an operand into K-major form) -------------------
+// c[m][n] = sum over splits (ascending) of part[split][m][n], rounded to bf16 once; four columns per thread.
 __global__ void __launch_bounds__(256)
-transpose_bf16_kernel(const __nv_bfloat16* __restrict__ in, __nv_bfloat16* __restrict__ out, int R, int Cn) {
-    __shared__ __nv_bfloat16 tile[64][66];
-    const int r0 = blockIdx.y * 64, c0 = blockIdx.x * 64;
-    const int tx = threadIdx.x % 32, ty = threadIdx.x / 32;          // 32 x 8
-    for (int i = ty; i < 64; i += 8) {
-        const int r = r0 + i;
-#pragma unroll
-        for (int j = 0; j < 2; j++) {
-            const int cc = c0 + tx * 2 + j;
-            tile[i][tx * 2 + j] = (r < R && cc < Cn) ? in[(int64_t)r * Cn + cc] : __float2bfloat16(0.f);
+fold_kernel(const float* __restrict__ part, __nv_bfloat16* __restrict__ c, int M, int N, int pitch, int splits) {
+    const int quads = pitch / 4;
+    const int64_t n = (int64_t)M * quads, plane = (int64_t)M * pitch;
+    const bool vec = N % 4 == 0 && ((uintptr_t)c & 7) == 0;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        float4 acc = __ldcs(reinterpret_cast<const float4*>(part) + i);
+        for (int s = 1; s < splits; s++) {
+            const float4 v = __ldcs(reinterpret_cast<const float4*>(part + s * plane) + i);
+            acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+        }
+        const int64_t m = i / quads; const int col = (int)(i - m * quads) * 4;
+        __nv_bfloat16* out = c + m * N + col;
+        const __nv_bfloat162 lo = __floats2bfloat162_rn(acc.x, acc.y), hi = __floats2bfloat162_rn(acc.z, acc.w);
+        if (vec) {
+            uint2 v; *reinterpret_cast<__nv_bfloat162*>(&v.x) = lo; *reinterpret_cast<__nv_bfloat162*>(&v.y) = hi;
+            *reinterpret_cast<uint2*>(out) = v;
+        } else {
+            out[0] = lo.x;
+            if (col + 1 < N) out[1] = lo.y;
+            if (col + 2 < N) out[2] = hi.x;
+            if (col + 3 < N) out[3] = hi.y;
         }
     }
-    __syncthreads();
-    for (int i = ty; i < 64; i += 8) {
-        const int cc = c0 + i;
+}
+
+// TMA wants rows at multiples of 16 bytes: [rows, cols] -> [rows, pitch] with pitch a multiple of 8, for an operand whose
+// contiguous extent is not one. Columns past cols are outside the tensor map and are not written.
+__global__ void __launch_bounds__(256)
+pad_rows_kernel(const __nv_bfloat16* __restrict__ in, __nv_bfloat16* __restrict__ out, int64_t rows, int cols, int pitch) {
+    const int chunks = pitch / 8;
+    const int64_t n = rows * chunks;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t r = i / chunks; const int c0 = (int)(i - r * chunks) * 8;
+        const __nv_bfloat16* p = in + r * cols + c0;
+        __align__(16) __nv_bfloat16 v[8];
 #pragma unroll
-        for (int j = 0; j < 2; j++) {
-            const int r = r0 + tx * 2 + j;
-            if (cc < Cn && r < R) out[(int64_t)cc * R + r] = tile[tx * 2 + j][i];
-        }
+        for (int e = 0; e < 8; e++) v[e] = c0 + e < cols ? p[e] : __float2bfloat16(0.f);
+        *reinterpret_cast<uint4*>(out + i * 8) = *reinterpret_cast<const uint4*>(v);
     }
 }
 
@@ -257,26 +316,12 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
     return fn;
 }
 
-// 2-D bf16 row-major [rows, cols] with a {BK, box_rows} box and 128-byte swizzle
-static bool make_map(CUtensorMap* map, const void* base, int64_t rows, int64_t cols, int box_rows) {
-    auto fn = encode_fn();
-    if (!fn) return false;
-    cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-    cuuint64_t strides[1] = {(cuuint64_t)cols * 2};
-    cuuint32_t box[2] = {(cuuint32_t)BK, (cuuint32_t)box_rows};
-    cuuint32_t estr[2] = {1, 1};
-    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
-                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    return r == CUDA_SUCCESS;
-}
-
-// 3-D bf16 [batch][rows][cols] with a {BK, box_rows, 1} box: one box has the shared-memory layout of the 2-D form
-static bool make_map_3d(CUtensorMap* map, const void* base, int64_t batch, int64_t rows, int64_t cols, int box_rows) {
+// bf16 [batch][rows][cols] with row pitch `pitch`, a {BK, box_rows, 1} box and 128-byte swizzle
+static bool make_map(CUtensorMap* map, const void* base, int64_t batch, int64_t rows, int64_t cols, int64_t pitch, int box_rows) {
     auto fn = encode_fn();
     if (!fn) return false;
     cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)rows, (cuuint64_t)batch};
-    cuuint64_t strides[2] = {(cuuint64_t)cols * 2, (cuuint64_t)rows * cols * 2};
+    cuuint64_t strides[2] = {(cuuint64_t)pitch * 2, (cuuint64_t)rows * pitch * 2};
     cuuint32_t box[3] = {(cuuint32_t)BK, (cuuint32_t)box_rows, 1};
     cuuint32_t estr[3] = {1, 1, 1};
     CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
@@ -285,116 +330,167 @@ static bool make_map_3d(CUtensorMap* map, const void* base, int64_t batch, int64
     return r == CUDA_SUCCESS;
 }
 
+template <bool PAIR, int MT>
+static const void* kernel_of(bool amn, bool bmn) {
+    return amn ? (bmn ? (const void*)gemm_bf16_kernel<PAIR, MT, true, true> : (const void*)gemm_bf16_kernel<PAIR, MT, true, false>)
+               : (bmn ? (const void*)gemm_bf16_kernel<PAIR, MT, false, true> : (const void*)gemm_bf16_kernel<PAIR, MT, false, false>);
+}
+static const void* kernel_of(bool pair, int mt, bool amn, bool bmn) {
+    return !pair ? kernel_of<false, 1>(amn, bmn) : mt == 1 ? kernel_of<true, 1>(amn, bmn) : kernel_of<true, 2>(amn, bmn);
+}
+static int smem_of(bool pair, int mt) {
+    return !pair ? Cfg<false, 1>::SMEM_BYTES : mt == 1 ? Cfg<true, 1>::SMEM_BYTES : Cfg<true, 2>::SMEM_BYTES;
+}
+
+// How many CTA pairs run at once (a persistent grid must not exceed it); 0 on error.
+static int pair_slots() {
+    static std::once_flag once;
+    static int slots = 0;
+    std::call_once(once, [] {
+        for (int pair = 0; pair < 2; pair++)
+            for (int mt = 1; mt <= 1 + pair; mt++)
+                for (int f = 0; f < 4; f++)
+                    if (cudaFuncSetAttribute(kernel_of(pair, mt, f & 1, f & 2), cudaFuncAttributeMaxDynamicSharedMemorySize, smem_of(pair, mt)) != cudaSuccess) return;
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension; at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+        cfg.gridDim = dim3(kNumSMs); cfg.blockDim = dim3(THREADS); cfg.dynamicSmemBytes = smem_of(true, 1); cfg.attrs = at; cfg.numAttrs = 1;
+        int n = 0;
+        if (cudaOccupancyMaxActiveClusters(&n, kernel_of(true, 1, false, false), &cfg) != cudaSuccess || n < 1) return;
+        slots = std::min(n, kNumSMs / 2);
+    });
+    return slots;
+}
+
+struct Plan { bool pair; int mt, bn, splits; double ns; };
+
+// Tile and split by estimated time. A k-block costs the larger of its MMAs (11 TFLOP/s per SM) and its operands' way from L2
+// (about 110 B per ns and SM); a tile adds its epilogue where no second accumulator hides it; split K adds the way of the partial
+// sums out and back and a second launch.
+static Plan plan_for(int64_t batch, int64_t M, int64_t N, int64_t K, bool bmn, bool may_split) {
+    Plan best{false, 1, MAX_BN, 1, 1e30};
+    const int64_t kb = (K + BK - 1) / BK;
+    const int pslots = pair_slots();
+    const char* fp = getenv("B200JT_GEMM_PAIR"); const char* fm = getenv("B200JT_GEMM_MT");      // read on every call:
+    const char* fb = getenv("B200JT_GEMM_BN"); const char* fs = getenv("B200JT_GEMM_SPLITS");    // tests force each variant in turn
+    for (int pair = 0; pair < 2; pair++) {
+        if ((fp && atoi(fp) != pair) || (pair && !pslots)) continue;
+        for (int mt = 1; mt <= 1 + pair; mt++) {
+            if (fm && atoi(fm) != mt && pair) continue;
+            const int tile_m = BM * mt * (1 + pair), slots = pair ? pslots : kNumSMs;
+            const int64_t tm = (M + tile_m - 1) / tile_m;
+            for (int bn = 32; bn <= MAX_BN; bn += 32) {
+                if (fb ? atoi(fb) != bn : bn > 32 && bn - 32 >= N) continue;
+                const int half = bn / (1 + pair);
+                const double feed = (mt * A_BYTES + (bmn ? (half + 63) / 64 * BOX_BYTES : half * BK * 2)) / 110.0;
+                const double mma = mt * std::max(bn, 64) * 1.5;
+                const double block = std::max(feed, mma) + 20;
+                const int64_t tiles = tm * ((N + bn - 1) / bn) * batch;
+                const double epi = mt * bn * 4.0;
+                int64_t tried = 0;
+                for (int q = 0; q < 3; q++) {
+                    int64_t s = q == 0 ? 1 : q == 1 ? slots / tiles : slots / tiles / 2;
+                    s = std::min(s, kb / 4);
+                    if (fs) s = std::min<int64_t>(atoi(fs), kb);
+                    if (s < 1 || !may_split) s = 1;
+                    if (s == tried) continue;
+                    tried = s;
+                    const double rounds = (double)((tiles * s + slots - 1) / slots);
+                    double ns = 2500 + rounds * ((kb + s - 1) / s * block + (mt == 2 ? epi : 0)) + epi;
+                    if (s > 1) ns += 3000 + (double)s * M * N * 8 / 4000;
+                    if (ns < best.ns) best = {pair != 0, mt, bn, (int)s, ns};
+                }
+            }
+        }
+    }
+    return best;
+}
+
+static int launch(const Plan& p, const void* a, const void* b, void* c, float* part, int64_t batch, int64_t a_batch, int64_t b_batch,
+                  int64_t M, int64_t N, int64_t K, int64_t pitch_a, int64_t pitch_b, bool amn, bool bmn, cudaStream_t st) {
+    const int ctas = p.pair ? 2 : 1, tile_m = BM * p.mt * ctas;
+    if (!pair_slots()) return fail(-4, "matmul: no room for the kernel's shared memory");
+    CUtensorMap ma, mb;
+    // K-major operands: boxes of 64 K-elements x rows; MN-major ones: boxes of 64 of their own elements x 64 K-rows
+    if (!(amn ? make_map(&ma, a, a_batch, K, M, pitch_a, 64) : make_map(&ma, a, a_batch, M, K, pitch_a, BM)) ||
+        !(bmn ? make_map(&mb, b, b_batch, K, N, pitch_b, 64) : make_map(&mb, b, b_batch, N, K, pitch_b, p.bn / ctas)))
+        return fail(-4, "matmul: cuTensorMapEncodeTiled failed");
+    GemmArgs A;
+    A.M = (int)M; A.N = (int)N; A.K = (int)K; A.bn = p.bn; A.k_blocks = (int)((K + BK - 1) / BK);
+    A.tiles_m = (int)((M + tile_m - 1) / tile_m); A.tiles_n = (int)((N + p.bn - 1) / p.bn);
+    A.batch = (int)batch; A.splits = p.splits; A.group = std::max(1, 1024 / tile_m);
+    A.a_batched = a_batch > 1; A.b_batched = b_batch > 1; A.pitch = (int)((N + 3) / 4 * 4);
+    const int64_t units = (int64_t)A.tiles_m * A.tiles_n * batch * p.splits;
+    if (units >= (1LL << 30)) return fail(-1, "matmul: too many tiles");
+    A.units = (int)units;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension; at[0].val.clusterDim.x = ctas; at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3((unsigned)(std::min<int64_t>(units, p.pair ? pair_slots() : kNumSMs) * ctas));
+    cfg.blockDim = dim3(THREADS); cfg.dynamicSmemBytes = smem_of(p.pair, p.mt); cfg.stream = st; cfg.attrs = at; cfg.numAttrs = p.pair ? 1 : 0;
+    void* args[] = {&ma, &mb, &c, &part, &A};
+    B200JT_CUDA(cudaLaunchKernelExC(&cfg, kernel_of(p.pair, p.mt, amn, bmn), args));
+    if (p.splits > 1) {
+        fold_kernel<<<grid_for(M * (A.pitch / 4), 256), 256, 0, st>>>(part, (__nv_bfloat16*)c, A.M, A.N, A.pitch, p.splits);
+        B200JT_LAUNCH_CHECK();
+    }
+    return 0;
+}
+
+inline int64_t pitch8(int64_t n) { return (n + 7) / 8 * 8; }
+inline size_t round256(size_t n) { return (n + 255) & ~(size_t)255; }
+
 }  // namespace tc
 
+// Any extents (an operand whose contiguous extent is not a multiple of 8 is first copied to TMA's pitch) once the product is
+// large enough to pay for a pipeline's fill and drain.
 bool matmul_tc_supported(int64_t M, int64_t N, int64_t K, const void* a, const void* b, const void* c) {
-    // TMA: 16-byte aligned bases and row pitches (K % 8); tiny problems stay on the CUDA-core kernel
-    return K % 8 == 0 && K >= 64 && M >= 128 && N >= 64 && M < (1LL << 31) && N < (1LL << 31) && K < (1LL << 31) &&
+    return K >= 32 && (double)M * N * K >= (double)(1 << 18) && M < (1LL << 30) && N < (1LL << 30) && K < (1LL << 30) &&
            ((uintptr_t)a % 16 == 0) && ((uintptr_t)b % 16 == 0) && ((uintptr_t)c % 2 == 0) && tc::encode_fn() != nullptr;
 }
 
-static bool b_mn_direct(int64_t N, bool trans_b) {
-    const char* e = getenv("B200JT_GEMM_BMN");
-    return !trans_b && N % 8 == 0 && !(e && atoi(e) == 0);
-}
-
 size_t matmul_tc_workspace(int64_t M, int64_t N, int64_t K, bool trans_a, bool trans_b) {
-    // A that is not K-major is transposed into the workspace first; B [K, N] is consumed directly as an MN-major operand
+    using namespace tc;
+    const int64_t ca = trans_a ? M : K, cb = trans_b ? K : N;
     size_t bytes = 0;
-    if (trans_a) bytes += (size_t)M * K * 2;
-    if (!trans_b && !b_mn_direct(N, trans_b)) bytes += (size_t)N * K * 2;
+    if (ca % 8) bytes += round256((size_t)(trans_a ? K : M) * pitch8(ca) * 2);
+    if (cb % 8) bytes += round256((size_t)(trans_b ? N : K) * pitch8(cb) * 2);
+    const Plan p = plan_for(1, M, N, K, !trans_b, true);
+    if (p.splits > 1) bytes += (size_t)p.splits * M * ((N + 3) / 4 * 4) * 4;
     return bytes;
 }
 
 int matmul_tc(const void* a, const void* b, void* c, int64_t M, int64_t N, int64_t K, bool trans_a, bool trans_b,
               void* workspace, cudaStream_t st) {
     using namespace tc;
-    const __nv_bfloat16* ak = (const __nv_bfloat16*)a;      // [M, K]
-    const __nv_bfloat16* bk = (const __nv_bfloat16*)b;      // [N, K]
     unsigned char* ws = (unsigned char*)workspace;
-    if (trans_a) {   // a is [K, M]
-        dim3 g((unsigned)((M + 63) / 64), (unsigned)((K + 63) / 64));
-        transpose_bf16_kernel<<<g, 256, 0, st>>>((const __nv_bfloat16*)a, (__nv_bfloat16*)ws, (int)K, (int)M);
-        ak = (const __nv_bfloat16*)ws; ws += (size_t)M * K * 2;
-    }
-    const bool bmn = b_mn_direct(N, trans_b);
-    if (!trans_b && !bmn) {  // b is [K, N]
-        dim3 g((unsigned)((N + 63) / 64), (unsigned)((K + 63) / 64));
-        transpose_bf16_kernel<<<g, 256, 0, st>>>((const __nv_bfloat16*)b, (__nv_bfloat16*)ws, (int)K, (int)N);
-        bk = (const __nv_bfloat16*)ws;
-    }
+    const Plan p = plan_for(1, M, N, K, !trans_b, true);
+    auto padded = [&](const void*& q, int64_t rows, int64_t cols) {
+        if (cols % 8 == 0) return cols;
+        const int64_t pitch = pitch8(cols);
+        pad_rows_kernel<<<grid_for(rows * (pitch / 8), 256), 256, 0, st>>>((const __nv_bfloat16*)q, (__nv_bfloat16*)ws, rows, (int)cols, (int)pitch);
+        q = ws; ws += round256((size_t)rows * pitch * 2);
+        return pitch;
+    };
+    const int64_t pa = trans_a ? padded(a, K, M) : padded(a, M, K);
+    const int64_t pb = trans_b ? padded(b, N, K) : padded(b, K, N);
     B200JT_LAUNCH_CHECK();
-    CUtensorMap ma, mb;
-    // K-major operands: boxes of 64 K-elements x rows; MN-major B: boxes of 64 N-elements x 64 K-rows of b[K, N]
-    if (!make_map(&ma, ak, M, K, BM) || !(bmn ? make_map(&mb, b, K, N, 64) : make_map(&mb, bk, N, K, BN)))
-        return fail(-4, "matmul: cuTensorMapEncodeTiled failed");
-    static std::once_flag once;
-    static cudaError_t attr_err = cudaSuccess;
-    std::call_once(once, [] {
-        attr_err = cudaFuncSetAttribute(gemm_bf16_kernel<1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<1>::SMEM_BYTES);
-        if (attr_err == cudaSuccess) attr_err = cudaFuncSetAttribute(gemm_bf16_kernel<2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<2>::SMEM_BYTES);
-        if (attr_err == cudaSuccess) attr_err = cudaFuncSetAttribute(gemm_bf16_kernel<1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<1>::SMEM_BYTES);
-        if (attr_err == cudaSuccess) attr_err = cudaFuncSetAttribute(gemm_bf16_kernel<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<2>::SMEM_BYTES);
-    });
-    B200JT_CUDA(attr_err);
-    // 256-row tiles when they still fill the machine for several waves, 128-row tiles otherwise
-    const int64_t tiles2 = ((M + 2 * BM - 1) / (2 * BM)) * ((N + BN - 1) / BN);
-    const char* genv = getenv("B200JT_GEMM_G");
-    const int group = genv ? atoi(genv) : 8;
-    const char* force = getenv("B200JT_GEMM_MT");
-    const bool two = force ? atoi(force) == 2 : tiles2 >= 4 * kNumSMs;
-    // MN-major B: 64-column chunks are 8 KB apart (leading offset), 8-row groups along K 1 KB apart (stride offset)
-    const uint32_t lbo = 64 * BK * 2, sbo = 1024;
-    const int64_t tiles1 = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
-    const int grid = (int)std::min<int64_t>(two ? tiles2 : tiles1, kNumSMs);
-#define B200JT_GEMM(MT_, BMN_) gemm_bf16_kernel<MT_, BMN_><<<grid, THREADS, Cfg<MT_>::SMEM_BYTES, st>>>( \
-        ma, mb, (__nv_bfloat16*)c, (int)M, (int)N, (int)K, group, lbo, sbo)
-    if (two) { if (bmn) B200JT_GEMM(2, true); else B200JT_GEMM(2, false); }
-    else     { if (bmn) B200JT_GEMM(1, true); else B200JT_GEMM(1, false); }
-#undef B200JT_GEMM
-    B200JT_LAUNCH_CHECK();
-    return 0;
+    return launch(p, a, b, c, (float*)ws, 1, 1, 1, M, N, K, pa, pb, trans_a, !trans_b, st);
 }
 
-// One launch for `batch` products c[i] = a[i or 0] . b[i or 0] (a [.., M, K] K-major; b [.., K, N] consumed MN-major, or
-// [.., N, K] when trans_b). The caller has checked batched_matmul_tc_supported.
+// One launch for `batch` products c[i] = a[i or 0] . b[i or 0]: no scratch, so operands whose pitches suit TMA as they are.
 bool batched_matmul_tc_supported(int64_t batch, int64_t M, int64_t N, int64_t K, bool trans_a, bool trans_b,
                                  const void* a, const void* b, const void* c) {
-    if (trans_a || !matmul_tc_supported(M, N, K, a, b, c) || batch >= (1LL << 31)) return false;
-    if ((M * K) % 8 != 0 || (N * K) % 8 != 0) return false;            // 16-byte batch pitch of the tensor maps
-    return trans_b || b_mn_direct(N, trans_b);
+    if (K < 64 || M < 128 || N < 64 || !matmul_tc_supported(M, N, K, a, b, c) || batch >= (1LL << 31)) return false;
+    if ((trans_a ? M : K) % 8 != 0 || (trans_b ? K : N) % 8 != 0) return false;
+    return batch * ((M + 127) / 128) * ((N + 31) / 32) < (1LL << 30);
 }
 
 int batched_matmul_tc(const void* a, const void* b, void* c, int64_t batch, int64_t a_batch, int64_t b_batch,
-                      int64_t M, int64_t N, int64_t K, bool trans_b, cudaStream_t st) {
+                      int64_t M, int64_t N, int64_t K, bool trans_a, bool trans_b, cudaStream_t st) {
     using namespace tc;
-    const bool bmn = !trans_b;
-    CUtensorMap ma, mb;
-    if (!make_map_3d(&ma, a, a_batch, M, K, BM) ||
-        !(bmn ? make_map_3d(&mb, b, b_batch, K, N, 64) : make_map_3d(&mb, b, b_batch, N, K, BN)))
-        return fail(-4, "batched matmul: cuTensorMapEncodeTiled failed");
-    static std::once_flag once;
-    static cudaError_t attr_err = cudaSuccess;
-    std::call_once(once, [] {
-        attr_err = cudaFuncSetAttribute(gemm_bf16_kernel<1, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<1>::SMEM_BYTES);
-        if (attr_err == cudaSuccess) attr_err = cudaFuncSetAttribute(gemm_bf16_kernel<2, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<2>::SMEM_BYTES);
-        if (attr_err == cudaSuccess) attr_err = cudaFuncSetAttribute(gemm_bf16_kernel<1, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<1>::SMEM_BYTES);
-        if (attr_err == cudaSuccess) attr_err = cudaFuncSetAttribute(gemm_bf16_kernel<2, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<2>::SMEM_BYTES);
-    });
-    B200JT_CUDA(attr_err);
-    const int64_t tiles2 = ((M + 2 * BM - 1) / (2 * BM)) * ((N + BN - 1) / BN) * batch;
-    const int64_t tiles1 = ((M + BM - 1) / BM) * ((N + BN - 1) / BN) * batch;
-    if (tiles1 >= (1LL << 31)) return fail(-1, "batched matmul: too many tiles");
-    const bool two = tiles2 >= 4 * kNumSMs && M > BM;
-    const uint32_t lbo = 64 * BK * 2, sbo = 1024;
-    const int grid = (int)std::min<int64_t>(two ? tiles2 : tiles1, kNumSMs);
-#define B200JT_BGEMM(MT_, BMN_) gemm_bf16_kernel<MT_, BMN_, true><<<grid, THREADS, Cfg<MT_>::SMEM_BYTES, st>>>( \
-        ma, mb, (__nv_bfloat16*)c, (int)M, (int)N, (int)K, 8, lbo, sbo, (int)batch, a_batch > 1 ? 1 : 0, b_batch > 1 ? 1 : 0)
-    if (two) { if (bmn) B200JT_BGEMM(2, true); else B200JT_BGEMM(2, false); }
-    else     { if (bmn) B200JT_BGEMM(1, true); else B200JT_BGEMM(1, false); }
-#undef B200JT_BGEMM
-    B200JT_LAUNCH_CHECK();
-    return 0;
+    return launch(plan_for(batch, M, N, K, !trans_b, false), a, b, c, nullptr, batch, a_batch, b_batch, M, N, K,
+                  trans_a ? M : K, trans_b ? K : N, trans_a, !trans_b, st);
 }
 
 int tc_status_fetch_and_clear() { return tc::status_fetch_and_clear(); }

@@ -46,3 +46,45 @@ def test_convolution_and_weight_gradient(n, ci, h, w, co, k, s, p, d, bn, monkey
     C.call("b200jt_conv2d_backward_w_tc", *args, ptr, size)
     near(dw, wd.grad)
     assert C.lib.b200jt_device_status() == 0
+
+
+# (M, N, K): extents around the tiles (128 / 256 / 512 rows, 32 .. 256 columns, 64 of K), pitches that are not multiples of 8,
+# products below one tile, K long enough to be split
+SIZES = [(64, 64, 64), (16, 4096, 512), (129, 33, 77), (513, 257, 130), (300, 10, 1000), (128, 256, 4096), (1031, 519, 321),
+         (2, 1000, 2048), (520, 601, 40), (4096, 64, 96)]
+VARIANTS = [{}, {"PAIR": 0, "BN": 32}, {"PAIR": 0, "BN": 224, "SPLITS": 3}, {"PAIR": 1, "MT": 1, "BN": 96}, {"PAIR": 1, "MT": 1, "BN": 256},
+            {"PAIR": 1, "MT": 2, "BN": 160, "SPLITS": 2}, {"PAIR": 1, "MT": 2, "BN": 256}]
+
+
+@pytest.mark.parametrize("variant", VARIANTS, ids=lambda v: "-".join(f"{k}{x}" for k, x in v.items()) or "chosen")
+@pytest.mark.parametrize("ta,tb", [(0, 0), (0, 1), (1, 0), (1, 1)])
+def test_matmul(ta, tb, variant, monkeypatch):
+    for k, v in variant.items():
+        monkeypatch.setenv("B200JT_GEMM_" + k, str(v))
+    for m, n, k in SIZES:
+        a = torch.randn(*((k, m) if ta else (m, k)), device="cuda").bfloat16()
+        b = torch.randn(*((n, k) if tb else (k, n)), device="cuda").bfloat16()
+        c = torch.full((m, n), float("nan"), device="cuda").bfloat16()
+        args = (C.desc(a), C.desc(b), C.desc(c), ta, tb)
+        size, ptr, ws = C.workspace("b200jt_matmul_workspace", *args)
+        want = (a.double().t() if ta else a.double()) @ (b.double().t() if tb else b.double())
+        C.call("b200jt_matmul", *args, ptr, size)
+        near(c, want)
+        if ta == 0 and n * m < 4096:                        # 2-byte aligned operand: the CUDA-core kernel
+            a1 = torch.randn(a.numel() + 1, device="cuda").bfloat16()[1:].view_as(a)
+            C.call("b200jt_matmul", C.desc(a1), *args[1:], ptr, size)
+            near(c, a1.double() @ (b.double().t() if tb else b.double()))
+    assert C.lib.b200jt_device_status() == 0
+
+
+@pytest.mark.parametrize("pair", [0, 1])
+@pytest.mark.parametrize("ta,tb", [(0, 0), (0, 1), (1, 0), (1, 1)])
+def test_batched_matmul(ta, tb, pair, monkeypatch):
+    monkeypatch.setenv("B200JT_GEMM_PAIR", str(pair))
+    for ba, bb, m, n, k in [(3, 3, 128, 64, 64), (1, 5, 136, 72, 200), (4, 1, 520, 264, 72)]:
+        a = torch.randn(ba, *((k, m) if ta else (m, k)), device="cuda").bfloat16()
+        b = torch.randn(bb, *((n, k) if tb else (k, n)), device="cuda").bfloat16()
+        c = torch.full((max(ba, bb), m, n), float("nan"), device="cuda").bfloat16()
+        C.call("b200jt_batched_matmul", C.desc(a), C.desc(b), C.desc(c), ta, tb)
+        near(c, (a.double().transpose(1, 2) if ta else a.double()) @ (b.double().transpose(1, 2) if tb else b.double()))
+    assert C.lib.b200jt_device_status() == 0
