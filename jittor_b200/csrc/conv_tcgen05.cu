@@ -7,8 +7,9 @@
 //               operands are K-major and every TMA box starts at a channel offset that is a multiple of 64 (the
 //               16-byte start rule); the spatial shift of a tap is carried by the H/W box coordinates, which may be
 //               negative or past the edge -- TMA zero-fills, which is exactly the reindex overflow value 0;
-//   tile        128 pixels (two 8x8 spatial patches, each one 4-D TMA box of 64 rows x 128 B) x 256 output channels;
-//   pipeline    same persistent warp-specialised ring as the GEMM (TMA warp, MMA warp, 4 epilogue warps, TMEM
+//   tile        128 pixels (two spatial patches of 64, each one 4-D TMA box of 64 rows x 128 B) x up to 256 output
+//               channels, for one CTA or twice the pixels for a pair of CTAs;
+//   pipeline    same persistent warp-specialised ring as the GEMM (TMA warp, MMA warp, 8 epilogue warps, TMEM
 //               double buffering); strides 1..4 through the traversal stride of the x tensor map;
 //   epilogue    tcgen05.ld -> bf16 -> y in NCHW; optionally per-channel sum / sum of squares of the stored values
 //               (the two reduce.mean of BatchNorm, python/jittor/nn.py:674-675) accumulated per CTA in shared memory
@@ -24,25 +25,31 @@ namespace tcconv {
 using namespace tc;
 
 constexpr int BM = 128, BN = 256, BK = 64;
-constexpr int PATCH = 8;                            // spatial patch edge: 8 x 8 = 64 pixels = half a tile
-constexpr int STAGES = 4;
-constexpr int A_BYTES = BM * BK * 2, B_BYTES = BN * BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;
+constexpr int A_BYTES = BM * BK * 2;
+// PAIR: the two CTAs of a cluster work on one tile of 256 pixels (tcgen05 cta_group::2). Each loads its own 128 pixels and HALF
+// of the weights, the leader's MMA reads both: 32 KB instead of 48 KB per stage and SM at 256 output channels. A tile alone on
+// its SM waits for the latency of its loads, so a ring holds as many stages as fit.
+template <int BN_T, bool PAIR> struct Ring {
+    static constexpr int STAGE_BYTES = A_BYTES + BN_T * BK * 2 / (PAIR ? 2 : 1);
+    static constexpr int STAGES = (192 * 1024) / STAGE_BYTES < 8 ? (192 * 1024) / STAGE_BYTES : 8;
+};
+constexpr int RING_BYTES = 192 * 1024;
 constexpr int STATS_MAX_CO = 512;                   // widest layer whose statistics the epilogue can keep per CTA
 constexpr int STATS_BYTES = 2 * STATS_MAX_CO * 4;
-constexpr int OUT_STAGE_BYTES = 2 * 64 * 64 * 2;      // TMA-store staging: 2 patches x 64 channels x 64 pixels
-constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256 + STATS_BYTES + OUT_STAGE_BYTES;
-constexpr int THREADS = 192;
-// cost per FLOP of 128-wide and 64-wide tiles relative to 256-wide ones (the feed from L2, not the tensor pipe, bounds them)
-constexpr double kNarrowTilePenalty = 1.5, kThinTilePenalty = 2.5;
+constexpr int OUT_STAGE_BYTES = 8 * 32 * 32 * 2;      // one 32 channel x 32 pixel square per epilogue warp
+constexpr int SMEM_BYTES = RING_BYTES + 1024 + 256 + STATS_BYTES + OUT_STAGE_BYTES;
+constexpr int THREADS = 320;                         // producer, MMA and 8 epilogue warps
 // Channel pitch of the channels-last copies: TMA wants row pitches of 16 bytes. Channels past C are outside the tensor map and
 // read as zero, so any channel count runs here.
 inline int pitch8(int c) { return (c + 7) / 8 * 8; }
 
 struct ConvArgs {
     int N, C, H, W, Co, KH, KW, OH, OW, sh, sw, ph, pw, dh, dw;
+    int pw_log;                      // a patch is 64 pixels, half a tile: (64 >> pw_log) rows of (1 << pw_log) pixels
     int tiles_h, tiles_w;            // patches per image
     int64_t patches;                 // N * tiles_h * tiles_w
     int tiles_m, tiles_n;
+    int vec;                         // pixels per store of y: the largest of 8, 4, 2, 1 that divides OW (and y's alignment)
     int last_k;                      // MMA steps of 16 channels in a tap's last channel block
 };
 
@@ -50,52 +57,57 @@ __device__ __forceinline__ void patch_coords(const ConvArgs& A, int64_t q, int& 
     const int per_img = A.tiles_h * A.tiles_w;
     n = (int)(q / per_img);
     const int r = (int)(q - (int64_t)n * per_img);
-    h0 = (r / A.tiles_w) * PATCH;
-    w0 = (r % A.tiles_w) * PATCH;
+    h0 = (r / A.tiles_w) * (64 >> A.pw_log);
+    w0 = (r % A.tiles_w) << A.pw_log;
 }
 
-// OUT == 1: the epilogue stages 64 channels x 128 pixels of bf16 in shared memory ([patch][channel][8x8]) and writes
-// them to y (NCHW) with two 4-D TMA box stores; edges are clipped by the tensor map. Needs OW % 8 == 0 (16-byte row
-// pitch); otherwise (OUT == 0) the lanes store their values directly. OUT == 2: y is NHWC ("acdb"), a lane stores the 32
-// consecutive channels of its pixel as four 16-byte vectors.
-// BN_T: output channels per tile (256, or 128 when that fills the last wave of the persistent grid better; the
-// shared-memory ring keeps the 256-channel stage size either way).
-template <int OUT, int BN_T>
+__device__ __forceinline__ int first_block(int tm, int k_blocks) { return (int)((tm * 7u) % (unsigned)k_blocks); }
+
+// NCHW y: a warp turns its 32 pixels x 32 channels around in shared memory and stores rows of up to 8 pixels. (TMA box stores
+// of [8][8] pixels move a row of 16 bytes in 1.7 ns, whatever there is to it: 6.8 us for a 128 x 256 tile.)
+// NHWC ("acdb"): a lane stores the 32 consecutive channels of its pixel as four 16-byte vectors.
+// BN_T: output channels per tile (256, or less where that fills the last wave of the persistent grid better).
+// The epilogue's eight warps are two per TMEM lane quadrant, each with every other 32 channels: four warps took longer than the
+// main loop of a 1 x 1 layer (64 x 64 x 56 x 56 -> 256 channels with
+// statistics, layout pass included: 142 us with four warps and box stores, 87 us now).
+// Each tile walks K from a start of its own. All tiles read the same weights: in step with one another they queue at the L2
+// slices that hold the current 32 KB (7 x 432 x 28 x 28 -> 320 channels, 3 x 3: 60 us
+// in step, 54 us this way).
+template <bool NHWC, int BN_T, bool PAIR>
 __global__ void __launch_bounds__(THREADS, 1)
 conv_bf16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
-                 const __grid_constant__ CUtensorMap map_y,
                  __nv_bfloat16* __restrict__ y, float* __restrict__ stats, const __grid_constant__ ConvArgs A) {
+    constexpr int CTAS = PAIR ? 2 : 1, STAGES = Ring<BN_T, PAIR>::STAGES, STAGE_BYTES = Ring<BN_T, PAIR>::STAGE_BYTES;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    uint64_t* bars = (uint64_t*)(smem + STAGES * STAGE_BYTES);
-    uint64_t* full = bars;
+    uint64_t* bars = (uint64_t*)(smem + RING_BYTES);
+    uint64_t* full = bars;                       // a pair uses the leader's
     uint64_t* empty = bars + STAGES;
-    uint64_t* acc_full = bars + 2 * STAGES;
+    uint64_t* acc_full = bars + 2 * STAGES;      // acc_empty: a pair uses the leader's
     uint64_t* acc_empty = bars + 2 * STAGES + 2;
     uint32_t* tmem_slot = (uint32_t*)(bars + 2 * STAGES + 4);
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
-    float* sstat = (float*)(smem + STAGES * STAGE_BYTES + 256);      // [2][STATS_MAX_CO] per-CTA channel sums
-    unsigned char* stage_out = smem + STAGES * STAGE_BYTES + 256 + STATS_BYTES;   // [2 patches][64 ch][64 px] bf16
-    constexpr bool TMA_OUT = OUT == 1;
+    float* sstat = (float*)(smem + RING_BYTES + 256);      // [2][STATS_MAX_CO] per-CTA channel sums
+    unsigned char* stage_out = smem + RING_BYTES + 256 + STATS_BYTES;   // [8 warps][32 ch][32 px] bf16
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int rank = PAIR ? (int)cluster_rank() : 0;
+    const int first = blockIdx.x / CTAS, step = gridDim.x / CTAS;
     const int total = A.tiles_m * A.tiles_n;
     const int cblocks = (A.C + BK - 1) / BK;
     const int k_blocks = A.KH * A.KW * cblocks;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; s++) { mbar_init(full + s, 1); mbar_init(empty + s, 1); }
-        for (int b = 0; b < 2; b++) { mbar_init(acc_full + b, 1); mbar_init(acc_empty + b, 4); }
+        for (int b = 0; b < 2; b++) { mbar_init(acc_full + b, 1); mbar_init(acc_empty + b, 8 * CTAS); }
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     for (int i = threadIdx.x; i < 2 * STATS_MAX_CO; i += blockDim.x) sstat[i] = 0.f;
-    if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(tmem_slot)) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
+    if (warp == 1) tmem_alloc<CTAS>(tmem_slot);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if (PAIR) cluster_sync();                 // the peer's barriers exist before anything signals them
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = *tmem_slot;
 
@@ -103,22 +115,27 @@ conv_bf16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         if (lane == 0) {
             int stage = 0; uint32_t phase = 0;
             bool ok = true;
-            for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
+            for (int t = first; t < total && ok; t += step) {
                 const int tm = t / A.tiles_n, tn = t - tm * A.tiles_n;
                 int n0, h0, w0, n1, h1, w1;
-                patch_coords(A, 2 * (int64_t)tm, n0, h0, w0);
-                patch_coords(A, 2 * (int64_t)tm + 1, n1, h1, w1);       // past the last patch: n1 >= N, zero-filled
+                patch_coords(A, 2 * ((int64_t)tm * CTAS + rank), n0, h0, w0);
+                patch_coords(A, 2 * ((int64_t)tm * CTAS + rank) + 1, n1, h1, w1);       // past the last patch: n1 >= N, zero-filled
+                int tap = first_block(tm, k_blocks) / cblocks, cb = first_block(tm, k_blocks) - tap * cblocks;
+                int kh = tap / A.KW, kw = tap - kh * A.KW;
                 for (int kb = 0; kb < k_blocks; kb++) {
-                    const int tap = kb / cblocks, cb = kb - tap * cblocks;
-                    const int kh = tap / A.KW, kw = tap - kh * A.KW;
                     const int dy = kh * A.dh - A.ph, dx = kw * A.dw - A.pw;
                     if (!(ok = mbar_wait(empty + stage, phase ^ 1, abort_flag, 11))) break;
                     unsigned char* sa = smem + stage * STAGE_BYTES;
-                    mbar_expect_tx(full + stage, A_BYTES + BN_T * BK * 2);
-                    // a box covers 8 x 8 OUTPUT pixels: with stride s the tensor map steps s input elements per box element
-                    tma_load_4d(sa, &map_x, full + stage, cb * BK, w0 * A.sw + dx, h0 * A.sh + dy, n0);
-                    tma_load_4d(sa + A_BYTES / 2, &map_x, full + stage, cb * BK, w1 * A.sw + dx, h1 * A.sh + dy, n1);
-                    tma_load_2d(sa + A_BYTES, &map_w, full + stage, cb * BK, tap * A.Co + tn * BN_T);
+                    if (rank == 0) mbar_expect_tx(full + stage, CTAS * A_BYTES + BN_T * BK * 2);      // both CTAs' bytes
+                    const uint32_t bar = PAIR ? leader_addr(full + stage) : smem_u32(full + stage);
+                    // a box covers 64 OUTPUT pixels: with stride s the tensor map steps s input elements per box element
+                    tma_load_tile<CTAS>(sa, &map_x, bar, cb * BK, w0 * A.sw + dx, h0 * A.sh + dy, n0);
+                    tma_load_tile<CTAS>(sa + A_BYTES / 2, &map_x, bar, cb * BK, w1 * A.sw + dx, h1 * A.sh + dy, n1);
+                    tma_load_tile<CTAS>(sa + A_BYTES, &map_w, bar, cb * BK, tap * A.Co + tn * BN_T + rank * (BN_T / CTAS));
+                    if (++cb == cblocks) {
+                        cb = 0; tap++;
+                        if (++kw == A.KW) { kw = 0; if (++kh == A.KH) { kh = 0; tap = 0; } }
+                    }
                     if (++stage == STAGES) { stage = 0; phase ^= 1; }
                 }
             }
@@ -128,18 +145,19 @@ conv_bf16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            constexpr uint32_t idesc = make_idesc(BM, BN_T);
+        if (lane == 0 && rank == 0) {
+            constexpr uint32_t idesc = make_idesc(BM * CTAS, BN_T);
             int stage = 0; uint32_t phase = 0;
             int it = 0;
             bool ok = true;
-            for (int t = blockIdx.x; t < total && ok; t += gridDim.x, it++) {
+            for (int t = first; t < total && ok; t += step, it++) {
                 const int buf = it & 1;
                 const uint32_t acc_phase = (it >> 1) & 1;
-                if (!(ok = mbar_wait(acc_empty + buf, acc_phase ^ 1, abort_flag, 12))) break;
+                if (!(ok = mbar_wait<PAIR>(acc_empty + buf, acc_phase ^ 1, abort_flag, 12))) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t tmem_d = tmem_base + buf * BN;
-                for (int kb = 0, cb = 0; kb < k_blocks; kb++) {
+                int cb = first_block(t / A.tiles_n, k_blocks) % cblocks;
+                for (int kb = 0; kb < k_blocks; kb++) {
                     if (!(ok = mbar_wait(full + stage, phase, abort_flag, 13))) break;
                     if (++cb == cblocks) cb = 0;
                     const int steps = cb == 0 ? A.last_k : BK / UMMA_K;          // no MMA on channels that do not exist
@@ -148,19 +166,19 @@ conv_bf16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                     const uint64_t da = make_smem_desc(sa), db = make_smem_desc(sa + A_BYTES);
 #pragma unroll
                     for (int k = 0; k < BK / UMMA_K; k++)
-                        if (k < steps) umma_f16(tmem_d, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
-                    umma_commit(empty + stage);
+                        if (k < steps) umma_f16<CTAS>(tmem_d, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
+                    umma_commit<CTAS>(empty + stage);
                     if (++stage == STAGES) { stage = 0; phase ^= 1; }
                 }
-                if (ok) umma_commit(acc_full + buf);
+                if (ok) umma_commit<CTAS>(acc_full + buf);
             }
         }
     } else {
-        const int quad = warp & 3;
+        const int quad = warp & 3, grp = (warp - 2) >> 2;
         int it = 0;
         bool ok = true;
         const int64_t plane = (int64_t)A.OH * A.OW;
-        for (int t = blockIdx.x; t < total && ok; t += gridDim.x, it++) {
+        for (int t = first; t < total && ok; t += step, it++) {
             const int tm = t / A.tiles_n, tn = t - tm * A.tiles_n;
             const int buf = it & 1;
             const uint32_t acc_phase = (it >> 1) & 1;
@@ -168,37 +186,29 @@ conv_bf16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            // this lane's pixel: row r of the tile = patch (r / 64), position (r % 64) = hh*8 + ww
+            // this lane's pixel: row r of the tile = patch (r / 64), position (r % 64) in row order
             const int r = quad * 32 + lane;
-            const int64_t q = 2 * (int64_t)tm + (r >> 6);
+            const int64_t q = 2 * ((int64_t)tm * CTAS + rank) + (r >> 6);
             int n, h0, w0;
             patch_coords(A, q, n, h0, w0);
-            const int oh = h0 + ((r & 63) >> 3), ow = w0 + (r & 7);
+            const int pw = 1 << A.pw_log;
+            const int oh = h0 + ((r & 63) >> A.pw_log), ow = w0 + (r & (pw - 1));
             const bool valid = q < A.patches && oh < A.OH && ow < A.OW;
-            __nv_bfloat16* yp = y + ((int64_t)n * A.Co) * plane + (int64_t)oh * A.OW + ow;
+            // the 8 pixels this lane stores: the (lane % 4)th of the warp's four runs, channels lane / 4 + 8 i of a chunk
+            const int run = (quad & 1) * 32 + (lane & 3) * 8, sow = w0 + (run & (pw - 1));
+            const int soh = h0 + (run >> A.pw_log), snw = A.OW - sow;
+            const bool svalid = q < A.patches && soh < A.OH && snw > 0;
+            __nv_bfloat16* yp = y + ((int64_t)n * A.Co + (lane >> 2)) * plane + (int64_t)soh * A.OW + sow;
+            __nv_bfloat16* square = reinterpret_cast<__nv_bfloat16*>(stage_out) + (warp - 2) * 1024;
             const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + buf * BN;
-            const bool issuer = threadIdx.x == 64;          // first epilogue thread drives the TMA stores
 #pragma unroll 1
-            for (int ch = 0; ch < BN_T / 32; ch++) {
+            for (int ch = grp; ch < BN_T / 32; ch += 2) {
                 const int co0 = tn * BN_T + ch * 32;
-                if (TMA_OUT && (ch & 1) == 0) {
-                    // staging buffer free again? (the previous round's stores must have read it)
-                    if (issuer) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-                    asm volatile("bar.sync 1, 128;" ::: "memory");
-                }
                 uint32_t v[32];
                 tmem_ld32(taddr + ch * 32, v);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                 float f[32];
-                if (TMA_OUT) {
-                    __nv_bfloat16* sp = reinterpret_cast<__nv_bfloat16*>(stage_out) + (r >> 6) * (64 * 64) + (ch & 1) * (32 * 64) + (r & 63);
-#pragma unroll
-                    for (int e = 0; e < 32; e++) {
-                        const __nv_bfloat16 b = __float2bfloat16(__uint_as_float(v[e]));
-                        sp[e * 64] = b;
-                        f[e] = (valid && co0 + e < A.Co) ? __bfloat162float(b) : 0.f;
-                    }
-                } else if (OUT == 2) {
+                if (NHWC) {
                     // NHWC: this lane's pixel, channels co0 .. co0 + 31 are contiguous
                     __align__(16) __nv_bfloat16 row[32];
 #pragma unroll
@@ -217,12 +227,35 @@ conv_bf16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                         }
                     }
                 } else {
+                    __syncwarp();
 #pragma unroll
                     for (int e = 0; e < 32; e++) {
                         const __nv_bfloat16 b = __float2bfloat16(__uint_as_float(v[e]));
-                        const bool st = valid && co0 + e < A.Co;
-                        if (st) yp[(int64_t)(co0 + e) * plane] = b;
-                        f[e] = st ? __bfloat162float(b) : 0.f;      // statistics of the value as stored
+                        square[e * 32 + lane] = b;
+                        f[e] = (valid && co0 + e < A.Co) ? __bfloat162float(b) : 0.f;      // statistics of the value as stored
+                    }
+                    __syncwarp();
+#pragma unroll
+                    for (int i = 0; i < 4; i++) {
+                        if (svalid && co0 + i * 8 + (lane >> 2) < A.Co) {
+                            const uint4 px = reinterpret_cast<const uint4*>(square)[i * 32 + lane];
+                            __nv_bfloat16* d = yp + (int64_t)(co0 + i * 8) * plane;
+                            if (A.vec == 8) *reinterpret_cast<uint4*>(d) = px;
+                            else if (A.vec == 4) {
+                                *reinterpret_cast<uint2*>(d) = make_uint2(px.x, px.y);
+                                if (snw > 4) *reinterpret_cast<uint2*>(d + 4) = make_uint2(px.z, px.w);
+                            } else {
+                                const uint32_t two[4] = {px.x, px.y, px.z, px.w};
+#pragma unroll
+                                for (int e = 0; e < 4; e++) {
+                                    if (A.vec == 2) { if (2 * e < snw) *reinterpret_cast<uint32_t*>(d + 2 * e) = two[e]; }
+                                    else {
+                                        if (2 * e < snw) reinterpret_cast<uint16_t*>(d)[2 * e] = (uint16_t)two[e];
+                                        if (2 * e + 1 < snw) reinterpret_cast<uint16_t*>(d)[2 * e + 1] = (uint16_t)(two[e] >> 16);
+                                    }
+                                }
+                            }
+                        }
                     }
                 }
                 if (stats) {
@@ -246,34 +279,15 @@ conv_bf16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                         atomicAdd(sstat + STATS_MAX_CO + co0 + lane, g[0]);
                     }
                 }
-                if (TMA_OUT && (ch & 1) == 1) {
-                    // 64 channels staged: make the writes visible to the async proxy, then two box stores
-                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                    asm volatile("bar.sync 1, 128;" ::: "memory");
-                    if (issuer) {
-                        const int cbase = tn * BN_T + (ch - 1) * 32;
-#pragma unroll
-                        for (int pp = 0; pp < 2; pp++) {
-                            const int64_t qq = 2 * (int64_t)tm + pp;
-                            if (qq < A.patches && cbase < A.Co) {
-                                int nn, hh0, ww0;
-                                patch_coords(A, qq, nn, hh0, ww0);
-                                asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%2, %3, %4, %5}], [%1];"
-                                             ::"l"(&map_y), "r"(smem_u32(stage_out + pp * (64 * 64 * 2))), "r"(ww0), "r"(hh0), "r"(cbase), "r"(nn) : "memory");
-                            }
-                        }
-                        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-                    }
-                }
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
-            if (lane == 0) mbar_arrive(acc_empty + buf);
+            if (lane == 0) { if (PAIR) mbar_arrive_leader(acc_empty + buf); else mbar_arrive(acc_empty + buf); }
         }
-        if (TMA_OUT && threadIdx.x == 64) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if (PAIR) cluster_sync();          // neither CTA leaves while the other may still signal it or read its tiles
     if (stats) {
         for (int i = threadIdx.x; i < A.Co; i += blockDim.x) {
             atomicAdd(stats + i, sstat[i]);
@@ -282,7 +296,7 @@ conv_bf16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     }
     if (warp == 1) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem_base) : "memory");
+        tmem_dealloc<CTAS>(tmem_base);
     }
 }
 
@@ -340,15 +354,15 @@ transpose_bf16_batched_kernel(const __nv_bfloat16* __restrict__ in, __nv_bfloat1
     }
 }
 
-static bool make_map_x(CUtensorMap* map, const void* base, const ConvShape& s) {
+static bool make_map_x(CUtensorMap* map, const void* base, const ConvShape& s, int pw_log) {
     auto fn = encode_fn();
     if (!fn) return false;
     cuuint64_t dims[4] = {(cuuint64_t)s.C, (cuuint64_t)s.W, (cuuint64_t)s.H, (cuuint64_t)s.N};
     const cuuint64_t cp = (cuuint64_t)pitch8(s.C) * 2;
     cuuint64_t strides[3] = {cp, s.W * cp, s.H * s.W * cp};
-    // strided convolution: the traversal stride of the map skips input pixels, so that a box still delivers 8 x 8 window
-    // origins; the box extent counts tensor elements, i.e. 8 * stride per axis (at most 8 * 8 = 64 <= 256)
-    cuuint32_t box[4] = {(cuuint32_t)BK, (cuuint32_t)(PATCH * s.sw), (cuuint32_t)(PATCH * s.sh), 1};
+    // strided convolution: the traversal stride of the map skips input pixels, so that a box still delivers 64 window
+    // origins; the box extent counts tensor elements, i.e. pixels * stride per axis (at most 64 * 4 = 256)
+    cuuint32_t box[4] = {(cuuint32_t)BK, (cuuint32_t)(s.sw << pw_log), (cuuint32_t)(s.sh * (64 >> pw_log)), 1};
     cuuint32_t estr[4] = {1, (cuuint32_t)s.sw, (cuuint32_t)s.sh, 1};
     return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, estr,
               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -366,16 +380,33 @@ static bool make_map_w(CUtensorMap* map, const void* base, const ConvShape& s, i
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-static bool make_map_y(CUtensorMap* map, const void* base, const ConvShape& s) {
-    auto fn = encode_fn();
-    if (!fn) return false;
-    cuuint64_t dims[4] = {(cuuint64_t)s.OW, (cuuint64_t)s.OH, (cuuint64_t)s.Co, (cuuint64_t)s.N};
-    cuuint64_t strides[3] = {(cuuint64_t)s.OW * 2, (cuuint64_t)s.OH * s.OW * 2, (cuuint64_t)s.Co * s.OH * s.OW * 2};
-    cuuint32_t box[4] = {PATCH, PATCH, 64, 1};
-    cuuint32_t estr[4] = {1, 1, 1, 1};
-    return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, estr,
-              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
-              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+template <bool NHWC>
+static const void* kernel_of(int bn, bool pair) {
+    return pair ? (bn == 256 ? (const void*)conv_bf16_kernel<NHWC, 256, true> : bn == 128 ? (const void*)conv_bf16_kernel<NHWC, 128, true>
+                                                                                       : (const void*)conv_bf16_kernel<NHWC, 64, true>)
+                : (bn == 256 ? (const void*)conv_bf16_kernel<NHWC, 256, false> : bn == 128 ? (const void*)conv_bf16_kernel<NHWC, 128, false>
+                                                                                        : (const void*)conv_bf16_kernel<NHWC, 64, false>);
+}
+static const void* kernel_of(bool nhwc, int bn, bool pair) { return nhwc ? kernel_of<true>(bn, pair) : kernel_of<false>(bn, pair); }
+
+// How many CTA pairs run at once (a persistent grid must not exceed it); 0 on error.
+static int pair_slots() {
+    static std::once_flag once;
+    static int slots = 0;
+    std::call_once(once, [] {
+        for (int out = 0; out < 2; out++)
+            for (int bn = 64; bn <= 256; bn *= 2)
+                for (int pair = 0; pair < 2; pair++)
+                    if (cudaFuncSetAttribute(kernel_of(out, bn, pair), cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) != cudaSuccess) return;
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension; at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+        cfg.gridDim = dim3(kNumSMs); cfg.blockDim = dim3(THREADS); cfg.dynamicSmemBytes = SMEM_BYTES; cfg.attrs = at; cfg.numAttrs = 1;
+        int n = 0;
+        if (cudaOccupancyMaxActiveClusters(&n, kernel_of(0, 256, true), &cfg) != cudaSuccess || n < 1) return;
+        slots = std::min(n, kNumSMs / 2);
+    });
+    return slots;
 }
 
 }  // namespace tcconv
@@ -408,9 +439,13 @@ size_t conv2d_tc_workspace(const ConvShape& s) {
     return xb + wb + 1024;
 }
 
-int conv2d_tc(const void* x, const void* w, void* y, float* stats, const ConvShape& s, void* workspace, cudaStream_t st,
+int conv2d_tc(const void* x, const void* w, void* y, float* stats, const ConvShape& shape, void* workspace, cudaStream_t st,
               const ConvLayout& lay) {
     using namespace tcconv;
+    ConvShape s = shape;
+    if (s.KH == 1 && s.KW == 1 && s.sh == 1 && s.sw == 1 && s.ph == 0 && s.pw == 0) {     // pixels are all alike: one row of them
+        s.W *= s.H; s.OW = s.W; s.H = s.OH = 1;
+    }
     unsigned char* ws = (unsigned char*)(((uintptr_t)workspace + 1023) & ~(uintptr_t)1023);
     // NHWC ("acdb") activations are what the kernel reads: no staging pass for x then
     __nv_bfloat16* xt = lay.x_nhwc ? (__nv_bfloat16*)const_cast<void*>(x) : (__nv_bfloat16*)ws;
@@ -431,44 +466,52 @@ int conv2d_tc(const void* x, const void* w, void* y, float* stats, const ConvSha
     ConvArgs A;
     A.N = s.N; A.C = s.C; A.H = s.H; A.W = s.W; A.Co = s.Co; A.KH = s.KH; A.KW = s.KW; A.OH = s.OH; A.OW = s.OW;
     A.sh = s.sh; A.sw = s.sw; A.ph = s.ph; A.pw = s.pw; A.dh = s.dh; A.dw = s.dw;
-    A.tiles_h = (s.OH + PATCH - 1) / PATCH; A.tiles_w = (s.OW + PATCH - 1) / PATCH;
-    A.patches = (int64_t)s.N * A.tiles_h * A.tiles_w;
-    A.tiles_m = (int)((A.patches + 1) / 2);
+    // Patch shape: the one that covers an image with the fewest patches, of equals the one with the longest rows (up to 32
+    // pixels: y is then written in whole sectors). 28 x 28: 14 patches of 4 x 16 instead of 16 of 8 x 8.
+    A.patches = INT64_MAX;
+    for (int l = 6; l >= 3; l--) {
+        const int th = (s.OH + (64 >> l) - 1) / (64 >> l), tw = (s.OW + (1 << l) - 1) >> l;
+        if ((int64_t)s.N * th * tw < A.patches || (l == 5 && (int64_t)s.N * th * tw == A.patches)) { A.patches = (int64_t)s.N * th * tw; A.tiles_h = th; A.tiles_w = tw; A.pw_log = l; }
+    }
     A.last_k = (s.C - (s.C + BK - 1) / BK * BK + BK + UMMA_K - 1) / UMMA_K;
-    // Tile width: the grid is persistent with a static round-robin, so its time is ceil(tiles / SMs) rounds. 128-wide
-    // tiles do a little worse per FLOP (more operand bytes per MMA) but halve the granularity of the last round.
-    auto rounds = [&](int bn) { const int64_t t = (int64_t)A.tiles_m * ((s.Co + bn - 1) / bn); return (double)((t + kNumSMs - 1) / kNumSMs) * bn; };
+    // Tile by estimated time: the grid is persistent with a static round-robin, so it takes ceil(tiles / slots) rounds, each of a
+    // tile's main loop and the part of its epilogue that the next tile's main loop does not hide (about half). A k-block of 64 channels
+    // measured 342, 354, 477 ns with 64, 128, 256 output channels and 347, 380, 445 ns on a pair: most of it is the feed of the
+    // x boxes (their 128 rows of 128 bytes), so narrow tiles feed the MMAs worse but leave less of the last round idle.
+    const int slots = pair_slots();
     const char* bn_env = getenv("B200JT_CONV_BN");          // read on every call: tests force each variant in turn
+    const char* pair_env = getenv("B200JT_CONV_PAIR");
     const int forced_bn = bn_env ? atoi(bn_env) : 0;
-    const double cost[3] = {rounds(256), rounds(128) * kNarrowTilePenalty, rounds(64) * kThinTilePenalty};
-    const int bn = forced_bn == 64 || forced_bn == 128 || forced_bn == 256 ? forced_bn
-                 : cost[2] < cost[1] && cost[2] < cost[0] ? 64 : cost[1] < cost[0] ? 128 : 256;
+    const int k_blocks = s.KH * s.KW * ((s.C + BK - 1) / BK);
+    bool pair = false; int bn = 256; double best = 1e30;
+    for (int p = 0; p < 2; p++) {
+        if ((pair_env && atoi(pair_env) != p) || (p && !slots)) continue;
+        for (int b = 64; b <= 256; b *= 2) {
+            if ((forced_bn == 64 || forced_bn == 128 || forced_bn == 256) && forced_bn != b) continue;
+            const int64_t t = (A.patches + 2 * p + 1) / (2 * p + 2) * ((s.Co + b - 1) / b);
+            const double block = 300 + (p ? 0.57 : 0.69) * b;
+            const double epilogue = 600 + b * (stats ? 23.0 : 12.5);
+            const int n = p ? slots : kNumSMs;
+            const double ns = (double)((t + n - 1) / n) * (k_blocks * block + 0.5 * epilogue + 250 * p) + epilogue;
+            if (ns < best) { best = ns; pair = p; bn = b; }
+        }
+    }
+    const int ctas = pair ? 2 : 1;
+    A.tiles_m = (int)((A.patches + 2 * ctas - 1) / (2 * ctas));
     A.tiles_n = (s.Co + bn - 1) / bn;
     CUtensorMap mx, mw;
-    if (!make_map_x(&mx, xt, s) || !make_map_w(&mw, wt, s, bn)) return fail(-4, "conv2d: cuTensorMapEncodeTiled failed");
-    static std::once_flag once;
-    static cudaError_t attr_err = cudaSuccess;
-    std::call_once(once, [] {
-        const void* kernels[] = {(const void*)conv_bf16_kernel<1, 256>, (const void*)conv_bf16_kernel<0, 256>,
-                                 (const void*)conv_bf16_kernel<1, 128>, (const void*)conv_bf16_kernel<0, 128>,
-                                 (const void*)conv_bf16_kernel<2, 256>, (const void*)conv_bf16_kernel<2, 128>,
-                                 (const void*)conv_bf16_kernel<1, 64>, (const void*)conv_bf16_kernel<0, 64>, (const void*)conv_bf16_kernel<2, 64>};
-        for (const void* k : kernels)
-            if (attr_err == cudaSuccess) attr_err = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-    });
-    B200JT_CUDA(attr_err);
-    // TMA stores need a 16-byte aligned base and row pitch
-    const bool tma_out = !lay.y_nhwc && (s.OW % 8 == 0) && ((uintptr_t)y % 16 == 0);
-    CUtensorMap my = mx;
-    if (tma_out && !make_map_y(&my, y, s)) return fail(-4, "conv2d: cuTensorMapEncodeTiled failed (y)");
+    if (!make_map_x(&mx, xt, s, A.pw_log) || !make_map_w(&mw, wt, s, bn / ctas)) return fail(-4, "conv2d: cuTensorMapEncodeTiled failed");
+    if (!slots) return fail(-4, "conv2d: no room for the kernel's shared memory");
+    A.vec = 8;
+    while (A.vec > 1 && (s.OW % A.vec || (uintptr_t)y % (2 * A.vec))) A.vec /= 2;
     float* fused = (stats && s.Co <= STATS_MAX_CO) ? stats : nullptr;
-    const int total = A.tiles_m * A.tiles_n;
-    const int grid = total < kNumSMs ? total : kNumSMs;
-    auto kern = bn == 256 ? (lay.y_nhwc ? conv_bf16_kernel<2, 256> : tma_out ? conv_bf16_kernel<1, 256> : conv_bf16_kernel<0, 256>)
-              : bn == 64  ? (lay.y_nhwc ? conv_bf16_kernel<2, 64> : tma_out ? conv_bf16_kernel<1, 64> : conv_bf16_kernel<0, 64>)
-                          : (lay.y_nhwc ? conv_bf16_kernel<2, 128> : tma_out ? conv_bf16_kernel<1, 128> : conv_bf16_kernel<0, 128>);
-    kern<<<grid, THREADS, SMEM_BYTES, st>>>(mx, mw, my, (__nv_bfloat16*)y, fused, A);
-    B200JT_LAUNCH_CHECK();
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension; at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3((unsigned)(std::min(A.tiles_m * A.tiles_n, pair ? slots : kNumSMs) * ctas));
+    cfg.blockDim = dim3(THREADS); cfg.dynamicSmemBytes = SMEM_BYTES; cfg.stream = st; cfg.attrs = at; cfg.numAttrs = pair ? 1 : 0;
+    void* args[] = {&mx, &mw, &y, &fused, &A};
+    B200JT_CUDA(cudaLaunchKernelExC(&cfg, kernel_of(lay.y_nhwc, bn, pair), args));
     return fused ? 1 : 0;      // 1: statistics were produced by the epilogue
 }
 

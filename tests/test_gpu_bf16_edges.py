@@ -16,13 +16,14 @@ def near(got, want):
 
 
 # channels below and across the 64-channel blocks, not multiples of 8; outputs smaller than a patch; 1 x 1 to 7 x 7 filters
-@pytest.mark.parametrize("bn", [None, 64])
+@pytest.mark.parametrize("bn,pair", [(None, None), (64, 0), (64, 1), (128, 1), (256, 1)])
 @pytest.mark.parametrize("n,ci,h,w,co,k,s,p,d", [
     (3, 8, 7, 7, 27, 3, 1, 1, 1), (2, 17, 9, 14, 16, 3, 1, 1, 1), (1, 63, 28, 28, 65, 1, 1, 0, 1), (2, 65, 16, 24, 130, 3, 2, 1, 1),
     (5, 33, 4, 5, 1, 2, 1, 1, 1), (2, 16, 56, 56, 112, 1, 2, 0, 1), (9, 129, 13, 8, 71, 5, 3, 2, 1), (1, 11, 40, 40, 300, 7, 4, 3, 2)])
-def test_convolution_and_weight_gradient(n, ci, h, w, co, k, s, p, d, bn, monkeypatch):
+def test_convolution_and_weight_gradient(n, ci, h, w, co, k, s, p, d, bn, pair, monkeypatch):
     if bn:
         monkeypatch.setenv("B200JT_CONV_BN", str(bn))
+        monkeypatch.setenv("B200JT_CONV_PAIR", str(pair))
     x = torch.randn(n, ci, h, w, device="cuda").bfloat16()
     wt = (torch.randn(co, ci, k, k, device="cuda") * 0.1).bfloat16()
     wd = wt.double().requires_grad_()

@@ -67,4 +67,4 @@ def test_batch_norm(n, c, h, w, relu, dtype, amp):
             if dtype == torch.float32:
                 near(a.torch(), b.torch(), 1e-4)
             else:
-                near(a.torch(), b.torch(), 4e-3 if amp == 0 else 1e-5)
+                near(a.torch(), b.torch(), 4e-3 if amp == 0 else 1e-3)    # amp 2 rounds as the graph does: at most a flip here and there
