@@ -380,6 +380,24 @@ static bool make_map_w(CUtensorMap* map, const void* base, const ConvShape& s, i
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// Pixels of a 1 x 1 layer are all alike: one row of them.
+static ConvShape flattened(ConvShape s) {
+    if (s.KH == 1 && s.KW == 1 && s.sh == 1 && s.sw == 1 && s.ph == 0 && s.pw == 0) { s.W *= s.H; s.OW = s.W; s.H = s.OH = 1; }
+    return s;
+}
+// Patch shape: the one that covers an image with the fewest patches, of equals the one with the longest rows (up to 32 pixels: y
+// is then written in whole sectors). 28 x 28: 14 patches of 4 x 16 instead of 16 of 8 x 8.
+struct Patches { int64_t count; int tiles_h, tiles_w, pw_log; };
+static Patches patches_of(const ConvShape& s) {
+    Patches best{INT64_MAX, 0, 0, 0};
+    for (int l = 6; l >= 3; l--) {
+        const int th = (s.OH + (64 >> l) - 1) / (64 >> l), tw = (s.OW + (1 << l) - 1) >> l;
+        const int64_t n = (int64_t)s.N * th * tw;
+        if (n < best.count || (l == 5 && n == best.count)) best = {n, th, tw, l};
+    }
+    return best;
+}
+
 template <bool NHWC>
 static const void* kernel_of(int bn, bool pair) {
     return pair ? (bn == 256 ? (const void*)conv_bf16_kernel<NHWC, 256, true> : bn == 128 ? (const void*)conv_bf16_kernel<NHWC, 128, true>
@@ -442,10 +460,7 @@ size_t conv2d_tc_workspace(const ConvShape& s) {
 int conv2d_tc(const void* x, const void* w, void* y, float* stats, const ConvShape& shape, void* workspace, cudaStream_t st,
               const ConvLayout& lay) {
     using namespace tcconv;
-    ConvShape s = shape;
-    if (s.KH == 1 && s.KW == 1 && s.sh == 1 && s.sw == 1 && s.ph == 0 && s.pw == 0) {     // pixels are all alike: one row of them
-        s.W *= s.H; s.OW = s.W; s.H = s.OH = 1;
-    }
+    const ConvShape s = flattened(shape);
     unsigned char* ws = (unsigned char*)(((uintptr_t)workspace + 1023) & ~(uintptr_t)1023);
     // NHWC ("acdb") activations are what the kernel reads: no staging pass for x then
     __nv_bfloat16* xt = lay.x_nhwc ? (__nv_bfloat16*)const_cast<void*>(x) : (__nv_bfloat16*)ws;
@@ -466,13 +481,8 @@ int conv2d_tc(const void* x, const void* w, void* y, float* stats, const ConvSha
     ConvArgs A;
     A.N = s.N; A.C = s.C; A.H = s.H; A.W = s.W; A.Co = s.Co; A.KH = s.KH; A.KW = s.KW; A.OH = s.OH; A.OW = s.OW;
     A.sh = s.sh; A.sw = s.sw; A.ph = s.ph; A.pw = s.pw; A.dh = s.dh; A.dw = s.dw;
-    // Patch shape: the one that covers an image with the fewest patches, of equals the one with the longest rows (up to 32
-    // pixels: y is then written in whole sectors). 28 x 28: 14 patches of 4 x 16 instead of 16 of 8 x 8.
-    A.patches = INT64_MAX;
-    for (int l = 6; l >= 3; l--) {
-        const int th = (s.OH + (64 >> l) - 1) / (64 >> l), tw = (s.OW + (1 << l) - 1) >> l;
-        if ((int64_t)s.N * th * tw < A.patches || (l == 5 && (int64_t)s.N * th * tw == A.patches)) { A.patches = (int64_t)s.N * th * tw; A.tiles_h = th; A.tiles_w = tw; A.pw_log = l; }
-    }
+    const Patches pt = patches_of(s);
+    A.patches = pt.count; A.tiles_h = pt.tiles_h; A.tiles_w = pt.tiles_w; A.pw_log = pt.pw_log;
     A.last_k = (s.C - (s.C + BK - 1) / BK * BK + BK + UMMA_K - 1) / UMMA_K;
     // Tile by estimated time: the grid is persistent with a static round-robin, so it takes ceil(tiles / slots) rounds, each of a
     // tile's main loop and the part of its epilogue that the next tile's main loop does not hide (about half). A k-block of 64 channels
@@ -520,7 +530,7 @@ int conv2d_tc(const void* x, const void* w, void* y, float* stats, const ConvSha
 // over (batch, rows, columns) of reindex(x) * broadcast(dy) that ConvTuner relays to cudnnConvolutionBackwardFilter
 // (python/jittor/extern/cuda/cudnn/ops/cudnn_conv_backward_w_op.cc:292). As a GEMM per filter tap:
 //   D[c, o] = sum over pixels of X_tap[pixel, c] * DY[pixel, o],     M = Cin (128 per CTA), N = Cout (256), K = N*OH*OW.
-// x and dy are first copied to NHWC, so a 4-D TMA box of 8 x 8 output pixels x 64 channels lands as 64 rows of 128 B with
+// x and dy are first copied to NHWC, so a 4-D TMA box of 64 output pixels x 64 channels lands as 64 rows of 128 B with
 // the channel axis contiguous: both operands are MN-major (their own axis contiguous, K = pixel strided), and the same box
 // geometry as the forward kernel carries the tap's shift and the stride in its coordinates. One CTA owns one
 // (tap, 128 input channels, 256 output channels) accumulator in TMEM and walks a contiguous range of pixel patches; the
@@ -530,7 +540,7 @@ namespace tcwgrad {
 
 using namespace tc;
 
-constexpr int BM = 128, PIX = 64, PATCH = 8, THREADS = 192;
+constexpr int BM = 128, PIX = 64, THREADS = 192;
 constexpr int CHUNK_BYTES = PIX * 64 * 2;                    // one box: 64 pixels x 64 channels of bf16
 // TAPS filter taps per CTA share the dy tile of a stage (their x tiles differ by the tap's shift): with two taps a stage is
 // 2 * 16 KB of x + 32 KB of dy for twice the MMAs, i.e. two thirds of the operand bytes per FLOP -- the feed from L2 into
@@ -543,7 +553,7 @@ template <int TAPS> struct Ring {
 
 struct WgradArgs {
     int N, C, H, W, Co, KH, KW, OH, OW, sh, sw, ph, pw, dh, dw;
-    int tiles_h, tiles_w;            // patches per image
+    int tiles_h, tiles_w, pw_log;    // patches per image, their shape
     int64_t patches;                 // N * tiles_h * tiles_w: the K axis in units of 64 pixels
     int tiles_m, tiles_n, splits, groups;      // groups: ceil(taps / TAPS) tap groups
 };
@@ -619,7 +629,7 @@ wgrad_bf16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
             // pixels past the edge of x (padding, ragged patches) and channels past C / Co are zero-filled by TMA
             if (owns)
                 tma_load_4d(smem + stage * MAX_STAGE_BYTES + lane * CHUNK_BYTES, map, full + stage, c0,
-                            tw * PATCH * sw + ox, th * PATCH * sh + oy, n);
+                            (tw << A.pw_log) * sw + ox, th * (64 >> A.pw_log) * sh + oy, n);
             if (++tw == A.tiles_w) { tw = 0; if (++th == A.tiles_h) { th = 0; n++; } }
             if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
@@ -704,15 +714,15 @@ wgrad_fold_kernel(const float* __restrict__ part, __nv_bfloat16* __restrict__ dw
     }
 }
 
-// NHWC tensor [N][H][W][C] as a 4-D map whose box is 64 channels x (8 * sw) x (8 * sh) x 1 with traversal strides
+// NHWC tensor [N][H][W][C] as a 4-D map whose box is 64 channels x a patch (times the strides) x 1 with traversal strides
 // (1, sw, sh, 1): 64 pixels x 128 B in shared memory.
-static bool make_map_nhwc(CUtensorMap* map, const void* base, int N, int H, int W, int C, int sh, int sw) {
+static bool make_map_nhwc(CUtensorMap* map, const void* base, int N, int H, int W, int C, int sh, int sw, int pw_log) {
     auto fn = encode_fn();
     if (!fn) return false;
     cuuint64_t dims[4] = {(cuuint64_t)C, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)N};
     const cuuint64_t cp = (cuuint64_t)tcconv::pitch8(C) * 2;
     cuuint64_t strides[3] = {cp, W * cp, (cuuint64_t)H * W * cp};
-    cuuint32_t box[4] = {64, (cuuint32_t)(PATCH * sw), (cuuint32_t)(PATCH * sh), 1};
+    cuuint32_t box[4] = {64, (cuuint32_t)(sw << pw_log), (cuuint32_t)(sh * (64 >> pw_log)), 1};
     cuuint32_t estr[4] = {1, (cuuint32_t)sw, (cuuint32_t)sh, 1};
     return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, estr,
               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -730,7 +740,7 @@ static Plan plan_for(const ConvShape& s) {
     p.groups = (taps + p.taps_per_cta - 1) / p.taps_per_cta;
     p.tiles_m = (s.C + BM - 1) / BM;
     p.tiles_n = (s.Co + p.bn - 1) / p.bn;
-    p.patches = (int64_t)s.N * ((s.OH + PATCH - 1) / PATCH) * ((s.OW + PATCH - 1) / PATCH);
+    p.patches = tcconv::patches_of(s).count;
     // fill the GPU once when the accumulators alone do not; every split keeps at least 8 patches (512 pixels) of K
     auto splits_for = [&](int64_t groups) {
         const int64_t base = groups * p.tiles_m * p.tiles_n;
@@ -757,14 +767,16 @@ bool conv2d_wgrad_tc_supported(const ConvShape& s, const void* x, const void* dy
 }
 
 size_t conv2d_wgrad_tc_workspace(const ConvShape& s) {
-    const tcwgrad::Plan p = tcwgrad::plan_for(s);
+    const tcwgrad::Plan p = tcwgrad::plan_for(tcconv::flattened(s));
     return p.xb + p.dyb + p.pb + 1024;
 }
 
-int conv2d_wgrad_tc(const void* x, const void* dy, void* dw, const ConvShape& s, void* workspace, cudaStream_t st,
+int conv2d_wgrad_tc(const void* x, const void* dy, void* dw, const ConvShape& shape, void* workspace, cudaStream_t st,
                     const ConvLayout& lay) {
     using namespace tcwgrad;
+    const ConvShape s = tcconv::flattened(shape);
     const Plan p = plan_for(s);
+    const tcconv::Patches pt = tcconv::patches_of(s);
     unsigned char* ws = (unsigned char*)(((uintptr_t)workspace + 1023) & ~(uintptr_t)1023);
     // channels-last ("acdb") x / dy are what the kernel reads: no copy on that side (lay.y_nhwc describes dy)
     __nv_bfloat16* xt = lay.x_nhwc ? (__nv_bfloat16*)const_cast<void*>(x) : (__nv_bfloat16*)ws;
@@ -784,10 +796,10 @@ int conv2d_wgrad_tc(const void* x, const void* dy, void* dw, const ConvShape& s,
     WgradArgs A;
     A.N = s.N; A.C = s.C; A.H = s.H; A.W = s.W; A.Co = s.Co; A.KH = s.KH; A.KW = s.KW; A.OH = s.OH; A.OW = s.OW;
     A.sh = s.sh; A.sw = s.sw; A.ph = s.ph; A.pw = s.pw; A.dh = s.dh; A.dw = s.dw;
-    A.tiles_h = (s.OH + PATCH - 1) / PATCH; A.tiles_w = (s.OW + PATCH - 1) / PATCH;
+    A.tiles_h = pt.tiles_h; A.tiles_w = pt.tiles_w; A.pw_log = pt.pw_log;
     A.patches = p.patches; A.tiles_m = p.tiles_m; A.tiles_n = p.tiles_n; A.splits = p.splits; A.groups = p.groups;
     CUtensorMap mx, mdy;
-    if (!make_map_nhwc(&mx, xt, s.N, s.H, s.W, s.C, s.sh, s.sw) || !make_map_nhwc(&mdy, dyt, s.N, s.OH, s.OW, s.Co, 1, 1))
+    if (!make_map_nhwc(&mx, xt, s.N, s.H, s.W, s.C, s.sh, s.sw, pt.pw_log) || !make_map_nhwc(&mdy, dyt, s.N, s.OH, s.OW, s.Co, 1, 1, pt.pw_log))
         return fail(-4, "conv2d_backward_w: cuTensorMapEncodeTiled failed");
     static std::once_flag once;
     static cudaError_t attr_err = cudaSuccess;

@@ -113,6 +113,29 @@ reduce_row_kernel(const void* __restrict__ x, int xdt, void* __restrict__ out, i
         C acc = reduce_init<C>(op, ydt);
         // [r0, r1) in units of the flattened reduced space; split into sweeps over the innermost axis
         int64_t r = r0;
+        if (A.nr == 2 && inner < 4 * (int64_t)blockDim.x) {
+            // Short runs of contiguous elements (a mean over batch, rows and columns of small images): a sweep per run would
+            // leave most threads idle and wait for memory run by run, so the threads stride the flattened space instead, eight
+            // loads in flight. 202 runs of 49 for each of 150 outputs: 244 us by sweeps, REDAFTER us.
+            const uint32_t in = (uint32_t)inner, dq = blockDim.x / in, dr = blockDim.x - dq * in;
+            const int64_t ostride = A.rstride[0];
+            r += threadIdx.x;
+            int64_t q = r / in;
+            uint32_t i = (uint32_t)(r - q * in);
+            auto advance = [&] { q += dq; i += dr; if (i >= in) { i -= in; q++; } r += blockDim.x; };
+            while (r < r1) {
+                C v[8];
+#pragma unroll
+                for (int u = 0; u < 8; u++) {
+                    v[u] = op == OP_MEAN ? (C)0 : reduce_init<C>(op, ydt);
+                    if (r < r1) v[u] = load_x<TX, C>(x, xdt, base + q * ostride + i * istride);
+                    advance();
+                }
+#pragma unroll
+                for (int u = 0; u < 8; u++) acc = reduce_combine<C>(op, acc, op == OP_MEAN ? v[u] * rcount : v[u]);
+            }
+            r = r1;
+        }
         while (r < r1) {
             const int64_t outer = r / inner, i0 = r - outer * inner;
             const int64_t i1 = (r1 - r) < (inner - i0) ? i0 + (r1 - r) : inner;

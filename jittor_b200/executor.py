@@ -438,6 +438,14 @@ def conv_dgrad_plan(v, dy, w, geo):
         from . import var as V
         wf = V.reindex(w, [Ci, Co, KH, KW], ["i1", "i0", f"{KH - 1}-i2", f"{KW - 1}-i3"])
         return Plan([dy, wf], lambda: run_conv2d(dy, wf, (1, 1, fp, fq, dh, dw), v.dtype))
+    if fp >= 0 and fq >= 0 and dy.dtype == "bfloat16" and Co >= 8 and max(sh, sw) <= 4:
+        # Strided: the same convolution over dy with sh - 1, sw - 1 zeros between its pixels. It multiplies sh * sw times as much,
+        # on the tensor cores: 136 x 208 x 4 x 4 -> 32 x 7 x 7 (3 x 3) took 280 us as a gather on the CUDA cores.
+        from . import var as V
+        H, W = v.shape[2] - 2 * fp + dh * (KH - 1), v.shape[3] - 2 * fq + dw * (KW - 1)
+        spread = V.reindex(dy, [dy.shape[0], Co, H, W], ["i0", "i1", f"i2/{sh}", f"i3/{sw}"], 0, [f"i2%{sh}||i3%{sw}"])
+        wf = V.reindex(w, [Ci, Co, KH, KW], ["i1", "i0", f"{KH - 1}-i2", f"{KW - 1}-i3"])
+        return Plan([spread, wf], lambda: run_conv2d(spread, wf, (1, 1, fp, fq, dh, dw), v.dtype))
     return Plan([dy, w], lambda: run_conv2d_transpose(dy, w, geo, 1, list(v.shape), v.dtype))
 
 
