@@ -290,6 +290,10 @@ int b200jt_conv2d_formats(const b200jt_tensor* x, const b200jt_tensor* w, const 
 int b200jt_conv2d_transpose(const b200jt_tensor* x, const b200jt_tensor* w, const b200jt_tensor* y,
                             int stride_h, int stride_w, int pad_h, int pad_w, int dil_h, int dil_w, int groups, void* stream);
 
+/* y[n,c,h,w] = x[n,c,h/sh,w/sw] where sh divides h and sw divides w (and the quotients are inside x), zero elsewhere; bfloat16.
+ * The convolution that gives a strided convolution's input gradient reads dy in this form. */
+int b200jt_spread2d(const b200jt_tensor* x, const b200jt_tensor* y, int stride_h, int stride_w, void* stream);
+
 /* dw[o,c,kh,kw] = sum over (n,oh,ow) of dy[n,o,oh,ow] * x[n,c,oh*stride-pad+kh*dil, ...]: the weight gradient of conv2d
  * (groups == 1), fp32 accumulation. Replaces the relay CudnnConvBackwardWOp(Var* x, Var* y, int kh, int kw, int strideh, ...),
  * python/jittor/extern/cuda/cudnn/ops/cudnn_conv_backward_w_op.h:20, which ConvTuner selects for

@@ -254,6 +254,44 @@ extern "C" int b200jt_conv2d_transpose(const b200jt_tensor* x, const b200jt_tens
     return conv2d_transpose_simt(x->ptr, w->ptr, y->ptr, x->dtype, s, (cudaStream_t)stream);
 }
 
+// One thread writes 8 pixels of a row (16 bytes where the rows allow): bound by the write of y, which is sh * sw times x.
+__global__ void __launch_bounds__(256)
+spread2d_kernel(const uint16_t* __restrict__ x, uint16_t* __restrict__ y, int64_t rows, int h_in, int w_in, int h_out, int w_out, int sh, int sw,
+                int vec) {
+    const int chunks = (w_out + 7) / 8;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < rows * chunks; i += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t row = i / chunks; const int w0 = (int)(i - row * chunks) * 8;
+        const int64_t plane = row / h_out; const int h = (int)(row - plane * h_out), hi = h / sh;
+        const uint16_t* src = x + (plane * h_in + hi) * w_in;
+        const bool live = hi * sh == h && hi < h_in;
+        __align__(16) uint16_t v[8];
+#pragma unroll
+        for (int e = 0; e < 8; e++) {
+            const int wi = (w0 + e) / sw;
+            v[e] = live && wi * sw == w0 + e && wi < w_in ? src[wi] : (uint16_t)0;
+        }
+        uint16_t* d = y + row * w_out + w0;
+        if (vec) *reinterpret_cast<uint4*>(d) = *reinterpret_cast<const uint4*>(v);
+        else {
+#pragma unroll
+            for (int e = 0; e < 8; e++) if (w0 + e < w_out) d[e] = v[e];
+        }
+    }
+}
+
+extern "C" int b200jt_spread2d(const b200jt_tensor* x, const b200jt_tensor* y, int sh, int sw, void* stream) {
+    B200JT_CHECK_ARG(valid_tensor(x) && valid_tensor(y) && x->ndim == 4 && y->ndim == 4, "spread2d takes NCHW tensors");
+    B200JT_CHECK_ARG(x->dtype == B200JT_BFLOAT16 && y->dtype == B200JT_BFLOAT16, "spread2d takes bfloat16 tensors");
+    B200JT_CHECK_ARG(sh > 0 && sw > 0 && x->shape[0] == y->shape[0] && x->shape[1] == y->shape[1], "spread2d: bad strides or shapes");
+    if (numel(y) == 0) return 0;
+    const int64_t rows = y->shape[0] * y->shape[1] * y->shape[2], work = rows * ((y->shape[3] + 7) / 8);
+    const int vec = y->shape[3] % 8 == 0 && (uintptr_t)y->ptr % 16 == 0;
+    spread2d_kernel<<<grid_for(work, 256), 256, 0, (cudaStream_t)stream>>>((const uint16_t*)x->ptr, (uint16_t*)y->ptr, rows, (int)x->shape[2],
+                                                                         (int)x->shape[3], (int)y->shape[2], (int)y->shape[3], sh, sw, vec);
+    B200JT_LAUNCH_CHECK();
+    return 0;
+}
+
 extern "C" int b200jt_conv2d_backward_w(const b200jt_tensor* x, const b200jt_tensor* dy, const b200jt_tensor* dw,
                                         int sh, int sw, int ph, int pw, int dh, int dw_, void* stream) {
     ConvShape s;

@@ -443,9 +443,13 @@ def conv_dgrad_plan(v, dy, w, geo):
         # on the tensor cores: 136 x 208 x 4 x 4 -> 32 x 7 x 7 (3 x 3) took 280 us as a gather on the CUDA cores.
         from . import var as V
         H, W = v.shape[2] - 2 * fp + dh * (KH - 1), v.shape[3] - 2 * fq + dw * (KW - 1)
-        spread = V.reindex(dy, [dy.shape[0], Co, H, W], ["i0", "i1", f"i2/{sh}", f"i3/{sw}"], 0, [f"i2%{sh}||i3%{sw}"])
         wf = V.reindex(w, [Ci, Co, KH, KW], ["i1", "i0", f"{KH - 1}-i2", f"{KW - 1}-i3"])
-        return Plan([spread, wf], lambda: run_conv2d(spread, wf, (1, 1, fp, fq, dh, dw), v.dtype))
+
+        def run():
+            spread = _empty([dy.shape[0], Co, H, W], "bfloat16")
+            C.call("b200jt_spread2d", C.desc(dy._data.view(list(dy.shape))), C.desc(spread), sh, sw)
+            return _conv2d(spread, _cast(wf._data, "bfloat16"), (1, 1, fp, fq, dh, dw), v.dtype)
+        return Plan([dy, wf], run)
     return Plan([dy, w], lambda: run_conv2d_transpose(dy, w, geo, 1, list(v.shape), v.dtype))
 
 
@@ -565,18 +569,20 @@ def run_conv2d_transpose(x, w, geo, groups, out_shape, out_dtype):
 
 
 def run_conv2d(x, w, geo, out_dtype, stats=None, groups=1):
+    return _conv2d(x._data, _cast(w._data, x.dtype), geo, out_dtype, stats, groups)
+
+
+def _conv2d(xd, wd, geo, out_dtype, stats=None, groups=1):
     sh, sw, ph, pw, dh, dw = geo
-    N, Ci, H, W = x.shape
-    Co, _, KH, KW = w.shape
+    N, Ci, H, W = xd.shape
+    Co, _, KH, KW = wd.shape
     OH = (H + 2 * ph - KH * dh + dh - 1) // sh + 1
     OW = (W + 2 * pw - KW * dw + dw - 1) // sw + 1
-    xd, wd = x._data, w._data
-    wd = _cast(wd, x.dtype)
-    out = _empty([N, Co, OH, OW], x.dtype)
+    out = _empty([N, Co, OH, OW], C.DTYPE_NAMES[xd.dtype])
     args = (C.desc(xd), C.desc(wd), C.desc(out), sh, sw, ph, pw, dh, dw, groups)
     nbytes, wsp, ws = C.workspace("b200jt_conv2d_workspace", *args)
     C.call("b200jt_conv2d", *args, stats.data_ptr() if stats is not None else None, wsp, nbytes,
-           what=lambda: f"conv2d x{list(x.shape)} w{list(w.shape)} geo{geo}")
+           what=lambda: f"conv2d x{list(xd.shape)} w{list(wd.shape)} geo{geo}")
     return _cast(out, out_dtype)
 
 

@@ -2,7 +2,8 @@
 import pytest
 import torch
 
-from jittor_b200 import _capi as C
+import jittor_b200 as jt
+from jittor_b200 import _capi as C, nn
 
 pytestmark = pytest.mark.gpu
 
@@ -89,3 +90,29 @@ def test_batched_matmul(ta, tb, pair, monkeypatch):
         C.call("b200jt_batched_matmul", C.desc(a), C.desc(b), C.desc(c), ta, tb)
         near(c, (a.double().transpose(1, 2) if ta else a.double()) @ (b.double().transpose(1, 2) if tb else b.double()))
     assert C.lib.b200jt_device_status() == 0
+
+
+@pytest.mark.parametrize("n,ci,h,w,co,k,s,p,d", [(3, 5, 27, 33, 8, 3, 2, 1, 1), (2, 70, 16, 16, 9, 1, 2, 0, 1), (4, 16, 29, 24, 24, 5, 3, 2, 1),
+                                                 (2, 8, 40, 23, 64, 2, 4, 0, 1), (1, 24, 21, 21, 16, 3, 2, 2, 2), (2, 9, 9, 9, 4, 3, 2, 1, 1)])
+def test_strided_input_gradient(n, ci, h, w, co, k, s, p, d):
+    x, wt = torch.randn(n, ci, h, w, device="cuda").bfloat16(), (torch.randn(co, ci, k, k, device="cuda") * 0.1).bfloat16()
+    vx = jt.array(x)
+    y = nn.conv2d(vx, jt.array(wt), None, s, p, d)
+    dy = torch.randn(*y.shape, device="cuda").bfloat16()
+    got = jt.grad((y * jt.array(dy)).sum(), vx).torch()
+    xd = x.double().requires_grad_()
+    torch.nn.functional.conv2d(xd, wt.double(), None, s, p, d).backward(dy.double())
+    near(got, xd.grad)
+
+
+@pytest.mark.parametrize("shape", [(3, 5, 1, 300), (202, 7, 7, 7), (37, 3, 1, 1023), (9, 4, 16, 16), (600, 2, 1, 1), (300, 150, 2, 3)])
+@pytest.mark.parametrize("op", ["mean", "add", "maximum"])
+def test_reduction_over_short_rows(shape, op):
+    x = torch.randn(*shape, device="cuda")
+    y = torch.empty(1, shape[1], 1, 1, device="cuda")
+    args = (C.desc(x), C.desc(y), op.encode(), 0b1101)
+    size, ptr, ws = C.workspace("b200jt_reduce_workspace", *args)
+    C.call("b200jt_reduce", *args, ptr, size)
+    xd = x.double()
+    want = xd.amax((0, 2, 3)) if op == "maximum" else xd.mean((0, 2, 3)) if op == "mean" else xd.sum((0, 2, 3))
+    assert torch.allclose(y.flatten().double(), want, rtol=1e-5, atol=1e-5 * float(xd.abs().sum((0, 2, 3)).max() if op == "add" else 1))
