@@ -199,6 +199,7 @@ conv_bf16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             const int soh = h0 + (run >> A.pw_log), snw = A.OW - sow;
             const bool svalid = q < A.patches && soh < A.OH && snw > 0;
             __nv_bfloat16* yp = y + ((int64_t)n * A.Co + (lane >> 2)) * plane + (int64_t)soh * A.OW + sow;
+            __nv_bfloat16* yl = y + (int64_t)n * A.Co * plane + (int64_t)oh * A.OW + ow;           // this lane's own pixel
             __nv_bfloat16* square = reinterpret_cast<__nv_bfloat16*>(stage_out) + (warp - 2) * 1024;
             const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + buf * BN;
 #pragma unroll 1
@@ -235,6 +236,11 @@ conv_bf16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                         f[e] = (valid && co0 + e < A.Co) ? __bfloat162float(b) : 0.f;      // statistics of the value as stored
                     }
                     __syncwarp();
+                    if (A.vec == 1) {           // rows start anywhere: a channel at a time, neighbouring lanes on neighbouring pixels
+#pragma unroll
+                        for (int e = 0; e < 32; e++)
+                            if (valid && co0 + e < A.Co) yl[(int64_t)(co0 + e) * plane] = square[e * 32 + lane];
+                    } else {
 #pragma unroll
                     for (int i = 0; i < 4; i++) {
                         if (svalid && co0 + i * 8 + (lane >> 2) < A.Co) {
@@ -247,15 +253,10 @@ conv_bf16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                             } else {
                                 const uint32_t two[4] = {px.x, px.y, px.z, px.w};
 #pragma unroll
-                                for (int e = 0; e < 4; e++) {
-                                    if (A.vec == 2) { if (2 * e < snw) *reinterpret_cast<uint32_t*>(d + 2 * e) = two[e]; }
-                                    else {
-                                        if (2 * e < snw) reinterpret_cast<uint16_t*>(d)[2 * e] = (uint16_t)two[e];
-                                        if (2 * e + 1 < snw) reinterpret_cast<uint16_t*>(d)[2 * e + 1] = (uint16_t)(two[e] >> 16);
-                                    }
-                                }
+                                for (int e = 0; e < 4; e++) if (2 * e < snw) *reinterpret_cast<uint32_t*>(d + 2 * e) = two[e];
                             }
                         }
+                    }
                     }
                 }
                 if (stats) {
