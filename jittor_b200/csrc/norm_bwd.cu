@@ -250,24 +250,27 @@ __device__ __forceinline__ bool passes(const BnArgs& g, const BnChannel& k, floa
     return (g.round == 2 ? bf(p) : p) + k.b > 0.f;
 }
 
-// A cluster of up to 8 CTAs per channel: CTA j takes the planes n = j, j + cluster size, ..., LANES threads to a plane, and the
-// CTAs' sums meet through distributed shared memory in rank order. With the graph's rounding a first sweep forms
+// A cluster of up to 8 CTAs per channel: CTA j takes the planes n = j, j + cluster size, ..., as one run of N-element vectors over
+// all its threads (a plane at a time left 158 of 256 threads idle at 28 x 28: 64 x 128 x 28 x 28 29 us, BNAFTER us this way),
+// and the CTAs' sums meet through distributed shared memory in rank order. With the graph's rounding a first sweep forms
 // E[bfloat16(x * x)] (the second sweep reads x from L2). sums: [4][C] = dbeta, dgamma, that mean square, the gradient of w.
-template <typename TX, typename TD, int N, int LANES>
+template <typename TX, typename TD, int N>
 __global__ void __launch_bounds__(256)
 bn_bwd_sums_kernel(const TX* __restrict__ x, const TD* __restrict__ dy, float* __restrict__ sums, const BnArgs g) {
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
-    const int c = blockIdx.y, t = threadIdx.x % LANES, p0 = threadIdx.x / LANES;
+    const int c = blockIdx.y;
     const int rank = (int)cluster.block_rank(), size = (int)cluster.num_blocks();
-    constexpr int PER = 256 / LANES;
-    const int hw = (int)g.HW;
+    const int hv = (int)g.HW / N, dj = 256 / hv, di = 256 - dj * hv, j0 = threadIdx.x / hv, i0 = threadIdx.x - j0 * hv;
+    const int total = (g.N_ - rank + size - 1) / size * hv;
     __shared__ float sm[32], mine[4];
     auto planes = [&](auto&& f) {
-        for (int n = rank * PER + p0; n < g.N_; n += size * PER) {
-            const int64_t at = ((int64_t)n * g.C + c) * g.HW;
-#pragma unroll 2
-            for (int i = t * N; i < hw; i += LANES * N) f(at + i);
+        int j = j0, i = i0;
+#pragma unroll 4
+        for (int v = threadIdx.x; v < total; v += 256) {
+            f(((int64_t)(rank + j * size) * g.C + c) * g.HW + i * N);
+            j += dj; i += di;
+            if (i >= hv) { i -= hv; j++; }
         }
     };
     float square = 0.f;
@@ -404,11 +407,11 @@ int run_ln(const T* x, const T* dy, const float* gamma, T* dx, float* params, fl
 #undef B200JT_LN
 }
 
-template <typename TX, typename TD, int N, int LANES>
+template <typename TX, typename TD, int N>
 int launch_bn_sums(const b200jt_tensor* x, const b200jt_tensor* dy, float* sums, const BnArgs& g, cudaStream_t st) {
-    // enough CTAs for four per SM, at most a cluster of 8 and a plane for each
+    // as many CTAs as run at once, four per SM; at most a cluster of 8, a plane for each and a vector for each thread
     int size = 1;
-    while (size < 8 && size * g.C < 4 * (kNumSMs - sm_reserve()) && size * 2 * (256 / LANES) <= g.N_) size *= 2;
+    while (size < 8 && size * 2 * g.C <= 4 * (kNumSMs - sm_reserve()) && size * 2 <= g.N_ && g.N_ / (size * 2) * (g.HW / N) >= 256) size *= 2;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(size, g.C);
     cfg.blockDim = dim3(256);
@@ -418,16 +421,14 @@ int launch_bn_sums(const b200jt_tensor* x, const b200jt_tensor* dy, float* sums,
     at.val.clusterDim.x = (unsigned)size; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
     cfg.attrs = &at;
     cfg.numAttrs = 1;
-    B200JT_CUDA(cudaLaunchKernelEx(&cfg, bn_bwd_sums_kernel<TX, TD, N, LANES>, (const TX*)x->ptr, (const TD*)dy->ptr, sums, g));
+    B200JT_CUDA(cudaLaunchKernelEx(&cfg, bn_bwd_sums_kernel<TX, TD, N>, (const TX*)x->ptr, (const TD*)dy->ptr, sums, g));
     return 0;
 }
 
 template <typename TX, typename TD, int V>
 int run_bn_sums(const b200jt_tensor* x, const b200jt_tensor* dy, float* sums, const BnArgs& g, cudaStream_t st) {
     const bool vec = g.HW % V == 0 && (uintptr_t)x->ptr % 16 == 0 && (uintptr_t)dy->ptr % 16 == 0;
-    const bool small = g.HW <= (vec ? 64 * V : 128);
-    if (vec) return small ? launch_bn_sums<TX, TD, V, 32>(x, dy, sums, g, st) : launch_bn_sums<TX, TD, V, 256>(x, dy, sums, g, st);
-    return small ? launch_bn_sums<TX, TD, 1, 32>(x, dy, sums, g, st) : launch_bn_sums<TX, TD, 1, 256>(x, dy, sums, g, st);
+    return vec ? launch_bn_sums<TX, TD, V>(x, dy, sums, g, st) : launch_bn_sums<TX, TD, 1>(x, dy, sums, g, st);
 }
 
 template <typename TX, typename TD, int V>
