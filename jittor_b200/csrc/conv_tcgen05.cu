@@ -302,16 +302,18 @@ conv_bf16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
 }
 
 // ---- layout passes -----------------------------------------------------------------------------------------
-// in[b][R][Cn] -> out[b][Cn][pitch] (bf16; pitch >= R is a multiple of 8, the elements past R are zero), 64x64 tiles, 16-byte
-// global accesses on both sides. The tile is kept as 32-bit pairs with an odd pitch (33 words) so that the column reads of the
-// second phase spread over the banks. Block (0,0,0) also zeroes `zero[0..n_zero)`. The first wz slices (blockIdx.z < wz) of
-// the same grid re-order the weights instead (w[Co][C][taps] -> wt[taps][Co][wpitch]), so that both layout passes of a
-// convolution are one launch.
+// in[b][R][Cn] -> out[b][Cn][pitch] (bf16; pitch >= R is a multiple of 8, the elements past R are zero), tiles of TR rows x 64
+// columns, 16-byte global accesses on both sides. HBM sets the time as long as whole runs are written: TR = 128 writes 256 bytes
+// at a time (256 x 256 x 56 x 56: 126 us, 6.5 TB/s; 128 bytes at a time 169 us, 64 bytes 194 us). The tile is kept as 32-bit pairs,
+// word w of row r at w ^ (r / 8) ^ (r % 4), which spreads both the rows of the first phase and the columns of the second over all banks.
+// Block (0,0,0) also zeroes `zero[0..n_zero)`. The first wz slices (blockIdx.z < wz) of the same grid re-order the weights
+// instead (w[Co][C][taps] -> wt[taps][Co][wpitch]), so that both layout passes of a convolution are one launch.
+template <int TR>
 __global__ void __launch_bounds__(256)
 transpose_bf16_batched_kernel(const __nv_bfloat16* __restrict__ in, __nv_bfloat16* __restrict__ out, int R, int Cn, int pitch, int wz,
                               const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ wt, int Co, int C, int taps, int wpitch,
                               float* __restrict__ zero, int n_zero, int w_ohwi) {
-    __shared__ __nv_bfloat16 tile[64][66];
+    __shared__ uint32_t tile[TR][32];
     if (zero && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0)       // the statistics the conv epilogue adds into
         for (int i = threadIdx.x; i < n_zero; i += blockDim.x) zero[i] = 0.f;
     if ((int)blockIdx.z < wz) {
@@ -327,33 +329,50 @@ transpose_bf16_batched_kernel(const __nv_bfloat16* __restrict__ in, __nv_bfloat1
     }
     const int64_t boff = (int64_t)((int)blockIdx.z - wz) * R * Cn;
     out += (int64_t)((int)blockIdx.z - wz) * pitch * Cn;
-    const int r0 = blockIdx.y * 64, c0 = blockIdx.x * 64;
+    const int r0 = blockIdx.y * TR, c0 = blockIdx.x * 64;
     const int j = threadIdx.x & 7, i = threadIdx.x >> 3;          // 8 chunks of 8 elements x 32 rows
     const bool vec_in = (Cn % 8 == 0);
+    uint4 v[TR / 32];
 #pragma unroll
-    for (int p = 0; p < 2; p++) {
+    for (int p = 0; p < TR / 32; p++) {
         const int r = r0 + i + p * 32, c = c0 + j * 8;
-        __align__(16) __nv_bfloat16 v[8];
-        if (r < R && vec_in && c + 8 <= Cn) *reinterpret_cast<uint4*>(v) = __ldcs(reinterpret_cast<const uint4*>(in + boff + (int64_t)r * Cn + c));
-        else {
+        v[p] = make_uint4(0, 0, 0, 0);
+        if (r < R && vec_in && c + 8 <= Cn) v[p] = __ldcs(reinterpret_cast<const uint4*>(in + boff + (int64_t)r * Cn + c));
+        else if (r < R) {
+            __align__(16) __nv_bfloat16 one[8];
 #pragma unroll
-            for (int e = 0; e < 8; e++) v[e] = (r < R && c + e < Cn) ? in[boff + (int64_t)r * Cn + c + e] : __float2bfloat16(0.f);
+            for (int e = 0; e < 8; e++) one[e] = c + e < Cn ? in[boff + (int64_t)r * Cn + c + e] : __float2bfloat16(0.f);
+            v[p] = *reinterpret_cast<const uint4*>(one);
         }
-        uint32_t* row = reinterpret_cast<uint32_t*>(&tile[i + p * 32][0]);
+    }
 #pragma unroll
-        for (int e = 0; e < 4; e++) row[j * 4 + e] = reinterpret_cast<const uint32_t*>(v)[e];
+    for (int p = 0; p < TR / 32; p++) {
+        const int row = i + p * 32, x = (row >> 3) ^ (row & 3);
+        tile[row][(j * 4) ^ x] = v[p].x; tile[row][(j * 4 + 1) ^ x] = v[p].y;
+        tile[row][(j * 4 + 2) ^ x] = v[p].z; tile[row][(j * 4 + 3) ^ x] = v[p].w;
     }
     __syncthreads();
+    constexpr int OCT = TR / 8;                                   // a warp writes whole runs of TR elements
+    const int lane = threadIdx.x & 31, oct = lane % OCT, r = r0 + oct * 8;
+    if (r >= pitch) return;
 #pragma unroll
-    for (int p = 0; p < 2; p++) {
-        const int c = c0 + i + p * 32, r = r0 + j * 8;           // output row = input column
+    for (int p = 0; p < OCT / 8; p++) {
+        const int pair = lane / OCT * OCT + (threadIdx.x >> 5) + p * 8, c = c0 + 2 * pair;      // two output rows = input columns
         if (c >= Cn) continue;
-        __align__(16) __nv_bfloat16 v[8];
+        uint32_t u[8];
 #pragma unroll
-        for (int e = 0; e < 8; e++) v[e] = tile[j * 8 + e][i + p * 32];
-        if (r < pitch) __stcs(reinterpret_cast<uint4*>(out + (int64_t)c * pitch + r), *reinterpret_cast<uint4*>(v));
+        for (int e = 0; e < 8; e++) u[e] = tile[oct * 8 + e][pair ^ oct ^ (e & 3)];
+        uint4 lo, hi;
+        lo.x = __byte_perm(u[0], u[1], 0x5410); lo.y = __byte_perm(u[2], u[3], 0x5410);
+        lo.z = __byte_perm(u[4], u[5], 0x5410); lo.w = __byte_perm(u[6], u[7], 0x5410);
+        hi.x = __byte_perm(u[0], u[1], 0x7632); hi.y = __byte_perm(u[2], u[3], 0x7632);
+        hi.z = __byte_perm(u[4], u[5], 0x7632); hi.w = __byte_perm(u[6], u[7], 0x7632);
+        __stcs(reinterpret_cast<uint4*>(out + (int64_t)c * pitch + r), lo);
+        if (c + 1 < Cn) __stcs(reinterpret_cast<uint4*>(out + (int64_t)(c + 1) * pitch + r), hi);
     }
 }
+
+inline int layout_rows(int c) { return c > 64 ? 128 : 64; }       // tile rows of the pass for c channels
 
 static bool make_map_x(CUtensorMap* map, const void* base, const ConvShape& s, int pw_log) {
     auto fn = encode_fn();
@@ -470,12 +489,13 @@ int conv2d_tc(const void* x, const void* w, void* y, float* stats, const ConvSha
     const int HW = s.H * s.W;
     {   // x[N][C][HW] -> xt[N][HW][C], and the weights tap-major, in one launch
         const int64_t nw = (int64_t)s.Co * s.C * s.KH * s.KW;
-        const unsigned gx = (unsigned)((HW + 63) / 64), gy = (unsigned)((s.C + 63) / 64);
+        const unsigned gx = (unsigned)((HW + 63) / 64), gy = (unsigned)((s.C + layout_rows(s.C) - 1) / layout_rows(s.C));
         const int64_t per_slice = (int64_t)gx * gy * 256;
         const unsigned wz = (unsigned)std::min<int64_t>(32, std::max<int64_t>(1, (nw + per_slice - 1) / per_slice));
         dim3 g(gx, gy, (lay.x_nhwc ? 0u : (unsigned)s.N) + wz);          // the first wz slices re-order the weights
         float* zero = (stats && s.Co <= STATS_MAX_CO) ? stats : nullptr;   // zeroed here instead of by a memset node
-        transpose_bf16_batched_kernel<<<g, 256, 0, st>>>((const __nv_bfloat16*)x, xt, s.C, HW, cp, (int)wz,
+        const auto kernel = layout_rows(s.C) == 128 ? transpose_bf16_batched_kernel<128> : transpose_bf16_batched_kernel<64>;
+        kernel<<<g, 256, 0, st>>>((const __nv_bfloat16*)x, xt, s.C, HW, cp, (int)wz,
                                                           (const __nv_bfloat16*)w, wt, s.Co, s.C, s.KH * s.KW, cp, zero, 2 * s.Co, lay.w_ohwi ? 1 : 0);
         B200JT_LAUNCH_CHECK();
     }
@@ -785,13 +805,15 @@ int conv2d_wgrad_tc(const void* x, const void* dy, void* dw, const ConvShape& sh
     float* part = (float*)(ws + p.xb + p.dyb);
     const int HW = s.H * s.W, OHW = s.OH * s.OW;
     if (!lay.x_nhwc) {   // x[N][C][HW] -> [N][HW][C]
-        dim3 gx((unsigned)((HW + 63) / 64), (unsigned)((s.C + 63) / 64), (unsigned)s.N);
-        tcconv::transpose_bf16_batched_kernel<<<gx, 256, 0, st>>>((const __nv_bfloat16*)x, xt, s.C, HW, tcconv::pitch8(s.C), 0, nullptr, nullptr, 0, 0, 0, 0, nullptr, 0, 0);
+        dim3 gx((unsigned)((HW + 63) / 64), (unsigned)((s.C + tcconv::layout_rows(s.C) - 1) / tcconv::layout_rows(s.C)), (unsigned)s.N);
+        const auto kernel = tcconv::layout_rows(s.C) == 128 ? tcconv::transpose_bf16_batched_kernel<128> : tcconv::transpose_bf16_batched_kernel<64>;
+        kernel<<<gx, 256, 0, st>>>((const __nv_bfloat16*)x, xt, s.C, HW, tcconv::pitch8(s.C), 0, nullptr, nullptr, 0, 0, 0, 0, nullptr, 0, 0);
         B200JT_LAUNCH_CHECK();
     }
     if (!lay.y_nhwc) {   // dy[N][Co][OH*OW] -> [N][OH*OW][Co]
-        dim3 gy((unsigned)((OHW + 63) / 64), (unsigned)((s.Co + 63) / 64), (unsigned)s.N);
-        tcconv::transpose_bf16_batched_kernel<<<gy, 256, 0, st>>>((const __nv_bfloat16*)dy, dyt, s.Co, OHW, tcconv::pitch8(s.Co), 0, nullptr, nullptr, 0, 0, 0, 0, nullptr, 0, 0);
+        dim3 gy((unsigned)((OHW + 63) / 64), (unsigned)((s.Co + tcconv::layout_rows(s.Co) - 1) / tcconv::layout_rows(s.Co)), (unsigned)s.N);
+        const auto kernel = tcconv::layout_rows(s.Co) == 128 ? tcconv::transpose_bf16_batched_kernel<128> : tcconv::transpose_bf16_batched_kernel<64>;
+        kernel<<<gy, 256, 0, st>>>((const __nv_bfloat16*)dy, dyt, s.Co, OHW, tcconv::pitch8(s.Co), 0, nullptr, nullptr, 0, 0, 0, 0, nullptr, 0, 0);
         B200JT_LAUNCH_CHECK();
     }
     WgradArgs A;
