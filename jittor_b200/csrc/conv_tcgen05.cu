@@ -5,10 +5,10 @@
 //   GEMM view   M = N*OH*OW output pixels, N = Cout, K = KH*KW*Cin, walked tap by tap in 64-channel blocks;
 //   layout      x is first copied NCHW -> NHWC (channels innermost) and w OIHW -> [tap][Cout][Cin], so that both
 //               operands are K-major and every TMA box starts at a channel offset that is a multiple of 64 (the
-//               16-byte start rule); the spatial shift of a tap is carried by the H/W box coordinates, which may be
-//               negative or past the edge -- TMA zero-fills, which is exactly the reindex overflow value 0;
-//   tile        128 pixels (two spatial patches of 64, each one 4-D TMA box of 64 rows x 128 B) x up to 256 output
-//               channels, for one CTA or twice the pixels for a pair of CTAs;
+//               16-byte start rule); the spatial shift of a tap comes with the load, and what lies outside x is zero-filled,
+//               which is exactly the reindex overflow value 0;
+//   tile        128 consecutive output pixels (one im2col TMA load of 128 rows x 128 B per k-block: rows, images and
+//               padding are the map's business) x up to 256 output channels, or twice the pixels for a pair of CTAs;
 //   pipeline    same persistent warp-specialised ring as the GEMM (TMA warp, MMA warp, 8 epilogue warps, TMEM
 //               double buffering); strides 1..4 through the traversal stride of the x tensor map;
 //   epilogue    tcgen05.ld -> bf16 -> y in NCHW; optionally per-channel sum / sum of squares of the stored values
@@ -45,21 +45,11 @@ inline int pitch8(int c) { return (c + 7) / 8 * 8; }
 
 struct ConvArgs {
     int N, C, H, W, Co, KH, KW, OH, OW, sh, sw, ph, pw, dh, dw;
-    int pw_log;                      // a patch is 64 pixels, half a tile: (64 >> pw_log) rows of (1 << pw_log) pixels
-    int tiles_h, tiles_w;            // patches per image
-    int64_t patches;                 // N * tiles_h * tiles_w
+    int64_t pixels;                  // N * OH * OW
     int tiles_m, tiles_n;
-    int vec;                         // pixels per store of y: the largest of 8, 4, 2, 1 that divides OW (and y's alignment)
+    int vec;                         // pixels per store of y: 8 or 4 where OH * OW is a multiple (and y aligned), else 1
     int last_k;                      // MMA steps of 16 channels in a tap's last channel block
 };
-
-__device__ __forceinline__ void patch_coords(const ConvArgs& A, int64_t q, int& n, int& h0, int& w0) {
-    const int per_img = A.tiles_h * A.tiles_w;
-    n = (int)(q / per_img);
-    const int r = (int)(q - (int64_t)n * per_img);
-    h0 = (r / A.tiles_w) * (64 >> A.pw_log);
-    w0 = (r % A.tiles_w) << A.pw_log;
-}
 
 __device__ __forceinline__ int first_block(int tm, int k_blocks) { return (int)((tm * 7u) % (unsigned)k_blocks); }
 
@@ -117,20 +107,18 @@ conv_bf16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             bool ok = true;
             for (int t = first; t < total && ok; t += step) {
                 const int tm = t / A.tiles_n, tn = t - tm * A.tiles_n;
-                int n0, h0, w0, n1, h1, w1;
-                patch_coords(A, 2 * ((int64_t)tm * CTAS + rank), n0, h0, w0);
-                patch_coords(A, 2 * ((int64_t)tm * CTAS + rank) + 1, n1, h1, w1);       // past the last patch: n1 >= N, zero-filled
+                int64_t q = ((int64_t)tm * CTAS + rank) * BM;
+                if (q >= A.pixels) q = 0;                       // a pair's second half past the last pixel: any pixels, none is stored
+                const int n = (int)(q / (A.OH * A.OW)), in = (int)(q - (int64_t)n * (A.OH * A.OW));
+                const int h = in / A.OW * A.sh - A.ph, w = in % A.OW * A.sw - A.pw;
                 int tap = first_block(tm, k_blocks) / cblocks, cb = first_block(tm, k_blocks) - tap * cblocks;
                 int kh = tap / A.KW, kw = tap - kh * A.KW;
                 for (int kb = 0; kb < k_blocks; kb++) {
-                    const int dy = kh * A.dh - A.ph, dx = kw * A.dw - A.pw;
                     if (!(ok = mbar_wait(empty + stage, phase ^ 1, abort_flag, 11))) break;
                     unsigned char* sa = smem + stage * STAGE_BYTES;
                     if (rank == 0) mbar_expect_tx(full + stage, CTAS * A_BYTES + BN_T * BK * 2);      // both CTAs' bytes
                     const uint32_t bar = PAIR ? leader_addr(full + stage) : smem_u32(full + stage);
-                    // a box covers 64 OUTPUT pixels: with stride s the tensor map steps s input elements per box element
-                    tma_load_tile<CTAS>(sa, &map_x, bar, cb * BK, w0 * A.sw + dx, h0 * A.sh + dy, n0);
-                    tma_load_tile<CTAS>(sa + A_BYTES / 2, &map_x, bar, cb * BK, w1 * A.sw + dx, h1 * A.sh + dy, n1);
+                    tma_load_im2col<CTAS>(sa, &map_x, bar, cb * BK, w, h, n, kw * A.dw, kh * A.dh);
                     tma_load_tile<CTAS>(sa + A_BYTES, &map_w, bar, cb * BK, tap * A.Co + tn * BN_T + rank * (BN_T / CTAS));
                     if (++cb == cblocks) {
                         cb = 0; tap++;
@@ -186,20 +174,14 @@ conv_bf16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            // this lane's pixel: row r of the tile = patch (r / 64), position (r % 64) in row order
-            const int r = quad * 32 + lane;
-            const int64_t q = 2 * ((int64_t)tm * CTAS + rank) + (r >> 6);
-            int n, h0, w0;
-            patch_coords(A, q, n, h0, w0);
-            const int pw = 1 << A.pw_log;
-            const int oh = h0 + ((r & 63) >> A.pw_log), ow = w0 + (r & (pw - 1));
-            const bool valid = q < A.patches && oh < A.OH && ow < A.OW;
-            // the 8 pixels this lane stores: the (lane % 4)th of the warp's four runs, channels lane / 4 + 8 i of a chunk
-            const int run = (quad & 1) * 32 + (lane & 3) * 8, sow = w0 + (run & (pw - 1));
-            const int soh = h0 + (run >> A.pw_log), snw = A.OW - sow;
-            const bool svalid = q < A.patches && soh < A.OH && snw > 0;
-            __nv_bfloat16* yp = y + ((int64_t)n * A.Co + (lane >> 2)) * plane + (int64_t)soh * A.OW + sow;
-            __nv_bfloat16* yl = y + (int64_t)n * A.Co * plane + (int64_t)oh * A.OW + ow;           // this lane's own pixel
+            // this lane's pixel, and the 8 pixels it stores: the (lane % 4)th of the warp's four runs, channels lane / 4 + 8 i of a chunk
+            const int64_t p0 = ((int64_t)tm * CTAS + rank) * BM + quad * 32, p = p0 + lane;
+            const bool valid = p < A.pixels;
+            auto plane_at = [&](int64_t q) { const int64_t n = q / plane; return y + n * (A.Co - 1) * plane + q; };
+            __nv_bfloat16* yl = NHWC ? y + p * A.Co : plane_at(p);
+            const int64_t run = p0 + (lane & 3) * 8;
+            __nv_bfloat16* y0 = plane_at(run) + (lane >> 2) * plane;
+            __nv_bfloat16* y1 = plane_at(run + 4) + (lane >> 2) * plane;
             __nv_bfloat16* square = reinterpret_cast<__nv_bfloat16*>(stage_out) + (warp - 2) * 1024;
             const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + buf * BN;
 #pragma unroll 1
@@ -218,7 +200,7 @@ conv_bf16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                         f[e] = (valid && co0 + e < A.Co) ? __bfloat162float(row[e]) : 0.f;
                     }
                     if (valid) {
-                        __nv_bfloat16* yq = y + (((int64_t)n * A.OH + oh) * A.OW + ow) * A.Co + co0;
+                        __nv_bfloat16* yq = yl + co0;
                         if (co0 + 32 <= A.Co && (A.Co & 7) == 0) {
 #pragma unroll
                             for (int q = 0; q < 4; q++) reinterpret_cast<uint4*>(yq)[q] = reinterpret_cast<const uint4*>(row)[q];
@@ -236,27 +218,23 @@ conv_bf16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                         f[e] = (valid && co0 + e < A.Co) ? __bfloat162float(b) : 0.f;      // statistics of the value as stored
                     }
                     __syncwarp();
-                    if (A.vec == 1) {           // rows start anywhere: a channel at a time, neighbouring lanes on neighbouring pixels
+                    if (A.vec == 1) {           // planes start anywhere: a channel at a time, neighbouring lanes on neighbouring pixels
 #pragma unroll
                         for (int e = 0; e < 32; e++)
                             if (valid && co0 + e < A.Co) yl[(int64_t)(co0 + e) * plane] = square[e * 32 + lane];
                     } else {
 #pragma unroll
-                    for (int i = 0; i < 4; i++) {
-                        if (svalid && co0 + i * 8 + (lane >> 2) < A.Co) {
-                            const uint4 px = reinterpret_cast<const uint4*>(square)[i * 32 + lane];
-                            __nv_bfloat16* d = yp + (int64_t)(co0 + i * 8) * plane;
-                            if (A.vec == 8) *reinterpret_cast<uint4*>(d) = px;
-                            else if (A.vec == 4) {
-                                *reinterpret_cast<uint2*>(d) = make_uint2(px.x, px.y);
-                                if (snw > 4) *reinterpret_cast<uint2*>(d + 4) = make_uint2(px.z, px.w);
-                            } else {
-                                const uint32_t two[4] = {px.x, px.y, px.z, px.w};
-#pragma unroll
-                                for (int e = 0; e < 4; e++) if (2 * e < snw) *reinterpret_cast<uint32_t*>(d + 2 * e) = two[e];
+                        for (int i = 0; i < 4; i++) {
+                            if (co0 + i * 8 + (lane >> 2) < A.Co) {
+                                const uint4 px = reinterpret_cast<const uint4*>(square)[i * 32 + lane];
+                                const int64_t d = (int64_t)(co0 + i * 8) * plane;
+                                if (A.vec == 8) { if (run < A.pixels) *reinterpret_cast<uint4*>(y0 + d) = px; }
+                                else {
+                                    if (run < A.pixels) *reinterpret_cast<uint2*>(y0 + d) = make_uint2(px.x, px.y);
+                                    if (run + 4 < A.pixels) *reinterpret_cast<uint2*>(y1 + d) = make_uint2(px.z, px.w);
+                                }
                             }
                         }
-                    }
                     }
                 }
                 if (stats) {
@@ -374,20 +352,26 @@ transpose_bf16_batched_kernel(const __nv_bfloat16* __restrict__ in, __nv_bfloat1
 
 inline int layout_rows(int c) { return c > 64 ? 128 : 64; }       // tile rows of the pass for c channels
 
-static bool make_map_x(CUtensorMap* map, const void* base, const ConvShape& s, int pw_log) {
-    auto fn = encode_fn();
+// Channels-last tensor [N][H][W][C] read as windows: `pixels` window origins x 64 channels per load. The bounding box holds the
+// origins (the corners: padding before, and padding minus the filter's reach after), the traversal strides are the convolution's,
+// the tap's shift comes with the load. Outside the tensor -- padding, channels past C, images past N -- reads as zero.
+static bool make_map_im2col(CUtensorMap* map, const void* base, int N, int H, int W, int C, int sh, int sw, int ph, int pw, int reach_h, int reach_w, int pixels) {
+    auto fn = encode_im2col_fn();
     if (!fn) return false;
-    cuuint64_t dims[4] = {(cuuint64_t)s.C, (cuuint64_t)s.W, (cuuint64_t)s.H, (cuuint64_t)s.N};
-    const cuuint64_t cp = (cuuint64_t)pitch8(s.C) * 2;
-    cuuint64_t strides[3] = {cp, s.W * cp, s.H * s.W * cp};
-    // strided convolution: the traversal stride of the map skips input pixels, so that a box still delivers 64 window
-    // origins; the box extent counts tensor elements, i.e. pixels * stride per axis (at most 64 * 4 = 256)
-    cuuint32_t box[4] = {(cuuint32_t)BK, (cuuint32_t)(s.sw << pw_log), (cuuint32_t)(s.sh * (64 >> pw_log)), 1};
-    cuuint32_t estr[4] = {1, (cuuint32_t)s.sw, (cuuint32_t)s.sh, 1};
-    return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, estr,
+    cuuint64_t dims[4] = {(cuuint64_t)C, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)N};
+    const cuuint64_t cp = (cuuint64_t)pitch8(C) * 2;
+    cuuint64_t strides[3] = {cp, W * cp, (cuuint64_t)H * W * cp};
+    int lower[2] = {-pw, -ph}, upper[2] = {pw - reach_w, ph - reach_h};
+    cuuint32_t estr[4] = {1, (cuuint32_t)sw, (cuuint32_t)sh, 1};
+    return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, lower, upper, BK, (cuuint32_t)pixels, estr,
               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
+// the corners and shifts an im2col map can hold
+static bool im2col_fits(const ConvShape& s) {
+    return s.ph <= 127 && s.pw <= 127 && (s.KH - 1) * (int64_t)s.dh <= 127 && (s.KW - 1) * (int64_t)s.dw <= 127;
+}
+
 static bool make_map_w(CUtensorMap* map, const void* base, const ConvShape& s, int bn) {
     auto fn = encode_fn();
     if (!fn) return false;
@@ -398,24 +382,6 @@ static bool make_map_w(CUtensorMap* map, const void* base, const ConvShape& s, i
     return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
-// Pixels of a 1 x 1 layer are all alike: one row of them.
-static ConvShape flattened(ConvShape s) {
-    if (s.KH == 1 && s.KW == 1 && s.sh == 1 && s.sw == 1 && s.ph == 0 && s.pw == 0) { s.W *= s.H; s.OW = s.W; s.H = s.OH = 1; }
-    return s;
-}
-// Patch shape: the one that covers an image with the fewest patches, of equals the one with the longest rows (up to 32 pixels: y
-// is then written in whole sectors). 28 x 28: 14 patches of 4 x 16 instead of 16 of 8 x 8.
-struct Patches { int64_t count; int tiles_h, tiles_w, pw_log; };
-static Patches patches_of(const ConvShape& s) {
-    Patches best{INT64_MAX, 0, 0, 0};
-    for (int l = 6; l >= 3; l--) {
-        const int th = (s.OH + (64 >> l) - 1) / (64 >> l), tw = (s.OW + (1 << l) - 1) >> l;
-        const int64_t n = (int64_t)s.N * th * tw;
-        if (n < best.count || (l == 5 && n == best.count)) best = {n, th, tw, l};
-    }
-    return best;
 }
 
 template <bool NHWC>
@@ -449,16 +415,14 @@ static int pair_slots() {
 
 }  // namespace tcconv
 
-// Any channel counts (the channels-last copies are padded to TMA's pitch, missing channels read as zero) and any extents, as
-// long as an 8 x 8 patch is at least an eighth full and there are the 8 channels that half of the smallest MMA step needs:
-// below that the padding costs more than the CUDA-core kernel. 304 -> 48 channels of 56 x 56, 18 images: 1.98 ms on the CUDA
-// cores, 0.21 ms here; 40 -> 27 channels of 7 x 7, 218 images: 106 us and 24 us.
+// Any channel counts (the channels-last copies are padded to TMA's pitch, missing channels read as zero) and any extents, down
+// to the 8 channels that half of the smallest MMA step needs: below that the padding costs more than the CUDA-core kernel.
+// 304 -> 48 channels of 56 x 56, 18 images: 1.98 ms on the CUDA cores; 40 -> 27 channels of 7 x 7, 218 images: 106 us.
 bool conv2d_tc_supported(const ConvShape& s, const void* x, const void* w, const void* y) {
     const int64_t px = (int64_t)s.N * s.OH * s.OW;
-    const int64_t patches = (int64_t)s.N * ((s.OH + 7) / 8) * ((s.OW + 7) / 8);
-    return s.sh >= 1 && s.sh <= 4 && s.sw >= 1 && s.sw <= 4 && px >= 8 * patches && s.C >= 8 && ((uintptr_t)x % 16 == 0) &&
+    return s.sh >= 1 && s.sh <= 4 && s.sw >= 1 && s.sw <= 4 && px >= 16 && s.C >= 8 && tcconv::im2col_fits(s) && ((uintptr_t)x % 16 == 0) &&
            ((uintptr_t)w % 2 == 0) && ((uintptr_t)y % 2 == 0) && (int64_t)s.Co * s.KH * s.KW < (1LL << 31) && s.N <= 65000 &&
-           patches * ((s.Co + 63) / 64) < (1LL << 31) && tc::encode_fn() != nullptr;
+           (int64_t)s.OH * s.OW < (1LL << 31) && px / 128 * ((s.Co + 63) / 64) < (1LL << 30) && tc::encode_fn() != nullptr && tc::encode_im2col_fn() != nullptr;
 }
 
 // The channels-last layouts are read and written where they lie and keep the rules they are documented with.
@@ -477,10 +441,9 @@ size_t conv2d_tc_workspace(const ConvShape& s) {
     return xb + wb + 1024;
 }
 
-int conv2d_tc(const void* x, const void* w, void* y, float* stats, const ConvShape& shape, void* workspace, cudaStream_t st,
+int conv2d_tc(const void* x, const void* w, void* y, float* stats, const ConvShape& s, void* workspace, cudaStream_t st,
               const ConvLayout& lay) {
     using namespace tcconv;
-    const ConvShape s = flattened(shape);
     unsigned char* ws = (unsigned char*)(((uintptr_t)workspace + 1023) & ~(uintptr_t)1023);
     // NHWC ("acdb") activations are what the kernel reads: no staging pass for x then
     __nv_bfloat16* xt = lay.x_nhwc ? (__nv_bfloat16*)const_cast<void*>(x) : (__nv_bfloat16*)ws;
@@ -502,8 +465,7 @@ int conv2d_tc(const void* x, const void* w, void* y, float* stats, const ConvSha
     ConvArgs A;
     A.N = s.N; A.C = s.C; A.H = s.H; A.W = s.W; A.Co = s.Co; A.KH = s.KH; A.KW = s.KW; A.OH = s.OH; A.OW = s.OW;
     A.sh = s.sh; A.sw = s.sw; A.ph = s.ph; A.pw = s.pw; A.dh = s.dh; A.dw = s.dw;
-    const Patches pt = patches_of(s);
-    A.patches = pt.count; A.tiles_h = pt.tiles_h; A.tiles_w = pt.tiles_w; A.pw_log = pt.pw_log;
+    A.pixels = (int64_t)s.N * s.OH * s.OW;
     A.last_k = (s.C - (s.C + BK - 1) / BK * BK + BK + UMMA_K - 1) / UMMA_K;
     // Tile by estimated time: the grid is persistent with a static round-robin, so it takes ceil(tiles / slots) rounds, each of a
     // tile's main loop and the part of its epilogue that the next tile's main loop does not hide (about half). A k-block of 64 channels
@@ -519,7 +481,7 @@ int conv2d_tc(const void* x, const void* w, void* y, float* stats, const ConvSha
         if ((pair_env && atoi(pair_env) != p) || (p && !slots)) continue;
         for (int b = 64; b <= 256; b *= 2) {
             if ((forced_bn == 64 || forced_bn == 128 || forced_bn == 256) && forced_bn != b) continue;
-            const int64_t t = (A.patches + 2 * p + 1) / (2 * p + 2) * ((s.Co + b - 1) / b);
+            const int64_t t = (A.pixels + BM * (p + 1) - 1) / (BM * (p + 1)) * ((s.Co + b - 1) / b);
             const double block = 300 + (p ? 0.57 : 0.69) * b;
             const double epilogue = 600 + b * (stats ? 23.0 : 12.5);
             const int n = p ? slots : kNumSMs;
@@ -528,13 +490,14 @@ int conv2d_tc(const void* x, const void* w, void* y, float* stats, const ConvSha
         }
     }
     const int ctas = pair ? 2 : 1;
-    A.tiles_m = (int)((A.patches + 2 * ctas - 1) / (2 * ctas));
+    A.tiles_m = (int)((A.pixels + BM * ctas - 1) / (BM * ctas));
     A.tiles_n = (s.Co + bn - 1) / bn;
     CUtensorMap mx, mw;
-    if (!make_map_x(&mx, xt, s, A.pw_log) || !make_map_w(&mw, wt, s, bn / ctas)) return fail(-4, "conv2d: cuTensorMapEncodeTiled failed");
+    if (!make_map_im2col(&mx, xt, s.N, s.H, s.W, s.C, s.sh, s.sw, s.ph, s.pw, s.dh * (s.KH - 1), s.dw * (s.KW - 1), BM) || !make_map_w(&mw, wt, s, bn / ctas)) return fail(-4, "conv2d: cuTensorMapEncodeTiled failed");
     if (!slots) return fail(-4, "conv2d: no room for the kernel's shared memory");
     A.vec = 8;
-    while (A.vec > 1 && (s.OW % A.vec || (uintptr_t)y % (2 * A.vec))) A.vec /= 2;
+    while (A.vec > 1 && ((int64_t)s.OH * s.OW % A.vec || (uintptr_t)y % (2 * A.vec))) A.vec /= 2;
+    if (A.vec == 2) A.vec = 1;
     float* fused = (stats && s.Co <= STATS_MAX_CO) ? stats : nullptr;
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute at[1];
@@ -551,10 +514,10 @@ int conv2d_tc(const void* x, const void* w, void* y, float* stats, const ConvSha
 // over (batch, rows, columns) of reindex(x) * broadcast(dy) that ConvTuner relays to cudnnConvolutionBackwardFilter
 // (python/jittor/extern/cuda/cudnn/ops/cudnn_conv_backward_w_op.cc:292). As a GEMM per filter tap:
 //   D[c, o] = sum over pixels of X_tap[pixel, c] * DY[pixel, o],     M = Cin (128 per CTA), N = Cout (256), K = N*OH*OW.
-// x and dy are first copied to NHWC, so a 4-D TMA box of 64 output pixels x 64 channels lands as 64 rows of 128 B with
+// x and dy are first copied to NHWC, so an im2col TMA load of 64 output pixels x 64 channels lands as 64 rows of 128 B with
 // the channel axis contiguous: both operands are MN-major (their own axis contiguous, K = pixel strided), and the same box
 // geometry as the forward kernel carries the tap's shift and the stride in its coordinates. One CTA owns one
-// (tap, 128 input channels, 256 output channels) accumulator in TMEM and walks a contiguous range of pixel patches; the
+// (tap, 128 input channels, 256 output channels) accumulator in TMEM and walks a contiguous range of 64-pixel blocks; the
 // K axis is split over `splits` CTAs per accumulator to fill the GPU, each writing fp32 partial sums that a second kernel
 // adds in split order (deterministic) and stores as bf16 in OIHW order.
 namespace tcwgrad {
@@ -574,8 +537,7 @@ template <int TAPS> struct Ring {
 
 struct WgradArgs {
     int N, C, H, W, Co, KH, KW, OH, OW, sh, sw, ph, pw, dh, dw;
-    int tiles_h, tiles_w, pw_log;    // patches per image, their shape
-    int64_t patches;                 // N * tiles_h * tiles_w: the K axis in units of 64 pixels
+    int64_t blocks;                  // the K axis in units of 64 consecutive output pixels
     int tiles_m, tiles_n, splits, groups;      // groups: ceil(taps / TAPS) tap groups
 };
 
@@ -603,8 +565,8 @@ wgrad_bf16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     const int tn = tile % A.tiles_n, tm = tile / A.tiles_n;
     const int tap0 = group * TAPS;
     const int ntap = min(TAPS, taps - tap0);                 // the last group of an odd tap count holds one tap
-    const int64_t p0 = A.patches * split / A.splits, p1 = A.patches * (split + 1) / A.splits;
-    const int k_blocks = (int)(p1 - p0);                     // >= 1: the host keeps splits <= patches
+    const int64_t p0 = A.blocks * split / A.splits, p1 = A.blocks * (split + 1) / A.splits;
+    const int k_blocks = (int)(p1 - p0);                     // >= 1: the host keeps splits <= blocks
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; s++) { mbar_init(full + s, 1); mbar_init(empty + s, 1); }
@@ -622,21 +584,19 @@ wgrad_bf16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     const uint32_t tmem_base = *tmem_slot;
 
     if (warp == 0) {
-        // The whole warp walks the patches; lane 0 waits for the slot and announces the bytes, then every lane that owns a box
+        // The whole warp walks the blocks; lane 0 waits for the slot and announces the bytes, then every lane that owns a box
         // issues it: chunk j of a stage belongs to lane j -- x chunks of tap 0, x chunks of tap 1, then the dy chunks.
         const bool is_x = lane < TAPS * XBOX;
         const int t = is_x ? lane / XBOX : 0;                 // which of this CTA's taps the lane's x box serves
         const int tap = min(tap0 + t, taps - 1);
         const int kh = tap / A.KW, kw = tap - kh * A.KW;
-        const int per_img = A.tiles_h * A.tiles_w;
-        int n = (int)(p0 / per_img);
-        const int r0 = (int)(p0 - (int64_t)n * per_img);
-        int th = r0 / A.tiles_w, tw = r0 - th * A.tiles_w;
+        const int plane = A.OH * A.OW;
+        int n = (int)(p0 * PIX / plane), in = (int)(p0 * PIX - (int64_t)n * plane);
         const bool owns = is_x ? t < ntap : lane < TAPS * XBOX + YBOX;
         const CUtensorMap* map = is_x ? &map_x : &map_dy;
         const int c0 = is_x ? tm * BM + (lane - t * XBOX) * 64 : tn * BN_T + (lane - TAPS * XBOX) * 64;
-        const int sw = is_x ? A.sw : 1, sh = is_x ? A.sh : 1;
-        const int ox = is_x ? kw * A.dw - A.pw : 0, oy = is_x ? kh * A.dh - A.ph : 0;
+        const int sw = is_x ? A.sw : 1, sh = is_x ? A.sh : 1, pw = is_x ? A.pw : 0, ph = is_x ? A.ph : 0;
+        const int dw = is_x ? kw * A.dw : 0, dh = is_x ? kh * A.dh : 0;
         const uint32_t stage_bytes = (uint32_t)(ntap * XBOX + YBOX) * CHUNK_BYTES;
         int stage = 0; uint32_t phase = 0;
         bool ok = true;
@@ -647,11 +607,12 @@ wgrad_bf16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
             }
             ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
             if (!ok) break;
-            // pixels past the edge of x (padding, ragged patches) and channels past C / Co are zero-filled by TMA
-            if (owns)
-                tma_load_4d(smem + stage * MAX_STAGE_BYTES + lane * CHUNK_BYTES, map, full + stage, c0,
-                            (tw << A.pw_log) * sw + ox, th * (64 >> A.pw_log) * sh + oy, n);
-            if (++tw == A.tiles_w) { tw = 0; if (++th == A.tiles_h) { th = 0; n++; } }
+            // pixels outside x or past the last image and channels past C / Co are zero-filled by TMA
+            if (owns) {
+                const int oh = in / A.OW, ow = in - oh * A.OW;
+                tma_load_im2col<1>(smem + stage * MAX_STAGE_BYTES + lane * CHUNK_BYTES, map, smem_u32(full + stage), c0, ow * sw - pw, oh * sh - ph, n, dw, dh);
+            }
+            for (in += PIX; in >= plane; in -= plane) n++;
             if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
         if (!ok && lane == 0) {
@@ -735,22 +696,7 @@ wgrad_fold_kernel(const float* __restrict__ part, __nv_bfloat16* __restrict__ dw
     }
 }
 
-// NHWC tensor [N][H][W][C] as a 4-D map whose box is 64 channels x a patch (times the strides) x 1 with traversal strides
-// (1, sw, sh, 1): 64 pixels x 128 B in shared memory.
-static bool make_map_nhwc(CUtensorMap* map, const void* base, int N, int H, int W, int C, int sh, int sw, int pw_log) {
-    auto fn = encode_fn();
-    if (!fn) return false;
-    cuuint64_t dims[4] = {(cuuint64_t)C, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)N};
-    const cuuint64_t cp = (cuuint64_t)tcconv::pitch8(C) * 2;
-    cuuint64_t strides[3] = {cp, W * cp, (cuuint64_t)H * W * cp};
-    cuuint32_t box[4] = {64, (cuuint32_t)(sw << pw_log), (cuuint32_t)(sh * (64 >> pw_log)), 1};
-    cuuint32_t estr[4] = {1, (cuuint32_t)sw, (cuuint32_t)sh, 1};
-    return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, estr,
-              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
-struct Plan { int bn, taps_per_cta, groups, tiles_m, tiles_n, splits; int64_t patches; size_t xb, dyb, pb; };
+struct Plan { int bn, taps_per_cta, groups, tiles_m, tiles_n, splits; int64_t blocks; size_t xb, dyb, pb; };
 
 static Plan plan_for(const ConvShape& s) {
     Plan p;
@@ -761,11 +707,11 @@ static Plan plan_for(const ConvShape& s) {
     p.groups = (taps + p.taps_per_cta - 1) / p.taps_per_cta;
     p.tiles_m = (s.C + BM - 1) / BM;
     p.tiles_n = (s.Co + p.bn - 1) / p.bn;
-    p.patches = tcconv::patches_of(s).count;
-    // fill the GPU once when the accumulators alone do not; every split keeps at least 8 patches (512 pixels) of K
+    p.blocks = ((int64_t)s.N * s.OH * s.OW + PIX - 1) / PIX;
+    // fill the GPU once when the accumulators alone do not; every split keeps at least 8 blocks (512 pixels) of K
     auto splits_for = [&](int64_t groups) {
         const int64_t base = groups * p.tiles_m * p.tiles_n;
-        return std::max<int64_t>(1, std::min<int64_t>(base >= kNumSMs ? 1 : kNumSMs / base, p.patches / 8));
+        return std::max<int64_t>(1, std::min<int64_t>(base >= kNumSMs ? 1 : kNumSMs / base, p.blocks / 8));
     };
     p.splits = (int)splits_for(p.groups);
     p.xb = ((size_t)s.N * s.H * s.W * tcconv::pitch8(s.C) * 2 + 1023) & ~(size_t)1023;
@@ -782,22 +728,20 @@ static Plan plan_for(const ConvShape& s) {
 // channels of 56 x 56 (3 x 3 filter, 18 images).
 bool conv2d_wgrad_tc_supported(const ConvShape& s, const void* x, const void* dy, const void* dw) {
     const int64_t taps = (int64_t)s.KH * s.KW;
-    return s.groups == 1 && s.sh >= 1 && s.sh <= 4 && s.sw >= 1 && s.sw <= 4 && s.N <= 65000 &&
+    return s.groups == 1 && s.sh >= 1 && s.sh <= 4 && s.sw >= 1 && s.sw <= 4 && s.N <= 65000 && tcconv::im2col_fits(s) && (int64_t)s.OH * s.OW < (1LL << 31) &&
            taps * ((s.C + 127) / 128) * ((s.Co + 255) / 256) <= (1 << 20) &&
-           ((uintptr_t)x % 16 == 0) && ((uintptr_t)dy % 16 == 0) && ((uintptr_t)dw % 2 == 0) && tc::encode_fn() != nullptr;
+           ((uintptr_t)x % 16 == 0) && ((uintptr_t)dy % 16 == 0) && ((uintptr_t)dw % 2 == 0) && tc::encode_im2col_fn() != nullptr;
 }
 
 size_t conv2d_wgrad_tc_workspace(const ConvShape& s) {
-    const tcwgrad::Plan p = tcwgrad::plan_for(tcconv::flattened(s));
+    const tcwgrad::Plan p = tcwgrad::plan_for(s);
     return p.xb + p.dyb + p.pb + 1024;
 }
 
-int conv2d_wgrad_tc(const void* x, const void* dy, void* dw, const ConvShape& shape, void* workspace, cudaStream_t st,
+int conv2d_wgrad_tc(const void* x, const void* dy, void* dw, const ConvShape& s, void* workspace, cudaStream_t st,
                     const ConvLayout& lay) {
     using namespace tcwgrad;
-    const ConvShape s = tcconv::flattened(shape);
     const Plan p = plan_for(s);
-    const tcconv::Patches pt = tcconv::patches_of(s);
     unsigned char* ws = (unsigned char*)(((uintptr_t)workspace + 1023) & ~(uintptr_t)1023);
     // channels-last ("acdb") x / dy are what the kernel reads: no copy on that side (lay.y_nhwc describes dy)
     __nv_bfloat16* xt = lay.x_nhwc ? (__nv_bfloat16*)const_cast<void*>(x) : (__nv_bfloat16*)ws;
@@ -819,11 +763,11 @@ int conv2d_wgrad_tc(const void* x, const void* dy, void* dw, const ConvShape& sh
     WgradArgs A;
     A.N = s.N; A.C = s.C; A.H = s.H; A.W = s.W; A.Co = s.Co; A.KH = s.KH; A.KW = s.KW; A.OH = s.OH; A.OW = s.OW;
     A.sh = s.sh; A.sw = s.sw; A.ph = s.ph; A.pw = s.pw; A.dh = s.dh; A.dw = s.dw;
-    A.tiles_h = pt.tiles_h; A.tiles_w = pt.tiles_w; A.pw_log = pt.pw_log;
-    A.patches = p.patches; A.tiles_m = p.tiles_m; A.tiles_n = p.tiles_n; A.splits = p.splits; A.groups = p.groups;
+    A.blocks = p.blocks; A.tiles_m = p.tiles_m; A.tiles_n = p.tiles_n; A.splits = p.splits; A.groups = p.groups;
     CUtensorMap mx, mdy;
-    if (!make_map_nhwc(&mx, xt, s.N, s.H, s.W, s.C, s.sh, s.sw, pt.pw_log) || !make_map_nhwc(&mdy, dyt, s.N, s.OH, s.OW, s.Co, 1, 1, pt.pw_log))
-        return fail(-4, "conv2d_backward_w: cuTensorMapEncodeTiled failed");
+    if (!tcconv::make_map_im2col(&mx, xt, s.N, s.H, s.W, s.C, s.sh, s.sw, s.ph, s.pw, s.dh * (s.KH - 1), s.dw * (s.KW - 1), PIX) ||
+        !tcconv::make_map_im2col(&mdy, dyt, s.N, s.OH, s.OW, s.Co, 1, 1, 0, 0, 0, 0, PIX))
+        return fail(-4, "conv2d_backward_w: cuTensorMapEncodeIm2col failed");
     static std::once_flag once;
     static cudaError_t attr_err = cudaSuccess;
     std::call_once(once, [] {

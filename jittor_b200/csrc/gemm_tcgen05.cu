@@ -316,6 +316,19 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
     return fn;
 }
 
+PFN_cuTensorMapEncodeIm2col_v12000 encode_im2col_fn() {
+    static PFN_cuTensorMapEncodeIm2col_v12000 fn = nullptr;
+    static std::once_flag once;
+    std::call_once(once, [] {
+        void* p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeIm2col", &p, cudaEnableDefault, &q) == cudaSuccess &&
+            q == cudaDriverEntryPointSuccess)
+            fn = (PFN_cuTensorMapEncodeIm2col_v12000)p;
+    });
+    return fn;
+}
+
 // bf16 [batch][rows][cols] with row pitch `pitch`, a {BK, box_rows, 1} box and 128-byte swizzle
 static bool make_map(CUtensorMap* map, const void* base, int64_t batch, int64_t rows, int64_t cols, int64_t pitch, int box_rows) {
     auto fn = encode_fn();

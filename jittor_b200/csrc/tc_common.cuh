@@ -79,14 +79,15 @@ __device__ __forceinline__ void tma_load_tile(void* dst, const CUtensorMap* map,
         asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
                      ::"r"(smem_u32(dst)), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2) : "memory");
 }
+// im2col: the map's count of pixels from (w, h, n) on, in the order w, h, n of the map's bounding box, each shifted by (dw, dh).
 template <int CTAS>
-__device__ __forceinline__ void tma_load_tile(void* dst, const CUtensorMap* map, uint32_t bar, int c0, int c1, int c2, int c3) {
+__device__ __forceinline__ void tma_load_im2col(void* dst, const CUtensorMap* map, uint32_t bar, int c, int w, int h, int n, int dw, int dh) {
     if (CTAS == 2)
-        asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%3, %4, %5, %6}], [%2];"
-                     ::"r"(smem_u32(dst)), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3) : "memory");
+        asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.im2col.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%3, %4, %5, %6}], [%2], {%7, %8};"
+                     ::"r"(smem_u32(dst)), "l"(map), "r"(bar), "r"(c), "r"(w), "r"(h), "r"(n), "h"((uint16_t)dw), "h"((uint16_t)dh) : "memory");
     else
-        asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
-                     ::"r"(smem_u32(dst)), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3) : "memory");
+        asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.im2col.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2], {%7, %8};"
+                     ::"r"(smem_u32(dst)), "l"(map), "r"(bar), "r"(c), "r"(w), "r"(h), "r"(n), "h"((uint16_t)dw), "h"((uint16_t)dh) : "memory");
 }
 template <int CTAS>
 __device__ __forceinline__ void tma_load_tile(void* dst, const CUtensorMap* map, uint32_t bar, int c0, int c1) {
@@ -172,12 +173,8 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* r) {
 }
 
 
-__device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1, int c2, int c3) {
-    asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
-                 ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(c3) : "memory");
-}
-
 PFN_cuTensorMapEncodeTiled_v12000 encode_fn();
+PFN_cuTensorMapEncodeIm2col_v12000 encode_im2col_fn();
 
 // Reads and clears this translation unit's status word (call after synchronising).
 static inline int status_fetch_and_clear() {
