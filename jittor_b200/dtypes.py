@@ -32,9 +32,19 @@ _ALIASES = {"float": "float32", "int": "int32", "double": "float64", "half": "fl
 
 class DType(str):
     """A dtype name that also compares equal to the numpy dtype of the same name and to the reference's short names
-    ("float", "int", "double", "half": python/jittor/src/misc/nano_string.cc aliases)."""
+    ("float", "int", "double", "half": python/jittor/src/misc/nano_string.cc aliases). One object per name, so that comparing
+    two of them is comparing pointers."""
+    _made = {}
+
+    def __new__(cls, name):
+        self = cls._made.get(name)
+        if self is None:
+            self = cls._made[name] = str.__new__(cls, name)
+        return self
 
     def __eq__(self, other):
+        if self is other:
+            return True
         if isinstance(other, str):
             return str.__eq__(self, _ALIASES.get(other, other))
         try:
@@ -43,7 +53,7 @@ class DType(str):
             return False
 
     def __ne__(self, other):
-        return not self.__eq__(other)
+        return self is not other and not self.__eq__(other)
 
     __hash__ = str.__hash__
 
@@ -145,7 +155,18 @@ def unary_dtype_infer(op, x):
     return DType(x)
 
 
+_REDUCE_CACHE = {}
+
+
 def reduce_dtype_infer(op, x):
+    key = (op, str(x), _FLAGS.amp_reg)
+    r = _REDUCE_CACHE.get(key)
+    if r is None:
+        r = _REDUCE_CACHE[key] = _reduce_dtype_infer(op, x)
+    return r
+
+
+def _reduce_dtype_infer(op, x):
     if x == "bool":
         return DType("int32")
     isf = is_float(x) or op in FLOAT_OPS

@@ -112,9 +112,20 @@ def _matmul_record(a, b, trans_b, amp, graph):
     """A 2-D product as a record where the contraction kernels take it (float32 / bfloat16 on both sides), else its graph."""
     if a.dtype != b.dtype or a.dtype not in ("float32", "bfloat16") or amp & dtypes.AMP_PREFER32 or a.is_scalar or b.is_scalar:
         return graph()
-    with flag_scope(amp_reg=amp):
-        dtype = dtypes.reduce_dtype_infer("add", dtypes.binary_dtype_infer("multiply", a.dtype, b.dtype))
-    return relay.matmul(a, b, False, trans_b, dtype, graph)
+    return relay.matmul(a, b, False, trans_b, _product_sum_dtype(a.dtype, b.dtype, False, False, amp), graph)
+
+
+_PRODUCT_SUM = {}
+
+
+def _product_sum_dtype(x, w, xscalar, wscalar, amp):
+    """dtype of sum(x * w) under the flags `amp`."""
+    key = (x, w, xscalar, wscalar, amp)
+    r = _PRODUCT_SUM.get(key)
+    if r is None:
+        with flag_scope(amp_reg=amp):
+            r = _PRODUCT_SUM[key] = dtypes.reduce_dtype_infer("add", dtypes.binary_dtype_infer("multiply", x, w, xscalar, wscalar))
+    return r
 
 
 def matmul(a, b):
@@ -268,8 +279,7 @@ def conv2d(x, weight, bias=None, stride=1, padding=0, dilation=1, groups=1):
     # The four-op graph is written down when something reads it (jt.grad, a consumer's pattern match, the fuser); a plain
     # forward call runs from the relay record alone: the executor would only find the same operands and geometry in the
     # index strings. Shape and dtype are what the graph's own inference gives.
-    with flag_scope(amp_reg=amp):
-        ydt = dtypes.reduce_dtype_infer("add", dtypes.binary_dtype_infer("multiply", x.dtype, weight.dtype, x.is_scalar, weight.is_scalar))
+    ydt = _product_sum_dtype(x.dtype, weight.dtype, x.is_scalar, weight.is_scalar, amp)
     y = V.LazyVar([N, out_channels, oh, ow], ydt, lambda: graph()._op)
     y._relay = ("conv2d", x, weight, stride + padding + dilation, 1)
     if x.dtype in ("float32", "bfloat16") and weight.dtype == x.dtype:
@@ -427,9 +437,9 @@ class LayerNorm(Module):
 
 
 def layer_norm(x, normalized_shape, weight=None, bias=None, eps=1e-5):
-    m = LayerNorm(normalized_shape, eps, weight is not None)
+    m = LayerNorm(normalized_shape, eps, False)
     if weight is not None:
-        m.weight, m.bias = to_var(weight), to_var(bias)
+        m.elementwise_affine, m.weight, m.bias = True, to_var(weight), to_var(bias)
     return m(x)
 
 

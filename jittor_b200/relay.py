@@ -13,6 +13,7 @@ import weakref
 import torch
 
 from . import _capi as C
+from . import dtypes
 from . import var as V
 from .flags import flags, flag_scope
 
@@ -44,7 +45,6 @@ def lazy(shape, dtype, record, build):
 
 def _graph_grad(y, dout, x):
     """d(y . dout) / dx by the per-op rules of y's graph."""
-    from .grad import backprop
     g = backprop(y, dout, [x], through_graph=y)[0]
     return g if g.dtype == x.dtype else g.cast(x.dtype)
 
@@ -56,12 +56,11 @@ def plan(v):
 
 
 def _plan(leaves, run):
-    from .executor import Plan
-    return Plan(leaves, run)
+    return E.Plan(leaves, run)
 
 
 # ------------------------------------------------------------------------------------------------ matmul
-_MM = ("float32", "bfloat16")
+_MM = (dtypes.DType("float32"), dtypes.DType("bfloat16"))
 
 
 def matmul(a, b, ta, tb, dtype, build):
@@ -84,7 +83,6 @@ def matmul(a, b, ta, tb, dtype, build):
 
 
 def _plan_matmul(v, r):
-    from . import executor as E
     _, a, b, ta, tb = r
     return _plan([a, b], lambda: E.run_matmul(a, b, ta, tb, v.dtype))
 
@@ -101,7 +99,6 @@ def conv_vjp(y, x, w, geo):
 
 
 def _plan_conv(v, r):
-    from . import executor as E
     kind, x, w, geo, groups = r
     if x.dtype not in _MM or w.dtype not in _MM:
         return None
@@ -111,19 +108,16 @@ def _plan_conv(v, r):
 
 
 def _plan_conv_dx(v, r):
-    from . import executor as E
     return E.conv_dgrad_plan(v, r[1], r[2], r[3])
 
 
 def _plan_conv_dw(v, r):
-    from . import executor as E
     _, x, dy, geo, wshape = r
     return _plan([x, dy], lambda: E.run_conv2d_backward_w(x, dy, geo, list(wshape), v.dtype))
 
 
 # ------------------------------------------------------------------------------------------------ softmax
 def softmax(x, log, rows, cols, build, backward):
-    from . import executor as E
     if x.dtype not in _MM or rows * cols == 0:
         return None
     if _recognised(("softmax", str(x.dtype), log, x.ndim, rows == 1 and x.ndim > 1, flags._v["amp_reg"]), build, E._match_softmax) != x.dtype:
@@ -196,7 +190,6 @@ MAX_NORM_COLS = 8192        # rows the gradient kernel keeps in registers
 
 def layer_norm(x, weight, bias, eps, k, build):
     """LayerNorm over the last k axes; None if the graph has to be written."""
-    from . import executor as E
     cols = 1
     for s in x._shape[x.ndim - k:]:
         cols *= s
@@ -284,7 +277,6 @@ def ahead(roots):
 def batch_norm(module, x, weight, bias, eps, build):
     """Training BatchNorm of one process; None if the graph has to be written. build() returns (normalised x, batch mean,
     batch variance)."""
-    from . import executor as E
     if x.ndim < 3 or x.dtype not in _MM or x.numel() == 0:
         return None
     cn = x._shape[1]
@@ -316,8 +308,7 @@ def relu_of(x, build):
     r = x._relay
     if r is None or r[0] != "batch_norm" or x._data is not None:
         return None
-    from . import dtypes as dt
-    dtype = dt.binary_dtype_infer("add", x.dtype, "float32", False, True)
+    dtype = dtypes.binary_dtype_infer("add", x.dtype, "float32", False, True)
     if dtype not in _MM:
         return None
     y = lazy(x.shape, dtype, ("batch_norm_relu", x), build)
@@ -353,7 +344,6 @@ def _run_bn_stats(xd):
 
 
 def _plan_batch_norm(v, r):
-    from . import executor as E
     root = v if r[0] == "batch_norm" else r[1]
     _, x, g, b, eps, stats = root._relay
     return E.batch_norm_plan(v, x, ("var", g) if g is not None else ("const", 1.0), ("var", b) if b is not None else ("const", 0.0),
@@ -395,3 +385,6 @@ _PLANS = {"matmul": _plan_matmul, "conv2d": _plan_conv, "conv2d_transpose": _pla
           "softmax": _plan_softmax, "mean_pool_dx": _plan_mean_pool_dx, "layer_norm": _plan_layer_norm, "layer_norm_dx": _plan_layer_norm_dx,
           "layer_norm_params": _plan_layer_norm_params, "part": _plan_part, "batch_norm": _plan_batch_norm,
           "batch_norm_relu": _plan_batch_norm, "batch_norm_sums": _plan_bn_sums, "batch_norm_dx": _plan_bn_dx}
+
+from . import executor as E             # noqa: E402  (imports this module)
+from .grad import backprop              # noqa: E402
