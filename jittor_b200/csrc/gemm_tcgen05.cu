@@ -16,6 +16,7 @@
 #include "tc_common.cuh"
 
 #include <algorithm>
+#include <cstring>
 #include <mutex>
 
 namespace b200jt {
@@ -380,7 +381,7 @@ struct Plan { bool pair; int mt, bn, splits; double ns; };
 // Tile and split by estimated time. A k-block costs the larger of its MMAs (11 TFLOP/s per SM) and its operands' way from L2
 // (about 110 B per ns and SM); a tile adds its epilogue where no second accumulator hides it; split K adds the way of the partial
 // sums out and back and a second launch.
-static Plan plan_for(int64_t batch, int64_t M, int64_t N, int64_t K, bool bmn, bool may_split) {
+static Plan estimate(int64_t batch, int64_t M, int64_t N, int64_t K, bool bmn, bool may_split) {
     Plan best{false, 1, MAX_BN, 1, 1e30};
     const int64_t kb = (K + BK - 1) / BK;
     const int pslots = pair_slots();
@@ -417,6 +418,20 @@ static Plan plan_for(int64_t batch, int64_t M, int64_t N, int64_t K, bool bmn, b
         }
     }
     return best;
+}
+
+// The estimate runs over some 70 candidates (1.5 us): each thread keeps its last 64 plans.
+static Plan plan_for(int64_t batch, int64_t M, int64_t N, int64_t K, bool bmn, bool may_split) {
+    if (getenv("B200JT_GEMM_PAIR") || getenv("B200JT_GEMM_MT") || getenv("B200JT_GEMM_BN") || getenv("B200JT_GEMM_SPLITS"))
+        return estimate(batch, M, N, K, bmn, may_split);
+    struct Entry { int64_t key[5] = {-1, 0, 0, 0, 0}; Plan p; };
+    static thread_local Entry kept[64];
+    const int64_t key[5] = {batch, M, N, K, (int64_t)bmn * 2 + may_split};
+    uint64_t h = 0;
+    for (int64_t k : key) h = (h ^ (uint64_t)k) * 0x9E3779B97F4A7C15ull;
+    Entry& e = kept[h >> 58];
+    if (memcmp(e.key, key, sizeof(key)) != 0) { e.p = estimate(batch, M, N, K, bmn, may_split); memcpy(e.key, key, sizeof(key)); }
+    return e.p;
 }
 
 static int launch(const Plan& p, const void* a, const void* b, void* c, float* part, int64_t batch, int64_t a_batch, int64_t b_batch,
