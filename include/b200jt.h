@@ -290,9 +290,13 @@ int b200jt_conv2d_formats(const b200jt_tensor* x, const b200jt_tensor* w, const 
 int b200jt_conv2d_transpose(const b200jt_tensor* x, const b200jt_tensor* w, const b200jt_tensor* y,
                             int stride_h, int stride_w, int pad_h, int pad_w, int dil_h, int dil_w, int groups, void* stream);
 
-/* y[n,c,h,w] = x[n,c,h/sh,w/sw] where sh divides h and sw divides w (and the quotients are inside x), zero elsewhere; bfloat16.
- * The convolution that gives a strided convolution's input gradient reads dy in this form. */
-int b200jt_spread2d(const b200jt_tensor* x, const b200jt_tensor* y, int stride_h, int stride_w, void* stream);
+/* dx of y = conv2d(x, w) (groups == 1) for bfloat16 on the tensor cores; w is the forward filter [Cout, Cin, KH, KW]. The
+ * workspace query returns 0 for what this entry does not take (b200jt_conv2d_transpose takes everything). */
+size_t b200jt_conv2d_backward_x_workspace(const b200jt_tensor* dy, const b200jt_tensor* w, const b200jt_tensor* dx,
+                                          int stride_h, int stride_w, int pad_h, int pad_w, int dil_h, int dil_w);
+int b200jt_conv2d_backward_x(const b200jt_tensor* dy, const b200jt_tensor* w, const b200jt_tensor* dx,
+                             int stride_h, int stride_w, int pad_h, int pad_w, int dil_h, int dil_w,
+                             void* workspace, size_t workspace_bytes, void* stream);
 
 /* dw[o,c,kh,kw] = sum over (n,oh,ow) of dy[n,o,oh,ow] * x[n,c,oh*stride-pad+kh*dil, ...]: the weight gradient of conv2d
  * (groups == 1), fp32 accumulation. Replaces the relay CudnnConvBackwardWOp(Var* x, Var* y, int kh, int kw, int strideh, ...),

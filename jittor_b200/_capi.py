@@ -109,7 +109,8 @@ SIGNATURES = [
     ("b200jt_bn_apply", _i, [_TP, _FP, _d, _FP, _FP, _d, _i, _TP, _FP, _FP, _d, _vp]),
     ("b200jt_pool2d", _i, [_TP, _TP, _vp, ctypes.c_char_p, _i, _i, _i, _i, _i, _i, _i, _vp]),
     ("b200jt_pool2d_backward", _i, [_TP, _TP, _TP, _TP, ctypes.c_char_p, _i, _i, _i, _i, _i, _i, _i, _vp]),
-    ("b200jt_spread2d", _i, [_TP, _TP, _i, _i, _vp]),
+    ("b200jt_conv2d_backward_x_workspace", _sz, [_TP, _TP, _TP, _i, _i, _i, _i, _i, _i]),
+    ("b200jt_conv2d_backward_x", _i, [_TP, _TP, _TP, _i, _i, _i, _i, _i, _i, _vp, _sz, _vp]),
     ("b200jt_pool2d_taps", _i, [_TP, _TP, _vp, ctypes.c_char_p, _i, _i, _i, _i, _i, _i, _vp]),
     ("b200jt_pool2d_backward_taps", _i, [_vp, _TP, _TP, _i, _i, _i, _i, _i, _i, _vp]),
     ("b200jt_pool2d_backward_indices", _i, [_TP, _TP, _vp, _TP, _TP, _i, _i, _i, _i, _i, _i, _vp]),

@@ -132,7 +132,8 @@ extern "C" size_t b200jt_conv2d_formats_workspace(const b200jt_tensor* x, const 
     b200jt_tensor xl, wl, yl; ConvLayout lay; ConvShape s;
     if (conv_formats(x, w, y, xformat, wformat, yformat, &xl, &wl, &yl, &lay)) return 0;
     if (conv_shape(&xl, &wl, &yl, sh, sw, ph, pw, dh, dw, 1, &s)) return 0;
-    if (x->dtype == B200JT_BFLOAT16 && conv2d_tc_supported(s, x->ptr, w->ptr, y->ptr) && formats_run_here(lay, conv2d_tc_layout_supported(s))) return conv2d_tc_workspace(s);
+    if (x->dtype == B200JT_BFLOAT16 && conv2d_tc_supported(s, x->ptr, w->ptr, y->ptr) &&
+        formats_run_here(lay, conv2d_tc_layout_supported(s))) return conv2d_tc_workspace(s);
     return 0;
 }
 
@@ -149,7 +150,7 @@ extern "C" int b200jt_conv2d_formats(const b200jt_tensor* x, const b200jt_tensor
     if (rc) return rc;
     if (numel(y) == 0) return 0;
     if (!(x->dtype == B200JT_BFLOAT16 && conv2d_tc_supported(s, x->ptr, w->ptr, y->ptr) && conv2d_tc_layout_supported(s) &&
-          ((uintptr_t)y->ptr % 16 == 0)))
+          (uintptr_t)x->ptr % 16 == 0 && (uintptr_t)y->ptr % 16 == 0))
         return fail(-5, "b200jt_conv2d_formats: acdb / ohwi layouts run on the tensor-core kernel only (bfloat16, in channels a "
                         "multiple of 8 and >= 64, out channels >= 64, at least 1024 output pixels, 16-byte aligned tensors)");
     const size_t need = conv2d_tc_workspace(s);
@@ -188,7 +189,7 @@ extern "C" int b200jt_conv2d_backward_w_formats(const b200jt_tensor* x, const b2
     if (rc) return rc;
     if (numel(dw) == 0) return 0;
     if (!(x->dtype == B200JT_BFLOAT16 && conv2d_wgrad_tc_supported(s, x->ptr, dy->ptr, dw->ptr) &&
-          conv2d_wgrad_tc_layout_supported(s)))
+          conv2d_wgrad_tc_layout_supported(s) && (uintptr_t)x->ptr % 16 == 0 && (uintptr_t)dy->ptr % 16 == 0))
         return fail(-5, "b200jt_conv2d_backward_w_formats: acdb / ohwi layouts run on the tensor-core kernel only (bfloat16, in and "
                         "out channels multiples of 8 and >= 64, outputs of at least 8 x 8 per image and 4096 pixels in all, "
                         "16-byte aligned x and dy)");
@@ -279,17 +280,51 @@ spread2d_kernel(const uint16_t* __restrict__ x, uint16_t* __restrict__ y, int64_
     }
 }
 
-extern "C" int b200jt_spread2d(const b200jt_tensor* x, const b200jt_tensor* y, int sh, int sw, void* stream) {
-    B200JT_CHECK_ARG(valid_tensor(x) && valid_tensor(y) && x->ndim == 4 && y->ndim == 4, "spread2d takes NCHW tensors");
-    B200JT_CHECK_ARG(x->dtype == B200JT_BFLOAT16 && y->dtype == B200JT_BFLOAT16, "spread2d takes bfloat16 tensors");
-    B200JT_CHECK_ARG(sh > 0 && sw > 0 && x->shape[0] == y->shape[0] && x->shape[1] == y->shape[1], "spread2d: bad strides or shapes");
-    if (numel(y) == 0) return 0;
-    const int64_t rows = y->shape[0] * y->shape[1] * y->shape[2], work = rows * ((y->shape[3] + 7) / 8);
-    const int vec = y->shape[3] % 8 == 0 && (uintptr_t)y->ptr % 16 == 0;
-    spread2d_kernel<<<grid_for(work, 256), 256, 0, (cudaStream_t)stream>>>((const uint16_t*)x->ptr, (uint16_t*)y->ptr, rows, (int)x->shape[2],
-                                                                         (int)x->shape[3], (int)y->shape[2], (int)y->shape[3], sh, sw, vec);
-    B200JT_LAUNCH_CHECK();
-    return 0;
+// dx of y = conv2d(x, w) as a convolution of dy: filter of output channels x input channels with the taps reversed, stride 1, the
+// padding that is left of the filter's reach, over dy with stride - 1 zeros between its pixels. That multiplies stride_h * stride_w
+// times as much, on the tensor cores: 136 x 208 x 4 x 4 -> 32 x 7 x 7 (3 x 3, stride 2) took 280 us as a gather on the CUDA cores.
+static bool backward_x_shape(const b200jt_tensor* dy, const b200jt_tensor* w, const b200jt_tensor* dx, int sh, int sw, int ph, int pw, int dh, int dw,
+                             ConvShape* s, size_t* spread) {
+    ConvShape f;
+    if (conv_shape(dx, w, dy, sh, sw, ph, pw, dh, dw, 1, &f) || dy->dtype != B200JT_BFLOAT16 || numel(dy) == 0 || numel(dx) == 0) return false;
+    const int64_t reach_h = (int64_t)dh * (f.KH - 1), reach_w = (int64_t)dw * (f.KW - 1);
+    if (reach_h < ph || reach_w < pw || sh > 4 || sw > 4) return false;
+    *s = f;
+    s->C = f.Co; s->Co = f.C; s->OH = f.H; s->OW = f.W; s->sh = s->sw = 1;
+    s->ph = (int)reach_h - ph; s->pw = (int)reach_w - pw;
+    s->H = f.H - 2 * s->ph + (int)reach_h; s->W = f.W - 2 * s->pw + (int)reach_w;       // dy with its zeros
+    const bool strided = sh > 1 || sw > 1;
+    *spread = strided ? ((size_t)s->N * s->C * s->H * s->W * 2 + 1023) / 1024 * 1024 + 1024 : 0;
+    return s->H > 0 && s->W > 0 && (strided || (s->H == f.OH && s->W == f.OW)) && conv2d_tc_supported(*s, strided ? nullptr : dy->ptr, w->ptr, dx->ptr);
+}
+
+extern "C" size_t b200jt_conv2d_backward_x_workspace(const b200jt_tensor* dy, const b200jt_tensor* w, const b200jt_tensor* dx,
+                                                     int sh, int sw, int ph, int pw, int dh, int dw) {
+    ConvShape s; size_t spread;
+    return backward_x_shape(dy, w, dx, sh, sw, ph, pw, dh, dw, &s, &spread) ? spread + conv2d_tc_workspace(s) : 0;
+}
+
+extern "C" int b200jt_conv2d_backward_x(const b200jt_tensor* dy, const b200jt_tensor* w, const b200jt_tensor* dx,
+                                        int sh, int sw, int ph, int pw, int dh, int dw, void* workspace, size_t workspace_bytes, void* stream) {
+    ConvShape s; size_t spread;
+    if (!backward_x_shape(dy, w, dx, sh, sw, ph, pw, dh, dw, &s, &spread))
+        return fail(-5, "b200jt_conv2d_backward_x: runs on the tensor-core kernel only (bfloat16, padding within the filter's reach, strides up to 4)");
+    const size_t need = spread + conv2d_tc_workspace(s);
+    B200JT_CHECK_ARG(workspace_bytes >= need && workspace, "workspace too small: need " + std::to_string(need) + " bytes");
+    cudaStream_t st = (cudaStream_t)stream;
+    const void* src = dy->ptr;
+    if (spread) {
+        uint16_t* z = (uint16_t*)(((uintptr_t)workspace + 1023) & ~(uintptr_t)1023);
+        const int64_t rows = (int64_t)s.N * s.C * s.H;
+        spread2d_kernel<<<grid_for(rows * ((s.W + 7) / 8), 256), 256, 0, st>>>((const uint16_t*)dy->ptr, z, rows, (int)dy->shape[2], (int)dy->shape[3],
+                                                                             s.H, s.W, sh, sw, s.W % 8 == 0);
+        B200JT_LAUNCH_CHECK();
+        src = z;
+    }
+    ConvLayout lay;
+    lay.w_grad = true;
+    const int rc = conv2d_tc(src, w->ptr, dx->ptr, nullptr, s, (char*)workspace + spread, st, lay);
+    return rc == 1 ? 0 : rc;
 }
 
 extern "C" int b200jt_conv2d_backward_w(const b200jt_tensor* x, const b200jt_tensor* dy, const b200jt_tensor* dw,

@@ -285,12 +285,14 @@ conv_bf16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
 // at a time (256 x 256 x 56 x 56: 126 us, 6.5 TB/s; 128 bytes at a time 169 us, 64 bytes 194 us). The tile is kept as 32-bit pairs,
 // word w of row r at w ^ (r / 8) ^ (r % 4), which spreads both the rows of the first phase and the columns of the second over all banks.
 // Block (0,0,0) also zeroes `zero[0..n_zero)`. The first wz slices (blockIdx.z < wz) of the same grid re-order the weights
-// instead (w[Co][C][taps] -> wt[taps][Co][wpitch]), so that both layout passes of a convolution are one launch.
+// instead (w -> wt[taps][Co][wpitch]; w_mode 0: w[Co][C][taps], 1: w[Co][taps][C], 2: w[C][Co][taps] with the taps reversed, the
+// filter of the input gradient), the next a.n slices are a's images and the rest b's: the layout passes of a convolution, of its
+// input gradient and of its weight gradient are one launch each.
+struct LayoutJob { const __nv_bfloat16* in = nullptr; __nv_bfloat16* out = nullptr; int R = 0, Cn = 0, pitch = 0, n = 0; };
 template <int TR>
 __global__ void __launch_bounds__(256)
-transpose_bf16_batched_kernel(const __nv_bfloat16* __restrict__ in, __nv_bfloat16* __restrict__ out, int R, int Cn, int pitch, int wz,
-                              const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ wt, int Co, int C, int taps, int wpitch,
-                              float* __restrict__ zero, int n_zero, int w_ohwi) {
+transpose_bf16_batched_kernel(const __grid_constant__ LayoutJob a, const __grid_constant__ LayoutJob b, int wz, const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ wt, int Co, int C, int taps, int wpitch,
+                              float* __restrict__ zero, int n_zero, int w_mode) {
     __shared__ uint32_t tile[TR][32];
     if (zero && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0)       // the statistics the conv epilogue adds into
         for (int i = threadIdx.x; i < n_zero; i += blockDim.x) zero[i] = 0.f;
@@ -301,15 +303,23 @@ transpose_bf16_batched_kernel(const __nv_bfloat16* __restrict__ in, __nv_bfloat1
         for (int64_t i = blk * blockDim.x + threadIdx.x; i < n; i += nblk * blockDim.x) {
             const int c = (int)(i % C); const int64_t t2 = i / C;
             const int co = (int)(t2 % Co); const int tap = (int)(t2 / Co);
-            wt[t2 * wpitch + c] = w_ohwi ? w[((int64_t)co * taps + tap) * C + c] : w[((int64_t)co * C + c) * taps + tap];
+            wt[t2 * wpitch + c] = w[w_mode == 0 ? ((int64_t)co * C + c) * taps + tap : w_mode == 1 ? ((int64_t)co * taps + tap) * C + c
+                                                : ((int64_t)c * Co + co) * taps + (taps - 1 - tap)];
         }
         return;
     }
-    const int64_t boff = (int64_t)((int)blockIdx.z - wz) * R * Cn;
-    out += (int64_t)((int)blockIdx.z - wz) * pitch * Cn;
+    const int slice = (int)blockIdx.z - wz;
+    const bool second = slice >= a.n;
+    const LayoutJob& job = second ? b : a;
+    const int64_t image = second ? slice - a.n : slice;
+    const int R = job.R, Cn = job.Cn, pitch = job.pitch;
     const int r0 = blockIdx.y * TR, c0 = blockIdx.x * 64;
+    if (r0 >= R || c0 >= Cn) return;
+    const __nv_bfloat16* __restrict__ in = job.in;
+    const int64_t boff = image * R * Cn;
+    __nv_bfloat16* __restrict__ out = job.out + image * pitch * Cn;
     const int j = threadIdx.x & 7, i = threadIdx.x >> 3;          // 8 chunks of 8 elements x 32 rows
-    const bool vec_in = (Cn % 8 == 0);
+    const bool vec_in = Cn % 8 == 0 && ((uintptr_t)in & 15) == 0;
     uint4 v[TR / 32];
 #pragma unroll
     for (int p = 0; p < TR / 32; p++) {
@@ -420,7 +430,7 @@ static int pair_slots() {
 // 304 -> 48 channels of 56 x 56, 18 images: 1.98 ms on the CUDA cores; 40 -> 27 channels of 7 x 7, 218 images: 106 us.
 bool conv2d_tc_supported(const ConvShape& s, const void* x, const void* w, const void* y) {
     const int64_t px = (int64_t)s.N * s.OH * s.OW;
-    return s.sh >= 1 && s.sh <= 4 && s.sw >= 1 && s.sw <= 4 && px >= 16 && s.C >= 8 && tcconv::im2col_fits(s) && ((uintptr_t)x % 16 == 0) &&
+    return s.sh >= 1 && s.sh <= 4 && s.sw >= 1 && s.sw <= 4 && px >= 16 && s.C >= 8 && tcconv::im2col_fits(s) && ((uintptr_t)x % 2 == 0) &&
            ((uintptr_t)w % 2 == 0) && ((uintptr_t)y % 2 == 0) && (int64_t)s.Co * s.KH * s.KW < (1LL << 31) && s.N <= 65000 &&
            (int64_t)s.OH * s.OW < (1LL << 31) && px / 128 * ((s.Co + 63) / 64) < (1LL << 30) && tc::encode_fn() != nullptr && tc::encode_im2col_fn() != nullptr;
 }
@@ -452,14 +462,15 @@ int conv2d_tc(const void* x, const void* w, void* y, float* stats, const ConvSha
     const int HW = s.H * s.W;
     {   // x[N][C][HW] -> xt[N][HW][C], and the weights tap-major, in one launch
         const int64_t nw = (int64_t)s.Co * s.C * s.KH * s.KW;
+        const LayoutJob job{(const __nv_bfloat16*)x, xt, s.C, HW, cp, lay.x_nhwc ? 0 : s.N};
         const unsigned gx = (unsigned)((HW + 63) / 64), gy = (unsigned)((s.C + layout_rows(s.C) - 1) / layout_rows(s.C));
         const int64_t per_slice = (int64_t)gx * gy * 256;
         const unsigned wz = (unsigned)std::min<int64_t>(32, std::max<int64_t>(1, (nw + per_slice - 1) / per_slice));
-        dim3 g(gx, gy, (lay.x_nhwc ? 0u : (unsigned)s.N) + wz);          // the first wz slices re-order the weights
+        dim3 g(gx, gy, (unsigned)job.n + wz);          // the first wz slices re-order the weights
         float* zero = (stats && s.Co <= STATS_MAX_CO) ? stats : nullptr;   // zeroed here instead of by a memset node
         const auto kernel = layout_rows(s.C) == 128 ? transpose_bf16_batched_kernel<128> : transpose_bf16_batched_kernel<64>;
-        kernel<<<g, 256, 0, st>>>((const __nv_bfloat16*)x, xt, s.C, HW, cp, (int)wz,
-                                                          (const __nv_bfloat16*)w, wt, s.Co, s.C, s.KH * s.KW, cp, zero, 2 * s.Co, lay.w_ohwi ? 1 : 0);
+        kernel<<<g, 256, 0, st>>>(job, LayoutJob(), (int)wz, (const __nv_bfloat16*)w, wt, s.Co, s.C, s.KH * s.KW, cp, zero, 2 * s.Co,
+                                  lay.w_grad ? 2 : lay.w_ohwi ? 1 : 0);
         B200JT_LAUNCH_CHECK();
     }
     ConvArgs A;
@@ -730,7 +741,7 @@ bool conv2d_wgrad_tc_supported(const ConvShape& s, const void* x, const void* dy
     const int64_t taps = (int64_t)s.KH * s.KW;
     return s.groups == 1 && s.sh >= 1 && s.sh <= 4 && s.sw >= 1 && s.sw <= 4 && s.N <= 65000 && tcconv::im2col_fits(s) && (int64_t)s.OH * s.OW < (1LL << 31) &&
            taps * ((s.C + 127) / 128) * ((s.Co + 255) / 256) <= (1 << 20) &&
-           ((uintptr_t)x % 16 == 0) && ((uintptr_t)dy % 16 == 0) && ((uintptr_t)dw % 2 == 0) && tc::encode_im2col_fn() != nullptr;
+           ((uintptr_t)x % 2 == 0) && ((uintptr_t)dy % 2 == 0) && ((uintptr_t)dw % 2 == 0) && tc::encode_im2col_fn() != nullptr;
 }
 
 size_t conv2d_wgrad_tc_workspace(const ConvShape& s) {
@@ -748,17 +759,21 @@ int conv2d_wgrad_tc(const void* x, const void* dy, void* dw, const ConvShape& s,
     __nv_bfloat16* dyt = lay.y_nhwc ? (__nv_bfloat16*)const_cast<void*>(dy) : (__nv_bfloat16*)(ws + p.xb);
     float* part = (float*)(ws + p.xb + p.dyb);
     const int HW = s.H * s.W, OHW = s.OH * s.OW;
-    if (!lay.x_nhwc) {   // x[N][C][HW] -> [N][HW][C]
-        dim3 gx((unsigned)((HW + 63) / 64), (unsigned)((s.C + tcconv::layout_rows(s.C) - 1) / tcconv::layout_rows(s.C)), (unsigned)s.N);
-        const auto kernel = tcconv::layout_rows(s.C) == 128 ? tcconv::transpose_bf16_batched_kernel<128> : tcconv::transpose_bf16_batched_kernel<64>;
-        kernel<<<gx, 256, 0, st>>>((const __nv_bfloat16*)x, xt, s.C, HW, tcconv::pitch8(s.C), 0, nullptr, nullptr, 0, 0, 0, 0, nullptr, 0, 0);
-        B200JT_LAUNCH_CHECK();
-    }
-    if (!lay.y_nhwc) {   // dy[N][Co][OH*OW] -> [N][OH*OW][Co]
-        dim3 gy((unsigned)((OHW + 63) / 64), (unsigned)((s.Co + tcconv::layout_rows(s.Co) - 1) / tcconv::layout_rows(s.Co)), (unsigned)s.N);
-        const auto kernel = tcconv::layout_rows(s.Co) == 128 ? tcconv::transpose_bf16_batched_kernel<128> : tcconv::transpose_bf16_batched_kernel<64>;
-        kernel<<<gy, 256, 0, st>>>((const __nv_bfloat16*)dy, dyt, s.Co, OHW, tcconv::pitch8(s.Co), 0, nullptr, nullptr, 0, 0, 0, 0, nullptr, 0, 0);
-        B200JT_LAUNCH_CHECK();
+    {   // x[N][C][HW] -> [N][HW][C] and dy[N][Co][OH*OW] -> [N][OH*OW][Co]
+        using tcconv::LayoutJob; using tcconv::layout_rows; using tcconv::pitch8;
+        const LayoutJob jobs[2] = {{(const __nv_bfloat16*)x, xt, s.C, HW, pitch8(s.C), lay.x_nhwc ? 0 : s.N},
+                                   {(const __nv_bfloat16*)dy, dyt, s.Co, OHW, pitch8(s.Co), lay.y_nhwc ? 0 : s.N}};
+        const bool together = s.N <= 32000;                      // grid z
+        for (int q = 0; q < (together ? 1 : 2); q++) {
+            const LayoutJob a = jobs[q], b = together ? jobs[1] : LayoutJob();
+            if (a.n + b.n == 0) continue;
+            const int rows = std::max(a.n ? layout_rows(a.R) : 64, b.n ? layout_rows(b.R) : 64);
+            const int r = std::max(a.n ? a.R : 0, b.n ? b.R : 0), cols = std::max(a.n ? a.Cn : 0, b.n ? b.Cn : 0);
+            const dim3 g((unsigned)((cols + 63) / 64), (unsigned)((r + rows - 1) / rows), (unsigned)(a.n + b.n));
+            const auto kernel = rows == 128 ? tcconv::transpose_bf16_batched_kernel<128> : tcconv::transpose_bf16_batched_kernel<64>;
+            kernel<<<g, 256, 0, st>>>(a, b, 0, nullptr, nullptr, 0, 0, 0, 0, nullptr, 0, 0);
+            B200JT_LAUNCH_CHECK();
+        }
     }
     WgradArgs A;
     A.N = s.N; A.C = s.C; A.H = s.H; A.W = s.W; A.Co = s.Co; A.KH = s.KH; A.KW = s.KW; A.OH = s.OH; A.OW = s.OW;

@@ -9,7 +9,7 @@ struct ConvShape {
     int groups = 1;
 };
 // Memory layouts other than the default NCHW / OIHW (tensor-core path only): x and y as NHWC ("acdb"), w as OHWI ("ohwi").
-struct ConvLayout { bool x_nhwc = false, w_ohwi = false, y_nhwc = false; };
+struct ConvLayout { bool x_nhwc = false, w_ohwi = false, y_nhwc = false, w_grad = false; };     // w_grad: w[C][Co][taps], taps from the last
 
 int matmul_simt(const void* a, const void* b, void* c, int dtype, int64_t M, int64_t N, int64_t K,
                 bool trans_a, bool trans_b, cudaStream_t st);

@@ -431,6 +431,7 @@ def _match_conv_dgrad(v):
 
 
 def conv_dgrad_plan(v, dy, w, geo):
+    """The plan of a graph that was matched: stride-1 bf16 as the convolution it is with flipped, transposed weights."""
     Co, Ci, KH, KW = w.shape
     sh, sw, ph, pw, dh, dw = geo
     fp, fq = dh * (KH - 1) - ph, dw * (KW - 1) - pw
@@ -438,19 +439,22 @@ def conv_dgrad_plan(v, dy, w, geo):
         from . import var as V
         wf = V.reindex(w, [Ci, Co, KH, KW], ["i1", "i0", f"{KH - 1}-i2", f"{KW - 1}-i3"])
         return Plan([dy, wf], lambda: run_conv2d(dy, wf, (1, 1, fp, fq, dh, dw), v.dtype))
-    if fp >= 0 and fq >= 0 and dy.dtype == "bfloat16" and Co >= 8 and max(sh, sw) <= 4:
-        # Strided: the same convolution over dy with sh - 1, sw - 1 zeros between its pixels. It multiplies sh * sw times as much,
-        # on the tensor cores: 136 x 208 x 4 x 4 -> 32 x 7 x 7 (3 x 3) took 280 us as a gather on the CUDA cores.
-        from . import var as V
-        H, W = v.shape[2] - 2 * fp + dh * (KH - 1), v.shape[3] - 2 * fq + dw * (KW - 1)
-        wf = V.reindex(w, [Ci, Co, KH, KW], ["i1", "i0", f"{KH - 1}-i2", f"{KW - 1}-i3"])
+    return conv_dx_plan(v, dy, w, geo)
 
-        def run():
-            spread = _empty([dy.shape[0], Co, H, W], "bfloat16")
-            C.call("b200jt_spread2d", C.desc(dy._data.view(list(dy.shape))), C.desc(spread), sh, sw)
-            return _conv2d(spread, _cast(wf._data, "bfloat16"), (1, 1, fp, fq, dh, dw), v.dtype)
-        return Plan([dy, wf], run)
-    return Plan([dy, w], lambda: run_conv2d_transpose(dy, w, geo, 1, list(v.shape), v.dtype))
+
+def conv_dx_plan(v, dy, w, geo):
+    """bf16 in one call on the tensor cores (any stride up to 4); what that does not take as the transposed convolution."""
+    def run():
+        if dy.dtype == "bfloat16":
+            out = _empty(list(v.shape), "bfloat16")
+            args = (C.desc(dy._data.view(list(dy.shape))), C.desc(_cast(w._data, "bfloat16")), C.desc(out), *geo)
+            nbytes, wsp, ws = C.workspace("b200jt_conv2d_backward_x_workspace", *args)
+            if nbytes:
+                C.call("b200jt_conv2d_backward_x", *args, wsp, nbytes,
+                       what=lambda: f"conv2d_backward_x dy{list(dy.shape)} w{list(w.shape)} geo{geo}")
+                return _cast(out, v.dtype)
+        return run_conv2d_transpose(dy, w, geo, 1, list(v.shape), v.dtype)
+    return Plan([dy, w], run)
 
 
 def _match_conv_wgrad(v):
@@ -569,11 +573,8 @@ def run_conv2d_transpose(x, w, geo, groups, out_shape, out_dtype):
 
 
 def run_conv2d(x, w, geo, out_dtype, stats=None, groups=1):
-    return _conv2d(x._data, _cast(w._data, x.dtype), geo, out_dtype, stats, groups)
-
-
-def _conv2d(xd, wd, geo, out_dtype, stats=None, groups=1):
     sh, sw, ph, pw, dh, dw = geo
+    xd, wd = x._data, _cast(w._data, x.dtype)
     N, Ci, H, W = xd.shape
     Co, _, KH, KW = wd.shape
     OH = (H + 2 * ph - KH * dh + dh - 1) // sh + 1

@@ -108,7 +108,7 @@ def _plan_conv(v, r):
 
 
 def _plan_conv_dx(v, r):
-    return E.conv_dgrad_plan(v, r[1], r[2], r[3])
+    return E.conv_dx_plan(v, r[1], r[2], r[3])
 
 
 def _plan_conv_dw(v, r):

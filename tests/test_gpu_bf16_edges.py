@@ -43,6 +43,7 @@ def test_convolution_and_weight_gradient(n, ci, h, w, co, k, s, p, d, bn, pair, 
     dy = torch.randn(*want.shape, device="cuda").bfloat16()
     want.backward(dy.double())
     dw = torch.full(list(wt.shape), float("nan"), device="cuda").bfloat16()
+    dy = torch.cat([dy.flatten()[:1], dy.flatten()])[1:].view_as(dy)               # 2-byte aligned
     args = (C.desc(x), C.desc(dy), C.desc(dw), *geo)
     size, ptr, ws = C.workspace("b200jt_conv2d_backward_w_workspace", *args)
     C.call("b200jt_conv2d_backward_w_tc", *args, ptr, size)
