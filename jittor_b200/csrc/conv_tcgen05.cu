@@ -58,11 +58,10 @@ __device__ __forceinline__ int first_block(int tm, int k_blocks) { return (int)(
 // NHWC ("acdb"): a lane stores the 32 consecutive channels of its pixel as four 16-byte vectors.
 // BN_T: output channels per tile (256, or less where that fills the last wave of the persistent grid better).
 // The epilogue's eight warps are two per TMEM lane quadrant, each with every other 32 channels: four warps took longer than the
-// main loop of a 1 x 1 layer (64 x 64 x 56 x 56 -> 256 channels with
-// statistics, layout pass included: 142 us with four warps and box stores, 87 us now).
+// main loop of a 1 x 1 layer (64 x 64 x 56 x 56 -> 256 channels with statistics, layout pass included: 142 us with four warps and
+// box stores, 87 us now).
 // Each tile walks K from a start of its own. All tiles read the same weights: in step with one another they queue at the L2
-// slices that hold the current 32 KB (7 x 432 x 28 x 28 -> 320 channels, 3 x 3: 60 us
-// in step, 54 us this way).
+// slices that hold the current 32 KB (7 x 432 x 28 x 28 -> 320 channels, 3 x 3: 60 us in step, 54 us this way).
 template <bool NHWC, int BN_T, bool PAIR>
 __global__ void __launch_bounds__(THREADS, 1)
 conv_bf16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,

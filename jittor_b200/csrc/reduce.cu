@@ -116,7 +116,7 @@ reduce_row_kernel(const void* __restrict__ x, int xdt, void* __restrict__ out, i
         if (A.nr == 2 && inner < 4 * (int64_t)blockDim.x) {
             // Short runs of contiguous elements (a mean over batch, rows and columns of small images): a sweep per run would
             // leave most threads idle and wait for memory run by run, so the threads stride the flattened space instead, eight
-            // loads in flight. 202 runs of 49 for each of 150 outputs: 244 us by sweeps, REDAFTER us.
+            // loads in flight. 202 runs of 49 for each of 150 outputs: 244 us by sweeps, 11 us this way.
             const uint32_t in = (uint32_t)inner, dq = blockDim.x / in, dr = blockDim.x - dq * in;
             const int64_t ostride = A.rstride[0];
             r += threadIdx.x;
