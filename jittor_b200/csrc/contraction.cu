@@ -1,6 +1,6 @@
 // C entry points of the two contraction relays (matmul, conv2d): argument checks and the choice
-// between the tcgen05 tensor-core kernels (bfloat16, tile-aligned shapes) and the CUDA-core kernels
-// (float32, or shapes the tensor-core tiles do not cover).
+// between the tcgen05 tensor-core kernels (bfloat16), the float32 kernel and the older CUDA-core kernels (groups, tiny
+// bfloat16 problems, operands at odd addresses).
 #include "gemm_simt.cuh"
 
 using namespace b200jt;

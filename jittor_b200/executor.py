@@ -501,8 +501,8 @@ def _wgrad_as_conv(xd, dyd, geo, w_shape):
     x[n,c,oh*s-p+kh*d, ...] IS a convolution of x with the batch and channel axes exchanged (images = in channels, channels =
     batch) by dy with its two leading axes exchanged as the filter (out channels = o, in channels = n, an OH x OW window),
     with the roles of stride and dilation exchanged; its [C, Co, KH, KW] result only needs its leading axes swapped back.
-    cuDNN has a dedicated kernel for this (cudnn_conv_backward_w_op.cc:292); here the forward kernel serves, at the price of
-    8x8 output patches of which KH x KW pixels are real. Returns None when the shapes miss the tensor-core path."""
+    cuDNN has a dedicated kernel for this (cudnn_conv_backward_w_op.cc:292); here the forward kernel serves
+    where the dedicated one does not. Returns None when the shapes miss the tensor-core path."""
     sh, sw, ph, pw, dh, dw = geo
     Co, Ci, KH, KW = w_shape
     N, _, H, W = xd.shape
