@@ -8,7 +8,7 @@
 //   warp 1     MMA issuer: one lane issues tcgen05.mma.kind::f16 (M = 128 per CTA, N <= 256, K = 16) on shared-memory
 //              descriptors, for one CTA or for a pair of CTAs; accumulators live in TMEM; tcgen05.commit releases ring
 //              slots / publishes accumulators;
-//   warps 2-5  epilogue: tcgen05.ld (32 lanes x 32 columns), fp32 -> bf16, 16-byte global stores.
+//   warps 2-9  epilogue: tcgen05.ld (32 lanes x 32 columns), fp32 -> bf16, 16-byte global stores.
 // Work items are scheduled statically in groups of tile-rows for L2 reuse; one CTA per SM. Ragged M/N/K edges rely on TMA
 // zero fill and masked stores. No load is multicast.
 // Every mbarrier wait is bounded: on expiry the CTA records a status word, stops issuing, drains and frees TMEM.
@@ -27,8 +27,8 @@ constexpr int BM = 128, BK = 64;                    // rows of one CTA's MMA til
 constexpr int MAX_BN = 256;
 constexpr int A_BYTES = BM * BK * 2;
 constexpr int BOX_BYTES = 64 * BK * 2;              // one MN-major box: 64 elements of the operand's own axis x 64 of K
-constexpr int THREADS = 192;                        // 6 warps
-constexpr int EPI_PITCH = 34;                       // bf16 per staged row of a ragged store
+constexpr int THREADS = 320;                        // producer, MMA and 8 epilogue warps
+constexpr int EPI_PITCH = 40;                       // bf16 per staged row: 16-byte aligned, eight rows on different banks
 
 // What bounds a large product is the tensor pipe as long as the operands' way from L2 into shared memory stays below it: a
 // 128 x 256 tile per SM takes 48 KB per 4.2 MFLOP, a 256 x 256 tile per CTA pair 32 KB per SM, a 512 x 256 tile per pair 48 KB
@@ -43,7 +43,7 @@ template <bool PAIR, int MT> struct Cfg {
     static constexpr int B_BYTES = MAX_BN / CTAS * BK * 2;
     static constexpr int STAGE_BYTES = MT * A_BYTES + B_BYTES;
     static constexpr int STAGES = (192 * 1024) / STAGE_BYTES;
-    static constexpr int EPI_BYTES = 4 * 32 * EPI_PITCH * 2;
+    static constexpr int EPI_BYTES = 8 * 32 * EPI_PITCH * 2;
     static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*alignment slack*/ + 256 /*barriers*/ + EPI_BYTES;
     static constexpr int NBUF = 2 / MT;             // accumulator sets in the 512 TMEM columns
     static constexpr int TILE_M = CTAS * MT * BM;
@@ -101,7 +101,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; s++) { mbar_init(full + s, 1); mbar_init(empty + s, 1); }
-        for (int b = 0; b < NBUF; b++) { mbar_init(acc_full + b, 1); mbar_init(acc_empty + b, 4 * CTAS); }
+        for (int b = 0; b < NBUF; b++) { mbar_init(acc_full + b, 1); mbar_init(acc_empty + b, 8 * CTAS); }
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -185,12 +185,14 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             }
         }
     } else {
-        // ---------------- epilogue: warps 2..5 own TMEM lane quadrants (warp % 4) ----------------
-        const int quad = warp & 3;
+        // ---------------- epilogue: two warps per TMEM lane quadrant (warp % 4), each with every other 32 columns ----------------
+        // Products with a short K are all epilogue: with one warp per quadrant and a
+        // lane to a row 15416 x 962 x 128 took 52 us, 8000 x 1001 x 256 34 us; 40 and 28 us this way.
+        const int quad = warp & 3, grp = (warp - 2) >> 2;
         int it = 0;
         bool ok = true;
         const bool vec_ok = (A.N % 8 == 0) && (((uintptr_t)c & 15) == 0);
-        __nv_bfloat16* rows = reinterpret_cast<__nv_bfloat16*>(epi) + quad * (32 * EPI_PITCH);
+        __nv_bfloat16* rows = reinterpret_cast<__nv_bfloat16*>(epi) + (warp - 2) * (32 * EPI_PITCH);
         for (int u = first; u < A.units && ok; u += step, it++) {
             const Unit w = unit_at(A, u);
             const int buf = it % NBUF;
@@ -203,9 +205,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             for (int j = 0; j < MT; j++) {
                 const int row0 = w.tm * F::TILE_M + (j * CTAS + rank) * BM + quad * 32, row = row0 + lane;
                 const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + buf * (MT * MAX_BN) + j * MAX_BN;
-                __nv_bfloat16* crow = c + ((int64_t)w.batch * A.M + row) * A.N;
 #pragma unroll 1
-                for (int ch = 0; ch < A.bn; ch += 32) {
+                for (int ch = grp * 32; ch < A.bn; ch += 64) {
                     const int col0 = w.tn * A.bn + ch;
                     if (row0 >= A.M || col0 >= A.N) break;       // uniform over the warp
                     uint32_t r[32];
@@ -224,25 +225,24 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                     __align__(16) __nv_bfloat162 h[16];
 #pragma unroll
                     for (int e = 0; e < 16; e++) h[e] = __floats2bfloat162_rn(__uint_as_float(r[2 * e]), __uint_as_float(r[2 * e + 1]));
+                    // turned around in shared memory: a warp then writes 64 bytes of a row at a time
+                    __syncwarp();
+#pragma unroll
+                    for (int q = 0; q < 4; q++) reinterpret_cast<uint4*>(rows + lane * EPI_PITCH)[q] = reinterpret_cast<const uint4*>(h)[q];
+                    __syncwarp();
+                    __nv_bfloat16* c0 = c + ((int64_t)w.batch * A.M + row0) * A.N + col0;
                     if (vec_ok) {
-                        if (row < A.M) {
+                        const int at = (lane & 3) * 8;
 #pragma unroll
-                            for (int q = 0; q < 4; q++)
-                                if (col0 + q * 8 < A.N)
-                                    *reinterpret_cast<uint4*>(crow + col0 + q * 8) = reinterpret_cast<const uint4*>(h)[q];
+                        for (int q = 0; q < 4; q++) {
+                            const int i = q * 8 + (lane >> 2);
+                            if (row0 + i < A.M && col0 + at < A.N)
+                                *reinterpret_cast<uint4*>(c0 + (int64_t)i * A.N + at) = *reinterpret_cast<const uint4*>(rows + i * EPI_PITCH + at);
                         }
-                    } else {
-                        // rows start at any multiple of 2 bytes: turned around in shared memory, a warp then writes 64 B of a row at a time
-                        __syncwarp();
-#pragma unroll
-                        for (int e = 0; e < 16; e++) *reinterpret_cast<__nv_bfloat162*>(rows + lane * EPI_PITCH + 2 * e) = h[e];
-                        __syncwarp();
-                        if (col0 + lane < A.N) {
-                            __nv_bfloat16* q = c + ((int64_t)w.batch * A.M + row0) * A.N + col0 + lane;
+                    } else if (col0 + lane < A.N) {               // rows start at any multiple of 2 bytes
 #pragma unroll 8
-                            for (int i = 0; i < 32; i++)
-                                if (row0 + i < A.M) q[(int64_t)i * A.N] = rows[i * EPI_PITCH + lane];
-                        }
+                        for (int i = 0; i < 32; i++)
+                            if (row0 + i < A.M) c0[(int64_t)i * A.N + lane] = rows[i * EPI_PITCH + lane];
                     }
                 }
             }
