@@ -208,22 +208,31 @@ class Recorder:
         self.ok = True
         self.thread = threading.get_ident()   # what other threads launch meanwhile is not part of this graph
         self.steps = []
-        self.spans = []                       # (base, bytes) per buffer
+        self.spans = []                       # (base, bytes, dtype) per buffer
         self.keep = []                        # nothing is freed while recording, so an address names one buffer
         for t in leaves:
             self._add(t)
 
     def _add(self, t):
-        self.spans.append((t.data_ptr(), t.numel() * t.element_size()))
+        self.spans.append((t.data_ptr(), t.numel() * t.element_size(), t.dtype))
         self.keep.append(t)
         return len(self.spans) - 1
 
     def locate(self, ptr):
         for k in range(len(self.spans) - 1, -1, -1):
-            base, n = self.spans[k]
+            base, n, _ = self.spans[k]
             if n and base <= ptr < base + n:
                 return k, ptr - base
         raise _NotReplayable(f"pointer {ptr:#x} belongs to no buffer of the plan")
+
+    def locate_result(self, t):
+        """A buffer that holds all of t as elements of its dtype (leaves may share memory in part, or as another dtype)."""
+        ptr, size = t.data_ptr(), t.numel() * t.element_size()
+        for k in range(len(self.spans) - 1, -1, -1):
+            base, n, dtype = self.spans[k]
+            if base <= ptr and ptr + size <= base + n and dtype == t.dtype:
+                return k, ptr - base
+        raise _NotReplayable("a result in no buffer of the plan")
 
     def alloc(self, t):
         k = self._add(t)

@@ -5,8 +5,8 @@
 // same few graphs over and over with other tensors, so the first sync of a graph runs the Python planner with every
 // allocation and library call written to a tape (executor.py), and later syncs of a graph of the same structure replay that
 // tape from here: one walk over the graph makes its signature (op kinds, attributes, shapes, dtypes, how nodes share
-// inputs, alignment of the leaves), a hash lookup finds the tape, and its calls run with the new pointers. Results are not
-// kept: every replay allocates its outputs and launches every kernel again.
+// inputs, alignment of the leaves and which of them share memory), a hash lookup finds the tape, and its calls run with the
+// new pointers. Results are not kept: every replay allocates its outputs and launches every kernel again.
 #include <Python.h>
 #include <structmember.h>
 
@@ -17,6 +17,7 @@
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+#include <algorithm>
 #include <cstring>
 #include <deque>
 #include <memory>
@@ -295,6 +296,25 @@ struct Walk {
         PyObject* f = PyDict_GetItem(h_flags, name);
         if (f) value(f);
     }
+    // A tape knows a leaf by its addresses: leaves that share memory (assign, a realised reshape, two Vars of one torch tensor)
+    // and leaves that do not are different graphs. For each leaf that starts inside another one: which, and how far in. That
+    // fixes every address of a group of overlapping leaves relative to the others'.
+    void sharing() {
+        struct Span { uintptr_t at, end; size_t leaf; };
+        std::vector<Span> spans;
+        spans.reserve(leaves.size());
+        for (size_t i = 0; i < leaves.size(); i++) {
+            const at::Tensor& t = THPVariable_Unpack(leaves[i]->data);
+            const uintptr_t at = (uintptr_t)t.const_data_ptr();
+            if (t.numel()) spans.push_back({at, at + (size_t)t.numel() * t.element_size(), i});
+        }
+        std::sort(spans.begin(), spans.end(), [](const Span& a, const Span& b) { return a.at != b.at ? a.at < b.at : a.leaf < b.leaf; });
+        Span last{0, 0, 0};                      // the span that reaches furthest so far
+        for (const Span& s : spans) {
+            if (s.at < last.end) { tag('o'); num((int64_t)s.leaf); num((int64_t)last.leaf); num((int64_t)(s.at - last.at)); }
+            if (s.end > last.end) last = s;
+        }
+    }
     void run(const std::vector<VarObj*>& roots) {
         key.reserve(2048);
         flag(s_fuse); flag(s_wgrad);
@@ -320,6 +340,7 @@ struct Walk {
             }
             tag('r'); num(index[root]);
         }
+        if (ok) sharing();
     }
 };
 

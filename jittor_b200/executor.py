@@ -76,7 +76,7 @@ def _record(roots, nodes, leaves):
             if v._data.numel() == 0 or not v._data.is_contiguous():
                 return None
             try:
-                buf, off = rec.locate(v._data.data_ptr())
+                buf, off = rec.locate_result(v._data)
             except C._NotReplayable:
                 return None
             results.append((i, buf, off, tuple(v._data.shape)))

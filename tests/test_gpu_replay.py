@@ -76,6 +76,36 @@ def test_replay_gives_the_planners_bits(graph, skew):
                 assert torch.equal(x, y)
 
 
+def pair(s, sharing):
+    """Two leaves of one structure: of their own, or in one memory."""
+    if sharing == "overlap":
+        t = data(s, 80).torch()
+        return jt.array(t[:64].view(4, 16)), jt.array(t[16:].view(4, 16))
+    a = data(s, 4, 16)
+    if sharing == "assign":
+        return a, data(s + 1, 4, 16).assign(a)
+    if sharing == "reshape":
+        return a, a.reshape([64]).sync().reshape([4, 16]).sync()
+    if sharing == "tensor":
+        return a, jt.array(a.torch())
+    return a, data(s + 1, 4, 16)
+
+
+@pytest.mark.parametrize("first,second", [(k, "own") for k in ("assign", "reshape", "tensor", "overlap")]
+                         + [("own", k) for k in ("assign", "reshape", "tensor", "overlap")] + [("overlap", "tensor"), ("tensor", "overlap")])
+def test_leaves_that_share_memory_are_a_graph_of_their_own(first, second):
+    def run(s, sharing):
+        a, b = pair(s, sharing)
+        return values([(a - b) * data(s + 2, 4, 16), a + a, b.sum(1), b.reshape([2, 32])])
+    want = []
+    for s, sharing in ((1, first), (5, second), (9, first)):
+        C.host.clear()
+        want.append(run(s, sharing))
+    C.host.clear()
+    for w, (s, sharing) in zip(want, ((1, first), (5, second), (9, first))):
+        assert all(torch.equal(x, y) for x, y in zip(w, run(s, sharing)))
+
+
 def test_threads_and_streams_share_the_tapes():
     want = {s: values(softmax(s, 0)) for s in range(4)}
     bad = []
