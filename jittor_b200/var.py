@@ -6,6 +6,7 @@ Every call records a node with inferred shape and dtype and computes nothing; `s
 `.numpy()` hand the graph to the executor (executor.py), which recognises the chains the reference
 fuses (conv, matmul, softmax, LayerNorm, BatchNorm) and launches the CUDA kernels through the C ABI.
 """
+import copyreg
 import numbers
 
 import numpy as np
@@ -34,6 +35,17 @@ class Shape(list):
 Op = host.Op                     # kind, inputs (list), attrs (dict): csrc/host.cpp
 
 
+def _make_op(kind, inputs, attrs):
+    return Op(kind, inputs, **attrs)
+
+
+def _bare(cls):
+    return cls.__new__(cls)
+
+
+copyreg.pickle(Op, lambda op: (_make_op, (op.kind, op.inputs, op.attrs)))
+
+
 def _check_shape(shape):
     shape = [int(s) for s in shape]
     if len(shape) > MAX_DIMS:
@@ -51,6 +63,32 @@ class Var(host.VarBase):
     `_const` (the Python number this Var was made from, if any), `_pending` (handle of a collective still in flight on
     another stream), `_relay`, `_vjp`, `_bn_running`, `_stop_grad`, `_stop_fuse`, `compile_options`."""
     __array_priority__ = 100
+
+    # ---- copies -------------------------------------------------------------------------------
+    _STATE = ("_shape", "_dtype", "_data", "_name", "_const", "_bn_running", "is_scalar", "_stop_grad", "_stop_fuse", "compile_options")
+
+    def __copy__(self):
+        """A Var of the same value, producer and layer record."""
+        op = self._op                           # written down now: a builder belongs to the Var it was made for
+        v = type(self).__new__(type(self))
+        for n in self._STATE + ("_pending", "_relay", "_vjp"):
+            setattr(v, n, getattr(self, n))
+        v._op = op
+        v.__dict__.update(self.__dict__)
+        return v
+
+    def __getstate__(self):
+        """What a Var that stands alone (deepcopy, pickle) keeps: a layer's record and rule name the Vars they were made with,
+        so the layer goes along as its graph."""
+        self.wait()
+        return {"_op": self._op, **{n: getattr(self, n) for n in self._STATE}, **self.__dict__}
+
+    def __setstate__(self, state):
+        for n, value in state.items():
+            setattr(self, n, value)
+
+    def __reduce_ex__(self, protocol):
+        return _bare, (type(self),), self.__getstate__()
 
     # ---- metadata -----------------------------------------------------------------------------
     @property

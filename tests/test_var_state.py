@@ -1,0 +1,80 @@
+"""What a Var holds besides its value: copies and pickles of it. No GPU: the values are CPU tensors that nothing computes with."""
+import copy
+import pickle
+
+import numpy as np
+import pytest
+import torch
+
+import jittor_b200 as jt
+from jittor_b200 import nn, pool
+from jittor_b200 import var as V
+
+
+def leaf(*shape, dtype=torch.float32):
+    t = torch.arange(int(np.prod(shape)), dtype=torch.float32).reshape(shape).to(dtype)
+    return V.Var(list(shape), str(dtype).split(".")[1], data=t)
+
+
+def layers():
+    x = leaf(2, 3, 8, 8)
+    bn = nn.BatchNorm(3)
+    return {"leaf": x, "expression": (x * 2.0 + x).sum(1), "constant": jt.array(2.5), "conv2d": nn.conv2d(x, leaf(4, 3, 3, 3), None, 1, 1),
+            "matmul": nn.matmul(leaf(4, 5), leaf(5, 6)), "softmax": nn.softmax(x, -1), "layer_norm": nn.layer_norm(x, (8,), leaf(8), leaf(8)),
+            "batch_norm_relu": nn.relu(bn(x)), "index": x[1], "mean_pool": pool.avg_pool2d(x, 2, 2)}
+
+
+def same(a, b):
+    assert list(a.shape) == list(b.shape) and a.dtype == b.dtype and a.is_scalar == b.is_scalar and a._const == b._const
+    assert a.is_stop_grad() == b.is_stop_grad() and a.is_stop_fuse() == b.is_stop_fuse() and a.name() == b.name()
+    assert (a._data is None) == (b._data is None) and (a._data is None or torch.equal(a._data, b._data))
+    assert (a._op is None) == (b._op is None) and (a._op is None or (a._op.kind == b._op.kind and len(a._op.inputs) == len(b._op.inputs)))
+
+
+@pytest.mark.parametrize("how", [copy.copy, copy.deepcopy, lambda v: pickle.loads(pickle.dumps(v))], ids=["copy", "deepcopy", "pickle"])
+@pytest.mark.parametrize("kind", sorted(layers()))
+def test_copies_of_a_var(kind, how):
+    v = layers()[kind]
+    v.name("v")
+    v.stop_grad()
+    v.stop_fuse()
+    v.compile_options["G"] = 1
+    v.note = "kept"
+    c = how(v)
+    same(v, c)
+    assert c is not v and c.note == "kept" and c.compile_options == {"G": 1}
+    c.start_grad()
+    assert v.is_stop_grad()
+
+
+def test_copies_share_or_own_their_memory():
+    x = leaf(3, 4)
+    assert copy.copy(x)._data is x._data
+    assert copy.deepcopy(x)._data.data_ptr() != x._data.data_ptr()
+    pair = copy.deepcopy([x, x * 2.0])
+    assert pair[1]._op.inputs[0] is pair[0]
+
+
+class Net(nn.Module):
+    def __init__(self):
+        self.norms, self.table, self.head = [nn.BatchNorm(4), nn.LayerNorm(6)], {"a": leaf(5, 2)}, leaf(2, 3)
+
+
+@pytest.mark.parametrize("how", [copy.deepcopy, lambda m: pickle.loads(pickle.dumps(m))], ids=["deepcopy", "pickle"])
+def test_copies_of_a_module(how):
+    net = Net()
+    twin = how(net)
+    assert len(twin.parameters()) == len(net.parameters()) == 8
+    for a, b in zip(net.parameters(), twin.parameters()):
+        assert a is not b
+        same(a, b)
+
+
+def test_gradients_flow_through_a_copied_graph():
+    """A deep copy of a layer's result and its input is differentiated with respect to the copied input."""
+    x = leaf(4, 6)
+    y = nn.softmax(x, -1)
+    x2, y2 = copy.deepcopy((x, y))
+    assert jt.grad(y2.sum(), x2)._op.kind != "fill"          # a Var no gradient reaches gets zeros
+    assert jt.grad(y2.sum(), x)._op.kind == "fill"
+    assert jt.grad(copy.copy(y).sum(), x)._op.kind != "fill"
