@@ -1101,7 +1101,8 @@ PyObject* m_optim_step(PyObject*, PyObject* args) {
                 if (!py) return nullptr;
                 at += (sizes[i] + 3) / 4 * 4;
                 Py_XSETREF(v->data, py);
-                Py_CLEAR(v->builder);
+                // as Var.assign: nothing describes the value it held before
+                Py_CLEAR(v->builder); Py_CLEAR(v->relay); Py_CLEAR(v->vjp); Py_CLEAR(v->bn_running); Py_CLEAR(v->konst);
                 Py_XSETREF(v->op, Py_NewRef(Py_None));
             }
         }

@@ -345,6 +345,8 @@ def _run_bn_stats(xd):
 
 def _plan_batch_norm(v, r):
     root = v if r[0] == "batch_norm" else r[1]
+    if root._relay is None:                 # the normalised Var was assigned to: the ReLU is of its new value
+        return None
     _, x, g, b, eps, stats = root._relay
     return E.batch_norm_plan(v, x, ("var", g) if g is not None else ("const", 1.0), ("var", b) if b is not None else ("const", 0.0),
                              eps, r[0] != "batch_norm", False, root, stats)

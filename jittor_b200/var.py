@@ -194,6 +194,7 @@ class Var(host.VarBase):
         other = to_var(other)
         other.sync()
         self._shape, self._dtype, self._data, self._op = other._shape, other._dtype, other._data, None
+        self._relay = self._vjp = self._bn_running = self._const = None        # what described the value it held before
         return self
 
     update = assign

@@ -1,4 +1,4 @@
-"""What a Var holds besides its value: copies and pickles of it. No GPU: the values are CPU tensors that nothing computes with."""
+"""What a Var holds besides its value: copies and pickles of it, assignment over it. No GPU: the values are CPU tensors that nothing computes with."""
 import copy
 import pickle
 
@@ -55,6 +55,12 @@ def test_copies_share_or_own_their_memory():
     assert pair[1]._op.inputs[0] is pair[0]
 
 
+def reaches(y, x):
+    """Whether a gradient of y reaches x (a Var that none reaches gets zeros)."""
+    g = jt.grad(y, x)
+    return g._op.kind != "fill"
+
+
 class Net(nn.Module):
     def __init__(self):
         self.norms, self.table, self.head = [nn.BatchNorm(4), nn.LayerNorm(6)], {"a": leaf(5, 2)}, leaf(2, 3)
@@ -75,6 +81,32 @@ def test_gradients_flow_through_a_copied_graph():
     x = leaf(4, 6)
     y = nn.softmax(x, -1)
     x2, y2 = copy.deepcopy((x, y))
-    assert jt.grad(y2.sum(), x2)._op.kind != "fill"          # a Var no gradient reaches gets zeros
-    assert jt.grad(y2.sum(), x)._op.kind == "fill"
-    assert jt.grad(copy.copy(y).sum(), x)._op.kind != "fill"
+    assert reaches(y2.sum(), x2) and not reaches(y2.sum(), x)
+    assert reaches(copy.copy(y).sum(), x)
+
+
+@pytest.mark.parametrize("kind", ["softmax", "log_softmax", "layer_norm", "matmul", "conv2d", "batch_norm", "batch_norm_relu", "mean_pool"])
+def test_an_assigned_var_is_a_leaf(kind):
+    """assign() over a layer's result: no gradient reaches the layer's input, in whatever way it is looked for."""
+    x = leaf(8, 8) if kind == "matmul" else leaf(2, 4, 8, 8)
+    y = {"softmax": lambda: nn.softmax(x, -1), "log_softmax": lambda: nn.log_softmax(x, -1), "layer_norm": lambda: nn.layer_norm(x, (8,), leaf(8), leaf(8)),
+         "matmul": lambda: nn.matmul(x, leaf(8, 3)), "conv2d": lambda: nn.conv2d(x, leaf(4, 4, 3, 3), None, 1, 1), "batch_norm": lambda: nn.BatchNorm(4)(x),
+         "batch_norm_relu": lambda: nn.relu(nn.BatchNorm(4)(x)), "mean_pool": lambda: pool.avg_pool2d(x, 2, 2)}[kind]()
+    assert reaches(y.sum(), x)
+    y.assign(leaf(3, 5))
+    assert y._op is None and y._relay is None and y._vjp is None and y._bn_running is None and list(y.shape) == [3, 5]
+    assert not reaches((y * y).sum(), x)
+
+
+def test_a_constant_that_was_assigned_is_no_constant():
+    s = jt.array(0.0)
+    s.assign(leaf(1))
+    assert s._const is None
+
+
+def test_relu_of_an_assigned_norm_is_of_the_new_value():
+    h = nn.BatchNorm(4)(leaf(2, 4, 8, 8))
+    y = nn.relu(h)
+    h.assign(leaf(2, 4, 8, 8))
+    from jittor_b200 import relay
+    assert relay.plan(y) is None and y._op.kind == "ternary" and y._op.inputs[1] is h
