@@ -154,11 +154,12 @@ def _plan_mean_pool_dx(v, r):
 
 
 # ------------------------------------------------------------------------------------------------ parameters of the norms
-def _param(p, n):
-    """A float32 Var of n elements, "const" for the neutral Python number, or None for what the kernels do not take."""
+def _param(p, shape, neutral):
+    """A float32 Var of that shape, "const" for the neutral Python number, or None for what the records do not hold: other
+    numbers, arrays, and shapes that the graph would stretch or refuse."""
     if isinstance(p, V.Var):
-        return p if p.dtype == "float32" and p.numel() == n else None
-    return "const"
+        return p if p.dtype == "float32" and p._const is None and list(p.shape) == list(shape) else None
+    return "const" if isinstance(p, (int, float)) and p == neutral else None
 
 
 def _var_or_none(p):
@@ -193,10 +194,10 @@ def layer_norm(x, weight, bias, eps, k, build):
     cols = 1
     for s in x._shape[x.ndim - k:]:
         cols *= s
-    g, b = _param(weight, cols), _param(bias, cols)
+    g, b = _param(weight, x._shape[x.ndim - k:], 1), _param(bias, x._shape[x.ndim - k:], 0)
     if g is None or b is None or x.dtype not in _MM or x.numel() == 0:
         return None
-    key = ("layer_norm", str(x.dtype), x.ndim, k, isinstance(g, str) and weight, isinstance(b, str) and bias, flags._v["amp_reg"])
+    key = ("layer_norm", str(x.dtype), x.ndim, k, isinstance(g, str), isinstance(b, str), flags._v["amp_reg"])
     if _recognised(key, build, E._match_layernorm) != x.dtype:
         return None
     g, b = _var_or_none(g), _var_or_none(b)
@@ -280,10 +281,10 @@ def batch_norm(module, x, weight, bias, eps, build):
     if x.ndim < 3 or x.dtype not in _MM or x.numel() == 0:
         return None
     cn = x._shape[1]
-    g, b = _param(weight, cn), _param(bias, cn)
+    g, b = _param(weight, [cn], 1), _param(bias, [cn], 0)
     if g is None or b is None or cn > 2048:
         return None
-    key = ("batch_norm", str(x.dtype), x.ndim, isinstance(g, str) and weight, isinstance(b, str) and bias, flags._v["amp_reg"])
+    key = ("batch_norm", str(x.dtype), x.ndim, isinstance(g, str), isinstance(b, str), flags._v["amp_reg"])
     dtype = _recognised(key, lambda: build()[0], E._match_batchnorm)
     if dtype not in _MM:
         return None

@@ -1,5 +1,6 @@
 """Gradient kernels of LayerNorm and training BatchNorm (csrc/norm_bwd.cu) and the one-element row kernels (csrc/rownorm.cu) at
 the edges of their register tiles, against float64 and, for bfloat16 BatchNorm, against the meta-op graph they stand for."""
+import numpy as np
 import pytest
 import torch
 
@@ -68,3 +69,22 @@ def test_batch_norm(n, c, h, w, relu, dtype, amp):
                 near(a.torch(), b.torch(), 1e-4)
             else:
                 near(a.torch(), b.torch(), 4e-3 if amp == 0 else 1e-3)    # amp 2 rounds as the graph does: at most a flip here and there
+
+
+@pytest.mark.parametrize("weight,bias", [(2.0, 0.5), (0.0, 1.0), (np.full(6, 2.0, np.float32), np.full(6, 0.5, np.float32)), (1.0, -3.0)])
+@pytest.mark.parametrize("relu", [False, True])
+def test_batch_norm_with_numbers_for_parameters(weight, bias, relu):
+    x, dy = torch.randn(5, 6, 7, 9, device="cuda") + 0.2, torch.randn(5, 6, 7, 9, device="cuda")
+    bn, vx = nn.BatchNorm(6), jt.array(x)
+    bn.weight, bn.bias = weight, bias
+    y = nn.relu(bn(vx)) if relu else bn(vx)
+    dx = jt.grad((y * jt.array(dy)).sum(), vx)
+    jt.sync([y, dx])
+    xd = x.double().requires_grad_()
+    w, b = (torch.as_tensor(p, device="cuda").double().expand(6) for p in (weight, bias))
+    ref = torch.nn.functional.batch_norm(xd, None, None, w, b, True, eps=1e-5)
+    ref = torch.relu(ref) if relu else ref
+    ref.backward(dy.double())
+    near(y.torch(), ref.detach(), 1e-5)
+    near(dx.torch(), xd.grad, 1e-4)
+    near(bn.running_mean.torch(), 0.1 * x.double().mean((0, 2, 3)), 1e-5)

@@ -1,4 +1,4 @@
-"""What a Var holds besides its value: copies and pickles of it, assignment over it. No GPU: the values are CPU tensors that nothing computes with."""
+"""What a Var holds besides its value: copies and pickles of it, assignment over it, which layers carry a record. No GPU: the values are CPU tensors that nothing computes with."""
 import copy
 import pickle
 
@@ -110,3 +110,31 @@ def test_relu_of_an_assigned_norm_is_of_the_new_value():
     h.assign(leaf(2, 4, 8, 8))
     from jittor_b200 import relay
     assert relay.plan(y) is None and y._op.kind == "ternary" and y._op.inputs[1] is h
+
+
+@pytest.mark.parametrize("weight,bias,recorded", [(1.0, 0.0, True), (1, 0, True), (2.0, 0.0, False), (1.0, 0.5, False), (0, 0, False), ((4,), (4,), True),
+                                                  ((4,), 0.0, True), (2.0, (4,), False), ((1, 1), 0.0, False)])
+def test_norms_with_numbers_for_parameters(weight, bias, recorded):
+    """A record holds float32 parameters of the layer's shape or none; any other weight or bias goes into the graph."""
+    def par(p):
+        return leaf(*p) if isinstance(p, tuple) else p
+    bn = nn.BatchNorm(4)
+    bn.weight, bn.bias = par(weight), par(bias)
+    if weight != (1, 1):
+        assert (bn(leaf(2, 4, 3, 3))._relay is not None) == recorded
+    ln = nn.LayerNorm(4)
+    ln.weight, ln.bias = par(weight), par(bias)
+    assert (ln(leaf(6, 4))._relay is not None) == recorded
+
+
+def test_a_norm_refuses_parameters_that_its_graph_refuses():
+    ln = nn.LayerNorm((4, 6))
+    assert ln(leaf(2, 4, 6))._relay is not None
+    ln.weight = leaf(24)
+    with pytest.raises(ValueError):
+        ln(leaf(2, 4, 6))
+    bn = nn.BatchNorm(4)
+    assert bn(leaf(2, 4, 3, 3))._relay is not None
+    bn.weight = leaf(2, 2)
+    with pytest.raises(ValueError):
+        bn(leaf(2, 4, 3, 3))
