@@ -927,10 +927,17 @@ PyObject* m_backprop(PyObject*, PyObject* args) {
     }
     struct Frame { PyObject *v, *inputs; bool rule; Py_ssize_t next; };
     std::vector<Frame> stack;
+    // A rule that passes over a Var the program holds (its third element): the graph is followed where the gradient of that
+    // Var is asked for, ends there, or another value was assigned to it.
+    auto stops_inside = [&](PyObject* vjp) {
+        if (PyTuple_GET_SIZE(vjp) < 3) return false;
+        PyObject* inner = PyTuple_GET_ITEM(vjp, 2);
+        return wanted.count(inner) > 0 || V(inner)->stop_grad || none(V(inner)->relay);
+    };
     auto push = [&](PyObject* v) -> bool {
         Frame f{v, nullptr, false, 0};
         if (!wanted.count(v) && !V(v)->stop_grad) {                                    // no gradient flows through stop_grad Vars
-            if (!none(V(v)->vjp) && v != through) { f.inputs = PyTuple_GET_ITEM(V(v)->vjp, 0); f.rule = true; }
+            if (!none(V(v)->vjp) && v != through && !stops_inside(V(v)->vjp)) { f.inputs = PyTuple_GET_ITEM(V(v)->vjp, 0); f.rule = true; }
             else {
                 PyObject* op = var_get_op(V(v), nullptr);
                 if (!op) return false;

@@ -6,7 +6,8 @@ matmul_tuner.cc:21-102, conv_tuner.cc:218-411). Here the caller hands the execut
 wrote; the graph itself is a builder that runs only when something reads `Var._op` -- another matcher, the fuser, or
 jt.grad when it differentiates a gradient. First-order gradients come from `Var._vjp`: (inputs, rule), where
 rule(y, dout, wanted) gives one gradient per input, again as records, whose builders derive the same gradient from the
-graph by the per-op rules. A record is only made for shapes, dtypes and flags whose graph the executor's matcher recognises
+graph by the per-op rules; a rule that takes two of the program's steps at once names the Var between them, and the graph
+is followed when the gradient of that one is asked for or ends there. A record is only made for shapes, dtypes and flags whose graph the executor's matcher recognises
 (`_recognised`), so a layer runs the same kernels with or without it."""
 import weakref
 
@@ -334,7 +335,7 @@ def _bn_vjp(y, root, relu):
         for p, want in zip(params, wanted[1:]):
             out.append(_part(sums, cn if p is g else 0, p.shape, lambda p=p: _graph_grad(y, dout, p)) if want else None)
         return out
-    y._vjp = ((x,) + params, rule)
+    y._vjp = ((x,) + params, rule, root) if relu else ((x,) + params, rule)
 
 
 def _run_bn_stats(xd):

@@ -1,4 +1,5 @@
-"""What a Var holds besides its value: copies and pickles of it, assignment over it, which layers carry a record. No GPU: the values are CPU tensors that nothing computes with."""
+"""What a Var holds besides its value: copies and pickles of it, assignment over it, which layers carry a record,
+which Vars a gradient reaches. No GPU: the values are CPU tensors that nothing computes with."""
 import copy
 import pickle
 
@@ -138,3 +139,19 @@ def test_a_norm_refuses_parameters_that_its_graph_refuses():
     bn.weight = leaf(2, 2)
     with pytest.raises(ValueError):
         bn(leaf(2, 4, 3, 3))
+
+
+def test_a_gradient_reaches_the_norm_under_a_relu():
+    """relu(batch_norm(x)) is one record; its gradient still reaches the normalised Var, and ends there when told to."""
+    x = leaf(2, 4, 3, 3)
+    h = nn.BatchNorm(4)(x)
+    y = nn.relu(h)
+    assert reaches(y.sum(), h) and reaches(y.sum(), x)
+    gh, gx = jt.grad((y * y).sum(), [h, x])
+    assert gh._op.kind != "fill" and gx._op.kind == "fill"            # a target takes the gradient: it does not go on from there
+    h.stop_grad()
+    assert not reaches(y.sum(), x)
+    h.start_grad()
+    assert jt.grad(y.sum(), x)._relay[0] == "batch_norm_dx"           # one step where nothing asks for h
+    h.assign(leaf(2, 4, 3, 3))
+    assert not reaches(y.sum(), x) and reaches(y.sum(), h)
