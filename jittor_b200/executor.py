@@ -114,6 +114,9 @@ def _run_plans(roots):
             stack.pop()
             pending_update = v._bn_running
             if pending_update is not None:          # a BatchNorm output computed op by op: move its running statistics now
+                if pending_update[1] is None:
+                    v._op                           # a record: writing its graph fills in the batch statistics
+                    pending_update = v._bn_running
                 v._bn_running = None
                 module, xmean, xvar = pending_update
                 module._update_running(xmean, xvar)

@@ -88,3 +88,18 @@ def test_batch_norm_with_numbers_for_parameters(weight, bias, relu):
     near(y.torch(), ref.detach(), 1e-5)
     near(dx.torch(), xd.grad, 1e-4)
     near(bn.running_mean.torch(), 0.1 * x.double().mean((0, 2, 3)), 1e-5)
+
+
+@pytest.mark.parametrize("replaced", ["float64", "shape"])
+def test_running_statistics_the_kernel_does_not_move(replaced):
+    """Statistics of another dtype or shape than the kernel's float32 [C] move through the graph's."""
+    x = torch.randn(5, 6, 7, 9, device="cuda") + 0.2
+    want = 0.1 * x.double().mean((0, 2, 3))
+    for _ in range(3):                                    # planned, then from what the first run left
+        bn = nn.BatchNorm(6)
+        if replaced == "float64":
+            bn.running_mean, bn.running_var = jt.zeros((6,), "float64"), jt.ones((6,), "float64")
+        else:
+            bn.running_mean, bn.running_var = jt.zeros((1,)), jt.ones((1,))
+        bn(jt.array(x)).sync()
+        near(bn.running_mean.torch(), want, 1e-5)
