@@ -178,10 +178,14 @@ PyGetSetDef var_getset[] = {
 struct Walk {
     std::string key;
     std::vector<VarObj*> nodes, leaves;
+    std::vector<PyObject*> held;                     // every Var met: Python that runs meanwhile (a builder, a wait, another thread) may drop it
     std::unordered_map<const void*, int> index;      // Var -> number: leaves and nodes share one numbering in visiting order
     bool ok = true;
     int count = 0;
 
+    Walk() = default;
+    Walk(const Walk&) = delete;
+    ~Walk() { for (PyObject* o : held) Py_DECREF(o); }
     void raw(const void* p, size_t n) { key.append((const char*)p, n); }
     void num(int64_t v) { raw(&v, sizeof v); }
     void tag(char c) { key.push_back(c); }
@@ -327,7 +331,10 @@ struct Walk {
             if (!index.count(root)) { index.emplace(root, -1); stack.push_back({root, {}, 0}); }
             while (ok && !stack.empty()) {
                 Frame& f = stack.back();
-                if (f.next == 0 && f.kids.empty() && none(f.v->data)) children(f.v, f.kids);
+                if (f.next == 0 && f.kids.empty() && none(f.v->data)) {
+                    children(f.v, f.kids);
+                    for (VarObj* k : f.kids) held.push_back(Py_NewRef((PyObject*)k));
+                }
                 if (!ok) break;
                 if (f.next < f.kids.size()) {
                     VarObj* k = f.kids[f.next++];
@@ -404,9 +411,9 @@ struct Tape {
     std::deque<std::vector<const char*>> string_lists;
     std::deque<std::vector<int64_t>> longs;
     std::deque<std::vector<int32_t>> ints;
-    std::vector<at::Tensor> bufs;
 };
-std::unordered_map<std::string, std::unique_ptr<Tape>> g_tapes;      // null: the planner has to run every time
+// null: the planner has to run every time. Shared: a replay keeps its tape while another thread clears the map.
+std::unordered_map<std::string, std::shared_ptr<Tape>> g_tapes;
 
 // One argument of a recorded call: (code, payload...), written by _capi.Recorder.
 bool add_arg(Tape& t, Step& st, PyObject* a) {
@@ -487,9 +494,9 @@ bool ints_of(PyObject* tuple, std::vector<int64_t>& out) {
 }
 
 // spec: (number of buffers, steps, results, nodes whose running statistics moved, plans) from executor._record
-std::unique_ptr<Tape> build_tape(PyObject* spec, int n_leaves) {
+std::shared_ptr<Tape> build_tape(PyObject* spec, int n_leaves) {
     PyObject *steps, *results, *bn;
-    auto t = std::make_unique<Tape>();
+    auto t = std::make_shared<Tape>();
     if (!PyArg_ParseTuple(spec, "iO!O!O!i", &t->n_bufs, &PyList_Type, &steps, &PyList_Type, &results, &PyList_Type, &bn, &t->n_plans))
         return nullptr;
     t->n_leaves = n_leaves;
@@ -557,43 +564,36 @@ std::unique_ptr<Tape> build_tape(PyObject* spec, int n_leaves) {
     return t;
 }
 
+// Buffers belong to the call. Slots and descriptors belong to the tape: a step writes its own and is launched with the
+// interpreter lock held all the while, so that two threads in one tape do not see each other's.
 bool replay(Tape& t, const Walk& w) {
-    t.bufs.assign((size_t)t.n_bufs, at::Tensor());
-    struct Clear { Tape& t; ~Clear() { t.bufs.clear(); } } clear{t};
-    for (int i = 0; i < t.n_leaves; i++) {
-        VarObj* v = w.leaves[i];
-        if (!none(v->pending)) {                           // produced by a collective on another stream
-            PyObject* r = PyObject_CallMethodNoArgs((PyObject*)v, s_wait);
-            if (!r) return false;
-            Py_DECREF(r);
-        }
-        t.bufs[i] = THPVariable_Unpack(v->data);
-    }
+    std::vector<at::Tensor> bufs((size_t)t.n_bufs);
+    for (int i = 0; i < t.n_leaves; i++) bufs[i] = THPVariable_Unpack(w.leaves[i]->data);
     const auto device = c10::Device(c10::kCUDA, c10::cuda::current_device());
     void* stream = (void*)c10::cuda::getCurrentCUDAStream().stream();
     for (Step& st : t.steps) {
         if (st.kind == Step::ALLOC) {
-            t.bufs[st.buf] = at::Tensor(at::detail::empty_cuda(st.sizes, st.type, device, std::nullopt));
+            bufs[st.buf] = at::Tensor(at::detail::empty_cuda(st.sizes, st.type, device, std::nullopt));
             continue;
         }
-        if (st.kind == Step::FILL) { t.bufs[st.buf].fill_(st.value); continue; }
+        if (st.kind == Step::FILL) { bufs[st.buf].fill_(st.value); continue; }
         for (Patch& p : st.patches) {
-            const at::Tensor& b = t.bufs[p.buf];
+            const at::Tensor& b = bufs[p.buf];
             *p.where = b.defined() ? (char*)b.data_ptr() + p.off : nullptr;
         }
-        for (auto& n : st.nbytes) st.slots[n.first].i = t.bufs[n.second].defined() ? t.bufs[n.second].numel() : 0;
+        for (auto& n : st.nbytes) st.slots[n.first].i = bufs[n.second].defined() ? bufs[n.second].numel() : 0;
         if (st.stream >= 0) st.slots[st.stream].p = stream;
         const int64_t rc = st.entry->invoke(st.entry->fn, st.slots.data());
         if (st.kind == Step::WORKSPACE) {
-            if (rc > 0) t.bufs[st.buf] = at::Tensor(at::detail::empty_cuda({rc}, at::kByte, device, std::nullopt));
+            if (rc > 0) bufs[st.buf] = at::Tensor(at::detail::empty_cuda({rc}, at::kByte, device, std::nullopt));
         } else if (rc != 0) {
             PyErr_Format(h_error, "%s: %s (status %d)", st.entry->name + 7, g_last_error ? g_last_error() : "", (int)rc);
             return false;
         }
-        for (int b : st.release) t.bufs[b].reset();
+        for (int b : st.release) bufs[b].reset();
     }
     for (const Result& r : t.results) {
-        at::Tensor out = t.bufs[r.buf];
+        at::Tensor out = bufs[r.buf];
         if (!r.same) {
             int64_t n = 1;
             for (int64_t d : r.shape) n *= d;
@@ -1122,7 +1122,7 @@ PyObject* m_optim_step(PyObject*, PyObject* args) {
 
 // ------------------------------------------------------------------------------------------------ module functions
 // realize(roots) -> True when every root is computed; False: the caller has to run the Python planner.
-PyObject* m_realize(PyObject*, PyObject* arg) {
+PyObject* m_realize(PyObject* self, PyObject* arg) {
     PyObject* seq = PySequence_Fast(arg, "realize: a list of Vars");
     if (!seq) return nullptr;
     struct Hold { PyObject* o; ~Hold() { Py_DECREF(o); } } hold{seq};
@@ -1134,14 +1134,24 @@ PyObject* m_realize(PyObject*, PyObject* arg) {
     }
     if (roots.empty()) Py_RETURN_TRUE;
     if (g_recording || !h_record) Py_RETURN_FALSE;
-    Walk w;
     try {
+        Walk w;
         w.run(roots);
         if (!w.ok) Py_RETURN_FALSE;
+        bool waited = false;
+        for (VarObj* v : w.leaves)
+            if (!none(v->pending)) {                        // produced by a collective on another stream
+                PyObject* r = PyObject_CallMethodNoArgs((PyObject*)v, s_wait);
+                if (!r) return nullptr;
+                Py_DECREF(r);
+                waited = true;
+            }
+        if (waited) return m_realize(self, arg);            // other threads ran: the graph is looked at again
         auto it = g_tapes.find(w.key);
         if (it != g_tapes.end()) {
-            if (!it->second) Py_RETURN_FALSE;
-            if (!replay(*it->second, w)) return nullptr;
+            const std::shared_ptr<Tape> tape = it->second;
+            if (!tape) Py_RETURN_FALSE;
+            if (!replay(*tape, w)) return nullptr;
             Py_RETURN_TRUE;
         }
         PyObject* nodes = PyList_New((Py_ssize_t)w.nodes.size());
@@ -1155,7 +1165,7 @@ PyObject* m_realize(PyObject*, PyObject* arg) {
         Py_DECREF(leaves);
         if (!spec) return nullptr;
         if (g_tapes.size() >= 4096) g_tapes.clear();          // programs with endless shapes: start over rather than grow
-        std::unique_ptr<Tape> tape;
+        std::shared_ptr<Tape> tape;
         if (spec != Py_None) {
             tape = build_tape(spec, (int)w.leaves.size());
             if (!tape) { Py_DECREF(spec); if (!PyErr_Occurred()) PyErr_SetString(PyExc_RuntimeError, "tape: malformed record"); return nullptr; }

@@ -125,6 +125,39 @@ def test_threads_and_streams_share_the_tapes():
     assert not bad
 
 
+class Handle:
+    """Stands for a collective in flight: waiting for it lets another thread run."""
+    def __init__(self, meanwhile):
+        self.meanwhile = meanwhile
+
+    def wait(self):
+        t = threading.Thread(target=self.meanwhile)
+        t.start()
+        t.join()
+
+
+@pytest.mark.parametrize("meanwhile", ["replay", "other", "clear"])
+def test_a_wait_lets_other_threads_into_the_tapes(meanwhile):
+    """A leaf that is still in flight is waited for before a tape is touched; what runs meanwhile does not disturb it."""
+    want, other, seen = values(softmax(3, 0)), values(softmax(7, 0)), []
+
+    def run():
+        if meanwhile == "clear":
+            C.host.clear()
+        else:
+            seen.append(values(softmax(7, 0) if meanwhile == "replay" else softmax(7, 1)))
+
+    values(softmax(1, 0))                                     # recorded
+    x, dy = data(3, 20, 300), data(4, 20, 300)
+    x._pending, dy._pending = Handle(run), Handle(run)
+    y = nn.softmax(x, -1)
+    got = values([y, jt.grad((y * dy).sum(), x)])
+    assert x._pending is None and dy._pending is None
+    assert all(torch.equal(a, b) for a, b in zip(want, got))
+    if meanwhile == "replay":
+        assert len(seen) == 2 and all(torch.equal(a, b) for s in seen for a, b in zip(other, s))
+
+
 @pytest.mark.parametrize("kind", ["sgd", "nesterov", "adam", "adamw", "rmsprop"])
 def test_many_tensor_update_has_the_bits_of_the_op_by_op_rule(kind):
     from jittor_b200 import optim
