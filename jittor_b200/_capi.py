@@ -279,8 +279,8 @@ class Recorder:
             except _NotReplayable:
                 self.ok = False
 
-    def call(self, name, args):
-        self.note(lambda: self.steps.append(("call", -1, name, self._args(name, args) + [("z",)])))
+    def call(self, name, args, what):
+        self.note(lambda: self.steps.append(("call", -1, name, self._args(name, args) + [("z",)], what)))
 
     def workspace(self, name, args, t):
         k = self._add(t)
@@ -325,7 +325,7 @@ def workspace(name, *args):
 def call(name, *args, what=None):
     """Launches entry point `name` on the current stream (its last argument)."""
     rc = getattr(lib, name)(*args, stream_ptr())
-    if rc:
-        check(rc, what() if callable(what) else what or name)
-    if recording():
-        recorder.call(name, args)
+    if rc or recording():
+        what = what() if callable(what) else what or name
+        check(rc, what)
+        recorder.call(name, args, what)

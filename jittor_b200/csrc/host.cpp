@@ -15,6 +15,7 @@
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <algorithm>
@@ -397,6 +398,7 @@ struct Step {
     std::vector<Patch> patches;
     std::vector<std::pair<int, int>> nbytes;   // (slot, buffer): the size of a workspace passed beside its pointer
     int stream = -1;                       // slot of the stream
+    std::string what;                      // CALL: what an error is reported as
     std::vector<int> release;              // buffers nothing reads after this step
 };
 struct Result { int node, buf; bool same; int64_t off; std::vector<int64_t> shape; };
@@ -523,6 +525,11 @@ std::shared_ptr<Tape> build_tape(PyObject* spec, int n_leaves) {
             PyObject* args = PyTuple_GET_ITEM(s, 3);
             st.slots.reserve((size_t)PyList_GET_SIZE(args));
             for (Py_ssize_t k = 0; k < PyList_GET_SIZE(args); k++) if (!add_arg(*t, st, PyList_GET_ITEM(args, k))) return nullptr;
+            if (st.kind == Step::CALL) {
+                const char* what = PyUnicode_AsUTF8(PyTuple_GET_ITEM(s, 4));
+                if (!what) return nullptr;
+                st.what = what;
+            }
         }
         if (PyErr_Occurred()) return nullptr;
     }
@@ -587,7 +594,7 @@ bool replay(Tape& t, const Walk& w) {
         if (st.kind == Step::WORKSPACE) {
             if (rc > 0) bufs[st.buf] = at::Tensor(at::detail::empty_cuda({rc}, at::kByte, device, std::nullopt));
         } else if (rc != 0) {
-            PyErr_Format(h_error, "%s: %s (status %d)", st.entry->name + 7, g_last_error ? g_last_error() : "", (int)rc);
+            PyErr_Format(h_error, "%s: %s (status %d)", st.what.c_str(), g_last_error ? g_last_error() : "", (int)rc);
             return false;
         }
         for (int b : st.release) bufs[b].reset();
@@ -1086,7 +1093,8 @@ PyObject* m_optim_step(PyObject*, PyObject* args) {
     std::vector<double> h;
     for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(hyper); i++) h.push_back(PyFloat_AsDouble(PyTuple_GET_ITEM(hyper, i)));
     if (PyErr_Occurred()) return nullptr;
-    try {
+    HANDLE_TH_ERRORS
+    {
         const auto device = c10::Device(c10::kCUDA, c10::cuda::current_device());
         static const int slot[3] = {0, 2, 3};
         at::Tensor flat[3];
@@ -1113,11 +1121,9 @@ PyObject* m_optim_step(PyObject*, PyObject* args) {
                 Py_XSETREF(v->op, Py_NewRef(Py_None));
             }
         }
-    } catch (const std::exception& e) {
-        PyErr_SetString(h_error, e.what());
-        return nullptr;
     }
     Py_RETURN_TRUE;
+    END_HANDLE_TH_ERRORS
 }
 
 // ------------------------------------------------------------------------------------------------ module functions
@@ -1134,7 +1140,8 @@ PyObject* m_realize(PyObject* self, PyObject* arg) {
     }
     if (roots.empty()) Py_RETURN_TRUE;
     if (g_recording || !h_record) Py_RETURN_FALSE;
-    try {
+    HANDLE_TH_ERRORS                                        // torch's own errors: running out of memory is torch.OutOfMemoryError, as in the planner
+    {
         Walk w;
         w.run(roots);
         if (!w.ok) Py_RETURN_FALSE;
@@ -1174,11 +1181,8 @@ PyObject* m_realize(PyObject* self, PyObject* arg) {
         g_tapes.emplace(std::move(w.key), std::move(tape));
         Py_DECREF(spec);
         Py_RETURN_TRUE;
-    } catch (const std::exception& e) {
-        g_recording = false;
-        PyErr_SetString(h_error ? h_error : PyExc_RuntimeError, e.what());
-        return nullptr;
     }
+    END_HANDLE_TH_ERRORS
 }
 
 // setup(Shape, make_shape, DType, canon, record, error, flags dict, {symbol: address})

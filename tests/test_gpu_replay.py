@@ -158,6 +158,44 @@ def test_a_wait_lets_other_threads_into_the_tapes(meanwhile):
         assert len(seen) == 2 and all(torch.equal(a, b) for s in seen for a, b in zip(other, s))
 
 
+class limited_memory:
+    """Allocations beyond `spare` bytes fail, as on a GPU that is full."""
+    def __init__(self, spare):
+        self.spare = spare
+
+    def __enter__(self):
+        torch.cuda.empty_cache()
+        total = torch.cuda.get_device_properties(0).total_memory
+        torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + self.spare) / total)
+
+    def __exit__(self, *exc):
+        torch.cuda.set_per_process_memory_fraction(1.0)
+
+
+def test_running_out_of_memory_is_the_same_error_from_planner_and_replay():
+    x = data(1, 1, 1 << 20)
+    graph = lambda: (x * 3.0).broadcast([64, 1 << 20]).reindex([64, 1 << 20], ["i0", f"{(1 << 20) - 1}-i1"])
+    for prepared in (False, True):
+        C.host.clear()
+        if prepared:
+            want = graph().sync().torch().clone()             # recorded
+        with limited_memory(32 << 20), pytest.raises(torch.OutOfMemoryError):
+            graph().sync()
+        assert graph().sync().numel() == 64 << 20             # and it runs once there is room
+    assert torch.equal(graph().torch(), want)
+
+
+def test_a_recorded_launch_keeps_what_its_error_is_called():
+    t = torch.ones(8, device="cuda")
+    C.recorder = C.Recorder([t])
+    try:
+        C.call("b200jt_unary", C.desc(t), C.desc(t), b"negative", what=lambda: "negative [8]")
+        step = C.recorder.steps[-1]
+    finally:
+        C.recorder = None
+    assert step[0] == "call" and step[4] == "negative [8]"
+
+
 @pytest.mark.parametrize("kind", ["sgd", "nesterov", "adam", "adamw", "rmsprop"])
 def test_many_tensor_update_has_the_bits_of_the_op_by_op_rule(kind):
     from jittor_b200 import optim
