@@ -208,6 +208,8 @@ class Recorder:
         self.ok = True
         self.thread = threading.get_ident()   # what other threads launch meanwhile is not part of this graph
         self.steps = []
+        self.moves = []                       # (step, Var): the step moves the running statistics that Var was to move
+        self.computed = {}                    # id of a Var -> steps after which it has its value
         self.spans = []                       # (base, bytes, dtype) per buffer
         self.keep = []                        # nothing is freed while recording, so an address names one buffer
         for t in leaves:
@@ -281,6 +283,10 @@ class Recorder:
 
     def call(self, name, args, what):
         self.note(lambda: self.steps.append(("call", -1, name, self._args(name, args) + [("z",)], what)))
+
+    def moved(self, v):
+        """The next step moves v's running statistics."""
+        self.moves.append((len(self.steps), v))
 
     def workspace(self, name, args, t):
         k = self._add(t)

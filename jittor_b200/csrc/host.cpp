@@ -400,13 +400,13 @@ struct Step {
     int stream = -1;                       // slot of the stream
     std::string what;                      // CALL: what an error is reported as
     std::vector<int> release;              // buffers nothing reads after this step
+    std::vector<int> moved;                // CALL: nodes whose running statistics it moves; a later step may fail, and they move once
 };
-struct Result { int node, buf; bool same; int64_t off; std::vector<int64_t> shape; };
+struct Result { int node, buf; bool same; int64_t off; std::vector<int64_t> shape; size_t ready; };      // ready: steps after which it has its value
 struct Tape {
     int n_leaves = 0, n_bufs = 0, n_plans = 0;
     std::vector<Step> steps;
     std::vector<Result> results;
-    std::vector<int> bn_done;              // nodes whose running statistics the fused BatchNorm updated
     // storage behind the slots
     std::deque<std::vector<b200jt_tensor>> tensors;
     std::deque<std::string> strings;
@@ -495,7 +495,7 @@ bool ints_of(PyObject* tuple, std::vector<int64_t>& out) {
     return !PyErr_Occurred();
 }
 
-// spec: (number of buffers, steps, results, nodes whose running statistics moved, plans) from executor._record
+// spec: (number of buffers, steps, results, (step, node) whose running statistics move, plans) from executor._record
 std::shared_ptr<Tape> build_tape(PyObject* spec, int n_leaves) {
     PyObject *steps, *results, *bn;
     auto t = std::make_shared<Tape>();
@@ -544,6 +544,7 @@ std::shared_ptr<Tape> build_tape(PyObject* spec, int n_leaves) {
         out.buf = (int)PyLong_AsLong(PyTuple_GET_ITEM(r, 1));
         out.off = PyLong_AsLongLong(PyTuple_GET_ITEM(r, 2));
         if (!ints_of(PyTuple_GET_ITEM(r, 3), out.shape)) return nullptr;
+        out.ready = PyLong_AsSize_t(PyTuple_GET_ITEM(r, 4));
         out.same = false;
         // the buffer is allocated in its result's shape, so that no view is needed for it
         if (out.off == 0 && out.buf >= n_leaves && !kept[out.buf])
@@ -557,7 +558,12 @@ std::shared_ptr<Tape> build_tape(PyObject* spec, int n_leaves) {
         kept[out.buf] = 1;
         t->results.push_back(std::move(out));
     }
-    for (Py_ssize_t i = 0; i < PyList_GET_SIZE(bn); i++) t->bn_done.push_back((int)PyLong_AsLong(PyList_GET_ITEM(bn, i)));
+    for (Py_ssize_t i = 0; i < PyList_GET_SIZE(bn); i++) {
+        PyObject* m = PyList_GET_ITEM(bn, i);
+        const size_t step = PyLong_AsSize_t(PyTuple_GET_ITEM(m, 0));
+        if (step >= t->steps.size()) return nullptr;
+        t->steps[step].moved.push_back((int)PyLong_AsLong(PyTuple_GET_ITEM(m, 1)));
+    }
     std::vector<int> last((size_t)t->n_bufs, -1);
     for (size_t k = 0; k < t->steps.size(); k++) {
         Step& st = t->steps[k];
@@ -576,46 +582,61 @@ std::shared_ptr<Tape> build_tape(PyObject* spec, int n_leaves) {
 bool replay(Tape& t, const Walk& w) {
     std::vector<at::Tensor> bufs((size_t)t.n_bufs);
     for (int i = 0; i < t.n_leaves; i++) bufs[i] = THPVariable_Unpack(w.leaves[i]->data);
+    // Hands out what the first `steps` steps have computed. Where a step fails, what was computed before it stays, as in the
+    // planner: running statistics among it, which moved and are not moved again.
+    auto hand_out = [&](size_t steps) {
+        for (const Result& r : t.results) {
+            if (r.ready > steps) continue;
+            at::Tensor out = bufs[r.buf];
+            if (!r.same) {
+                int64_t n = 1;
+                for (int64_t d : r.shape) n *= d;
+                if (r.off == 0 && n == out.numel()) out = out.view(r.shape);
+                else {
+                    std::vector<int64_t> stride(r.shape.size(), 1);
+                    for (int i = (int)r.shape.size() - 2; i >= 0; i--) stride[i] = stride[i + 1] * r.shape[i + 1];
+                    out = out.as_strided(r.shape, stride, out.storage_offset() + r.off / (int64_t)out.element_size());
+                }
+            }
+            PyObject* py = THPVariable_Wrap(std::move(out));
+            if (!py) return false;
+            Py_XSETREF(w.nodes[r.node]->data, py);
+        }
+        return true;
+    };
     const auto device = c10::Device(c10::kCUDA, c10::cuda::current_device());
     void* stream = (void*)c10::cuda::getCurrentCUDAStream().stream();
-    for (Step& st : t.steps) {
-        if (st.kind == Step::ALLOC) {
-            bufs[st.buf] = at::Tensor(at::detail::empty_cuda(st.sizes, st.type, device, std::nullopt));
-            continue;
-        }
-        if (st.kind == Step::FILL) { bufs[st.buf].fill_(st.value); continue; }
-        for (Patch& p : st.patches) {
-            const at::Tensor& b = bufs[p.buf];
-            *p.where = b.defined() ? (char*)b.data_ptr() + p.off : nullptr;
-        }
-        for (auto& n : st.nbytes) st.slots[n.first].i = bufs[n.second].defined() ? bufs[n.second].numel() : 0;
-        if (st.stream >= 0) st.slots[st.stream].p = stream;
-        const int64_t rc = st.entry->invoke(st.entry->fn, st.slots.data());
-        if (st.kind == Step::WORKSPACE) {
-            if (rc > 0) bufs[st.buf] = at::Tensor(at::detail::empty_cuda({rc}, at::kByte, device, std::nullopt));
-        } else if (rc != 0) {
-            PyErr_Format(h_error, "%s: %s (status %d)", st.what.c_str(), g_last_error ? g_last_error() : "", (int)rc);
-            return false;
-        }
-        for (int b : st.release) bufs[b].reset();
-    }
-    for (const Result& r : t.results) {
-        at::Tensor out = bufs[r.buf];
-        if (!r.same) {
-            int64_t n = 1;
-            for (int64_t d : r.shape) n *= d;
-            if (r.off == 0 && n == out.numel()) out = out.view(r.shape);
-            else {
-                std::vector<int64_t> stride(r.shape.size(), 1);
-                for (int i = (int)r.shape.size() - 2; i >= 0; i--) stride[i] = stride[i + 1] * r.shape[i + 1];
-                out = out.as_strided(r.shape, stride, out.storage_offset() + r.off / (int64_t)out.element_size());
+    size_t at = 0;
+    try {
+        for (; at < t.steps.size(); at++) {
+            Step& st = t.steps[at];
+            if (st.kind == Step::ALLOC) {
+                bufs[st.buf] = at::Tensor(at::detail::empty_cuda(st.sizes, st.type, device, std::nullopt));
+                continue;
             }
+            if (st.kind == Step::FILL) { bufs[st.buf].fill_(st.value); continue; }
+            for (Patch& p : st.patches) {
+                const at::Tensor& b = bufs[p.buf];
+                *p.where = b.defined() ? (char*)b.data_ptr() + p.off : nullptr;
+            }
+            for (auto& n : st.nbytes) st.slots[n.first].i = bufs[n.second].defined() ? bufs[n.second].numel() : 0;
+            if (st.stream >= 0) st.slots[st.stream].p = stream;
+            const int64_t rc = st.entry->invoke(st.entry->fn, st.slots.data());
+            if (st.kind == Step::WORKSPACE) {
+                if (rc > 0) bufs[st.buf] = at::Tensor(at::detail::empty_cuda({rc}, at::kByte, device, std::nullopt));
+            } else if (rc != 0) {
+                const std::string why = g_last_error ? g_last_error() : "";
+                if (hand_out(at)) PyErr_Format(h_error, "%s: %s (status %d)", st.what.c_str(), why.c_str(), (int)rc);
+                return false;
+            }
+            for (int n : st.moved) Py_XSETREF(w.nodes[n]->bn_running, Py_NewRef(Py_None));
+            for (int b : st.release) bufs[b].reset();
         }
-        PyObject* py = THPVariable_Wrap(std::move(out));
-        if (!py) return false;
-        Py_XSETREF(w.nodes[r.node]->data, py);
+    } catch (...) {
+        if (!hand_out(at)) return false;
+        throw;
     }
-    for (int n : t.bn_done) Py_XSETREF(w.nodes[n]->bn_running, Py_NewRef(Py_None));
+    if (!hand_out(t.steps.size())) return false;
     g_plans += t.n_plans;
     g_replays++;
     return true;

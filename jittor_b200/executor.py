@@ -65,7 +65,6 @@ def _record(roots, nodes, leaves):
     """Runs the planner over `roots` with its allocations and launches recorded. Returns what host.cpp makes a tape of, or
     None if the run did something a tape does not hold."""
     before = counters["plans"]
-    bn = [v for v in nodes if v._bn_running is not None]
     C.recorder = rec = C.Recorder([v._data for v in leaves])
     try:
         _run_plans(roots)
@@ -79,13 +78,16 @@ def _record(roots, nodes, leaves):
                 buf, off = rec.locate_result(v._data)
             except C._NotReplayable:
                 return None
-            results.append((i, buf, off, tuple(v._data.shape)))
+            results.append((i, buf, off, tuple(v._data.shape), rec.computed.get(id(v), len(rec.steps))))
     finally:
         C.recorder = None
     if not rec.ok:
         return None
-    done = [i for i, v in enumerate(nodes) if v._bn_running is None and any(v is b for b in bn)]
-    return len(rec.spans), rec.steps, results, done, counters["plans"] - before
+    place = {id(v): i for i, v in enumerate(nodes)}
+    moves = [(step, place.get(id(v))) for step, v in rec.moves]
+    if any(i is None for _, i in moves):
+        return None
+    return len(rec.spans), rec.steps, results, moves, counters["plans"] - before
 
 
 def _run_plans(roots):
@@ -110,6 +112,8 @@ def _run_plans(roots):
             out = plan.run()
             counters["plans"] += 1
             v._data = out.reshape(list(v.shape))
+            if C.recording():
+                C.recorder.computed[id(v)] = len(C.recorder.steps)
             plans.pop(id(v), None)
             stack.pop()
             pending_update = v._bn_running
@@ -1088,6 +1092,8 @@ def batch_norm_plan(v, x, g, b, eps, relu, synced, root, stats_var):
         momentum = 0.0
         if running is not None and root._bn_running is not None:
             root._bn_running = None                # consumed here: the kernel updates the running statistics in place
+            if C.recording():
+                C.recorder.moved(root)
             rmp, rvp, momentum = running[0].running_mean._data.data_ptr(), running[0].running_var._data.data_ptr(), running[0].momentum
         C.call("b200jt_bn_apply", C.desc(xd), stats.data_ptr(), count, gt.data_ptr() if gt is not None else None,
                bt.data_ptr() if bt is not None else None, eps, int(relu), C.desc(out), rmp, rvp, float(momentum), what="bn_apply")

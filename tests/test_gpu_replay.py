@@ -185,6 +185,25 @@ def test_running_out_of_memory_is_the_same_error_from_planner_and_replay():
     assert torch.equal(graph().torch(), want)
 
 
+@pytest.mark.parametrize("prepared", [False, True])
+def test_running_statistics_move_once_when_a_later_step_fails(prepared):
+    x = torch.randn(4, 16, 8, 8, device="cuda") + 0.3
+
+    def graph():
+        bn = nn.BatchNorm(16)
+        y = nn.relu(bn(jt.array(x)))
+        return bn, y, (y.reshape([1, 4096]) * 2.0).broadcast([1 << 14, 4096]).reindex([1 << 14, 4096], ["i0", "4095-i1"])
+    C.host.clear()
+    if prepared:
+        jt.sync(list(graph()[1:]))
+    bn, y, wide = graph()
+    with limited_memory(32 << 20), pytest.raises(torch.OutOfMemoryError):
+        jt.sync([y, wide])
+    jt.sync([y, wide])
+    want = 0.1 * x.double().mean((0, 2, 3))
+    assert (bn.running_mean.torch().double() - want).abs().max() <= 1e-6
+
+
 def test_a_recorded_launch_keeps_what_its_error_is_called():
     t = torch.ones(8, device="cuda")
     C.recorder = C.Recorder([t])
