@@ -9,6 +9,7 @@ import os
 import threading
 
 import torch
+from torch.multiprocessing.reductions import StorageWeakRef
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "csrc", "libb200jt.so")
@@ -210,20 +211,18 @@ class Recorder:
         self.steps = []
         self.moves = []                       # (step, Var): the step moves the running statistics that Var was to move
         self.computed = {}                    # id of a Var -> steps after which it has its value
-        self.spans = []                       # (base, bytes, dtype) per buffer
-        self.keep = []                        # nothing is freed while recording, so an address names one buffer
+        self.spans = []                       # (base, bytes, dtype, storage) per buffer; of two with an address one is alive
         for t in leaves:
             self._add(t)
 
     def _add(self, t):
-        self.spans.append((t.data_ptr(), t.numel() * t.element_size(), t.dtype))
-        self.keep.append(t)
+        self.spans.append((t.data_ptr(), t.numel() * t.element_size(), t.dtype, StorageWeakRef(t.untyped_storage())))
         return len(self.spans) - 1
 
     def locate(self, ptr):
         for k in range(len(self.spans) - 1, -1, -1):
-            base, n, _ = self.spans[k]
-            if n and base <= ptr < base + n:
+            base, n, _, storage = self.spans[k]
+            if n and base <= ptr < base + n and not storage.expired():
                 return k, ptr - base
         raise _NotReplayable(f"pointer {ptr:#x} belongs to no buffer of the plan")
 
@@ -231,8 +230,8 @@ class Recorder:
         """A buffer that holds all of t as elements of its dtype (leaves may share memory in part, or as another dtype)."""
         ptr, size = t.data_ptr(), t.numel() * t.element_size()
         for k in range(len(self.spans) - 1, -1, -1):
-            base, n, dtype = self.spans[k]
-            if base <= ptr and ptr + size <= base + n and dtype == t.dtype:
+            base, n, dtype, storage = self.spans[k]
+            if base <= ptr and ptr + size <= base + n and dtype == t.dtype and not storage.expired():
                 return k, ptr - base
         raise _NotReplayable("a result in no buffer of the plan")
 

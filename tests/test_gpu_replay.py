@@ -204,6 +204,27 @@ def test_running_statistics_move_once_when_a_later_step_fails(prepared):
     assert (bn.running_mean.torch().double() - want).abs().max() <= 1e-6
 
 
+def test_recording_takes_no_more_memory_than_planning():
+    """Temporaries and workspaces (here the channels-last copies) are freed as they are when nothing is recorded."""
+    from jittor_b200 import executor
+    w = [data(k, 64, 64, 3, 3, dtype=torch.bfloat16) for k in range(4)]
+
+    def peak(run):
+        x = data(9, 16, 64, 56, 56, dtype=torch.bfloat16)
+        y = x
+        for k in w:
+            y = nn.conv2d(y, k, None, 1, 1)
+        torch.cuda.synchronize()
+        torch.cuda.reset_peak_memory_stats()
+        base = torch.cuda.memory_allocated()
+        run([y])
+        return torch.cuda.max_memory_allocated() - base
+    planned = peak(executor._realize)
+    C.host.clear()
+    assert peak(executor.realize) <= planned                  # recorded
+    assert peak(executor.realize) <= planned                  # replayed
+
+
 def test_a_recorded_launch_keeps_what_its_error_is_called():
     t = torch.ones(8, device="cuda")
     C.recorder = C.Recorder([t])
