@@ -33,7 +33,7 @@ namespace {
 
 // ------------------------------------------------------------------------------------------------ hooks set by the package
 PyObject *h_shape_type, *h_make_shape, *h_dtype_type, *h_canon, *h_record, *h_error, *h_flags;
-PyObject *s_running_mean, *s_running_var, *s_momentum, *s_wait, *s_sig, *s_also, *s_custom, *s_fuse, *s_wgrad, *s_collective;
+PyObject *s_running_mean, *s_running_var, *s_momentum, *s_wait, *s_sig, *s_also, *s_custom, *s_fuse, *s_wgrad, *s_collective, *s_value;
 long g_context = 0;          // host state that changes plans (SMs reserved for a collective): part of every signature
 bool g_recording = false;
 int64_t g_plans = 0, g_replays = 0, g_records = 0;
@@ -181,6 +181,7 @@ struct Walk {
     std::vector<VarObj*> nodes, leaves;
     std::vector<PyObject*> held;                     // every Var met: Python that runs meanwhile (a builder, a wait, another thread) may drop it
     std::unordered_map<const void*, int> index;      // Var -> number: leaves and nodes share one numbering in visiting order
+    std::vector<std::pair<size_t, size_t>> numbers;  // where the key holds the value of a Python number: (place, bytes)
     bool ok = true;
     int count = 0;
 
@@ -208,6 +209,17 @@ struct Walk {
         else if (is_var(v)) { tag('v'); num(index.count(v) ? index[v] : -1); }
         else ok = false;
     }
+    void number(PyObject* v) {
+        const size_t at = key.size();
+        value(v);
+        if (key.size() > at + 1) numbers.emplace_back(at + 1, key.size() - at - 1);       // what kind of number it is stays
+    }
+    // the key with every number the same
+    std::string skeleton() const {
+        std::string k = key;
+        for (auto& n : numbers) std::fill_n(k.begin() + n.first, n.second, '\0');
+        return k;
+    }
     void meta(VarObj* v) {
         PyObject* s = v->shape;
         if (!s || !PyList_Check(s)) { ok = false; return; }
@@ -215,7 +227,7 @@ struct Walk {
         tag((char)('A' + n));
         for (Py_ssize_t i = 0; i < n; i++) num(PyLong_AsLongLong(PyList_GET_ITEM(s, i)));
         text(v->dtype);
-        if (!none(v->konst)) { tag('c'); value(v->konst); }
+        if (!none(v->konst)) { tag('c'); number(v->konst); }
         tag((char)(v->stop_fuse * 2 + v->is_scalar));
     }
     static void vars_in(PyObject* t, std::vector<VarObj*>& out) {
@@ -274,7 +286,7 @@ struct Walk {
             else {
                 Py_ssize_t pos = 0;
                 PyObject *k, *x;
-                while (PyDict_Next(o->attrs, &pos, &k, &x)) { text(k); value(x); }
+                while (PyDict_Next(o->attrs, &pos, &k, &x)) { text(k); if (k == s_value) number(x); else value(x); }
             }
             value(o->inputs);
             if (PyObject* also = PyDict_GetItem(o->attrs, s_also)) value(also);
@@ -415,7 +427,31 @@ struct Tape {
     std::deque<std::vector<int32_t>> ints;
 };
 // null: the planner has to run every time. Shared: a replay keeps its tape while another thread clears the map.
-std::unordered_map<std::string, std::shared_ptr<Tape>> g_tapes;
+typedef std::unordered_map<std::string, std::shared_ptr<Tape>> Tapes;
+// Programs with endless shapes fill the map: when the newer half is full it becomes the older one, whose tapes are dropped
+// unless they were used since. A number that changes from call to call (a learning rate) makes a graph of its own each time,
+// which is not worth a record: after kMaxVariants of a structure that differ in their numbers only, others are planned.
+constexpr size_t kHalf = 2048;
+constexpr int kMaxVariants = 16;
+Tapes g_tapes, g_older;
+std::unordered_map<std::string, int> g_variants;
+void age_tapes() {
+    if (g_variants.size() >= 2 * kHalf) g_variants.clear();
+    if (g_tapes.size() < kHalf) return;
+    g_older = std::move(g_tapes);
+    g_tapes.clear();
+    g_variants.clear();
+}
+const std::shared_ptr<Tape>* find_tape(const std::string& key) {
+    auto it = g_tapes.find(key);
+    if (it != g_tapes.end()) return &it->second;
+    auto old = g_older.find(key);
+    if (old == g_older.end()) return nullptr;
+    std::shared_ptr<Tape> tape = std::move(old->second);
+    g_older.erase(old);
+    age_tapes();
+    return &g_tapes.emplace(key, std::move(tape)).first->second;
+}
 
 // One argument of a recorded call: (code, payload...), written by _capi.Recorder.
 bool add_arg(Tape& t, Step& st, PyObject* a) {
@@ -1175,13 +1211,13 @@ PyObject* m_realize(PyObject* self, PyObject* arg) {
                 waited = true;
             }
         if (waited) return m_realize(self, arg);            // other threads ran: the graph is looked at again
-        auto it = g_tapes.find(w.key);
-        if (it != g_tapes.end()) {
-            const std::shared_ptr<Tape> tape = it->second;
+        if (const std::shared_ptr<Tape>* found = find_tape(w.key)) {
+            const std::shared_ptr<Tape> tape = *found;
             if (!tape) Py_RETURN_FALSE;
             if (!replay(*tape, w)) return nullptr;
             Py_RETURN_TRUE;
         }
+        if (!w.numbers.empty() && ++g_variants[w.skeleton()] > kMaxVariants) Py_RETURN_FALSE;
         PyObject* nodes = PyList_New((Py_ssize_t)w.nodes.size());
         PyObject* leaves = PyList_New((Py_ssize_t)w.leaves.size());
         for (size_t i = 0; i < w.nodes.size(); i++) PyList_SET_ITEM(nodes, (Py_ssize_t)i, Py_NewRef((PyObject*)w.nodes[i]));
@@ -1192,7 +1228,7 @@ PyObject* m_realize(PyObject* self, PyObject* arg) {
         Py_DECREF(nodes);
         Py_DECREF(leaves);
         if (!spec) return nullptr;
-        if (g_tapes.size() >= 4096) g_tapes.clear();          // programs with endless shapes: start over rather than grow
+        age_tapes();
         std::shared_ptr<Tape> tape;
         if (spec != Py_None) {
             tape = build_tape(spec, (int)w.leaves.size());
@@ -1230,9 +1266,9 @@ PyObject* m_context(PyObject*, PyObject* n) {
     if (PyErr_Occurred()) return nullptr;
     Py_RETURN_NONE;
 }
-PyObject* m_clear(PyObject*, PyObject*) { g_tapes.clear(); Py_RETURN_NONE; }
+PyObject* m_clear(PyObject*, PyObject*) { g_tapes.clear(); g_older.clear(); g_variants.clear(); Py_RETURN_NONE; }
 PyObject* m_stats(PyObject*, PyObject*) {
-    return Py_BuildValue("{s:n,s:L,s:L}", "tapes", (Py_ssize_t)g_tapes.size(), "recorded", (long long)g_records, "replayed", (long long)g_replays);
+    return Py_BuildValue("{s:n,s:L,s:L}", "tapes", (Py_ssize_t)(g_tapes.size() + g_older.size()), "recorded", (long long)g_records, "replayed", (long long)g_replays);
 }
 PyObject* m_take_plans(PyObject*, PyObject*) {
     const long long n = g_plans;
@@ -1285,7 +1321,7 @@ PyMODINIT_FUNC PyInit__b200jt_host(void) {
         {&o_maximum, "maximum"}, {&o_minimum, "minimum"}, {&o_equal, "equal"}, {&o_negative, "negative"}, {&o_mean, "mean"}, {&o_log, "log"}, {&o_exp, "exp"}};
     for (auto& n : names) *n.at = PyUnicode_InternFromString(n.text);
     i_zero = PyLong_FromLong(0);
-    s_collective = PyUnicode_InternFromString("mpi_all_reduce");
+    s_collective = PyUnicode_InternFromString("mpi_all_reduce"); s_value = PyUnicode_InternFromString("value");
     s_wgrad = PyUnicode_InternFromString("b200_wgrad_tc");
     if (PyModule_AddObjectRef(m, "Op", (PyObject*)&OpType) < 0 || PyModule_AddObjectRef(m, "VarBase", (PyObject*)&VarType) < 0) return nullptr;
     return m;

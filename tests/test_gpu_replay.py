@@ -8,6 +8,7 @@ import torch
 
 import jittor_b200 as jt
 from jittor_b200 import _capi as C, nn, pool
+from jittor_b200 import var as V
 
 pytestmark = pytest.mark.gpu
 
@@ -223,6 +224,33 @@ def test_recording_takes_no_more_memory_than_planning():
     C.host.clear()
     assert peak(executor.realize) <= planned                  # recorded
     assert peak(executor.realize) <= planned                  # replayed
+
+
+def test_a_number_that_changes_is_not_recorded_for_ever():
+    x = data(1, 8, 32)
+    C.host.clear()
+    before = C.host.stats()
+    for k in range(100):
+        got = values([x * (1.0 + k) + 0.5, V.full([8, 32], k) * x])
+        assert torch.equal(got[0], x.torch() * (1.0 + k) + 0.5) and torch.equal(got[1], x.torch() * k)
+    after = C.host.stats()
+    assert after["recorded"] - before["recorded"] <= 16 and after["tapes"] <= 16
+    values([x * 3.0 + 0.5, V.full([8, 32], 2) * x])          # k = 2: one of the recorded ones
+    assert C.host.stats()["replayed"] == after["replayed"] + 1
+
+
+def test_a_graph_in_use_outlives_endless_shapes():
+    x = data(1, 1, 5000)
+    hot = lambda: (x * 2.0).sum(1).sync()
+    C.host.clear()
+    hot()
+    before = C.host.stats()["recorded"]
+    for n in range(1, 4301):
+        jt.array(x.torch()[:, :n]).exp().sync()
+        if n % 256 == 0:
+            hot()
+    stats = C.host.stats()
+    assert stats["recorded"] == before + 4300 and stats["tapes"] <= 4096
 
 
 def test_a_recorded_launch_keeps_what_its_error_is_called():
