@@ -261,13 +261,14 @@ bn_bwd_sums_kernel(const TX* __restrict__ x, const TD* __restrict__ dy, float* _
     cg::cluster_group cluster = cg::this_cluster();
     const int c = blockIdx.y;
     const int rank = (int)cluster.block_rank(), size = (int)cluster.num_blocks();
-    const int hv = (int)g.HW / N, dj = 256 / hv, di = 256 - dj * hv, j0 = threadIdx.x / hv, i0 = threadIdx.x - j0 * hv;
-    const int total = (g.N_ - rank + size - 1) / size * hv;
+    // a plane has fewer than 2^31 elements, a channel's planes together may have more
+    const unsigned hv = (unsigned)g.HW / N, dj = 256 / hv, di = 256 - dj * hv, j0 = threadIdx.x / hv, i0 = threadIdx.x - j0 * hv;
+    const int64_t total = (int64_t)((g.N_ - rank + size - 1) / size) * hv;
     __shared__ float sm[32], mine[4];
     auto planes = [&](auto&& f) {
-        int j = j0, i = i0;
+        unsigned j = j0, i = i0;
 #pragma unroll 4
-        for (int v = threadIdx.x; v < total; v += 256) {
+        for (int64_t v = threadIdx.x; v < total; v += 256) {
             f(((int64_t)(rank + j * size) * g.C + c) * g.HW + i * N);
             j += dj; i += di;
             if (i >= hv) { i -= hv; j++; }

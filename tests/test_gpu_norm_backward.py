@@ -103,3 +103,14 @@ def test_running_statistics_the_kernel_does_not_move(replaced):
             bn.running_mean, bn.running_var = jt.zeros((1,)), jt.ones((1,))
         bn(jt.array(x)).sync()
         near(bn.running_mean.torch(), want, 1e-5)
+
+
+def test_batch_norm_sums_over_more_than_2_31_elements_of_a_channel():
+    from jittor_b200 import _capi as C
+    n, h, w = 16, 32767, 32771                            # odd planes: one element per access, 2 * h * w > 2^31 of them for a CTA
+    x = torch.ones(n, 1, h, w, device="cuda", dtype=torch.bfloat16)
+    stats, sums = torch.zeros(2, device="cuda"), torch.empty(4, device="cuda")
+    C.call("b200jt_bn_backward_sums", C.desc(x), C.desc(x), stats.data_ptr(), float(n * h * w), None, None, 1e-5, 0, sums.data_ptr())
+    assert abs(sums[0].item() - n * h * w) <= 1e-6 * n * h * w          # each thread counts up to 2^23 ones: exact until the threads meet
+    del x
+    torch.cuda.empty_cache()
