@@ -453,8 +453,9 @@ def conv_dx_plan(v, dy, w, geo):
     """bf16 in one call on the tensor cores (any stride up to 4); what that does not take as the transposed convolution."""
     def run():
         if dy.dtype == "bfloat16":
+            wd = _cast(w._data, "bfloat16")                   # held until the launch: the workspace must not take its memory
             out = _empty(list(v.shape), "bfloat16")
-            args = (C.desc(dy._data.view(list(dy.shape))), C.desc(_cast(w._data, "bfloat16")), C.desc(out), *geo)
+            args = (C.desc(dy._data.view(list(dy.shape))), C.desc(wd), C.desc(out), *geo)
             nbytes, wsp, ws = C.workspace("b200jt_conv2d_backward_x_workspace", *args)
             if nbytes:
                 C.call("b200jt_conv2d_backward_x", *args, wsp, nbytes,

@@ -106,6 +106,22 @@ def test_strided_input_gradient(n, ci, h, w, co, k, s, p, d):
     near(got, xd.grad)
 
 
+def test_input_gradient_with_float32_weights():
+    """The weights are cast for the launch; the scratch memory allocated after that is not theirs."""
+    from jittor_b200 import executor
+    dy, w = torch.randn(2, 256, 14, 14, device="cuda").bfloat16(), torch.randn(256, 256, 3, 3, device="cuda") * 0.02
+    xd = torch.zeros(2, 256, 28, 28, device="cuda", dtype=torch.float64, requires_grad=True)
+    torch.nn.functional.conv2d(xd, w.bfloat16().double(), None, 2, 1).backward(dy.double())
+    plan = executor.conv_dx_plan(jt.Var([2, 256, 28, 28], "bfloat16"), jt.array(dy), jt.array(w), (2, 2, 1, 1, 1, 1))
+    C.recorder = rec = C.Recorder([p._data for p in plan.leaves])          # takes no pointer to memory that was given back
+    try:
+        got = plan.run()
+    finally:
+        C.recorder = None
+    assert rec.ok
+    near(got, xd.grad)
+
+
 @pytest.mark.parametrize("shape", [(3, 5, 1, 300), (202, 7, 7, 7), (37, 3, 1, 1023), (9, 4, 16, 16), (600, 2, 1, 1), (300, 150, 2, 3)])
 @pytest.mark.parametrize("op", ["mean", "add", "maximum"])
 def test_reduction_over_short_rows(shape, op):
