@@ -376,9 +376,11 @@ static bool make_map_im2col(CUtensorMap* map, const void* base, int N, int H, in
               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
-// the corners and shifts an im2col map can hold
+// The corners and shifts an im2col map of four axes can hold: corners of the bounding box from -128 to 127, shifts from 0 to 255.
+// 3 x 3 filters dilated by up to 127 with the padding that keeps the size fit.
 static bool im2col_fits(const ConvShape& s) {
-    return s.ph <= 127 && s.pw <= 127 && (s.KH - 1) * (int64_t)s.dh <= 127 && (s.KW - 1) * (int64_t)s.dw <= 127;
+    const auto fits = [](int64_t pad, int64_t reach) { return pad <= 128 && reach <= 255 && reach - pad <= 128 && pad - reach <= 127; };
+    return fits(s.ph, (s.KH - 1) * (int64_t)s.dh) && fits(s.pw, (s.KW - 1) * (int64_t)s.dw);
 }
 
 static bool make_map_w(CUtensorMap* map, const void* base, const ConvShape& s, int bn) {

@@ -106,6 +106,13 @@ def test_strided_input_gradient(n, ci, h, w, co, k, s, p, d):
     near(got, xd.grad)
 
 
+# filters that reach as far as an im2col map allows: corners at -128 and 127, shifts up to 255
+@pytest.mark.parametrize("n,ci,h,w,co,k,p,d", [(1, 64, 80, 72, 64, 3, 64, 64), (2, 8, 140, 131, 16, 3, 127, 127), (1, 16, 20, 9, 24, 2, 128, 255),
+                                               (1, 24, 150, 160, 8, 2, 0, 128), (1, 8, 30, 30, 8, 1, 127, 1)])
+def test_convolution_of_wide_reach(n, ci, h, w, co, k, p, d, monkeypatch):
+    test_convolution_and_weight_gradient(n, ci, h, w, co, k, 1, p, d, None, None, monkeypatch)
+
+
 def test_input_gradient_with_float32_weights():
     """The weights are cast for the launch; the scratch memory allocated after that is not theirs."""
     from jittor_b200 import executor
