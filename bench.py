@@ -3,7 +3,8 @@
     python bench.py [--gpus N] [--steps K] [--warmup W] [--workload c1|c2|c3|c4|c5|meta|fused|next] [--impl reference]
 
 One JSON line on stdout (rank 0). The default run measures c2 (the headline keys of the line) and then c1, c3, c4, c5 and
-the meta / fused / next sets with the same method into "workloads"; --workload X measures X alone. Workloads are the benchmark configurations:
+the meta / fused / next sets with the same method, whose values are in "workloads"; the full records, with every part's time
+and kernel, are one line on stderr. --workload X measures X alone. Workloads are the benchmark configurations:
     c1            reindex-lowered conv2d fp32 [4,32,32,32] * [64,32,3,3], L2 flushed before every repetition    (GB/s and TFLOP/s)
     c2 (default)  reindex_reduce scatter: 2^24 int32 -> 2^20 bins and 2^24 fp32 -> 4096 bins, uniform and Zipf(1.1)
                   indices, plus the 2x2 max-pool backward [64,128,56,56,2,2] -> [64,128,112,112]      (GB/s, HBM)
@@ -94,7 +95,7 @@ class C1ConvF32:
     N, C, H, W, CO = 4, 32, 32, 32, 64
     description = ("config 0: reindex-lowered conv2d fp32 [4,32,32,32] * [64,32,3,3] s1 p1 "
                    "(reindex -> broadcast -> multiply -> sum over [Cin,Kh,Kw], recognised and run as one CUDA-core implicit GEMM)")
-    kernel_of = {"conv-f32": "gemm_simt_deep_kernel<float, ConvLoader, 32, 32>"}
+    kernel_of = {"conv-f32": "contract_kernel<FWD> (float32)"}
     launches = {"conv-f32": 1}
     flush_l2 = True
     FLOP = 2 * 4 * 64 * 32 * 32 * 32 * 9
@@ -471,7 +472,7 @@ class C5ConvBN:
     kernel_of = {"conv": "conv_bf16_kernel (tcgen05)", "conv-bn-relu": "conv_bf16_kernel (tcgen05)",
                  "conv-acdb": "conv_bf16_kernel (tcgen05)", "conv-wgrad": "wgrad_bf16_kernel (tcgen05)",
                  "conv-wgrad-acdb": "wgrad_bf16_kernel (tcgen05)"}
-    launches = {"conv": 2, "conv-bn-relu": 3, "conv-acdb": 2, "conv-wgrad": 6, "conv-wgrad-acdb": 2}
+    launches = {"conv": 2, "conv-bn-relu": 3, "conv-acdb": 2, "conv-wgrad": 3, "conv-wgrad-acdb": 2}
     all_reduced = ("conv-bn-relu",)
     traffic = {"conv": 776.5e6, "conv-bn-relu": 776.5e6, "conv-acdb": 776.5e6, "conv-wgrad": 826.0e6, "conv-wgrad-acdb": 826.0e6}
 
@@ -705,11 +706,10 @@ class FusedChains:
     key, metric, unit, bound, dtype, scaling = "fused", "meta-op GB/s", "GB/s", "hbm", "f32", "weak"
     ROWS, COLS = 32768, 4096
     description = ("fused element-wise chains on [32768,4096] fp32, one launch of a kernel compiled for the chain each: x*w+b "
-                   "(w, b per column), relu(x+bias), (a*b).sum(1), (x-mean)/sqrt(mean(x*x)+eps) (three row statements), the "
-                   "gradient of LayerNorm w.r.t. x as jt.grad builds it (four row reduces), and the backward of nn.softmax "
-                   "(its own kernel from y and dy)")
+                   "(w, b per column), relu(x+bias), (a*b).sum(1), (x-mean)/sqrt(mean(x*x)+eps) (three row statements); the "
+                   "gradient of LayerNorm w.r.t. x and the backward of nn.softmax as jt.grad builds them (a kernel of their own each)")
     kernel_of = {"scale-shift": "chain_jit_map_kernel", "relu-bias": "chain_jit_map_kernel", "mul-rowsum": "chain_jit_rows_kernel",
-                 "centre-scale": "chain_jit_rows_kernel", "layernorm-bwd": "chain_jit_rows_kernel",
+                 "centre-scale": "chain_jit_rows_kernel", "layernorm-bwd": "layer_norm_bwd_kernel",
                  "softmax-bwd": "softmax_bwd_reg_kernel"}
     launches = {k: 1 for k in kernel_of}
 
@@ -738,7 +738,7 @@ class FusedChains:
             return (x * y).sum(1)
         if name == "centre-scale":
             return (x - x.mean(1, keepdims=True)) / ((x * x).mean(1, keepdims=True) + 1e-5).sqrt()
-        if name == "layernorm-bwd":        # d LayerNorm / dx as jt.grad builds it from the per-op rules: four row reduces, one program
+        if name == "layernorm-bwd":        # d LayerNorm / dx as jt.grad builds it
             return self.jt.grad((self.nn.layer_norm(x, (x.shape[-1],), self.w, self.b) * y).sum(), x)
         sm = next((s for v, s in zip(self.x, self.sm) if v is x), None)
         if sm is None:
@@ -811,17 +811,17 @@ class NextOps:
     ROWS, COLS, PICK = 1 << 20, 64, 1 << 19
     description = ("callers of the path: 3x3 stride-2 pad-1 max-pool forward and backward on [64,128,112,112] fp32, "
                    "getitem x[idx] of 2^19 rows out of [2^20,64] fp32, setitem x[idx] += v on the same shapes")
-    kernel_of = {"maxpool-fwd": "pool_fwd_s2_kernel", "maxpool-bwd": "pool_bwd_indices_s2_kernel",
+    kernel_of = {"maxpool-fwd": "pool_fwd_tile_kernel", "maxpool-bwd": "pool_bwd_tile_kernel",
                  "getitem-rows": "reindex_rows_kernel", "setitem-add-rows": "rr_rows_kernel (+ table copy)"}
     launches = {"maxpool-fwd": 1, "maxpool-bwd": 1, "getitem-rows": 1, "setitem-add-rows": 1}
-    traffic = {"maxpool-fwd": 584.9e6, "maxpool-bwd": 566.8e6, "getitem-rows": 241.1e6, "setitem-add-rows": 365.8e6}
+    traffic = {"maxpool-fwd": 520.5e6, "maxpool-bwd": 481.3e6, "getitem-rows": 225.5e6, "setitem-add-rows": 365.3e6}
 
     def work(self):
         n = int(np.prod(self.SHAPE)) * 4
         o = self.SHAPE[0] * self.SHAPE[1] * 56 * 56 * 4
         rows = self.PICK * self.COLS * 4
-        # backward: index map + output gradient in, input gradient out (x and y are not read by the index-based kernel)
-        return {"maxpool-fwd": n + o, "maxpool-bwd": n + 2 * o, "getitem-rows": 2 * rows + self.PICK * 4,
+        # a byte per output says which element of its window won: written forward, read backward instead of x and y
+        return {"maxpool-fwd": n + o + o // 4, "maxpool-bwd": n + o + o // 4, "getitem-rows": 2 * rows + self.PICK * 4,
                 "setitem-add-rows": 2 * self.ROWS * self.COLS * 4 + 2 * rows + self.PICK * 4}
 
     def setup(self, rank, world, jt, torch, multi):
@@ -933,6 +933,32 @@ def run_reference(args, rank, world):
             extra[key] = {"value": v2, "unit": w2.unit, "ms_per_step": ms2, "cores": os.cpu_count(), "kind": "port", "sample": sample2}
         out["workloads"] = extra
     print(json.dumps(out))
+
+
+def short(v):
+    """Numbers to six digits, in containers too."""
+    if isinstance(v, float):
+        return float(f"{v:.6g}")
+    if isinstance(v, dict):
+        return {k: short(x) for k, x in v.items()}
+    return [short(x) for x in v] if isinstance(v, list) else v
+
+
+def contract_line(full):
+    """What stdout carries: the headline workload's fields and the other workloads' values, in well under 3000 characters,
+    because whoever collects the line may keep the end of the output only. The parts, the spread and the other workloads'
+    records go to stderr as one line."""
+    out = {k: full[k] for k in ("metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step", "higher_is_better", "scaling", "vs_baseline",
+                                "dtype", "data", "config", "clocks", "e2e", "gpu_launches", "device_status")}
+    out["roofline"] = {k: full["roofline"][k] for k in ("bound", "kernel", "achieved", "peak", "unit", "frac", "peak_source", "step_frac")}
+    for k in ("parity_ok", "collective", "cpu_baseline", "gpu_launches_all_workloads"):
+        if full.get(k) is not None:
+            out[k] = full[k]
+    if "workloads" in full:
+        out["workloads"] = {key: {"value": r["value"], "unit": r["unit"], "ms_per_step": r["ms_per_step"], "frac": r["roofline"]["step_frac"],
+                                  "e2e": r["e2e"]["value"], "ok": bool(r.get("parity_ok", True)) and r["device_status"] == 0}
+                            for key, r in full["workloads"].items()}
+    return short(out)
 
 
 def percentile(sorted_vals, q):
@@ -1277,7 +1303,8 @@ def main():
             out["workloads"] = others
             out["gpu_launches_all_workloads"] = out["gpu_launches"] + sum(r["gpu_launches"] for r in others.values())
     if out is not None:
-        print(json.dumps(out))
+        print("[bench] " + json.dumps(short(out)), file=sys.stderr)
+        print(json.dumps(contract_line(out)))
 
 
 if __name__ == "__main__":

@@ -40,3 +40,35 @@ def test_workload_tables_are_consistent():
         assert set(getattr(wl, "traffic", {})) <= parts
         assert set(getattr(wl, "all_reduced", ())) <= parts
         assert wl.unit in ("GB/s", "TFLOP/s") and wl.bound in ("hbm", "tensor") and wl.scaling in ("weak", "strong")
+
+
+def test_the_line_of_a_default_run_is_short_and_complete():
+    """Built from records as measure() makes them, with every number at full length."""
+    sys.path.insert(0, ROOT)
+    import bench
+    x = 1234.5678901234567
+    clocks = {"sm_mhz": x, "sm_max_mhz": x, "reasons": ["hw_slowdown", "hw_thermal_slowdown", "sw_thermal_slowdown", "sw_power_cap"], "samples": 999,
+              "window": "timed region and untimed repeats of the same step"}
+
+    def record(key):
+        wl = bench.WORKLOADS[key]
+        kernel = max(wl().kernel_of.values(), key=len)
+        return {"metric": wl.metric, "value": x, "unit": wl.unit, "n_gpus": 8, "steps": 50, "warmup": 5, "ms_per_step": x, "higher_is_better": True,
+                "scaling": wl.scaling, "vs_baseline": None, "dtype": wl.dtype, "data": "synthetic",
+                "config": {"workload": wl.description, "algorithmic_work_per_step": 10 ** 13, "l2": "no flush: " + "x" * 70, "parallelism": "dp8"},
+                "clocks": clocks, "e2e": {"value": x, "unit": wl.unit, "ms_per_step": x, "h2d_bytes_per_step": 10 ** 10, "d2h_bytes_per_step": 10 ** 10},
+                "gpu_launches": 10 ** 4, "collective": "peer-kernel (NVLink loads/stores, one launch per rank)", "collective_overlap": True,
+                "roofline": {"bound": wl.bound, "kernel": kernel, "parts": list(wl().work()), "achieved": x, "peak": x, "unit": wl.unit, "frac": x,
+                             "peak_source": "measured (burst)", "traffic": x, "step_frac": x, "note": "n" * 400},
+                "parts": [{"part": p, "ms": x} for p in wl().work()], "stability": {"repetitions": 300, "ms_median": x}, "cuda_graph": True,
+                "parts_timing": "p" * 60, "device_status": 0, "parity_ok": True,
+                "cpu_baseline": {"value": x, "unit": wl.unit, "cores": 128, "kind": "port", "sample": "s" * 150}}
+    full = dict(record(bench.HEADLINE), workloads={k: record(k) for k in bench.CONFIGS}, gpu_launches_all_workloads=10 ** 5)
+    line = json.dumps(bench.contract_line(full))
+    assert len(line) < 2900
+    d = json.loads(line)
+    for key in ("metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step", "higher_is_better", "scaling", "vs_baseline", "dtype", "data",
+                "config", "clocks", "e2e", "gpu_launches", "roofline", "cpu_baseline", "parity_ok", "device_status"):
+        assert key in d, key
+    assert set(d["workloads"]) == set(bench.CONFIGS) and all(r["ok"] and r["value"] > 0 for r in d["workloads"].values())
+    assert set(d["clocks"]) >= {"sm_mhz", "sm_max_mhz", "reasons"} and set(d["e2e"]) >= {"value", "unit", "h2d_bytes_per_step", "d2h_bytes_per_step"}
