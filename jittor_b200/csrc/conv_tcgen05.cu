@@ -51,8 +51,6 @@ struct ConvArgs {
     int last_k;                      // MMA steps of 16 channels in a tap's last channel block
 };
 
-__device__ __forceinline__ int first_block(int tm, int k_blocks) { return (int)((tm * 7u) % (unsigned)k_blocks); }
-
 // NCHW y: a warp turns its 32 pixels x 32 channels around in shared memory and stores rows of up to 8 pixels. (TMA box stores
 // of [8][8] pixels move a row of 16 bytes in 1.7 ns, whatever there is to it: 6.8 us for a 128 x 256 tile.)
 // NHWC ("acdb"): a lane stores the 32 consecutive channels of its pixel as four 16-byte vectors.
@@ -60,8 +58,9 @@ __device__ __forceinline__ int first_block(int tm, int k_blocks) { return (int)(
 // The epilogue's eight warps are two per TMEM lane quadrant, each with every other 32 channels: four warps took longer than the
 // main loop of a 1 x 1 layer (64 x 64 x 56 x 56 -> 256 channels with statistics, layout pass included: 142 us with four warps and
 // box stores, 87 us now).
-// Each tile walks K from a start of its own. All tiles read the same weights: in step with one another they queue at the L2
-// slices that hold the current 32 KB (7 x 432 x 28 x 28 -> 320 channels, 3 x 3: 60 us in step, 54 us this way).
+// Every tile walks K from its first tap, so that an image gives the same bits wherever it stands in a batch. (Starts spread over
+// the tiles, which keeps them from reading the same weights at the same time, were no faster: 814 and 806 us for 256 x 256 x 56 x 56,
+// 50 and 50 us for 7 x 432 x 28 x 28 -> 320.)
 template <bool NHWC, int BN_T, bool PAIR>
 __global__ void __launch_bounds__(THREADS, 1)
 conv_bf16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
@@ -110,8 +109,7 @@ conv_bf16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                 if (q >= A.pixels) q = 0;                       // a pair's second half past the last pixel: any pixels, none is stored
                 const int n = (int)(q / (A.OH * A.OW)), in = (int)(q - (int64_t)n * (A.OH * A.OW));
                 const int h = in / A.OW * A.sh - A.ph, w = in % A.OW * A.sw - A.pw;
-                int tap = first_block(tm, k_blocks) / cblocks, cb = first_block(tm, k_blocks) - tap * cblocks;
-                int kh = tap / A.KW, kw = tap - kh * A.KW;
+                int tap = 0, cb = 0, kh = 0, kw = 0;
                 for (int kb = 0; kb < k_blocks; kb++) {
                     if (!(ok = mbar_wait(empty + stage, phase ^ 1, abort_flag, 11))) break;
                     unsigned char* sa = smem + stage * STAGE_BYTES;
@@ -121,7 +119,7 @@ conv_bf16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                     tma_load_tile<CTAS>(sa + A_BYTES, &map_w, bar, cb * BK, tap * A.Co + tn * BN_T + rank * (BN_T / CTAS));
                     if (++cb == cblocks) {
                         cb = 0; tap++;
-                        if (++kw == A.KW) { kw = 0; if (++kh == A.KH) { kh = 0; tap = 0; } }
+                        if (++kw == A.KW) { kw = 0; kh++; }
                     }
                     if (++stage == STAGES) { stage = 0; phase ^= 1; }
                 }
@@ -143,7 +141,7 @@ conv_bf16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                 if (!(ok = mbar_wait<PAIR>(acc_empty + buf, acc_phase ^ 1, abort_flag, 12))) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t tmem_d = tmem_base + buf * BN;
-                int cb = first_block(t / A.tiles_n, k_blocks) % cblocks;
+                int cb = 0;
                 for (int kb = 0; kb < k_blocks; kb++) {
                     if (!(ok = mbar_wait(full + stage, phase, abort_flag, 13))) break;
                     if (++cb == cblocks) cb = 0;

@@ -106,6 +106,14 @@ def test_strided_input_gradient(n, ci, h, w, co, k, s, p, d):
     near(got, xd.grad)
 
 
+@pytest.mark.parametrize("ci,h,w,co,k,s,p", [(96, 20, 20, 64, 3, 1, 1), (200, 9, 13, 300, 3, 1, 1), (64, 28, 28, 128, 5, 2, 2), (320, 7, 7, 96, 1, 1, 0)])
+def test_an_image_gives_the_same_bits_at_every_place_of_a_batch(ci, h, w, co, k, s, p):
+    x = torch.randn(1, ci, h, w, device="cuda").bfloat16().expand(37, -1, -1, -1).contiguous()
+    wt = jt.array((torch.randn(co, ci, k, k, device="cuda") * 0.1).bfloat16())
+    y = nn.conv2d(jt.array(x), wt, None, s, p)
+    assert all(torch.equal(y.torch()[0], image) for image in y.torch())
+
+
 # filters that reach as far as an im2col map allows: corners at -128 and 127, shifts up to 255
 @pytest.mark.parametrize("n,ci,h,w,co,k,p,d", [(1, 64, 80, 72, 64, 3, 64, 64), (2, 8, 140, 131, 16, 3, 127, 127), (1, 16, 20, 9, 24, 2, 128, 255),
                                                (1, 24, 150, 160, 8, 2, 0, 128), (1, 8, 30, 30, 8, 1, 127, 1)])
