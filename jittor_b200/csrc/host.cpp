@@ -136,8 +136,11 @@ PyObject* var_get_op(VarObj* self, void*) {
         PyObject* b = self->builder;
         self->builder = nullptr;
         PyObject* op = PyObject_CallNoArgs(b);
+        if (!op) {                                          // asked again it fails the same way
+            if (none(self->builder)) Py_XSETREF(self->builder, b); else Py_DECREF(b);
+            return nullptr;
+        }
         Py_DECREF(b);
-        if (!op) return nullptr;
         Py_XSETREF(self->op, op);
     }
     return Py_NewRef(self->op ? self->op : Py_None);

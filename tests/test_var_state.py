@@ -1,5 +1,5 @@
 """What a Var holds besides its value: copies and pickles of it, assignment over it, which layers carry a record,
-which Vars a gradient reaches. No GPU: the values are CPU tensors that nothing computes with."""
+which Vars a gradient reaches, what a producer that fails raises. No GPU: the values are CPU tensors that nothing computes with."""
 import copy
 import pickle
 
@@ -155,3 +155,22 @@ def test_a_gradient_reaches_the_norm_under_a_relu():
     assert jt.grad(y.sum(), x)._relay[0] == "batch_norm_dx"           # one step where nothing asks for h
     h.assign(leaf(2, 4, 3, 3))
     assert not reaches(y.sum(), x) and reaches(y.sum(), h)
+
+
+def test_a_producer_that_fails_raises_its_own_error_each_time():
+    def build():
+        raise ValueError("no such graph")
+    v = V.LazyVar([2], "float32", build)
+    for _ in range(3):
+        with pytest.raises(ValueError, match="no such graph"):
+            v._op
+    with pytest.raises(ValueError, match="no such graph"):
+        jt.grad((v * v).sum(), leaf(2))
+
+
+@pytest.mark.gpu
+def test_sync_of_a_producer_that_fails_raises_its_own_error():
+    def build():
+        raise ValueError("no such graph")
+    with pytest.raises(ValueError, match="no such graph"):
+        (V.LazyVar([2], "float32", build) * 2.0).sync()
