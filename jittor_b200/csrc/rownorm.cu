@@ -59,6 +59,10 @@ template <typename T> struct Single {
     static __device__ __forceinline__ void store(T* p, const float* in) { st1<T>(p, in[0]); }
 };
 
+// Softmax of a row is that of the row less any constant, and m * log2e overflows in a row of the type's lowest values (one that
+// is masked as a whole): below this maximum the row is shifted to 0 first.
+constexpr float kLowRow = -1e38f;
+
 __device__ __forceinline__ float ex2_approx(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -222,6 +226,13 @@ row_reg_kernel(const T* __restrict__ x, T* __restrict__ y, const float* __restri
 #pragma unroll
             for (int r = 0; r < RPI; r++) {
                 sum[r] = 0.f;
+                if (OP == ROW_SOFTMAX && m[r] < kLowRow) {
+#pragma unroll
+                    for (int k = 0; k < VPT; k++)
+#pragma unroll
+                        for (int e = 0; e < N; e++) if (t + k * GROUP < nvec) v[r][k][e] -= m[r];
+                    m[r] = 0.f;
+                }
 #pragma unroll
                 for (int k = 0; k < VPT; k++)
 #pragma unroll
@@ -345,6 +356,13 @@ row_cluster_kernel(const T* __restrict__ x, T* __restrict__ y, const float* __re
                 for (int e = 0; e < N; e++) m[0] = fmaxf(m[0], v[k][e]);
             cluster_reduce_n<CL, true, 1>(m, sm, xch, slot);
             float sum[1] = {0.f};
+            if (OP == ROW_SOFTMAX && m[0] < kLowRow) {
+#pragma unroll
+                for (int k = 0; k < VPT; k++)
+#pragma unroll
+                    for (int e = 0; e < N; e++) if (crank * 256 + t + k * 256 * CL < nvec) v[k][e] -= m[0];
+                m[0] = 0.f;
+            }
 #pragma unroll
             for (int k = 0; k < VPT; k++)
 #pragma unroll

@@ -114,3 +114,23 @@ def test_batch_norm_sums_over_more_than_2_31_elements_of_a_channel():
     assert abs(sums[0].item() - n * h * w) <= 1e-6 * n * h * w          # each thread counts up to 2^23 ones: exact until the threads meet
     del x
     torch.cuda.empty_cache()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("cols", [7, 255, 256, 1001, 1024, 4100, 8191, 8192, 16384, 32768, 40001])
+def test_softmax_of_rows_that_are_masked_as_a_whole(cols, dtype):
+    """Rows of the type's lowest value, as an additive mask leaves them, are rows of equal elements."""
+    low = torch.finfo(dtype).min
+    x = torch.full((4, cols), low, device="cuda", dtype=dtype)
+    x[1, cols // 2] = 1.0
+    x[2, 0], x[2, 1:] = -3e38, low
+    x[3] = torch.linspace(-2e38, -1.9e38, cols, device="cuda").to(dtype)
+    for log in (False, True):
+        got = nn.softmax(jt.array(x), -1, log).torch().double()
+        want = torch.log_softmax(x.double(), -1) if log else torch.softmax(x.double(), -1)
+        assert torch.isfinite(got[:2]).all() and not got.isnan().any()
+        tol = 1e-5 if dtype == torch.float32 else 2 ** -7
+        if log:                                               # differences of huge numbers: what float32 holds of them
+            assert torch.allclose(got[:1], want[:1], rtol=tol, atol=0)
+        else:
+            assert torch.allclose(got, want, rtol=tol, atol=1e-30)
