@@ -460,7 +460,7 @@ template <typename T, int OP>
 static int launch_rows(const T* x, T* y, const float* gamma, const float* beta, int64_t rows, int64_t cols,
                        float eps, cudaStream_t st) {
     constexpr int N = Vec16<T>::N;
-    const bool vec_ok = cols % N == 0 && ((uintptr_t)x % 16 == 0) && ((uintptr_t)y % 16 == 0);
+    const bool vec_ok = cols % N == 0 && (((uintptr_t)x | (uintptr_t)y | (uintptr_t)gamma | (uintptr_t)beta) & 15) == 0;
     const int64_t nvec = cols / N;
 #define B200JT_ROW(GROUP, VPT)                                                                      \
     do { const int rpc = 256 / GROUP;                                                               \

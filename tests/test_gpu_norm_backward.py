@@ -134,3 +134,18 @@ def test_softmax_of_rows_that_are_masked_as_a_whole(cols, dtype):
             assert torch.allclose(got[:1], want[:1], rtol=tol, atol=0)
         else:
             assert torch.allclose(got, want, rtol=tol, atol=1e-30)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("cols", [8, 256, 1024, 4096, 8192, 16384])
+@pytest.mark.parametrize("which", [(0,), (1,), (0, 1)])
+def test_layer_norm_parameters_at_odd_addresses(cols, dtype, which):
+    """Parameters that are views into a larger tensor, four bytes off, beside rows at 16-byte addresses."""
+    x = torch.randn(5, cols, device="cuda").to(dtype)
+    par = [1 + 0.1 * torch.randn(cols, device="cuda"), torch.randn(cols, device="cuda")]
+    for i in which:
+        par[i] = torch.cat([par[i][:1], par[i]])[1:]
+        assert par[i].data_ptr() % 16
+    y = nn.layer_norm(jt.array(x), (cols,), jt.array(par[0]), jt.array(par[1]))
+    want = torch.nn.functional.layer_norm(x.double(), (cols,), par[0].double(), par[1].double())
+    near(y.torch(), want, 1e-5 if dtype == torch.float32 else 6e-3)
