@@ -1125,7 +1125,9 @@ PyObject* m_setup_graph(PyObject*, PyObject* args) {
 }
 
 // optim_step(kind, params, grads, states0, states1 or None, hyper, nesterov) -> False where a tensor is not float32 on the GPU.
-// The new values of one step live in one flat buffer per slot; the Vars are rebound to views of it.
+// The new values of a step live in flat buffers per slot that hold up to kPackFloats elements of small parameters; the Vars are
+// rebound to views of them. Whoever keeps one parameter of a step keeps its buffer: 1 MB at most, or a large parameter's own.
+constexpr int64_t kPackFloats = 1 << 18;
 decltype(&b200jt_optim_step) g_optim = nullptr;
 PyObject* m_optim_step(PyObject*, PyObject* args) {
     const char* kind;
@@ -1138,7 +1140,6 @@ PyObject* m_optim_step(PyObject*, PyObject* args) {
     if (!g_optim || n == 0) Py_RETURN_FALSE;
     std::vector<const float*> in[4];
     std::vector<int64_t> sizes;
-    int64_t total = 0;
     for (int l = 0; l < (two ? 4 : 3); l++) {
         if (!PyList_Check(lists[l]) || PyList_GET_SIZE(lists[l]) != n) { PyErr_SetString(PyExc_ValueError, "optim_step: lists differ in length"); return nullptr; }
         for (Py_ssize_t i = 0; i < n; i++) {
@@ -1146,7 +1147,7 @@ PyObject* m_optim_step(PyObject*, PyObject* args) {
             if (!is_var(v) || none(V(v)->data) || !THPVariable_Check(V(v)->data)) Py_RETURN_FALSE;
             const at::Tensor& t = THPVariable_Unpack(V(v)->data);
             if (!t.is_cuda() || !t.is_contiguous() || t.scalar_type() != at::kFloat || (l && t.numel() != sizes[i])) Py_RETURN_FALSE;
-            if (l == 0) { sizes.push_back(t.numel()); total += (t.numel() + 3) / 4 * 4; }
+            if (l == 0) sizes.push_back(t.numel());
             in[l].push_back((const float*)t.const_data_ptr());
         }
     }
@@ -1157,24 +1158,29 @@ PyObject* m_optim_step(PyObject*, PyObject* args) {
     {
         const auto device = c10::Device(c10::kCUDA, c10::cuda::current_device());
         static const int slot[3] = {0, 2, 3};
-        at::Tensor flat[3];
+        std::vector<int64_t> total;                                        // of each buffer
+        std::vector<std::pair<size_t, int64_t>> place;                     // of each parameter: (buffer, offset)
+        for (int64_t s : sizes) {
+            const int64_t room = (s + 3) / 4 * 4;
+            if (total.empty() || total.back() + room > kPackFloats) total.push_back(0);
+            place.emplace_back(total.size() - 1, total.back());
+            total.back() += room;
+        }
+        std::vector<at::Tensor> flat[3];
         std::vector<float*> out[3];
         for (int o = 0; o < (two ? 3 : 2); o++) {
-            flat[o] = at::Tensor(at::detail::empty_cuda({total}, at::kFloat, device, std::nullopt));
-            float* base = (float*)flat[o].data_ptr();
-            for (int64_t s : sizes) { out[o].push_back(base); base += (s + 3) / 4 * 4; }
+            for (int64_t t : total) flat[o].push_back(at::Tensor(at::detail::empty_cuda({t}, at::kFloat, device, std::nullopt)));
+            for (auto& p : place) out[o].push_back((float*)flat[o][p.first].data_ptr() + p.second);
         }
         const int rc = g_optim(kind, (int)n, sizes.data(), in[0].data(), in[1].data(), in[2].data(), two ? in[3].data() : nullptr, out[0].data(), out[1].data(),
                                two ? out[2].data() : nullptr, h.data(), (int)h.size(), nesterov, (void*)c10::cuda::getCurrentCUDAStream().stream());
         if (rc) { PyErr_Format(h_error, "optim_step: %s (status %d)", g_last_error ? g_last_error() : "", rc); return nullptr; }
         for (int o = 0; o < (two ? 3 : 2); o++) {
-            int64_t at = 0;
             for (Py_ssize_t i = 0; i < n; i++) {
                 VarObj* v = V(PyList_GET_ITEM(lists[slot[o]], i));
                 const at::Tensor& old = THPVariable_Unpack(v->data);
-                PyObject* py = THPVariable_Wrap(flat[o].as_strided(old.sizes(), old.strides(), at));
+                PyObject* py = THPVariable_Wrap(flat[o][place[i].first].as_strided(old.sizes(), old.strides(), place[i].second));
                 if (!py) return nullptr;
-                at += (sizes[i] + 3) / 4 * 4;
                 Py_XSETREF(v->data, py);
                 // as Var.assign: nothing describes the value it held before
                 Py_CLEAR(v->builder); Py_CLEAR(v->relay); Py_CLEAR(v->vjp); Py_CLEAR(v->bn_running); Py_CLEAR(v->konst);

@@ -288,6 +288,28 @@ def test_many_tensor_update_has_the_bits_of_the_op_by_op_rule(kind):
         assert torch.equal(a, b)
 
 
+@pytest.mark.parametrize("kind", ["sgd", "adam"])
+def test_a_parameter_kept_from_a_step_keeps_little_else(kind):
+    from jittor_b200 import optim
+    params = [data(1, 1024, 4096), data(2, 10), data(3, 300, 1000), data(4, 7)]
+    opt = optim.SGD(params, 0.1, momentum=0.9) if kind == "sgd" else optim.Adam(params, 1e-3)
+    kept = []
+
+    def step():
+        loss = None
+        for p in params:
+            loss = (p * p).sum() if loss is None else loss + (p * p).sum()
+        opt.step(loss)
+    step()
+    step()
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated()
+    for _ in range(6):
+        step()
+        kept += [params[1].torch(), params[3].torch()]
+    assert torch.cuda.memory_allocated() - before <= 12 << 20           # two buffers of at most 1 MB a step; the weights are 17 MB
+
+
 @pytest.mark.parametrize("rows,dim,vocab,skew", [(1, 16, 5, 0), (3, 17, 2, 0), (127, 16, 3, 1), (129, 36, 40, 0), (1000, 64, 7, 0), (2500, 132, 900, 0), (40000, 20, 11, 0),
                                                  (90000, 128, 3000, 0)])
 def test_row_gather_and_folded_row_scatter(rows, dim, vocab, skew):
