@@ -336,7 +336,10 @@ struct Walk {
         }
     }
     void run(const std::vector<VarObj*>& roots) {
-        key.reserve(2048);
+        key.reserve(1 << 13);                            // a training step of a small network is 150 nodes and 10 KB
+        index.reserve(256);
+        held.reserve(256);
+        nodes.reserve(128);
         flag(s_fuse); flag(s_wgrad);
         num(g_context);
         if (c10::cuda::device_count() < 1) { ok = false; return; }
