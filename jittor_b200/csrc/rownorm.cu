@@ -226,7 +226,7 @@ row_reg_kernel(const T* __restrict__ x, T* __restrict__ y, const float* __restri
 #pragma unroll
             for (int r = 0; r < RPI; r++) {
                 sum[r] = 0.f;
-                if (OP == ROW_SOFTMAX && m[r] < kLowRow) {
+                if (OP == ROW_SOFTMAX && __builtin_expect(m[r] < kLowRow, 0)) {
 #pragma unroll
                     for (int k = 0; k < VPT; k++)
 #pragma unroll
@@ -356,7 +356,7 @@ row_cluster_kernel(const T* __restrict__ x, T* __restrict__ y, const float* __re
                 for (int e = 0; e < N; e++) m[0] = fmaxf(m[0], v[k][e]);
             cluster_reduce_n<CL, true, 1>(m, sm, xch, slot);
             float sum[1] = {0.f};
-            if (OP == ROW_SOFTMAX && m[0] < kLowRow) {
+            if (OP == ROW_SOFTMAX && __builtin_expect(m[0] < kLowRow, 0)) {
 #pragma unroll
                 for (int k = 0; k < VPT; k++)
 #pragma unroll
