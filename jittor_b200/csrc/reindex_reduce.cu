@@ -353,44 +353,66 @@ rr_flat_kernel(const T* __restrict__ y, T* __restrict__ x, const __grid_constant
 // Loads are issued UNROLL vectors ahead so that enough bytes are in flight per SM to cover HBM latency.
 // f(bin, value, valid) is called by all 32 lanes of a warp together (valid == false on lanes past the end), so
 // that warp-collective code may run inside it.
-template <typename T, typename E, int VEC, int UNROLL, typename F>
+// AHEAD: the next UNROLL vectors are loaded before the current ones are handed to f, for an f that takes as long as the loads.
+template <typename T, typename E, int VEC, int UNROLL, bool AHEAD = false, typename F>
 __device__ __forceinline__ void for_each_pair(const T* __restrict__ y, const E* __restrict__ idx, int64_t n, F&& f) {
     const int64_t n_vec = n / VEC;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     const int lane = threadIdx.x & 31;
-    for (int64_t w0 = blockIdx.x * (int64_t)blockDim.x + (threadIdx.x - lane); w0 < n_vec; w0 += stride * UNROLL) {
+    struct Batch { __align__(16) T val[UNROLL][VEC]; __align__(16) E ind[UNROLL][VEC]; };
+    auto load = [&](Batch& q, int64_t w0) {
         const int64_t v0 = w0 + lane;
-        __align__(16) T val[UNROLL][VEC];
-        __align__(16) E ind[UNROLL][VEC];
 #pragma unroll
         for (int u = 0; u < UNROLL; u++) {
             const int64_t v = v0 + u * stride;
             if (v < n_vec) {
-                if constexpr (VEC * sizeof(T) == 16) *reinterpret_cast<uint4*>(val[u]) = __ldcs(reinterpret_cast<const uint4*>(y) + v);
+                if constexpr (VEC * sizeof(T) == 16) *reinterpret_cast<uint4*>(q.val[u]) = __ldcs(reinterpret_cast<const uint4*>(y) + v);
                 else {
 #pragma unroll
-                    for (int e = 0; e < VEC; e++) val[u][e] = y[v * VEC + e];
+                    for (int e = 0; e < VEC; e++) q.val[u][e] = y[v * VEC + e];
                 }
-                if constexpr (VEC * sizeof(E) == 16) *reinterpret_cast<uint4*>(ind[u]) = __ldcs(reinterpret_cast<const uint4*>(idx) + v);
+                if constexpr (VEC * sizeof(E) == 16) *reinterpret_cast<uint4*>(q.ind[u]) = __ldcs(reinterpret_cast<const uint4*>(idx) + v);
                 else if constexpr (VEC * sizeof(E) == 32) {
-                    *reinterpret_cast<uint4*>(ind[u]) = __ldcs(reinterpret_cast<const uint4*>(idx) + 2 * v);
-                    *reinterpret_cast<uint4*>(ind[u] + VEC / 2) = __ldcs(reinterpret_cast<const uint4*>(idx) + 2 * v + 1);
+                    *reinterpret_cast<uint4*>(q.ind[u]) = __ldcs(reinterpret_cast<const uint4*>(idx) + 2 * v);
+                    *reinterpret_cast<uint4*>(q.ind[u] + VEC / 2) = __ldcs(reinterpret_cast<const uint4*>(idx) + 2 * v + 1);
                 } else {
 #pragma unroll
-                    for (int e = 0; e < VEC; e++) ind[u][e] = idx[v * VEC + e];
+                    for (int e = 0; e < VEC; e++) q.ind[u][e] = idx[v * VEC + e];
                 }
             } else {
 #pragma unroll
-                for (int e = 0; e < VEC; e++) { ind[u][e] = (E)-1; val[u][e] = T(); }
+                for (int e = 0; e < VEC; e++) { q.ind[u][e] = (E)-1; q.val[u][e] = T(); }
             }
         }
+    };
+    auto apply = [&](const Batch& q, int64_t w0) {
 #pragma unroll
         for (int u = 0; u < UNROLL; u++) {
             if (w0 + u * stride < n_vec) {                       // warp-uniform
-                const bool valid = v0 + u * stride < n_vec;
+                const bool valid = w0 + lane + u * stride < n_vec;
 #pragma unroll
-                for (int e = 0; e < VEC; e++) f((int64_t)ind[u][e], val[u][e], valid);
+                for (int e = 0; e < VEC; e++) f((int64_t)q.ind[u][e], q.val[u][e], valid);
             }
+        }
+    };
+    int64_t w0 = blockIdx.x * (int64_t)blockDim.x + (threadIdx.x - lane);
+    if constexpr (AHEAD) {
+        Batch p, q;
+        if (w0 < n_vec) load(p, w0);
+        while (w0 < n_vec) {
+            const int64_t w1 = w0 + stride * UNROLL;
+            load(q, w1);
+            apply(p, w0);
+            if (w1 >= n_vec) break;
+            w0 = w1 + stride * UNROLL;
+            load(p, w0);
+            apply(q, w1);
+        }
+    } else {
+        for (; w0 < n_vec; w0 += stride * UNROLL) {
+            Batch p;
+            load(p, w0);
+            apply(p, w0);
         }
     }
     for (int64_t w = n_vec * VEC + blockIdx.x * (int64_t)blockDim.x + (threadIdx.x - lane); w < n; w += stride) {
@@ -453,19 +475,20 @@ rr_direct_kernel(const T* __restrict__ y, const E* __restrict__ idx, T* __restri
 // with one atomic per warp and hot bin.
 constexpr int kHot = 4;
 
-template <typename T, typename E, int VEC>
+template <typename T, typename E, int VEC, bool ADD>
 __global__ void __launch_bounds__(kPrivThreads, 1)
 rr_privatised_kernel(const T* __restrict__ y, const E* __restrict__ idx, T* __restrict__ partial,
-                     int64_t n, int bins, int replicas, int op, bool is_bool, bool allow_hot) {
+                     int64_t n, int bins, int replicas, int op_, bool is_bool, bool allow_hot) {
+    const int op = ADD ? (int)OP_ADD : op_;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T* sm = reinterpret_cast<T*>(smem_raw);
     const int rstride = bins + 1;
     const T init = init_value<T>(op, is_bool);
     __shared__ int hot_bin[kHot];
     __shared__ unsigned warp_best[kPrivThreads / 32];
-    constexpr bool kHotPath = std::is_same<T, float>::value && VEC > 1;
+    constexpr bool kHotPath = ADD && std::is_same<T, float>::value && VEC > 1;
     bool use_hot = false;
-    if (kHotPath && allow_hot && op == OP_ADD && bins < 8192 && n / VEC >= (int64_t)gridDim.x * blockDim.x * 8) {
+    if (kHotPath && allow_hot && bins < 8192 && n / VEC >= (int64_t)gridDim.x * blockDim.x * 8) {
         // histogram of the sample in the (not yet initialised) replica area
         int* hist = reinterpret_cast<int*>(smem_raw);
         for (int i = threadIdx.x; i < bins; i += blockDim.x) hist[i] = 0;
@@ -512,7 +535,7 @@ rr_privatised_kernel(const T* __restrict__ y, const E* __restrict__ idx, T* __re
         int hb[kHot];
 #pragma unroll
         for (int k = 0; k < kHot; k++) hb[k] = use_hot ? hot_bin[k] : -2;
-        for_each_pair<T, E, VEC, 4>(y, idx, n, [&](int64_t b, T v, bool valid) {
+        for_each_pair<T, E, VEC, 2, true>(y, idx, n, [&](int64_t b, T v, bool valid) {
             const int bi = (int)b;
             bool hit = false;
 #pragma unroll
@@ -533,7 +556,7 @@ rr_privatised_kernel(const T* __restrict__ y, const E* __restrict__ idx, T* __re
             }
         }
     } else {
-        for_each_pair<T, E, VEC, 4>(y, idx, n, [&](int64_t b, T v, bool valid) {
+        for_each_pair<T, E, VEC, 2, true>(y, idx, n, [&](int64_t b, T v, bool valid) {
             if (valid && b >= 0 && b < bins) atomic_apply<T>(mine + b, v, op);
         });
     }
@@ -715,8 +738,10 @@ static int run_typed(const b200jt_tensor* y, const b200jt_tensor* x, int op, con
         const bool allow_hot = !(hot_env && hot_env[0] == '0');
         // the shared-memory opt-in is set once per instantiation, not on every launch
 #define B200JT_PRIV(E, V)                                                                                      \
-        do { auto k = rr_privatised_kernel<T, E, V>;                                                            \
-             static const cudaError_t attr_ = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kPrivMaxSmemBytes); \
+        do { auto k = op == OP_ADD ? rr_privatised_kernel<T, E, V, true> : rr_privatised_kernel<T, E, V, false>; \
+             static const cudaError_t attr_ = [] {                                                               \
+                 const cudaError_t e = cudaFuncSetAttribute(rr_privatised_kernel<T, E, V, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPrivMaxSmemBytes); \
+                 return e != cudaSuccess ? e : cudaFuncSetAttribute(rr_privatised_kernel<T, E, V, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPrivMaxSmemBytes); }(); \
              B200JT_CUDA(attr_);                                                                                  \
              k<<<priv_grid, kPrivThreads, plan.smem, st>>>(yp, (const E*)P.extras[0].ptr, partial, n, (int)bins,   \
                                                            plan.replicas, op, is_bool, allow_hot); } while (0)
