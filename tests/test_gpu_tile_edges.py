@@ -23,3 +23,18 @@ def test_few_bins(n, dtype, idx, op):
     else:
         want = torch.full((bins,), -1e9, device="cuda", dtype=torch.float64).scatter_reduce_(0, i[ok].long(), v[ok].double(), "amax")
     assert torch.equal(got.double(), want)
+
+
+# ---- softmax backward: rows in registers with the next one on its way, and rows of up to 16384 columns
+@pytest.mark.parametrize("log", [0, 1])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rows,cols", [(5, 8), (9500, 40), (2369, 2048), (4740, 1001), (3, 8192), (3, 8193), (150, 8200), (2, 12001), (2400, 16384), (2, 16383), (2, 16400)])
+def test_softmax_backward(rows, cols, dtype, log):
+    x = torch.randn(rows, cols, device="cuda")
+    y = (torch.log_softmax(x, 1) if log else torch.softmax(x, 1)).to(dtype)
+    dy, dx = torch.randn(rows, cols, device="cuda").to(dtype), torch.full((rows, cols), float("nan"), device="cuda", dtype=dtype)
+    C.call("b200jt_softmax_backward", C.desc(y), C.desc(dy), C.desc(dx), log)
+    yd, dd = y.double(), dy.double()
+    want = dd - yd.exp() * dd.sum(1, keepdim=True) if log else yd * (dd - (yd * dd).sum(1, keepdim=True))
+    tol = 2.0 ** -8 if dtype == torch.bfloat16 else 1e-5
+    assert (dx.double() - want).norm() <= tol * want.norm()
