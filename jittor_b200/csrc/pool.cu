@@ -290,7 +290,7 @@ static int window_code(const Geo& g) {
 // shared by the windows above and below, the place of a maximum comes from comparisons with the 3-input maximum, and the
 // position of the first extreme element is kept as ONE byte (its place in the window) instead of a 4-byte index -- the map
 // is written forward and read backward, 103 MB each way for [64,128,112,112] with int32. 3x3 s2 p1 on that shape, float32:
-// forward 0.142 -> 0.098 ms, backward 0.161 -> 0.086 ms (0.96 of HBM).
+// forward 0.142 -> 0.091 ms, backward 0.161 -> 0.086 ms (0.96 of HBM).
 template <typename T, int N> __device__ __forceinline__ void load_n(const T* p, float* o) {
     if constexpr (N == 1) o[0] = ld<T>(p);
     else if constexpr (sizeof(T) * N > 16) { load_n<T, N / 2>(p, o); load_n<T, N / 2>(p + N / 2, o + N / 2); }
@@ -323,8 +323,10 @@ template <typename T, int N, int A> __device__ __forceinline__ void load_row(con
     }
 }
 
-// output rows of a tile: enough loads in flight without running out of registers
+// output rows of a tile: enough loads in flight without running out of registers. Forward, float32 3x3 s2 p1 on [64,128,112,112]: 102 us
+// with 4 rows and 88 registers, 91 with 2 and 48; single outputs a thread (57 x 57) 43 with 4 and 47 with 2.
 constexpr int rows_up(int vo) { return vo >= 4 ? 2 : 4; }
+constexpr int rows_up_fwd(int vo) { return vo >= 2 ? 2 : 4; }
 struct TileMap {                                // flat thread index -> (plane, tile row, tile column)
     int cols, rows;
     int64_t threads;
@@ -350,7 +352,7 @@ struct TileMap {                                // flat thread index -> (plane, 
 template <typename T, bool MEAN, int K, int S, int PAD, int VO, int AX>
 __global__ void __launch_bounds__(256) pool_fwd_tile_kernel(const T* __restrict__ x, T* __restrict__ y, int32_t* __restrict__ indices,
                                                             uint8_t* __restrict__ taps, const Geo g, const TileMap map, float init, float sign) {
-    constexpr int RU = rows_up(VO), ROWS = (RU - 1) * S + K, SPAN = (VO - 1) * S + K;
+    constexpr int RU = rows_up_fwd(VO), ROWS = (RU - 1) * S + K, SPAN = (VO - 1) * S + K;
     constexpr int RIGHT = SPAN - PAD - VO * S > 0 ? SPAN - PAD - VO * S : 0;
     int64_t plane;
     int r, c;
@@ -572,7 +574,7 @@ static void launch_fwd(const T* xp, T* yp, int32_t* indices, uint8_t* taps, cons
             else init_f = __bfloat162float(init);
             const float sign = OP == 1 ? -1.f : 1.f;
             dispatch_tile<T>(g, xp, yp, taps, [&](auto k, auto s, auto p, auto vo, auto ax) {
-                const TileMap m = tile_map(g, g.OH, g.OW, rows_up(vo()), vo());
+                const TileMap m = tile_map(g, g.OH, g.OW, rows_up_fwd(vo()), vo());
                 pool_fwd_tile_kernel<T, OP == 2, k(), s(), p(), vo(), ax()><<<(unsigned)((m.threads + 255) / 256), 256, 0, st>>>(
                     xp, yp, indices, taps, g, m, init_f * sign, sign);
             });

@@ -38,3 +38,18 @@ def test_softmax_backward(rows, cols, dtype, log):
     want = dd - yd.exp() * dd.sum(1, keepdim=True) if log else yd * (dd - (yd * dd).sum(1, keepdim=True))
     tol = 2.0 ** -8 if dtype == torch.bfloat16 else 1e-5
     assert (dx.double() - want).norm() <= tol * want.norm()
+
+
+# ---- pooling forward: two rows of two outputs to a thread (csrc/pool.cu)
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("k,stride,pad", [(2, 2, 0), (3, 2, 1), (3, 2, 0), (3, 1, 1)])
+@pytest.mark.parametrize("h,w", [(3, 8), (5, 16), (8, 12), (11, 9), (10, 32), (13, 20)])
+def test_pool_forward(h, w, k, stride, pad, dtype):
+    import jittor_b200 as jt
+    from jittor_b200 import pool
+    x = torch.randn(3, 5, h, w, device="cuda").to(dtype)
+    got = pool.max_pool2d(jt.array(x), k, stride, pad).torch()
+    assert torch.equal(got, torch.nn.functional.max_pool2d(x, k, stride, pad))
+    got = pool.avg_pool2d(jt.array(x), k, stride, pad).torch()
+    want = torch.nn.functional.avg_pool2d(x.double(), k, stride, pad)
+    assert (got.double() - want).abs().max() <= (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -21) * want.abs().max()
