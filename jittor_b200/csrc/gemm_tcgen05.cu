@@ -52,30 +52,37 @@ template <bool PAIR, int MT> struct Cfg {
 struct GemmArgs {
     int M, N, K;
     int tiles_m, tiles_n, bn, k_blocks;
-    int units;                     // splits x batch x tiles_m x tiles_n work items
+    int units;                     // work items: batch x tiles, or `whole` tiles and then splits x the others
     int batch, splits, group;      // group: tile-rows that are walked together (L2 reuse of the Bt tiles)
+    int whole;                     // tiles that are not split (splits > 1)
     int a_batched, b_batched;      // an operand whose batch extent is 1 is shared by all products
-    int pitch;                     // of a row of partial sums (splits > 1)
 };
 
-struct Unit { int split, batch, tm, tn, kb0, kb1; };
+struct Unit { int batch, tm, tn, kb0, kb1, part; };      // part: place among the partial tiles, -1: the product itself
+__device__ __forceinline__ void tile_at(const GemmArgs& A, int t, int& tm, int& tn) {
+    const int per_group = A.group * A.tiles_n, g = t / per_group, r = t - g * per_group;
+    const int rows = min(A.group, A.tiles_m - g * A.group);
+    tm = g * A.group + r % rows; tn = r / rows;
+}
 __device__ __forceinline__ Unit unit_at(const GemmArgs& A, int u) {
     Unit w;
     const int tiles = A.tiles_m * A.tiles_n;
-    int i = u / tiles;
-    const int t = u - i * tiles;
-    w.split = i / A.batch; w.batch = i - w.split * A.batch;
-    const int per_group = A.group * A.tiles_n, g = t / per_group, r = t - g * per_group;
-    const int rows = min(A.group, A.tiles_m - g * A.group);
-    w.tm = g * A.group + r % rows; w.tn = r / rows;
-    w.kb0 = (int)((int64_t)A.k_blocks * w.split / A.splits);
-    w.kb1 = (int)((int64_t)A.k_blocks * (w.split + 1) / A.splits);
+    w.batch = 0; w.kb0 = 0; w.kb1 = A.k_blocks; w.part = -1;
+    if (A.splits == 1) { w.batch = u / tiles; u -= w.batch * tiles; }
+    else if (u >= A.whole) {
+        w.part = u - A.whole;
+        const int others = tiles - A.whole, split = w.part / others;
+        u -= split * others;
+        w.kb0 = (int)((int64_t)A.k_blocks * split / A.splits);
+        w.kb1 = (int)((int64_t)A.k_blocks * (split + 1) / A.splits);
+    }
+    tile_at(A, u, w.tm, w.tn);
     return w;
 }
 
 // AMN / BMN: the operand's own axis (M / N) is the contiguous one in memory; it is then loaded in 64 x 64 boxes and used
 // as an MN-major operand, so no operand is ever transposed by a pass of its own.
-// Accumulators leave as bf16 in c, or -- when K is split -- as fp32 partial sums in part[split][M][pitch], which
+// Accumulators leave as bf16 in c, or -- where K is split -- as fp32 partial tiles in part[split][split tile][TILE_M][bn], which
 // fold_kernel adds in split order. The tensor maps are 3-D ([batch][rows][cols]).
 template <bool PAIR, int MT, bool AMN, bool BMN>
 __global__ void __launch_bounds__(THREADS, 1)
@@ -212,13 +219,12 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                     uint32_t r[32];
                     tmem_ld32(taddr + ch, r);
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                    if (A.splits > 1) {
-                        float* prow = part + ((int64_t)w.split * A.M + row) * A.pitch + col0;
+                    if (w.part >= 0) {
+                        float* prow = part + ((int64_t)w.part * F::TILE_M + row - w.tm * F::TILE_M) * A.bn + ch;
                         if (row < A.M) {
 #pragma unroll
                             for (int q = 0; q < 8; q++)
-                                if (col0 + q * 4 < A.pitch)
-                                    *reinterpret_cast<uint4*>(prow + q * 4) = make_uint4(r[q * 4], r[q * 4 + 1], r[q * 4 + 2], r[q * 4 + 3]);
+                                *reinterpret_cast<uint4*>(prow + q * 4) = make_uint4(r[q * 4], r[q * 4 + 1], r[q * 4 + 2], r[q * 4 + 3]);
                         }
                         continue;
                     }
@@ -261,29 +267,33 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     }
 }
 
-// c[m][n] = sum over splits (ascending) of part[split][m][n], rounded to bf16 once; four columns per thread.
+// The split tiles' elements: sums over splits (ascending) of the partial tiles, rounded to bf16 once; four columns per thread.
 __global__ void __launch_bounds__(256)
-fold_kernel(const float* __restrict__ part, __nv_bfloat16* __restrict__ c, int M, int N, int pitch, int splits) {
-    const int quads = pitch / 4;
-    const int64_t n = (int64_t)M * quads, plane = (int64_t)M * pitch;
-    const bool vec = N % 4 == 0 && ((uintptr_t)c & 7) == 0;
+fold_kernel(const float* __restrict__ part, __nv_bfloat16* __restrict__ c, const __grid_constant__ GemmArgs A, int tile_m) {
+    const int quads = A.bn / 4, others = A.tiles_m * A.tiles_n - A.whole;
+    const int64_t per_tile = (int64_t)tile_m * quads, n = others * per_tile;
+    const bool vec = A.N % 4 == 0 && ((uintptr_t)c & 7) == 0;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const int t = (int)(i / per_tile), q = (int)(i - t * per_tile), r = q / quads;
+        int tm, tn;
+        tile_at(A, A.whole + t, tm, tn);
+        const int m = tm * tile_m + r, col = tn * A.bn + (q - r * quads) * 4;
+        if (m >= A.M || col >= A.N) continue;
         float4 acc = __ldcs(reinterpret_cast<const float4*>(part) + i);
-        for (int s = 1; s < splits; s++) {
-            const float4 v = __ldcs(reinterpret_cast<const float4*>(part + s * plane) + i);
+        for (int s = 1; s < A.splits; s++) {
+            const float4 v = __ldcs(reinterpret_cast<const float4*>(part) + s * n + i);
             acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
         }
-        const int64_t m = i / quads; const int col = (int)(i - m * quads) * 4;
-        __nv_bfloat16* out = c + m * N + col;
+        __nv_bfloat16* out = c + (int64_t)m * A.N + col;
         const __nv_bfloat162 lo = __floats2bfloat162_rn(acc.x, acc.y), hi = __floats2bfloat162_rn(acc.z, acc.w);
         if (vec) {
             uint2 v; *reinterpret_cast<__nv_bfloat162*>(&v.x) = lo; *reinterpret_cast<__nv_bfloat162*>(&v.y) = hi;
             *reinterpret_cast<uint2*>(out) = v;
         } else {
             out[0] = lo.x;
-            if (col + 1 < N) out[1] = lo.y;
-            if (col + 2 < N) out[2] = hi.x;
-            if (col + 3 < N) out[3] = hi.y;
+            if (col + 1 < A.N) out[1] = lo.y;
+            if (col + 2 < A.N) out[2] = hi.x;
+            if (col + 3 < A.N) out[3] = hi.y;
         }
     }
 }
@@ -376,13 +386,13 @@ static int pair_slots() {
     return slots;
 }
 
-struct Plan { bool pair; int mt, bn, splits; double ns; };
+struct Plan { bool pair; int mt, bn, splits; int64_t whole; double ns; };
 
 // Tile and split by estimated time. A k-block costs the larger of its MMAs (11 TFLOP/s per SM) and its operands' way from L2
 // (about 110 B per ns and SM); a tile adds its epilogue where no second accumulator hides it; split K adds the way of the partial
 // sums out and back and a second launch.
 static Plan estimate(int64_t batch, int64_t M, int64_t N, int64_t K, bool bmn, bool may_split) {
-    Plan best{false, 1, MAX_BN, 1, 1e30};
+    Plan best{false, 1, MAX_BN, 1, 0, 1e30};
     const int64_t kb = (K + BK - 1) / BK;
     const int pslots = pair_slots();
     const char* fp = getenv("B200JT_GEMM_PAIR"); const char* fm = getenv("B200JT_GEMM_MT");      // read on every call:
@@ -401,18 +411,27 @@ static Plan estimate(int64_t batch, int64_t M, int64_t N, int64_t K, bool bmn, b
                 const double block = std::max(feed, mma) + 20;
                 const int64_t tiles = tm * ((N + bn - 1) / bn) * batch;
                 const double epi = mt * bn * 4.0;
+                // K whole, or split where the tiles leave a round part empty: all of them when they do not fill one round, else those
+                // of the last round. 4096 x 4096 x 16384 (256 tiles of 256 x 256 on 74 pairs): 3 rounds and a half one instead of 4.
+                const int64_t last = tiles % slots, whole = tiles - last;
                 int64_t tried = 0;
                 for (int q = 0; q < 3; q++) {
-                    int64_t s = q == 0 ? 1 : q == 1 ? slots / tiles : slots / tiles / 2;
+                    int64_t s = q == 0 || last == 0 ? 1 : q == 1 ? slots / last : slots / last / 2;
                     s = std::min(s, kb / 4);
                     if (fs) s = std::min<int64_t>(atoi(fs), kb);
-                    if (s < 1 || !may_split) s = 1;
+                    if (s < 1 || !may_split || last == 0) s = 1;
                     if (s == tried) continue;
                     tried = s;
-                    const double rounds = (double)((tiles * s + slots - 1) / slots);
-                    double ns = 2500 + rounds * ((kb + s - 1) / s * block + (mt == 2 ? epi : 0)) + epi;
-                    if (s > 1) ns += 3000 + (double)s * M * N * 8 / 4000;
-                    if (ns < best.ns) best = {pair != 0, mt, bn, (int)s, ns};
+                    const int64_t kept = s == 1 ? 0 : whole;
+                    const double once = kb * block + (mt == 2 ? epi : 0);
+                    double ns = 2500 + epi;
+                    if (s == 1) ns += (double)((tiles + slots - 1) / slots) * once;
+                    else {
+                        const int64_t others = tiles - kept;
+                        ns += (double)(kept / slots) * once + (double)((others * s + slots - 1) / slots) * ((kb + s - 1) / s * block + (mt == 2 ? epi : 0)) +
+                              3000 + (double)s * others * tile_m * bn * 8 / 4000;
+                    }
+                    if (ns < best.ns) best = {pair != 0, mt, bn, (int)s, kept, ns};
                 }
             }
         }
@@ -447,8 +466,8 @@ static int launch(const Plan& p, const void* a, const void* b, void* c, float* p
     A.M = (int)M; A.N = (int)N; A.K = (int)K; A.bn = p.bn; A.k_blocks = (int)((K + BK - 1) / BK);
     A.tiles_m = (int)((M + tile_m - 1) / tile_m); A.tiles_n = (int)((N + p.bn - 1) / p.bn);
     A.batch = (int)batch; A.splits = p.splits; A.group = std::max(1, 1024 / tile_m);
-    A.a_batched = a_batch > 1; A.b_batched = b_batch > 1; A.pitch = (int)((N + 3) / 4 * 4);
-    const int64_t units = (int64_t)A.tiles_m * A.tiles_n * batch * p.splits;
+    A.a_batched = a_batch > 1; A.b_batched = b_batch > 1; A.whole = (int)p.whole;
+    const int64_t tiles = (int64_t)A.tiles_m * A.tiles_n, units = p.splits > 1 ? p.whole + (tiles - p.whole) * p.splits : tiles * batch;
     if (units >= (1LL << 30)) return fail(-1, "matmul: too many tiles");
     A.units = (int)units;
     cudaLaunchConfig_t cfg = {};
@@ -459,7 +478,7 @@ static int launch(const Plan& p, const void* a, const void* b, void* c, float* p
     void* args[] = {&ma, &mb, &c, &part, &A};
     B200JT_CUDA(cudaLaunchKernelExC(&cfg, kernel_of(p.pair, p.mt, amn, bmn), args));
     if (p.splits > 1) {
-        fold_kernel<<<grid_for(M * (A.pitch / 4), 256), 256, 0, st>>>(part, (__nv_bfloat16*)c, A.M, A.N, A.pitch, p.splits);
+        fold_kernel<<<grid_for((tiles - p.whole) * tile_m * (p.bn / 4), 256), 256, 0, st>>>(part, (__nv_bfloat16*)c, A, tile_m);
         B200JT_LAUNCH_CHECK();
     }
     return 0;
@@ -484,7 +503,10 @@ size_t matmul_tc_workspace(int64_t M, int64_t N, int64_t K, bool trans_a, bool t
     if (ca % 8) bytes += round256((size_t)(trans_a ? K : M) * pitch8(ca) * 2);
     if (cb % 8) bytes += round256((size_t)(trans_b ? N : K) * pitch8(cb) * 2);
     const Plan p = plan_for(1, M, N, K, !trans_b, true);
-    if (p.splits > 1) bytes += (size_t)p.splits * M * ((N + 3) / 4 * 4) * 4;
+    if (p.splits > 1) {
+        const int64_t tile_m = BM * p.mt * (1 + p.pair);
+        bytes += (size_t)p.splits * ((M + tile_m - 1) / tile_m * ((N + p.bn - 1) / p.bn) - p.whole) * tile_m * p.bn * 4;
+    }
     return bytes;
 }
 

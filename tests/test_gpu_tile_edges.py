@@ -1,10 +1,52 @@
 """Kernels at the sizes where their tiles, rings, splits and register rows begin and end, against float64 (or exactly)."""
+import os
+
 import pytest
 import torch
 
 from jittor_b200 import _capi as C
 
 pytestmark = pytest.mark.gpu
+
+
+class forced:
+    """Environment switches of the kernels' plans, for one block."""
+
+    def __init__(self, **names):
+        self.names = {"B200JT_" + k: str(v) for k, v in names.items()}
+
+    def __enter__(self):
+        self.old = {k: os.environ.get(k) for k in self.names}
+        os.environ.update(self.names)
+
+    def __exit__(self, *exc):
+        for k, v in self.old.items():
+            os.environ.pop(k) if v is None else os.environ.__setitem__(k, v)
+
+
+def matmul(a, b, ta, tb, scratch=True):
+    c = torch.full((a.shape[1 if ta else 0], b.shape[0 if tb else 1]), float("nan"), dtype=a.dtype, device="cuda")
+    args = (C.desc(a), C.desc(b), C.desc(c), int(ta), int(tb))
+    size, ptr, ws = C.workspace("b200jt_matmul_workspace", *args)
+    C.call("b200jt_matmul", *args, *((ptr, size) if scratch else (None, 0)))
+    return c
+
+
+def product(a, b, ta, tb):
+    return (a.double().t() if ta else a.double()) @ (b.double().t() if tb else b.double())
+
+
+# ---- bfloat16 products whose last round alone is split (csrc/gemm_tcgen05.cu)
+@pytest.mark.parametrize("ta,tb", [(0, 0), (1, 0), (0, 1)])
+@pytest.mark.parametrize("pair,mt,bn,splits,m,k,n", [(0, 1, 64, 2, 1300, 300, 1000), (0, 1, 32, 3, 1283, 200, 500), (1, 1, 64, 4, 2570, 260, 600),
+                                                     (1, 2, 32, 2, 5000, 136, 300)])
+def test_bf16_matmul_split_last_round(pair, mt, bn, splits, m, k, n, ta, tb):
+    a, b = torch.randn(*((k, m) if ta else (m, k)), device="cuda").bfloat16(), torch.randn(*((n, k) if tb else (k, n)), device="cuda").bfloat16()
+    with forced(GEMM_PAIR=pair, GEMM_MT=mt, GEMM_BN=bn, GEMM_SPLITS=splits):
+        c = matmul(a, b, ta, tb)
+    want = product(a, b, ta, tb)
+    assert (c.double() - want).abs().max() <= 2.0 ** -8 * want.abs().max()             # one rounding to bfloat16 of a float32 sum
+    assert C.lib.b200jt_device_status() == 0
 
 
 # ---- few bins (csrc/reindex_reduce.cu): whole, part and no batches of a thread's two vectors
