@@ -51,6 +51,37 @@ struct ConvArgs {
     int last_k;                      // MMA steps of 16 channels in a tap's last channel block
 };
 
+// A warp's square of 32 channels (rows of 64 bytes) x 32 pixels in shared memory, 16-byte chunks of a row at chunk ^ (row / 2 % 4): a
+// pixel per lane going in, eight chunks of two rows or one chunk of eight rows coming out all touch every bank once.
+__device__ __forceinline__ int square_chunk(int ch, int chunk) { return ch * 4 + (chunk ^ ((ch >> 1) & 3)); }
+__device__ __forceinline__ __nv_bfloat16* square_at(__nv_bfloat16* square, int ch, int px) { return square + square_chunk(ch, px >> 3) * 8 + (px & 7); }
+
+// Adds the square's channel sums and sums of squares to the CTA's: a lane reads its channel's 32 pixels and adds pairs of them with
+// packed float32 arithmetic. (A halving exchange between the lanes was 62 shuffles and 280 instructions for a square, half of the
+// epilogue of a 1 x 1 layer.)
+__device__ __forceinline__ void add_square_sums(const __nv_bfloat16* square, int co0, int Co, float* sstat) {
+    const int lane = threadIdx.x & 31;
+    unsigned long long s[2] = {0, 0}, q[2] = {0, 0};
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+        const uint4 v = reinterpret_cast<const uint4*>(square)[square_chunk(lane, c)];
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            unsigned long long two;
+            asm("mov.b64 %0, {%1, %2};" : "=l"(two) : "r"(w[i] << 16), "r"(w[i] & 0xffff0000u));
+            asm("add.rn.f32x2 %0, %0, %1;" : "+l"(s[i & 1]) : "l"(two));
+            asm("fma.rn.f32x2 %0, %1, %1, %0;" : "+l"(q[i & 1]) : "l"(two));
+        }
+    }
+    asm("add.rn.f32x2 %0, %0, %1;" : "+l"(s[0]) : "l"(s[1]));
+    asm("add.rn.f32x2 %0, %0, %1;" : "+l"(q[0]) : "l"(q[1]));
+    if (co0 + lane < Co) {
+        atomicAdd(sstat + co0 + lane, __uint_as_float((uint32_t)s[0]) + __uint_as_float((uint32_t)(s[0] >> 32)));
+        atomicAdd(sstat + STATS_MAX_CO + co0 + lane, __uint_as_float((uint32_t)q[0]) + __uint_as_float((uint32_t)(q[0] >> 32)));
+    }
+}
+
 // NCHW y: a warp turns its 32 pixels x 32 channels around in shared memory and stores rows of up to 8 pixels. (TMA box stores
 // of [8][8] pixels move a row of 16 bytes in 1.7 ns, whatever there is to it: 6.8 us for a 128 x 256 tile.)
 // NHWC ("acdb"): a lane stores the 32 consecutive channels of its pixel as four 16-byte vectors.
@@ -187,14 +218,14 @@ conv_bf16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                 uint32_t v[32];
                 tmem_ld32(taddr + ch * 32, v);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                float f[32];
+                __syncwarp();
                 if (NHWC) {
                     // NHWC: this lane's pixel, channels co0 .. co0 + 31 are contiguous
                     __align__(16) __nv_bfloat16 row[32];
 #pragma unroll
                     for (int e = 0; e < 32; e++) {
                         row[e] = __float2bfloat16(__uint_as_float(v[e]));
-                        f[e] = (valid && co0 + e < A.Co) ? __bfloat162float(row[e]) : 0.f;
+                        if (stats) *square_at(square, e, lane) = valid ? row[e] : __float2bfloat16(0.f);
                     }
                     if (valid) {
                         __nv_bfloat16* yq = yl + co0;
@@ -207,23 +238,18 @@ conv_bf16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                         }
                     }
                 } else {
-                    __syncwarp();
 #pragma unroll
-                    for (int e = 0; e < 32; e++) {
-                        const __nv_bfloat16 b = __float2bfloat16(__uint_as_float(v[e]));
-                        square[e * 32 + lane] = b;
-                        f[e] = (valid && co0 + e < A.Co) ? __bfloat162float(b) : 0.f;      // statistics of the value as stored
-                    }
+                    for (int e = 0; e < 32; e++) *square_at(square, e, lane) = __float2bfloat16(valid ? __uint_as_float(v[e]) : 0.f);
                     __syncwarp();
                     if (A.vec == 1) {           // planes start anywhere: a channel at a time, neighbouring lanes on neighbouring pixels
 #pragma unroll
                         for (int e = 0; e < 32; e++)
-                            if (valid && co0 + e < A.Co) yl[(int64_t)(co0 + e) * plane] = square[e * 32 + lane];
+                            if (valid && co0 + e < A.Co) yl[(int64_t)(co0 + e) * plane] = *square_at(square, e, lane);
                     } else {
 #pragma unroll
                         for (int i = 0; i < 4; i++) {
                             if (co0 + i * 8 + (lane >> 2) < A.Co) {
-                                const uint4 px = reinterpret_cast<const uint4*>(square)[i * 32 + lane];
+                                const uint4 px = reinterpret_cast<const uint4*>(square)[square_chunk(i * 8 + (lane >> 2), lane & 3)];
                                 const int64_t d = (int64_t)(co0 + i * 8) * plane;
                                 if (A.vec == 8) { if (run < A.pixels) *reinterpret_cast<uint4*>(y0 + d) = px; }
                                 else {
@@ -234,26 +260,9 @@ conv_bf16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                         }
                     }
                 }
-                if (stats) {
-                    // lanes are 32 pixels, f[] 32 channels: halving exchange leaves lane L with the sum of channel L
-                    float g[32];
-#pragma unroll
-                    for (int e = 0; e < 32; e++) g[e] = f[e] * f[e];
-#pragma unroll
-                    for (int s = 16; s > 0; s >>= 1) {
-                        const bool up = (lane & s) != 0;
-#pragma unroll
-                        for (int i = 0; i < s; i++) {
-                            const float keep = up ? f[i + s] : f[i], send = up ? f[i] : f[i + s];
-                            f[i] = keep + __shfl_xor_sync(0xffffffffu, send, s);
-                            const float keep2 = up ? g[i + s] : g[i], send2 = up ? g[i] : g[i + s];
-                            g[i] = keep2 + __shfl_xor_sync(0xffffffffu, send2, s);
-                        }
-                    }
-                    if (co0 + lane < A.Co) {
-                        atomicAdd(sstat + co0 + lane, f[0]);
-                        atomicAdd(sstat + STATS_MAX_CO + co0 + lane, g[0]);
-                    }
+                if (stats) {                    // of the values as stored, zero where there is no pixel
+                    if (NHWC) __syncwarp();
+                    add_square_sums(square, co0, A.Co, sstat);
                 }
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
