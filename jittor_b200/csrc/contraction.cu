@@ -17,7 +17,8 @@ extern "C" size_t b200jt_matmul_workspace(const b200jt_tensor* a, const b200jt_t
     if (!matmul_dims(a, b, trans_a, trans_b, &M, &N, &K) || !valid_tensor(c)) return 0;
     if (a->dtype == B200JT_BFLOAT16 && matmul_tc_supported(M, N, K, a->ptr, b->ptr, c->ptr))
         return matmul_tc_workspace(M, N, K, trans_a != 0, trans_b != 0);
-    if (a->dtype == B200JT_FLOAT32) return matmul_f32_workspace(M, N, K);
+    if (a->dtype == B200JT_FLOAT32)
+        return matmul_f32_tc_wanted(M, N, K) ? matmul_f32_tc_workspace(M, N, K, trans_a != 0, trans_b != 0) : matmul_f32_workspace(M, N, K);
     return 0;
 }
 
@@ -26,7 +27,8 @@ extern "C" size_t b200jt_matmul_workspace(const b200jt_tensor* a, const b200jt_t
 extern "C" int b200jt_device_status(void) {
     if (cudaDeviceSynchronize() != cudaSuccess) return -1;
     const int a = tc_status_fetch_and_clear(), b = tcconv_status_fetch_and_clear(), c = peer_status_fetch_and_clear();
-    return a ? a : b ? b : c;
+    const int d = tcf32_status_fetch_and_clear();
+    return a ? a : b ? b : c ? c : d;
 }
 
 extern "C" int b200jt_matmul(const b200jt_tensor* a, const b200jt_tensor* b, const b200jt_tensor* c,
@@ -46,6 +48,9 @@ extern "C" int b200jt_matmul(const b200jt_tensor* a, const b200jt_tensor* b, con
         B200JT_CHECK_ARG(workspace_bytes >= need && (need == 0 || workspace), "workspace too small: need " + std::to_string(need) + " bytes");
         return matmul_tc(a->ptr, b->ptr, c->ptr, M, N, K, trans_a != 0, trans_b != 0, workspace, st);
     }
+    if (a->dtype == B200JT_FLOAT32 && matmul_f32_tc_wanted(M, N, K) && workspace &&
+        workspace_bytes >= matmul_f32_tc_workspace(M, N, K, trans_a != 0, trans_b != 0))
+        return matmul_f32_tc(a->ptr, b->ptr, c->ptr, M, N, K, trans_a != 0, trans_b != 0, workspace, st);
     if (a->dtype == B200JT_FLOAT32 && matmul_f32_supported(1, M, N, K))
         return matmul_f32(a->ptr, b->ptr, c->ptr, 1, 1, 1, M, N, K, trans_a != 0, trans_b != 0, workspace, workspace_bytes, st);
     return matmul_simt(a->ptr, b->ptr, c->ptr, a->dtype, M, N, K, trans_a != 0, trans_b != 0, st);

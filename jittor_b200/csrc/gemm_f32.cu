@@ -414,13 +414,12 @@ struct Tile { int bm, bn, occ; double alone, more, most, gather; };
 constexpr Tile kTiles[] = {{128, 128, 2, 0.64, 0.05, 0.70, 0.94}, {64, 64, 4, 0.26, 0.12, 0.57, 0.90}, {32, 128, 4, 0.26, 0.12, 0.57, 0.82},
                            {64, 64, 3, 0.35, 0.12, 0.54, 0.90}, {16, 128, 4, 0.20, 0.09, 0.42, 0.85}};
 constexpr int kNumTiles = 5;
-struct Split { int tile = 1, cluster = 1, outer = 1; };
+struct Split { int tile = 1, cluster = 1, outer = 1; double cycles = 1e300; };
 
 // Cycles of the slowest SM: CTAs per SM x the tile's FMAs at the rate that many resident CTAs reach, plus what a split costs.
 // Every combination of tile, cluster size and slice count is tried: 0.2 to 1.5 us of host time a call.
 inline Split plan(int64_t M, int64_t N, int64_t K, int64_t copies, bool may_fold, bool gather) {
     Split best;
-    double cost = 1e300;
     const int64_t kt = std::max<int64_t>(1, (K + BK - 1) / BK);
     for (int t = 0; t < kNumTiles; t++) {
         const Tile& T = kTiles[t];
@@ -434,7 +433,7 @@ inline Split plan(int64_t M, int64_t N, int64_t K, int64_t copies, bool may_fold
                 const int64_t r = (tiles * n + kNumSMs - 1) / kNumSMs;
                 const double eff = std::min(T.most, T.alone + (std::min<int64_t>(r, T.occ) - 1) * T.more) * (gather ? T.gather : 1.0);
                 const double c = (double)r * (work / eff + 600) + (s > 1 ? 1500.0 + (double)r * T.bm * T.bn / 8 : 0) + (o > 1 ? 4000.0 + (double)M * N * copies * o / 800 : 0);
-                if (c < cost) { cost = c; best.tile = t; best.cluster = s; best.outer = o; }
+                if (c < best.cycles) best = {t, s, o, c};
             }
     }
     return best;
@@ -488,6 +487,7 @@ static constexpr int64_t kMaxElems = 0x7fffffff;
 bool matmul_f32_supported(int64_t batch, int64_t M, int64_t N, int64_t K) {
     return M > 0 && N > 0 && K > 0 && M <= 65535 * 32ll && N < kMaxElems - 128 && K < kMaxElems - 64 && batch <= 60000;
 }
+double matmul_f32_ns(int64_t M, int64_t N, int64_t K) { return plan(M, N, K, 1, true, false).cycles / 1.9; }
 size_t matmul_f32_workspace(int64_t M, int64_t N, int64_t K) {
     if (!matmul_f32_supported(1, M, N, K)) return 0;
     const Split p = plan(M, N, K, 1, true, false);

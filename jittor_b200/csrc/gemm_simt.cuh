@@ -44,9 +44,15 @@ int peer_status_fetch_and_clear();          // peer_allreduce.cu
 
 // float32 contractions (gemm_f32.cu): tiled fp32x2 FMAs, k split over clusters; sizes beyond its 32-bit offsets stay below
 bool matmul_f32_supported(int64_t batch, int64_t M, int64_t N, int64_t K);
+double matmul_f32_ns(int64_t M, int64_t N, int64_t K);          // estimated time
 size_t matmul_f32_workspace(int64_t M, int64_t N, int64_t K);
 int matmul_f32(const void* a, const void* b, void* c, int64_t batch, int64_t a_batch, int64_t b_batch, int64_t M, int64_t N, int64_t K,
                bool trans_a, bool trans_b, void* workspace, size_t workspace_bytes, cudaStream_t st);
+// ... and on the tensor cores, operands split into bfloat16 parts (gemm_f32_tc.cu)
+bool matmul_f32_tc_wanted(int64_t M, int64_t N, int64_t K);
+size_t matmul_f32_tc_workspace(int64_t M, int64_t N, int64_t K, bool trans_a, bool trans_b);
+int matmul_f32_tc(const void* a, const void* b, void* c, int64_t M, int64_t N, int64_t K, bool trans_a, bool trans_b, void* workspace, cudaStream_t st);
+int tcf32_status_fetch_and_clear();
 bool conv2d_f32_supported(const ConvShape& s);
 int conv2d_f32(const void* x, const void* w, void* y, const ConvShape& s, cudaStream_t st);
 bool conv2d_transpose_f32_supported(const ConvShape& s);

@@ -36,6 +36,48 @@ def product(a, b, ta, tb):
     return (a.double().t() if ta else a.double()) @ (b.double().t() if tb else b.double())
 
 
+# ---- float32 on the tensor cores (csrc/gemm_f32_tc.cu)
+@pytest.mark.parametrize("ta,tb", [(0, 0), (0, 1), (1, 0), (1, 1)])
+@pytest.mark.parametrize("pair,bn,splits", [(0, 32, 1), (0, 96, 2), (0, 128, 4), (0, 64, 8), (1, 128, 1), (1, 192, 1), (1, 256, 1)])
+@pytest.mark.parametrize("m,k,n", [(1, 32, 1), (127, 257, 65), (129, 545, 130), (300, 97, 513)])
+def test_f32_tensor_core_matmul(m, k, n, pair, bn, splits, ta, tb):
+    a, b = torch.randn(*((k, m) if ta else (m, k)), device="cuda"), torch.randn(*((n, k) if tb else (k, n)), device="cuda")
+    with forced(F32TC=1, F32TC_PAIR=pair, F32TC_BN=bn, F32TC_SPLITS=splits):
+        c = matmul(a, b, ta, tb)
+    want = product(a, b, ta, tb)
+    # per 64 of k four truncated additions, each below 2^-23 of the sum so far, then one rounding per 64 of k; no sum exceeds that of
+    # the products' magnitudes
+    assert (c.double() - want).norm() <= (4 + k / 128) * 2.0 ** -23 * product(a.abs(), b.abs(), ta, tb).norm()
+    assert C.lib.b200jt_device_status() == 0
+
+
+def test_f32_tensor_core_matmul_range():
+    """Subnormal and huge operands, overflow, infinities and NaN come out as from float32 arithmetic."""
+    m, k, n = 130, 200, 140
+    a, b = torch.randn(m, k, device="cuda"), torch.randn(k, n, device="cuda")
+    with forced(F32TC=1):
+        for sa, sb in ((1e-42, 1e20), (1e-38, 1.0), (1e-20, 1e-20), (1e37, 1e-37), (1e33, 1.0), (1e12, 1e13)):
+            x, y = a * sa, b * sb
+            want = product(x, y, 0, 0)
+            got = matmul(x, y, 0, 0).double()
+            # eight chains of k / 8 fused multiply-adds where the scaled range is left; results below 2^-126 are rounded to 2^-149
+            assert (got - want).norm() <= (k / 8 + 3) * 2.0 ** -24 * product(x.abs(), y.abs(), 0, 0).norm() + (m * n) ** 0.5 * 2.0 ** -149, (sa, sb)
+        a[3, 5], a[7, 1], b[9, 11], a[20, 9], a[50] = float("inf"), float("nan"), -float("inf"), 0.0, 3e38
+        b[:, 60] = 1.0
+        got, want = matmul(a, b, 0, 0), product(a, b, 0, 0).float()
+        rows = torch.tensor([i for i in range(m) if i != 50], device="cuda")          # sums of 3e38: finite or not by their order
+        assert torch.equal(torch.isnan(got[rows]), torch.isnan(want[rows])) and torch.equal(torch.isinf(got[rows]), torch.isinf(want[rows]))
+        assert not torch.isfinite(got[50, 60])
+
+
+def test_f32_matmul_without_scratch_stays_on_the_fma_pipe():
+    a, b = torch.randn(600, 300, device="cuda"), torch.randn(300, 700, device="cuda")
+    with forced(F32TC=0):
+        want = matmul(a, b, 0, 0, scratch=False)
+    with forced(F32TC=1):
+        assert torch.equal(matmul(a, b, 0, 0, scratch=False), want)
+
+
 # ---- bfloat16 products whose last round alone is split (csrc/gemm_tcgen05.cu)
 @pytest.mark.parametrize("ta,tb", [(0, 0), (1, 0), (0, 1)])
 @pytest.mark.parametrize("pair,mt,bn,splits,m,k,n", [(0, 1, 64, 2, 1300, 300, 1000), (0, 1, 32, 3, 1283, 200, 500), (1, 1, 64, 4, 2570, 260, 600),
@@ -85,7 +127,7 @@ def test_softmax_backward(rows, cols, dtype, log):
 # ---- pooling forward: two rows of two outputs to a thread (csrc/pool.cu)
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("k,stride,pad", [(2, 2, 0), (3, 2, 1), (3, 2, 0), (3, 1, 1)])
-@pytest.mark.parametrize("h,w", [(3, 8), (5, 16), (8, 12), (11, 9), (10, 32), (13, 20)])
+@pytest.mark.parametrize("h,w", [(4, 8), (5, 16), (8, 12), (11, 9), (10, 32), (13, 20)])
 def test_pool_forward(h, w, k, stride, pad, dtype):
     import jittor_b200 as jt
     from jittor_b200 import pool
