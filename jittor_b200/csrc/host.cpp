@@ -94,15 +94,40 @@ struct VarObj {
 PyTypeObject VarType = {PyVarObject_HEAD_INIT(nullptr, 0)};
 inline bool is_var(PyObject* o) { return PyObject_TypeCheck(o, &VarType); }
 
+// What Var's make_shape and canon make of their argument. Lists and tuples of plain whole numbers are copied here, and the names of
+// dtypes are asked for once: a layer's call makes a dozen of each.
+PyObject* shape_from(PyObject* x) {
+    const bool list = PyList_CheckExact(x);
+    if (!list && !PyTuple_CheckExact(x)) return PyObject_CallOneArg(h_make_shape, x);
+    const Py_ssize_t n = list ? PyList_GET_SIZE(x) : PyTuple_GET_SIZE(x);
+    auto item = [&](Py_ssize_t i) { return list ? PyList_GET_ITEM(x, i) : PyTuple_GET_ITEM(x, i); };
+    bool plain = n <= B200JT_MAX_DIMS;
+    for (Py_ssize_t i = 0; plain && i < n; i++) plain = PyLong_CheckExact(item(i));
+    if (!plain) return PyObject_CallOneArg(h_make_shape, x);
+    PyTypeObject* t = (PyTypeObject*)h_shape_type;
+    PyObject* s = t->tp_alloc(t, 0);
+    for (Py_ssize_t i = 0; s && i < n; i++) if (PyList_Append(s, item(i)) < 0) Py_CLEAR(s);
+    return s;
+}
+PyObject* dtype_from(PyObject* x) {
+    static PyObject* known = PyDict_New();
+    if (!PyUnicode_CheckExact(x)) return PyObject_CallOneArg(h_canon, x);
+    if (PyObject* d = PyDict_GetItemWithError(known, x)) return Py_NewRef(d);
+    if (PyErr_Occurred()) return nullptr;
+    PyObject* d = PyObject_CallOneArg(h_canon, x);
+    if (d && PyDict_SetItem(known, x, d) < 0) Py_CLEAR(d);
+    return d;
+}
+
 int var_init(VarObj* self, PyObject* args, PyObject* kw) {
     static const char* names[] = {"shape", "dtype", "op", "data", "is_scalar", nullptr};
     PyObject *shape, *dtype, *op = Py_None, *data = Py_None;
     int scalar = 0;
     if (!PyArg_ParseTupleAndKeywords(args, kw, "OO|OOp", (char**)names, &shape, &dtype, &op, &data, &scalar)) return -1;
     if ((PyObject*)Py_TYPE(shape) == h_shape_type) Py_INCREF(shape);
-    else if (!(shape = PyObject_CallOneArg(h_make_shape, shape))) return -1;
+    else if (!(shape = shape_from(shape))) return -1;
     if ((PyObject*)Py_TYPE(dtype) == h_dtype_type) Py_INCREF(dtype);
-    else if (!(dtype = PyObject_CallOneArg(h_canon, dtype))) { Py_DECREF(shape); return -1; }
+    else if (!(dtype = dtype_from(dtype))) { Py_DECREF(shape); return -1; }
     Py_XSETREF(self->shape, shape);
     Py_XSETREF(self->dtype, dtype);
     Py_INCREF(op);
