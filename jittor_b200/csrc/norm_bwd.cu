@@ -55,12 +55,13 @@ __device__ __forceinline__ float warp_sum(float v) {
     for (int d = 16; d > 0; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
     return v;
 }
-// Sums of NV values over the GROUP threads of a row (a warp, or the CTA of 256).
+// Sums of NV values over the GROUP threads of a row (a warp, or a CTA of up to 256).
+constexpr int cta_of(int group) { return group == 32 ? 256 : group; }
 template <int GROUP, int NV>
 __device__ __forceinline__ void row_sum(float (&v)[NV], float* sm) {
 #pragma unroll
     for (int i = 0; i < NV; i++) v[i] = warp_sum(v[i]);
-    if constexpr (GROUP == 256) {
+    if constexpr (GROUP > 32) {
         const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
         __syncthreads();
         if (lane == 0)
@@ -71,7 +72,7 @@ __device__ __forceinline__ void row_sum(float (&v)[NV], float* sm) {
         for (int i = 0; i < NV; i++) {
             float t = 0.f;
 #pragma unroll
-            for (int w = 0; w < 8; w++) t += sm[i * 8 + w];
+            for (int w = 0; w < GROUP / 32; w++) t += sm[i * 8 + w];
             v[i] = t;
         }
     }
@@ -80,10 +81,10 @@ __device__ __forceinline__ void row_sum(float (&v)[NV], float* sm) {
 // GROUP threads hold a row of x and of dy in registers (E elements each, in vectors of N) and keep their columns' sums for
 // dgamma / dbeta across the rows they visit; a CTA writes one pair of partial rows at the end.
 template <typename T, int N, int GROUP, int E, bool DX, bool PARAMS>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(cta_of(GROUP))
 layer_norm_bwd_kernel(const T* __restrict__ x, const T* __restrict__ dy, const float* __restrict__ gamma, T* __restrict__ dx,
                       float* __restrict__ partial, int64_t rows, int cols, float eps) {
-    constexpr int VPT = E / N, RPC = 256 / GROUP;
+    constexpr int VPT = E / N, RPC = cta_of(GROUP) / GROUP;
     __shared__ float sm[32];
     extern __shared__ float fold[];                             // GROUP == 32 and PARAMS: [2][cols]
     const int g = threadIdx.x / GROUP, t = threadIdx.x % GROUP;
@@ -158,7 +159,7 @@ layer_norm_bwd_kernel(const T* __restrict__ x, const T* __restrict__ dy, const f
     }
     if constexpr (PARAMS) {
         float* out = partial + (int64_t)blockIdx.x * 2 * cols;
-        if constexpr (GROUP == 256) {
+        if constexpr (GROUP > 32) {
 #pragma unroll
             for (int k = 0; k < VPT; k++) {
                 const int vi = t + k * GROUP;
@@ -187,21 +188,19 @@ layer_norm_bwd_kernel(const T* __restrict__ x, const T* __restrict__ dy, const f
     }
 }
 
-// out[i] = sum over p < parts of partial[p * n + i], in order of p within eight interleaved chains.
-__global__ void __launch_bounds__(256) fold_rows_kernel(const float* __restrict__ partial, float* __restrict__ out, int n, int parts) {
-    __shared__ float sm[8][33];
+// out[i] = sum over p < parts of partial[p * n + i], in order of p within 32 interleaved chains. (Eight of them were bound by their
+// length: 592 rows of 2002 sums 6.5 us.)
+__global__ void __launch_bounds__(1024) fold_rows_kernel(const float* __restrict__ partial, float* __restrict__ out, int n, int parts) {
+    __shared__ float sm[32][33];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, i = blockIdx.x * 32 + lane;
     float s = 0.f;
     if (i < n)
-        for (int p = w; p < parts; p += 8) s += partial[(int64_t)p * n + i];
+#pragma unroll 4
+        for (int p = w; p < parts; p += 32) s += partial[(int64_t)p * n + i];
     sm[w][lane] = s;
     __syncthreads();
-    if (w == 0 && i < n) {
-        float t = 0.f;
-#pragma unroll
-        for (int k = 0; k < 8; k++) t += sm[k][lane];
-        out[i] = t;
-    }
+    const float t = warp_sum(sm[lane][w]);                     // warp w adds the chains of column w
+    if (lane == 0 && blockIdx.x * 32 + w < n) out[blockIdx.x * 32 + w] = t;
 }
 
 // ---- BatchNorm ---------------------------------------------------------------------------------------------------------
@@ -371,37 +370,41 @@ bn_bwd_dx_kernel(const TX* __restrict__ x, const TD* __restrict__ dy, const floa
 // Rows stay in registers up to 8192 columns (32 elements a thread); the host keeps the op-by-op graph for longer ones.
 constexpr int kMaxCols = 8192;
 // Persistent CTAs: enough rows in flight to cover the latency of a row's reductions, few enough partial rows to fold.
-inline int ln_ctas(int64_t rows, int rpc, bool wide) {
+constexpr int kMostCtas = 8;                                   // per SM, over all forms below
+inline int ln_ctas(int64_t rows, int rpc, int per_sm) {
     const int64_t need = (rows + rpc - 1) / rpc;
-    return (int)std::max<int64_t>(1, std::min<int64_t>(need, (int64_t)(kNumSMs - sm_reserve()) * (wide ? 2 : 4)));
+    return (int)std::max<int64_t>(1, std::min<int64_t>(need, (int64_t)(kNumSMs - sm_reserve()) * per_sm));
 }
 
 template <typename T, int N, int GROUP, int E>
 int launch_ln(const T* x, const T* dy, const float* gamma, T* dx, float* params, float* partial, int64_t rows, int cols, float eps, int ctas, cudaStream_t st) {
     const size_t smem = params && GROUP == 32 ? sizeof(float) * 2 * cols : 0;
-    if (dx && params) layer_norm_bwd_kernel<T, N, GROUP, E, true, true><<<ctas, 256, smem, st>>>(x, dy, gamma, dx, partial, rows, cols, eps);
-    else if (dx) layer_norm_bwd_kernel<T, N, GROUP, E, true, false><<<ctas, 256, 0, st>>>(x, dy, gamma, dx, partial, rows, cols, eps);
-    else layer_norm_bwd_kernel<T, N, GROUP, E, false, true><<<ctas, 256, smem, st>>>(x, dy, gamma, dx, partial, rows, cols, eps);
+    if (dx && params) layer_norm_bwd_kernel<T, N, GROUP, E, true, true><<<ctas, cta_of(GROUP), smem, st>>>(x, dy, gamma, dx, partial, rows, cols, eps);
+    else if (dx) layer_norm_bwd_kernel<T, N, GROUP, E, true, false><<<ctas, cta_of(GROUP), 0, st>>>(x, dy, gamma, dx, partial, rows, cols, eps);
+    else layer_norm_bwd_kernel<T, N, GROUP, E, false, true><<<ctas, cta_of(GROUP), smem, st>>>(x, dy, gamma, dx, partial, rows, cols, eps);
     B200JT_LAUNCH_CHECK();
     if (params) {
-        fold_rows_kernel<<<(2 * cols + 31) / 32, 256, 0, st>>>(partial, params, 2 * cols, ctas);
+        fold_rows_kernel<<<(2 * cols + 31) / 32, 1024, 0, st>>>(partial, params, 2 * cols, ctas);
         B200JT_LAUNCH_CHECK();
     }
     return 0;
 }
 
-// A warp to a row of up to 512 columns (256 one by one: more registers per lane leave too few warps), a CTA beyond; 16-byte
-// vectors where columns and pointers allow, else one element. [5000, 1001] float32: 41 us with a warp to the row, 15 with a CTA.
+// A warp to a row of up to 512 columns (256 one by one), a CTA beyond; 16-byte vectors where columns and pointers allow, else one
+// element. CTAs as small as the rows: [50000, 768] bfloat16 165 us with 256 threads to the row, 81 with 128, float32 175 and 125;
+// [3000, 301] 9.7 and 4.9 with 64. Ragged rows: [60000, 301] 173 us with 256 threads, 65 with a warp, whose parameter sums a CTA adds
+// one warp after the other (10 us: worth it from some 8000 rows on); [100000, 1001] 350 with 256 threads, 369 with 128.
 template <typename T, int V>
 int run_ln(const T* x, const T* dy, const float* gamma, T* dx, float* params, float* partial, int64_t rows, int cols, float eps, cudaStream_t st) {
     const bool vec = cols % V == 0 && (uintptr_t)x % 16 == 0 && (uintptr_t)dy % 16 == 0 && (uintptr_t)dx % 16 == 0 && (uintptr_t)gamma % 16 == 0;
 #define B200JT_LN(GROUP, E)                                                                                                      \
-    do { const int ctas = ln_ctas(rows, 256 / GROUP, E > 16);                                                                    \
+    do { const int ctas = ln_ctas(rows, cta_of(GROUP) / GROUP, GROUP != 32 && GROUP < 256 ? kMostCtas : E > 16 ? 2 : 4);         \
          return vec ? launch_ln<T, V, GROUP, E>(x, dy, gamma, dx, params, partial, rows, cols, eps, ctas, st)                    \
                     : launch_ln<T, 1, GROUP, E>(x, dy, gamma, dx, params, partial, rows, cols, eps, ctas, st); } while (0)
     if (cols <= 256) B200JT_LN(32, 8);
-    if (cols <= 512 && vec) B200JT_LN(32, 16);
-    if (cols <= 1024 && !vec) return launch_ln<T, 1, 256, 4>(x, dy, gamma, dx, params, partial, rows, cols, eps, ln_ctas(rows, 1, false), st);
+    if (cols <= 512) { if (vec || rows >= 8192) B200JT_LN(32, 16); B200JT_LN(64, 8); }
+    if (cols <= 1024 && vec) B200JT_LN(128, 8);
+    if (cols <= 1024) return launch_ln<T, 1, 256, 4>(x, dy, gamma, dx, params, partial, rows, cols, eps, ln_ctas(rows, 1, 4), st);
     if (cols <= 2048) B200JT_LN(256, 8);
     if (cols <= 4096) B200JT_LN(256, 16);
     B200JT_LN(256, 32);
@@ -467,7 +470,7 @@ extern "C" size_t b200jt_layer_norm_backward_workspace(const b200jt_tensor* x, i
     if (!valid_tensor(x) || !want_params) return 0;
     const int64_t cols = x->shape[x->ndim - 1], rows = cols ? numel(x) / cols : 0;
     if (cols < 1 || cols > kMaxCols || rows < 1) return 0;
-    return sizeof(float) * 2 * cols * (size_t)ln_ctas(rows, 1, false);
+    return sizeof(float) * 2 * cols * (size_t)ln_ctas(rows, 1, kMostCtas);
 }
 
 extern "C" int b200jt_layer_norm_backward(const b200jt_tensor* x, const b200jt_tensor* gamma, const b200jt_tensor* dy, const b200jt_tensor* dx,

@@ -19,12 +19,16 @@ namespace b200jt {
 
 enum RowOp : int { ROW_SOFTMAX = 0, ROW_LOG_SOFTMAX = 1, ROW_LAYERNORM = 2 };
 
+constexpr int cta_of(int group) { return group == 32 ? 256 : group; }
+// sixteen CTAs of 256 threads' worth of rows for every SM, more rows than that go round
+inline unsigned row_grid(int64_t rows, int group) {
+    const int64_t rpc = cta_of(group) / group, most = (int64_t)kNumSMs * (group == 32 || group > 256 ? 16 : 4096 / group);
+    return (unsigned)std::min((rows + rpc - 1) / rpc, most);
+}
+
 template <typename T> struct Vec16;
 template <> struct Vec16<float> {
     static constexpr int N = 4;
-    using Raw = float4;
-    static __device__ __forceinline__ Raw raw(const float* p) { return __ldcs(reinterpret_cast<const float4*>(p)); }
-    static __device__ __forceinline__ void unpack(const Raw& v, float* out) { out[0] = v.x; out[1] = v.y; out[2] = v.z; out[3] = v.w; }
     static __device__ __forceinline__ void load(const float* p, float* out) {
         float4 v = __ldcs(reinterpret_cast<const float4*>(p)); out[0] = v.x; out[1] = v.y; out[2] = v.z; out[3] = v.w;
     }
@@ -60,9 +64,6 @@ template <> __device__ __forceinline__ void st1<__nv_bfloat16>(__nv_bfloat16* p,
 // One element per access, for rows that 16-byte vectors do not fit.
 template <typename T> struct Single {
     static constexpr int N = 1;
-    using Raw = T;
-    static __device__ __forceinline__ Raw raw(const T* p) { return *p; }
-    static __device__ __forceinline__ void unpack(const Raw& v, float* out) { out[0] = ld1<T>(&v); }
     static __device__ __forceinline__ void load(const T* p, float* out) { out[0] = ld1<T>(p); }
     static __device__ __forceinline__ void store(T* p, const float* in) { st1<T>(p, in[0]); }
 };
@@ -141,14 +142,14 @@ __device__ __forceinline__ void group_reduce_n(float (&v)[NV], float* sm) {
     }
 }
 
-// GROUP threads per row, VPT vectors per thread (V: 16 bytes, or one element); requires cols % V::N == 0 and
+// GROUP threads per row -- a warp, eight of them to a CTA, or a CTA of that size --, VPT vectors per thread (V: 16 bytes, or one element); requires cols % V::N == 0 and
 // cols <= GROUP * VPT * N. RPI rows are taken per round (their reductions share the shared-memory exchanges).
 template <typename T, typename V, int GROUP, int VPT, int OP>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(cta_of(GROUP))
 row_reg_kernel(const T* __restrict__ x, T* __restrict__ y, const float* __restrict__ gamma,
                const float* __restrict__ beta, int64_t rows, int cols, float eps) {
     constexpr int N = V::N;
-    constexpr int ROWS_PER_CTA = 256 / GROUP;
+    constexpr int ROWS_PER_CTA = cta_of(GROUP) / GROUP;
     constexpr int RPI = 1;          // two rows per round were measured slower (fewer CTAs in flight outweigh the shared exchange)
     __shared__ float sm[32];
     const int g = threadIdx.x / GROUP, t = threadIdx.x % GROUP;
@@ -471,15 +472,15 @@ static int launch_rows(const T* x, T* y, const float* gamma, const float* beta, 
     const bool vec_ok = cols % N == 0 && (((uintptr_t)x | (uintptr_t)y | (uintptr_t)gamma | (uintptr_t)beta) & 15) == 0;
     const int64_t nvec = cols / N;
 #define B200JT_ROW(GROUP, VPT)                                                                      \
-    do { const int rpc = 256 / GROUP;                                                               \
-         int64_t ctas = (rows + rpc - 1) / rpc;                                                     \
-         unsigned grid = (unsigned)(ctas < (int64_t)kNumSMs * 16 ? ctas : (int64_t)kNumSMs * 16);   \
-         row_reg_kernel<T, V, GROUP, VPT, OP><<<grid, 256, 0, st>>>(x, y, gamma, beta, rows, (int)cols, eps); } while (0)
+    row_reg_kernel<T, V, GROUP, VPT, OP><<<row_grid(rows, GROUP), cta_of(GROUP), 0, st>>>(x, y, gamma, beta, rows, (int)cols, eps)
     if (!vec_ok && cols <= 256 * 32) {
         using V = Single<T>;
+        // rows in flight cover the latency of a row's loads and reductions: [60000, 301] float32 softmax 77 us with 256 threads to
+        // the row, 24 with a warp; [20000, 777] bfloat16 29 and 21 with 128
         if (cols <= 32 * 8) B200JT_ROW(32, 8);
-        else if (cols <= 256 * 4) B200JT_ROW(256, 4);
-        else if (cols <= 256 * 8) B200JT_ROW(256, 8);
+        else if (cols <= 32 * 16) B200JT_ROW(32, 16);
+        else if (cols <= 128 * 8) B200JT_ROW(128, 8);
+        else if (cols <= 128 * 16) B200JT_ROW(128, 16);
         else if (cols <= 256 * 16) B200JT_ROW(256, 16);
         else B200JT_ROW(256, 32);
         B200JT_LAUNCH_CHECK();
@@ -517,59 +518,88 @@ static int launch_rows(const T* x, T* y, const float* gamma, const float* beta, 
 // dx = y * (dy - sum(y * dy))   for y = softmax(x),      dx = dy - exp(y) * sum(dy)   for y = log_softmax(x),
 // the two reductions of the reference's hand-written backward (python/jittor/other/code_softmax.py:109-147). The row of y
 // and of dy live in registers: one read of each, one write of dx.
-// The next row's vectors are loaded before this row's sum goes round the CTA, so that the loads do not wait for the barrier and the
-// stores: [32768, 4096] bfloat16 147 -> 121 us, [65536, 1024] 105 -> 63. Rows of 8193 to 16384 columns take a CTA of 1024
+// bfloat16: the next row's vectors are loaded, as they lie in memory, before this row's sum goes round the CTA, so that the loads do
+// not wait for the barrier and the stores: [32768, 4096] 147 -> 121 us, [65536, 1024] 105 -> 63. Rows of 8193 to 16384 columns take a CTA of 1024
 // threads ([8192, 16384] bfloat16: 270 us in two sweeps).
 template <typename T, typename V, int GROUP, int VPT, bool LOG>
-__global__ void __launch_bounds__(GROUP > 256 ? GROUP : 256)
+__global__ void __launch_bounds__(cta_of(GROUP))
 softmax_bwd_reg_kernel(const T* __restrict__ y, const T* __restrict__ dy, T* __restrict__ dx, int64_t rows, int cols) {
     constexpr int N = V::N;
-    constexpr int ROWS_PER_CTA = GROUP < 256 ? 256 / GROUP : 1;
+    constexpr int ROWS_PER_CTA = cta_of(GROUP) / GROUP;
     __shared__ float sm[32];
     const int g = threadIdx.x / GROUP, t = threadIdx.x % GROUP;
     const int nvec = cols / N;
-    typename V::Raw a[VPT], b[VPT];
-    auto load = [&](int64_t row) {
+    const int64_t step = (int64_t)gridDim.x * ROWS_PER_CTA;
+    // float32 rows have as many bytes in flight without, and one vector to a lane leaves room for more rows instead
+    constexpr bool AHEAD = sizeof(T) == 2 && N > 1 && (GROUP > 32 || VPT > 1) && VPT <= (GROUP > 512 ? 2 : 4);
+    // the CTA-wide reduction has a barrier inside: rows are taken in rounds the whole CTA goes through together
+    if constexpr (AHEAD) {
+        typename V::Raw a[VPT], b[VPT];
+        auto load = [&](int64_t row) {
 #pragma unroll
-        for (int k = 0; k < VPT; k++) {
-            const int vi = t + k * GROUP;
-            if (row < rows && vi < nvec) {
-                a[k] = V::raw(y + row * cols + (int64_t)vi * N);
-                b[k] = V::raw(dy + row * cols + (int64_t)vi * N);
+            for (int k = 0; k < VPT; k++) {
+                const int vi = t + k * GROUP;
+                if (row < rows && vi < nvec) {
+                    a[k] = V::raw(y + row * cols + (int64_t)vi * N);
+                    b[k] = V::raw(dy + row * cols + (int64_t)vi * N);
+                }
+            }
+        };
+        load((int64_t)blockIdx.x * ROWS_PER_CTA + g);
+        for (int64_t round0 = (int64_t)blockIdx.x * ROWS_PER_CTA; round0 < rows; round0 += step) {
+            const int64_t row = round0 + g;
+            const bool live = row < rows;
+            typename V::Raw ya[VPT], da[VPT];
+            float s = 0.f;
+#pragma unroll
+            for (int k = 0; k < VPT; k++) {
+                ya[k] = a[k]; da[k] = b[k];
+                float p[N], q[N];
+                V::unpack(ya[k], p); V::unpack(da[k], q);
+                if (live && t + k * GROUP < nvec)
+#pragma unroll
+                    for (int e = 0; e < N; e++) s += LOG ? q[e] : p[e] * q[e];
+            }
+            load(row + step);                               // in flight through the reduction and the stores
+            s = group_reduce<GROUP, false>(s, sm);
+#pragma unroll
+            for (int k = 0; k < VPT; k++) {
+                const int vi = t + k * GROUP;
+                if (live && vi < nvec) {
+                    float p[N], q[N], o[N];
+                    V::unpack(ya[k], p); V::unpack(da[k], q);
+#pragma unroll
+                    for (int e = 0; e < N; e++) o[e] = LOG ? q[e] - expf(p[e]) * s : p[e] * (q[e] - s);
+                    V::store(dx + row * cols + (int64_t)vi * N, o);
+                }
             }
         }
-    };
-    const int64_t step = (int64_t)gridDim.x * ROWS_PER_CTA;
-    // longer rows have enough in flight, and twice the registers would cost residency
-    constexpr bool AHEAD = VPT * (sizeof(typename V::Raw) < 4 ? 4 : sizeof(typename V::Raw)) <= (GROUP > 512 ? 32 : 64);
-    if (AHEAD) load((int64_t)blockIdx.x * ROWS_PER_CTA + g);
-    // the CTA-wide reduction has a barrier inside: rows are taken in rounds the whole CTA goes through together
-    for (int64_t round0 = (int64_t)blockIdx.x * ROWS_PER_CTA; round0 < rows; round0 += step) {
-        const int64_t row = round0 + g;
-        const bool live = row < rows;
-        if (!AHEAD) load(row);
-        typename V::Raw ya[VPT], da[VPT];
-        float s = 0.f;
+    } else {
+        for (int64_t round0 = (int64_t)blockIdx.x * ROWS_PER_CTA; round0 < rows; round0 += step) {
+            const int64_t row = round0 + g;
+            const bool live = row < rows;
+            float a[VPT][N], b[VPT][N];
+            float s = 0.f;
 #pragma unroll
-        for (int k = 0; k < VPT; k++) {
-            ya[k] = a[k]; da[k] = b[k];
-            float p[N], q[N];
-            V::unpack(ya[k], p); V::unpack(da[k], q);
-            if (live && t + k * GROUP < nvec)
+            for (int k = 0; k < VPT; k++) {
+                const int vi = t + k * GROUP;
+                if (live && vi < nvec) {
+                    V::load(y + row * cols + (int64_t)vi * N, a[k]);
+                    V::load(dy + row * cols + (int64_t)vi * N, b[k]);
 #pragma unroll
-                for (int e = 0; e < N; e++) s += LOG ? q[e] : p[e] * q[e];
-        }
-        if (AHEAD) load(row + step);                        // in flight through the reduction and the stores
-        s = group_reduce<GROUP, false>(s, sm);
+                    for (int e = 0; e < N; e++) s += LOG ? b[k][e] : a[k][e] * b[k][e];
+                }
+            }
+            s = group_reduce<GROUP, false>(s, sm);
 #pragma unroll
-        for (int k = 0; k < VPT; k++) {
-            const int vi = t + k * GROUP;
-            if (live && vi < nvec) {
-                float p[N], q[N], o[N];
-                V::unpack(ya[k], p); V::unpack(da[k], q);
+            for (int k = 0; k < VPT; k++) {
+                const int vi = t + k * GROUP;
+                if (live && vi < nvec) {
+                    float o[N];
 #pragma unroll
-                for (int e = 0; e < N; e++) o[e] = LOG ? q[e] - expf(p[e]) * s : p[e] * (q[e] - s);
-                V::store(dx + row * cols + (int64_t)vi * N, o);
+                    for (int e = 0; e < N; e++) o[e] = LOG ? b[k][e] - expf(a[k][e]) * s : a[k][e] * (b[k][e] - s);
+                    V::store(dx + row * cols + (int64_t)vi * N, o);
+                }
             }
         }
     }
@@ -598,13 +628,13 @@ static int launch_softmax_bwd(const T* y, const T* dy, T* dx, int64_t rows, int6
     const bool vec_ok = cols % N == 0 && ((uintptr_t)y % 16 == 0) && ((uintptr_t)dy % 16 == 0) && ((uintptr_t)dx % 16 == 0);
     const int64_t nvec = cols / N;
 #define B200JT_SB(GROUP, VPT)                                                                       \
-    do { const int rpc = GROUP < 256 ? 256 / GROUP : 1;                                             \
-         int64_t ctas = (rows + rpc - 1) / rpc;                                                     \
-         unsigned grid = (unsigned)(ctas < (int64_t)kNumSMs * 16 ? ctas : (int64_t)kNumSMs * 16);   \
-         softmax_bwd_reg_kernel<T, V, GROUP, VPT, LOG><<<grid, GROUP > 256 ? GROUP : 256, 0, st>>>(y, dy, dx, rows, (int)cols); } while (0)
+    softmax_bwd_reg_kernel<T, V, GROUP, VPT, LOG><<<row_grid(rows, GROUP), cta_of(GROUP), 0, st>>>(y, dy, dx, rows, (int)cols)
     if (!vec_ok && cols <= 1024 * 16) {
         using V = Single<T>;
+        // [60000, 301] float32: 66 us with 256 threads to the row, 40 with 64; [20000, 777] bfloat16 26 and 22 with 128
         if (cols <= 32 * 8) B200JT_SB(32, 8);
+        else if (cols <= 64 * 8) B200JT_SB(64, 8);
+        else if (cols <= 128 * 8 && sizeof(T) == 2) B200JT_SB(128, 8);
         else if (cols <= 256 * 4) B200JT_SB(256, 4);
         else if (cols <= 256 * 8) B200JT_SB(256, 8);
         else if (cols <= 256 * 16) B200JT_SB(256, 16);

@@ -137,3 +137,62 @@ def test_pool_forward(h, w, k, stride, pad, dtype):
     got = pool.avg_pool2d(jt.array(x), k, stride, pad).torch()
     want = torch.nn.functional.avg_pool2d(x.double(), k, stride, pad)
     assert (got.double() - want).abs().max() <= (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -21) * want.abs().max()
+
+
+# ---- ragged rows: a warp, or a CTA of 64 to 1024 threads, to the row (csrc/rownorm.cu, csrc/norm_bwd.cu)
+def placed(rows, cols, dtype, offset):
+    """A [rows, cols] tensor that starts `offset` elements into a guarded buffer, and a check that the guards are untouched."""
+    buf = torch.full((rows * cols + 32,), 7.0, device="cuda", dtype=dtype)
+    t = buf[offset:offset + rows * cols].view(rows, cols)
+
+    def guarded():
+        return bool((buf[:offset] == 7).all()) and bool((buf[offset + rows * cols:] == 7).all())
+    return t, guarded
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("offset", [0, 1, 3])
+@pytest.mark.parametrize("rows,cols", [(1, 1), (9, 33), (19, 256), (2500, 257), (8200, 259), (5, 512), (21, 515), (2377, 1001), (5, 1024), (7, 1027),
+                                       (601, 2051), (5, 4099), (3, 8191), (3, 8193)])
+def test_ragged_rows(rows, cols, offset, dtype):
+    tol = 2.0 ** -8 if dtype == torch.bfloat16 else 1e-5
+    v = torch.randn(rows, cols, device="cuda").to(dtype)
+    w = torch.randn(rows, cols, device="cuda").to(dtype)
+    x, _ = placed(rows, cols, dtype, offset)
+    dy, _ = placed(rows, cols, dtype, offset)
+    x.copy_(v)
+    dy.copy_(w)
+    d = x.double()
+
+    def near(got, want):
+        return (got.double() - want).norm() <= tol * want.norm() + 1e-30
+    for log in (0, 1):
+        y, kept = placed(rows, cols, dtype, offset)
+        C.call("b200jt_softmax", C.desc(x), C.desc(y), log)
+        assert near(y, torch.log_softmax(d, 1) if log else torch.softmax(d, 1)) and kept()
+        dx, kept = placed(rows, cols, dtype, offset)
+        C.call("b200jt_softmax_backward", C.desc(y), C.desc(dy), C.desc(dx), log)
+        yd, g = y.double(), dy.double()
+        assert near(dx, g - yd.exp() * g.sum(1, keepdim=True) if log else yd * (g - (yd * g).sum(1, keepdim=True))) and kept()
+    if cols < 2:
+        return
+    gamma, beta = torch.randn(cols, device="cuda"), torch.randn(cols, device="cuda")
+    y, kept = placed(rows, cols, dtype, offset)
+    C.call("b200jt_layer_norm", C.desc(x), C.desc(gamma), C.desc(beta), C.desc(y), 1e-5)
+    d.requires_grad_(True)
+    gd, bd = gamma.double().requires_grad_(True), beta.double().requires_grad_(True)
+    want = torch.nn.functional.layer_norm(d, (cols,), gd, bd, 1e-5)
+    assert near(y, want.detach()) and kept()
+    if cols > 8192:
+        return
+    for pointer in (gamma, None):
+        params = torch.full((2 * cols,), float("nan"), device="cuda")
+        dx, kept = placed(rows, cols, dtype, offset)
+        want = torch.nn.functional.layer_norm(d, (cols,), gd if pointer is not None else None, bd if pointer is not None else None, 1e-5)
+        wx = torch.autograd.grad(want, d, dy.double())[0]
+        n, p, ws = C.workspace("b200jt_layer_norm_backward_workspace", C.desc(x), 1)
+        C.call("b200jt_layer_norm_backward", C.desc(x), C.desc(gamma) if pointer is not None else None, C.desc(dy), C.desc(dx), params.data_ptr(), 1e-5, p, n)
+        xh = torch.nn.functional.layer_norm(d.detach(), (cols,), None, None, 1e-5)
+        # two columns: the gradient is what is left of a cancellation, and E[x^2] - E[x]^2 loses digits with it
+        assert (dx.double() - wx).norm() <= (tol if cols > 8 else 10 * tol) * (wx.norm() + 1e-2 * dy.double().norm()) and kept()
+        assert near(params[:cols], (xh * dy.double()).sum(0)) and near(params[cols:], dy.double().sum(0))
