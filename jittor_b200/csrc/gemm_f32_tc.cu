@@ -236,6 +236,10 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
             for (int i = 0; i < CHUNKS; i++) {
                 const int ch = grp * 32 + i * 64, col0 = tn * A.bn + ch;
                 if (ch >= A.bn || row0 >= A.M || col0 >= A.N) break;     // uniform over the warp
+                bool odd = false;
+#pragma unroll
+                for (int e = 0; e < 32; e++) odd |= !finite(acc[i][e]);
+                odd = __any_sync(0xffffffffu, odd);
                 __syncwarp();
 #pragma unroll
                 for (int e = 0; e < 32; e++) square[lane * TURN_PITCH + e] = acc[i][e];
@@ -243,11 +247,15 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
                 float* out = c + (int64_t)row0 * A.N + col0 + lane;
                 const int rows = min(32, A.M - row0);
                 if (col0 + lane < A.N) {
+                    if (!odd) {
 #pragma unroll 8
-                    for (int r = 0; r < rows; r++) {
-                        float v = square[r * TURN_PITCH + lane] * UNSCALE;
-                        if (!finite(v)) v = dot_again(A, row0 + r, col0 + lane);
-                        out[(int64_t)r * A.N] = v;
+                        for (int r = 0; r < rows; r++) out[(int64_t)r * A.N] = square[r * TURN_PITCH + lane] * UNSCALE;
+                    } else {
+                        for (int r = 0; r < rows; r++) {
+                            float v = square[r * TURN_PITCH + lane] * UNSCALE;
+                            if (!finite(v)) v = dot_again(A, row0 + r, col0 + lane);
+                            out[(int64_t)r * A.N] = v;
+                        }
                     }
                 }
             }
@@ -267,11 +275,11 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
             const int r = rank * rows + e / quads, q = (e % quads) * 4;
             const int m = tm * BM + r, n = tn * A.bn + q;
             if (m >= A.M || n >= A.N) continue;
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            for (int p = 0; p < splits; p++) {
-                const float4 w = *(const float4*)(cluster.map_shared_rank((float*)smem, p) + r * pitch + q);
-                v.x += w.x; v.y += w.y; v.z += w.z; v.w += w.w;
-            }
+            float4 w[MAX_SPLIT], v = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int p = 0; p < MAX_SPLIT; p++) if (p < splits) w[p] = *(const float4*)(cluster.map_shared_rank((float*)smem, p) + r * pitch + q);
+#pragma unroll
+            for (int p = 0; p < MAX_SPLIT; p++) if (p < splits) { v.x += w[p].x; v.y += w[p].y; v.z += w[p].z; v.w += w[p].w; }
             float o[4] = {v.x * UNSCALE, v.y * UNSCALE, v.z * UNSCALE, v.w * UNSCALE};
 #pragma unroll
             for (int i = 0; i < 4; i++)
@@ -379,8 +387,10 @@ struct Plan { bool tc, pair; int bn, splits; };
 // Tile, cluster and path by estimated time. A stage of 32 of K measured 0.84 us with 128 columns on a CTA (its 48 KB in and the
 // 96 KB that the MMAs read share the SM's 128 bytes a cycle) and 1.18 us with 256 on a pair; the split pass reads 4 bytes an
 // element and writes 6. The FMA kernel stays where that pass costs more than it gives -- few rows by a large matrix (16 x 4096 x
-// 4096: 32 and 61 us), small products (300 x 300 x 300: 10 and 14) -- and the estimates are within a fifth of the times
-// measured for 28 shapes; 500 x 777 x 1000: 31 and 20 us, 1024 x 1024 x 1024: 61 and 28, 4096 x 2048 x 4096: 1410 and 349.
+// 4096: 32 and 61 us), small products (300 x 300 x 300: 10 and 14), short K by a wide result (9472 x 39 x 1024: 26.3 and 26.6) --
+// and the estimates are within a fifth of the times measured for 28 shapes; 500 x 777 x 1000: 29 and 18 us, 1024 x 1024 x 1024: 61
+// and 28, 4096 x 2048 x 4096: 1410 and 349. 3 us in hand: of 54 products drawn from 16 to 9472 a side none was then slower than
+// the FMA kernel by more than the timer shows (with 1 us in hand, and half of what the stores take: 4588 x 72 x 3272, 64 and 69).
 static Plan estimate(int64_t M, int64_t N, int64_t K) {
     Plan best{false, false, 128, 1};
     double best_ns = 1e30;
@@ -397,13 +407,13 @@ static Plan estimate(int64_t M, int64_t N, int64_t K) {
                 const int s = 1 << i, at_once = pair ? slots().pair : slots().by_split[i];
                 if (fs && !pair ? atoi(fs) != s : s > 1 && (tiles > at_once || kb / s < 2)) continue;
                 if (s > kb || !at_once) continue;
-                const double ns = 4500 + 10.0 * (M * K + K * N) / 4000 + (double)((tiles + at_once - 1) / at_once) * ((double)((kb + s - 1) / s) * stage + bn * 8.0) + (s > 1 ? 1500 : 0);
+                const double ns = 4500 + 10.0 * (M * K + K * N) / 4000 + (double)((tiles + at_once - 1) / at_once) * ((double)((kb + s - 1) / s) * stage + bn * 16.0) + (s > 1 ? 1500 : 0);
                 if (ns < best_ns) { best_ns = ns; best = {true, pair != 0, bn, s}; }
             }
         }
     }
     const char* f = getenv("B200JT_F32TC");                 // read on every call: tests force each path in turn
-    best.tc = best_ns < 1e30 && (f ? atoi(f) != 0 : best_ns + 1000 < matmul_f32_ns(M, N, K));
+    best.tc = best_ns < 1e30 && (f ? atoi(f) != 0 : best_ns + 3000 < matmul_f32_ns(M, N, K));
     return best;
 }
 
