@@ -104,6 +104,25 @@ inline unsigned grid_for(int64_t work, int block, int ctas_per_sm = 8) {
     return (unsigned)(need < cap ? need : cap);
 }
 
+// A launch whose CTAs all run at once, for kernels that meet at a grid barrier (1.5 us on the device, where a second launch is 2.6 on
+// the host) and take any number of CTAs: where the GPU has room for fewer, that many.
+template <typename... P, typename... A>
+inline cudaError_t launch_cooperative(void (*kernel)(P...), unsigned grid, int block, size_t smem, cudaStream_t st, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative; at[0].val.cooperative = 1;
+    cfg.gridDim = dim3(grid); cfg.blockDim = dim3(block); cfg.dynamicSmemBytes = smem; cfg.stream = st; cfg.attrs = at; cfg.numAttrs = 1;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+    if (e != cudaErrorCooperativeLaunchTooLarge) return e;
+    cudaGetLastError();
+    int device = 0, sms = 0, per_sm = 0;
+    if ((e = cudaGetDevice(&device)) != cudaSuccess || (e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device)) != cudaSuccess ||
+        (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, smem)) != cudaSuccess) return e;
+    if (per_sm < 1 || (unsigned)(sms * per_sm) >= grid) return cudaErrorCooperativeLaunchTooLarge;
+    cfg.gridDim = dim3((unsigned)(sms * per_sm));
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // ---- reduce / binary op codes shared by several kernels -----------------------------------------
 enum OpCode : int {
     OP_ADD = 0, OP_SUB, OP_MUL, OP_DIV, OP_FLOORDIV, OP_MOD, OP_POW, OP_MAX, OP_MIN,

@@ -16,6 +16,7 @@
 #include "index_program.cuh"
 
 #include <algorithm>
+#include <cooperative_groups.h>
 
 namespace b200jt {
 
@@ -463,6 +464,8 @@ rr_direct_kernel(const T* __restrict__ y, const E* __restrict__ idx, T* __restri
 }
 
 // ---- privatised scatter, few bins ------------------------------------------------------------------
+// One cooperative launch: the CTAs publish their rows, meet at a grid barrier, and 32 bins at a time are folded in a fixed order by
+// 32 warps (2^24 float32 into 4096 Zipf bins: 49.2 us, against 52.8 with a second launch whose 8 warps folded).
 // smem layout: R replicas of `bins` elements at a stride of bins+1 (so that the replicas of one bin sit in
 // different banks); lane l of a warp updates replica (l % R), which spreads the same-bin lanes of skewed inputs.
 //
@@ -478,7 +481,7 @@ constexpr int kHot = 4;
 template <typename T, typename E, int VEC, bool ADD>
 __global__ void __launch_bounds__(kPrivThreads, 1)
 rr_privatised_kernel(const T* __restrict__ y, const E* __restrict__ idx, T* __restrict__ partial,
-                     int64_t n, int bins, int replicas, int op_, bool is_bool, bool allow_hot) {
+                     T* __restrict__ x, int64_t n, int bins, int replicas, int op_, bool is_bool, bool allow_hot) {
     const int op = ADD ? (int)OP_ADD : op_;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T* sm = reinterpret_cast<T*>(smem_raw);
@@ -567,27 +570,21 @@ rr_privatised_kernel(const T* __restrict__ y, const E* __restrict__ idx, T* __re
         for (int r = 1; r < replicas; r++) acc = apply_op<T>(op, acc, sm[r * rstride + b]);
         partial[(int64_t)blockIdx.x * bins + b] = acc;
     }
-}
-
-// Folds the per-CTA rows into x in a fixed order (deterministic): a CTA owns 32 bins, its 8 warps take the rows
-// r = w, w+8, ... (coalesced 128-byte reads), then warp 0 combines the 8 partial sums in warp order.
-template <typename T>
-__global__ void __launch_bounds__(256)
-rr_fold_partials_kernel(const T* __restrict__ partial, T* __restrict__ x, int bins, int rows, int op, bool is_bool) {
-    __shared__ T part[8][33];
+    cooperative_groups::this_grid().sync();
+    // the rows into x: warp w takes the rows w, w + 32, ... of 32 bins (128-byte reads), then folds the 32 partial results of bin w
+    T (*part)[33] = reinterpret_cast<T (*)[33]>(smem_raw);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     for (int b0 = blockIdx.x * 32; b0 < bins; b0 += gridDim.x * 32) {
-        const int b = b0 + lane;
-        T acc = init_value<T>(op, is_bool);
-        if (b < bins)
-            for (int r = w; r < rows; r += 8) acc = apply_op<T>(op, acc, partial[(int64_t)r * bins + b]);
+        T acc = init;
+        if (b0 + lane < bins)
+#pragma unroll 4
+            for (int r = w; r < (int)gridDim.x; r += 32) acc = apply_op<T>(op, acc, partial[(int64_t)r * bins + b0 + lane]);
         part[w][lane] = acc;
         __syncthreads();
-        if (w == 0 && b < bins) {
-            T t = part[0][lane];
-#pragma unroll
-            for (int k = 1; k < 8; k++) t = apply_op<T>(op, t, part[k][lane]);
-            x[b] = t;
+        if (lane == 0 && b0 + w < bins) {
+            T t = part[0][w];
+            for (int k = 1; k < 32; k++) t = apply_op<T>(op, t, part[k][w]);
+            x[b0 + w] = t;
         }
         __syncthreads();
     }
@@ -658,7 +655,7 @@ static RRPlan make_plan(const b200jt_tensor* y, const b200jt_tensor* x, int op, 
             plan.path = RRPlan::PRIVATISED;
             int r = (int)(kPrivMaxSmemBytes / ((bins + 1) * es));
             plan.replicas = r >= 8 ? 8 : r >= 4 ? 4 : r >= 2 ? 2 : 1;
-            plan.smem = (size_t)plan.replicas * (bins + 1) * es;
+            plan.smem = std::max<size_t>((size_t)plan.replicas * (bins + 1) * es, 32 * 33 * es);       // replicas, then the fold's square
             plan.workspace = (size_t)kPrivGrid * bins * es;
         } else {
             plan.path = RRPlan::DIRECT;
@@ -743,14 +740,11 @@ static int run_typed(const b200jt_tensor* y, const b200jt_tensor* x, int op, con
                  const cudaError_t e = cudaFuncSetAttribute(rr_privatised_kernel<T, E, V, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPrivMaxSmemBytes); \
                  return e != cudaSuccess ? e : cudaFuncSetAttribute(rr_privatised_kernel<T, E, V, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPrivMaxSmemBytes); }(); \
              B200JT_CUDA(attr_);                                                                                  \
-             k<<<priv_grid, kPrivThreads, plan.smem, st>>>(yp, (const E*)P.extras[0].ptr, partial, n, (int)bins,   \
-                                                           plan.replicas, op, is_bool, allow_hot); } while (0)
+             const E* idx = (const E*)P.extras[0].ptr;                                                            \
+             B200JT_CUDA(launch_cooperative(k, priv_grid, kPrivThreads, plan.smem, st, yp, idx, partial, xp, n, (int)bins, plan.replicas, op, is_bool, allow_hot)); } while (0)
         if (e64) { if (aligned) B200JT_PRIV(int64_t, VEC); else B200JT_PRIV(int64_t, 1); }
         else     { if (aligned) B200JT_PRIV(int32_t, VEC); else B200JT_PRIV(int32_t, 1); }
 #undef B200JT_PRIV
-        B200JT_LAUNCH_CHECK();
-        rr_fold_partials_kernel<T><<<grid_for((bins + 31) / 32 * 256, 256), 256, 0, st>>>(partial, xp, (int)bins, priv_grid, op, is_bool);
-        B200JT_LAUNCH_CHECK();
         return 0;
     }
     if (op != OP_VOID && bins > 0 && !(plan.path == RRPlan::INJECTIVE && plan.covers_all)) {

@@ -1,4 +1,5 @@
 """Kernels at the sizes where their tiles, rings, splits and register rows begin and end, against float64 (or exactly)."""
+import ctypes
 import os
 
 import pytest
@@ -107,6 +108,33 @@ def test_few_bins(n, dtype, idx, op):
     else:
         want = torch.full((bins,), -1e9, device="cuda", dtype=torch.float64).scatter_reduce_(0, i[ok].long(), v[ok].double(), "amax")
     assert torch.equal(got.double(), want)
+
+
+# the fold behind the grid barrier: part of 32 bins, more bins than one pass of the grid takes, fewer CTAs; also from a graph
+@pytest.mark.parametrize("reserve", [0, 64])
+@pytest.mark.parametrize("dtype,bins", [(torch.float32, 1), (torch.float32, 33), (torch.int32, 4737), (torch.float32, 20011), (torch.float64, 9500)])
+def test_few_bins_fold(dtype, bins, reserve):
+    n = 300007
+    v, i = torch.randint(-50, 50, (n,), device="cuda").to(dtype), torch.randint(0, bins, (n,), device="cuda", dtype=torch.int32)
+    want = torch.zeros(bins, device="cuda", dtype=torch.float64).index_add_(0, i.long(), v.double())
+    out = torch.empty(bins, dtype=dtype, device="cuda")
+    idx, none = C.strings(["@e0(i0)"]), C.strings([])
+    args = [C.desc(v), C.desc(out), b"add", idx, 1, none, 0, C.descs([i]), 1]
+    ws = torch.empty(int(C.lib.b200jt_reindex_reduce_workspace(*args)), dtype=torch.uint8, device="cuda")
+    run = lambda: C.call("b200jt_reindex_reduce", *args, ctypes.c_void_p(ws.data_ptr()), ws.numel())
+    C.check(C.lib.b200jt_set_sm_reserve(reserve), "set_sm_reserve")
+    try:
+        run()
+        assert torch.equal(out.double(), want)
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            run()
+        v.neg_()
+        g.replay()
+        g.replay()
+        assert torch.equal(out.double(), -want)
+    finally:
+        C.lib.b200jt_set_sm_reserve(0)
 
 
 # ---- softmax backward: rows in registers with the next one on its way, and rows of up to 16384 columns
