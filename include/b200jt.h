@@ -222,6 +222,9 @@ int b200jt_bn_backward_sums(const b200jt_tensor* x, const b200jt_tensor* dy, con
                             const float* beta, double eps, int relu, float* sums, void* stream);
 int b200jt_bn_backward_dx(const b200jt_tensor* x, const b200jt_tensor* dy, const float* stats, double count, const float* gamma,
                           const float* beta, double eps, int relu, const float* sums, const b200jt_tensor* dx, void* stream);
+/* Both, in one launch where shared memory holds the layer (up to 0.9 MB of x and dy a channel), else in two. */
+int b200jt_bn_backward(const b200jt_tensor* x, const b200jt_tensor* dy, const float* stats, double count, const float* gamma,
+                       const float* beta, double eps, int relu, float* sums, const b200jt_tensor* dx, void* stream);
 
 /* One optimiser step over `count` float32 parameters: kind "sgd" (hyper: lr, momentum, weight decay, 1 - dampening; s0 = velocity),
  * "adam" / "adamw" (b0, 1 - b0, b1, 1 - b1, step size, eps, weight decay or 1 - lr * weight decay, sqrt(1 - b1^n); s0 = second

@@ -88,6 +88,7 @@ SIGNATURES = [
     ("b200jt_layer_norm_backward", _i, [_TP, _TP, _TP, _TP, _FP, _d, _vp, _sz, _vp]),
     ("b200jt_bn_backward_sums", _i, [_TP, _TP, _FP, _d, _FP, _FP, _d, _i, _FP, _vp]),
     ("b200jt_bn_backward_dx", _i, [_TP, _TP, _FP, _d, _FP, _FP, _d, _i, _FP, _TP, _vp]),
+    ("b200jt_bn_backward", _i, [_TP, _TP, _FP, _d, _FP, _FP, _d, _i, _FP, _TP, _vp]),
     ("b200jt_optim_step", _i, [ctypes.c_char_p, _i, ctypes.POINTER(ctypes.c_int64)] + [ctypes.POINTER(_vp)] * 7
      + [ctypes.POINTER(_d), _i, _i, _vp]),
     ("b200jt_matmul_workspace", _sz, [_TP, _TP, _TP, _i, _i]),

@@ -420,7 +420,7 @@ Entry g_entries[] = {
     E(b200jt_conv2d_transpose), E(b200jt_conv2d_backward_w), E(b200jt_conv2d_backward_w_workspace), E(b200jt_conv2d_backward_w_tc),
     E(b200jt_conv2d_backward_w_formats_workspace), E(b200jt_conv2d_backward_w_formats), E(b200jt_bn_stats), E(b200jt_bn_apply),
     E(b200jt_layer_norm_backward_workspace), E(b200jt_layer_norm_backward), E(b200jt_bn_backward_sums),
-    E(b200jt_bn_backward_dx), E(b200jt_pool2d), E(b200jt_pool2d_backward), E(b200jt_pool2d_backward_indices), E(b200jt_pool2d_taps), E(b200jt_conv2d_backward_x), E(b200jt_conv2d_backward_x_workspace),
+    E(b200jt_bn_backward_dx), E(b200jt_bn_backward), E(b200jt_pool2d), E(b200jt_pool2d_backward), E(b200jt_pool2d_backward_indices), E(b200jt_pool2d_taps), E(b200jt_conv2d_backward_x), E(b200jt_conv2d_backward_x_workspace),
     E(b200jt_pool2d_backward_taps),
 };
 #undef E

@@ -1,8 +1,7 @@
 // Gradients of LayerNorm and training BatchNorm (with the ReLU that follows it) as the kernels read them, instead of the
 // op-by-op graph of the reverse rules: that graph is nine row or column reduces and a dozen full-size passes per layer
 // (LayerNorm [5000,1001] float32: 7 launches, 106 us; BatchNorm + ReLU [64,128,28,28] bfloat16: 23 launches, 190 us). Both are
-// bound by memory: x and dy are read once (LayerNorm) or twice, the second time from L2 for layers below its size
-// (BatchNorm), dx is written once, and everything per channel or column is folded in a fixed order.
+// bound by memory: x and dy are read once (LayerNorm, BatchNorm of layers that shared memory holds) or twice, dx is written once, and everything per channel or column is folded in a fixed order.
 //
 //   LayerNorm   xh = (x - mean) * rstd, g = dy * gamma:  dx = rstd * (g - mean(g) - xh * mean(g * xh)),
 //               dgamma = sum over rows of dy * xh, dbeta = sum of dy
@@ -13,6 +12,7 @@
 
 #include <algorithm>
 #include <cooperative_groups.h>
+#include <type_traits>
 
 namespace b200jt {
 namespace nbwd {
@@ -249,13 +249,126 @@ __device__ __forceinline__ bool passes(const BnArgs& g, const BnChannel& k, floa
     return (g.round == 2 ? bf(p) : p) + k.b > 0.f;
 }
 
+// What the sums of a channel become (in place), and the gradient of w in the rounded forms.
+__device__ __forceinline__ float bn_gradients(const BnArgs& g, const BnChannel& k, float& s0, float& s1) {
+    float dw = 0.f;
+    if (g.round == 2) {
+        s0 = bf(s0);
+        dw = bf(bf(s1) + bf(k.mean * -s0));
+        s1 = bf(dw / k.sd);
+    } else if (g.round == 1) {
+        dw = __fadd_rn(s1, __fmul_rn(k.mean, -s0));
+        s1 = dw / k.sd;
+    }
+    return dw;
+}
+// dx of one element, closed form w * d + p * x + q, rounded form ((w * d + x * p) + x * p) + q, each step to bfloat16
+struct BnDx { float p, q; };
+__device__ __forceinline__ BnDx bn_dx(const BnArgs& g, const BnChannel& k, int c, float s0, float s1, float dw) {
+    BnDx r;
+    if (g.round == 0) {
+        r.p = k.live ? -k.w * k.rstd * s1 * g.rcount : 0.f;
+        r.q = -k.w * s0 * g.rcount - r.p * k.mean;
+    } else {
+        const float gamma = g.gamma ? g.gamma[c] : 1.f;
+        float num = __fmul_rn(-dw, gamma), wd = __fmul_rn(k.w, -s0);
+        if (g.round == 2) num = bf(num);
+        const float dvar = k.live ? bf(bf(num / bf(k.sd * k.sd)) / bf(k.sd * 2.f)) : 0.f;
+        const float t = bf(k.mean * -dvar);
+        r.p = bf(dvar * g.rcount);
+        r.q = bf(bf(bf(bf(wd) + t) + t) * g.rcount);
+    }
+    return r;
+}
+__device__ __forceinline__ float bn_dx_of(const BnArgs& g, const BnChannel& k, const BnDx& r, float x, float dy) {
+    const float u = passes(g, k, x) ? dy : 0.f;
+    if (g.round == 0) return k.w * u + (r.p * x + r.q);
+    const float t = bf(x * r.p);
+    return bf(bf(bf(k.w * u) + t) + t) + r.q;                   // the store rounds the last sum
+}
+
+// One vector's part of the three passes over a layer: the sum of bfloat16(x * x), the two sums, dx.
+template <typename TX, typename TD, int N, bool HALF> struct BnPass {
+    static __device__ __forceinline__ void square(const TX* x, float& s) {
+        float a[N];
+        Vec<TX, N>::ld(x, a);
+#pragma unroll
+        for (int e = 0; e < N; e++) s += bf(a[e] * a[e]);
+    }
+    static __device__ __forceinline__ void sums(const BnArgs& g, const BnChannel& k, const TX* x, const TD* dy, float (&s)[2]) {
+        float a[N], d[N];
+        Vec<TX, N>::ld(x, a);
+        Vec<TD, N>::ld(dy, d);
+#pragma unroll
+        for (int e = 0; e < N; e++) {
+            const float v = passes(g, k, a[e]) ? d[e] : 0.f;
+            s[0] += v;
+            s[1] += g.round == 0 ? v * ((a[e] - k.mean) * k.rstd) : g.round == 2 ? bf(a[e] * v) : a[e] * v;
+        }
+    }
+    static __device__ __forceinline__ void grad(const BnArgs& g, const BnChannel& k, const BnDx& r, const TX* x, const TD* dy, TX* dx) {
+        float a[N], d[N];
+        Vec<TX, N>::ld(x, a);
+        Vec<TD, N>::ld(dy, d);
+#pragma unroll
+        for (int e = 0; e < N; e++) a[e] = bn_dx_of(g, k, r, a[e], d[e]);
+        Vec<TX, N>::st(dx, a);
+    }
+};
+// Every step in bfloat16 (g.round == 2, x and dy bfloat16): the passes are bound by their conversions, a dozen an element when each
+// rounds alone (64 x 128 x 28 x 28 in one launch: 24.6 us, in pairs 18.3; in two 29.2 and 25). The products' factors are all bfloat16, so that one packed multiplication rounds two of them as float32 and a
+// conversion would; sums stay float32 and are converted in pairs. x * w + b > 0 is x * w > -b: a float32 sum is 0 only if it is.
+struct Pair { float x, y; };
+__device__ __forceinline__ Pair floats(__nv_bfloat162 v) { const float2 f = __bfloat1622float2(v); return {f.x, f.y}; }
+__device__ __forceinline__ __nv_bfloat162 masked(const BnArgs& g, const BnChannel& k, __nv_bfloat162 a, __nv_bfloat162 d) {
+    if (!g.relu) return d;
+    const Pair p = floats(__hmul2_rn(a, __float2bfloat162_rn(k.w)));
+    unsigned v;
+    memcpy(&v, &d, 4);
+    v &= (p.x > -k.b ? 0xffffu : 0u) | (p.y > -k.b ? 0xffff0000u : 0u);
+    memcpy(&d, &v, 4);
+    return d;
+}
+template <> struct BnPass<__nv_bfloat16, __nv_bfloat16, 8, true> {
+    using B = __nv_bfloat16;
+    struct alignas(16) Pack { __nv_bfloat162 h[4]; };
+    static __device__ __forceinline__ void square(const B* x, float& s) {
+        const Pack a = *(const Pack*)x;
+#pragma unroll
+        for (int e = 0; e < 4; e++) { const Pair q = floats(__hmul2_rn(a.h[e], a.h[e])); s += q.x; s += q.y; }
+    }
+    static __device__ __forceinline__ void sums(const BnArgs& g, const BnChannel& k, const B* x, const B* dy, float (&s)[2]) {
+        const Pack a = *(const Pack*)x, d = *(const Pack*)dy;
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+            const __nv_bfloat162 v = masked(g, k, a.h[e], d.h[e]);
+            const Pair f = floats(v), q = floats(__hmul2_rn(a.h[e], v));
+            s[0] += f.x; s[0] += f.y;
+            s[1] += q.x; s[1] += q.y;
+        }
+    }
+    static __device__ __forceinline__ void grad(const BnArgs& g, const BnChannel& k, const BnDx& r, const B* x, const B* dy, B* dx) {
+        const Pack a = *(const Pack*)x, d = *(const Pack*)dy;
+        Pack o;
+        const __nv_bfloat162 w = __float2bfloat162_rn(k.w), p = __float2bfloat162_rn(r.p);
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+            const Pair u = floats(__hmul2_rn(w, masked(g, k, a.h[e], d.h[e]))), t = floats(__hmul2_rn(a.h[e], p));
+            const Pair y = floats(__floats2bfloat162_rn(u.x + t.x, u.y + t.y)), z = floats(__floats2bfloat162_rn(y.x + t.x, y.y + t.y));
+            o.h[e] = __floats2bfloat162_rn(z.x + r.q, z.y + r.q);
+        }
+        *(Pack*)dx = o;
+    }
+};
+
 // A cluster of up to 8 CTAs per channel: CTA j takes the planes n = j, j + cluster size, ..., as one run of N-element vectors over
 // all its threads (a plane at a time left 158 of 256 threads idle at 28 x 28: 64 x 128 x 28 x 28 29 us, 15.5 us this way),
 // and the CTAs' sums meet through distributed shared memory in rank order. With the graph's rounding a first sweep forms
 // E[bfloat16(x * x)] (the second sweep reads x from L2). sums: [4][C] = dbeta, dgamma, that mean square, the gradient of w.
-template <typename TX, typename TD, int N>
+template <typename TX, typename TD, int N, bool HALF>
 __global__ void __launch_bounds__(256)
 bn_bwd_sums_kernel(const TX* __restrict__ x, const TD* __restrict__ dy, float* __restrict__ sums, const BnArgs g) {
+    using Pass = BnPass<TX, TD, N, HALF>;
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
     const int c = blockIdx.y;
@@ -276,12 +389,7 @@ bn_bwd_sums_kernel(const TX* __restrict__ x, const TD* __restrict__ dy, float* _
     float square = 0.f;
     if (g.round > 0) {
         float s[1] = {0.f};
-        planes([&](int64_t i) {
-            float a[N];
-            Vec<TX, N>::ld(x + i, a);
-#pragma unroll
-            for (int e = 0; e < N; e++) s[0] += bf(a[e] * a[e]);
-        });
+        planes([&](int64_t i) { Pass::square(x + i, s[0]); });
         row_sum<256, 1>(s, sm);
         if (threadIdx.x == 0) mine[0] = s[0];
         cluster.sync();
@@ -290,59 +398,28 @@ bn_bwd_sums_kernel(const TX* __restrict__ x, const TD* __restrict__ dy, float* _
     }
     const BnChannel k = bn_channel(g, c, square);
     float s[2] = {0.f, 0.f};
-    planes([&](int64_t i) {
-        float a[N], d[N];
-        Vec<TX, N>::ld(x + i, a);
-        Vec<TD, N>::ld(dy + i, d);
-#pragma unroll
-        for (int e = 0; e < N; e++) {
-            const float v = passes(g, k, a[e]) ? d[e] : 0.f;
-            s[0] += v;
-            s[1] += g.round == 0 ? v * ((a[e] - k.mean) * k.rstd) : g.round == 2 ? bf(a[e] * v) : a[e] * v;
-        }
-    });
+    planes([&](int64_t i) { Pass::sums(g, k, x + i, dy + i, s); });
     row_sum<256, 2>(s, sm);
     if (threadIdx.x == 0) { mine[1] = s[0]; mine[2] = s[1]; }
     cluster.sync();
     if (rank == 0 && threadIdx.x == 0) {
-        float s0 = 0.f, s1 = 0.f, dw = 0.f;
+        float s0 = 0.f, s1 = 0.f;
         for (int r = 0; r < size; r++) { s0 += cluster.map_shared_rank(mine, r)[1]; s1 += cluster.map_shared_rank(mine, r)[2]; }
-        if (g.round == 2) {
-            s0 = bf(s0);
-            dw = bf(bf(s1) + bf(k.mean * -s0));
-            s1 = bf(dw / k.sd);
-        } else if (g.round == 1) {
-            dw = __fadd_rn(s1, __fmul_rn(k.mean, -s0));
-            s1 = dw / k.sd;
-        }
+        const float dw = bn_gradients(g, k, s0, s1);
         sums[c] = s0; sums[g.C + c] = s1; sums[2 * g.C + c] = square; sums[3 * g.C + c] = dw;
     }
     cluster.sync();                                             // no CTA leaves while its sums are read
 }
 
-// dx over the tensor as one stream of N-element vectors; the channels' coefficients are derived once per CTA:
-// closed form dx = w * d + p * x + q; rounded form dx = ((w * d + x * p) + x * p) + q, each step to bfloat16.
-template <typename TX, typename TD, int N>
+// dx over the tensor as one stream of N-element vectors; the channels' coefficients are derived once per CTA.
+template <typename TX, typename TD, int N, bool HALF>
 __global__ void __launch_bounds__(256)
 bn_bwd_dx_kernel(const TX* __restrict__ x, const TD* __restrict__ dy, const float* __restrict__ sums, TX* __restrict__ dx, const BnArgs g) {
     extern __shared__ float co[];                               // per channel: w, b, p, q
     for (int c = threadIdx.x; c < g.C; c += 256) {
         const BnChannel k = bn_channel(g, c, sums[2 * g.C + c]);
-        const float s0 = sums[c];
-        float p, q;
-        if (g.round == 0) {
-            p = k.live ? -k.w * k.rstd * sums[g.C + c] * g.rcount : 0.f;
-            q = -k.w * s0 * g.rcount - p * k.mean;
-        } else {
-            const float gamma = g.gamma ? g.gamma[c] : 1.f, dw = sums[3 * g.C + c];
-            float num = __fmul_rn(-dw, gamma), wd = __fmul_rn(k.w, -s0);
-            if (g.round == 2) num = bf(num);
-            const float dvar = k.live ? bf(bf(num / bf(k.sd * k.sd)) / bf(k.sd * 2.f)) : 0.f;
-            const float t = bf(k.mean * -dvar);
-            p = bf(dvar * g.rcount);
-            q = bf(bf(bf(bf(wd) + t) + t) * g.rcount);
-        }
-        co[c] = k.w; co[g.C + c] = k.b; co[2 * g.C + c] = p; co[3 * g.C + c] = q;
+        const BnDx r = bn_dx(g, k, c, sums[c], sums[g.C + c], sums[3 * g.C + c]);
+        co[c] = k.w; co[g.C + c] = k.b; co[2 * g.C + c] = r.p; co[3 * g.C + c] = r.q;
     }
     __syncthreads();
     const int64_t vpp = g.HW / N, nvec = (int64_t)g.N_ * g.C * vpp;
@@ -350,21 +427,79 @@ bn_bwd_dx_kernel(const TX* __restrict__ x, const TD* __restrict__ dy, const floa
         const int c = nvec < 0x7fffffff ? ((unsigned)v / (unsigned)vpp) % (unsigned)g.C : (int)((v / vpp) % g.C);
         BnChannel k;
         k.w = co[c]; k.b = co[g.C + c];
-        const float p = co[2 * g.C + c], q = co[3 * g.C + c];
-        float a[N], d[N];
-        Vec<TX, N>::ld(x + v * N, a);
-        Vec<TD, N>::ld(dy + v * N, d);
-#pragma unroll
-        for (int e = 0; e < N; e++) {
-            const float u = passes(g, k, a[e]) ? d[e] : 0.f;
-            if (g.round == 0) a[e] = k.w * u + (p * a[e] + q);
-            else {
-                const float t = bf(a[e] * p);
-                a[e] = bf(bf(bf(k.w * u) + t) + t) + q;         // the store rounds the last sum
-            }
-        }
-        Vec<TX, N>::st(dx + v * N, a);
+        const BnDx r = {co[2 * g.C + c], co[3 * g.C + c]};
+        BnPass<TX, TD, N, HALF>::grad(g, k, r, x + v * N, dy + v * N, dx + v * N);
     }
+}
+
+// Both of the above in one launch, for layers that shared memory holds: the CTAs of a channel's cluster keep their planes of x and dy
+// in it, so that these are read once, and nothing but the sums meets between the two parts. Each thread copies, and later reads,
+// its own vectors: the copies need no barrier. 64 x 128 x 28 x 28 bfloat16: 18.3 us, the two kernels 15.7 + 13.5 and a launch
+// between them; from cold caches 64 x 1024 x 14 x 14 82 and 138, float32 45 and 69.
+template <int BYTES>
+__device__ __forceinline__ void hold(void* to, const void* from) {
+    if constexpr (BYTES >= 16) {
+#pragma unroll
+        for (int b = 0; b < BYTES; b += 16)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(to) + b), "l"((const char*)from + b) : "memory");
+    } else if constexpr (BYTES == 4) *(float*)to = *(const float*)from;
+    else *(unsigned short*)to = *(const unsigned short*)from;
+}
+template <typename TX, typename TD, int N, bool HALF>
+__global__ void __launch_bounds__(256)
+bn_bwd_held_kernel(const TX* __restrict__ x, const TD* __restrict__ dy, float* __restrict__ sums, TX* __restrict__ dx, const BnArgs g) {
+    using Pass = BnPass<TX, TD, N, HALF>;
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    extern __shared__ __align__(16) unsigned char held[];
+    __shared__ float sm[32], mine[4];
+    const int c = blockIdx.y;
+    const int rank = (int)cluster.block_rank(), size = (int)cluster.num_blocks();
+    const unsigned hv = (unsigned)g.HW / N, dj = 256 / hv, di = 256 - dj * hv, j0 = threadIdx.x / hv, i0 = threadIdx.x - j0 * hv;
+    const int total = (int)((g.N_ - rank + size - 1) / size * hv), most = (int)((g.N_ + size - 1) / size * hv);
+    TX* hx = (TX*)held;
+    TD* hd = (TD*)(held + ((size_t)most * N * sizeof(TX) + 15) / 16 * 16);
+    auto planes = [&](auto&& f) {
+        unsigned j = j0, i = i0;
+#pragma unroll 4
+        for (int v = threadIdx.x; v < total; v += 256) {
+            f(v * N, ((int64_t)(rank + j * size) * g.C + c) * g.HW + i * N);
+            j += dj; i += di;
+            if (i >= hv) { i -= hv; j++; }
+        }
+    };
+    planes([&](int v, int64_t at) { hold<N * sizeof(TX)>(hx + v, x + at); });
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    planes([&](int v, int64_t at) { hold<N * sizeof(TD)>(hd + v, dy + at); });
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    float square = 0.f;
+    if (g.round > 0) {
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        float s[1] = {0.f};
+#pragma unroll 4
+        for (int v = threadIdx.x; v < total; v += 256) Pass::square(hx + v * N, s[0]);
+        row_sum<256, 1>(s, sm);
+        if (threadIdx.x == 0) mine[0] = s[0];
+        cluster.sync();
+        for (int r = 0; r < size; r++) square += cluster.map_shared_rank(mine, r)[0];
+        square *= g.rcount;
+    }
+    const BnChannel k = bn_channel(g, c, square);
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    float s[2] = {0.f, 0.f};
+#pragma unroll 4
+    for (int v = threadIdx.x; v < total; v += 256) Pass::sums(g, k, hx + v * N, hd + v * N, s);
+    row_sum<256, 2>(s, sm);
+    if (threadIdx.x == 0) { mine[1] = s[0]; mine[2] = s[1]; }
+    cluster.sync();
+    float s0 = 0.f, s1 = 0.f;
+    for (int r = 0; r < size; r++) { s0 += cluster.map_shared_rank(mine, r)[1]; s1 += cluster.map_shared_rank(mine, r)[2]; }
+    cluster.barrier_arrive();                                   // its sums are read; waited for at the end: no CTA leaves before
+    const float dw = bn_gradients(g, k, s0, s1);
+    if (rank == 0 && threadIdx.x == 0) { sums[c] = s0; sums[g.C + c] = s1; sums[2 * g.C + c] = square; sums[3 * g.C + c] = dw; }
+    const BnDx r = bn_dx(g, k, c, s0, s1, dw);
+    planes([&](int v, int64_t at) { Pass::grad(g, k, r, hx + v, hd + v, dx + at); });
+    cluster.barrier_wait();
 }
 
 // Rows stay in registers up to 8192 columns (32 elements a thread); the host keeps the op-by-op graph for longer ones.
@@ -411,21 +546,33 @@ int run_ln(const T* x, const T* dy, const float* gamma, T* dx, float* params, fl
 #undef B200JT_LN
 }
 
+// As many CTAs as run at once, four per SM; at most a cluster of 8, a plane for each and a vector for each thread.
+inline int bn_cluster(const BnArgs& g, int n) {
+    int size = 1;
+    while (size < 8 && size * 2 * g.C <= 4 * (kNumSMs - sm_reserve()) && size * 2 <= g.N_ && g.N_ / (size * 2) * (g.HW / n) >= 256) size *= 2;
+    return size;
+}
+inline void cluster_launch(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* at, int size, int C, cudaStream_t st) {
+    at->id = cudaLaunchAttributeClusterDimension;
+    at->val.clusterDim.x = (unsigned)size; at->val.clusterDim.y = 1; at->val.clusterDim.z = 1;
+    cfg->gridDim = dim3(size, C);
+    cfg->blockDim = dim3(256);
+    cfg->stream = st;
+    cfg->attrs = at;
+    cfg->numAttrs = 1;
+}
+template <typename TX, typename TD, int N> constexpr bool can_half = std::is_same<TX, __nv_bfloat16>::value && std::is_same<TD, __nv_bfloat16>::value && N == 8;
+template <typename TX, typename TD, int N> inline bool half_steps(const BnArgs& g) { return can_half<TX, TD, N> && g.round == 2; }
+// A layer is held with four CTAs to an SM where a cluster of 8 allows it, and with two at the least (bfloat16 256 x 256 x 28 x 28,
+// 98 KB each: 135 us, 149 in two kernels; float32 128 x 128 x 28 x 28: 55 and 63); one alone would load, add and store in turn.
+constexpr int64_t kHeldWanted = 55 << 10, kHeldMost = 112 << 10;
+
 template <typename TX, typename TD, int N>
 int launch_bn_sums(const b200jt_tensor* x, const b200jt_tensor* dy, float* sums, const BnArgs& g, cudaStream_t st) {
-    // as many CTAs as run at once, four per SM; at most a cluster of 8, a plane for each and a vector for each thread
-    int size = 1;
-    while (size < 8 && size * 2 * g.C <= 4 * (kNumSMs - sm_reserve()) && size * 2 <= g.N_ && g.N_ / (size * 2) * (g.HW / N) >= 256) size *= 2;
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(size, g.C);
-    cfg.blockDim = dim3(256);
-    cfg.stream = st;
     cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = (unsigned)size; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    B200JT_CUDA(cudaLaunchKernelEx(&cfg, bn_bwd_sums_kernel<TX, TD, N>, (const TX*)x->ptr, (const TD*)dy->ptr, sums, g));
+    cluster_launch(&cfg, &at, bn_cluster(g, N), g.C, st);
+    B200JT_CUDA(cudaLaunchKernelEx(&cfg, half_steps<TX, TD, N>(g) ? bn_bwd_sums_kernel<TX, TD, N, can_half<TX, TD, N>> : bn_bwd_sums_kernel<TX, TD, N, false>, (const TX*)x->ptr, (const TD*)dy->ptr, sums, g));
     return 0;
 }
 
@@ -441,10 +588,42 @@ int run_bn_dx(const b200jt_tensor* x, const b200jt_tensor* dy, const float* sums
     const int64_t n = (int64_t)g.N_ * g.C * g.HW / (vec ? V : 1);
     const unsigned grid = grid_for(n, 256, 6);
     const size_t smem = sizeof(float) * 4 * g.C;
-    if (vec) bn_bwd_dx_kernel<TX, TD, V><<<grid, 256, smem, st>>>((const TX*)x->ptr, (const TD*)dy->ptr, sums, (TX*)dx->ptr, g);
-    else bn_bwd_dx_kernel<TX, TD, 1><<<grid, 256, smem, st>>>((const TX*)x->ptr, (const TD*)dy->ptr, sums, (TX*)dx->ptr, g);
+    if (vec && half_steps<TX, TD, V>(g)) bn_bwd_dx_kernel<TX, TD, V, can_half<TX, TD, V>><<<grid, 256, smem, st>>>((const TX*)x->ptr, (const TD*)dy->ptr, sums, (TX*)dx->ptr, g);
+    else if (vec) bn_bwd_dx_kernel<TX, TD, V, false><<<grid, 256, smem, st>>>((const TX*)x->ptr, (const TD*)dy->ptr, sums, (TX*)dx->ptr, g);
+    else bn_bwd_dx_kernel<TX, TD, 1, false><<<grid, 256, smem, st>>>((const TX*)x->ptr, (const TD*)dy->ptr, sums, (TX*)dx->ptr, g);
     B200JT_LAUNCH_CHECK();
     return 0;
+}
+
+// 0: done; 1: the layer is not held (b200jt_bn_backward then runs the two kernels)
+template <typename TX, typename TD, int N>
+int launch_bn_held(const b200jt_tensor* x, const b200jt_tensor* dy, float* sums, const b200jt_tensor* dx, const BnArgs& g, cudaStream_t st) {
+    const int64_t plane = g.HW * (int64_t)(sizeof(TX) + sizeof(TD));
+    int size = bn_cluster(g, N);
+    while (size < 8 && size * 2 <= g.N_ && (g.N_ + size - 1) / size * plane > kHeldWanted) size *= 2;
+    const int64_t smem = (g.N_ + size - 1) / size * plane + 16;
+    if (smem > kHeldMost) return 1;
+    const auto kernel = half_steps<TX, TD, N>(g) ? bn_bwd_held_kernel<TX, TD, N, can_half<TX, TD, N>> : bn_bwd_held_kernel<TX, TD, N, false>;
+    static const cudaError_t attr = [] {
+        const cudaError_t e = cudaFuncSetAttribute(bn_bwd_held_kernel<TX, TD, N, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kHeldMost);
+        return e != cudaSuccess ? e : cudaFuncSetAttribute(bn_bwd_held_kernel<TX, TD, N, can_half<TX, TD, N>>, cudaFuncAttributeMaxDynamicSharedMemorySize, kHeldMost);
+    }();
+    B200JT_CUDA(attr);
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute at{};
+    cluster_launch(&cfg, &at, size, g.C, st);
+    cfg.dynamicSmemBytes = (size_t)smem;
+    B200JT_CUDA(cudaLaunchKernelEx(&cfg, kernel, (const TX*)x->ptr, (const TD*)dy->ptr, sums, (TX*)dx->ptr, g));
+    return 0;
+}
+
+template <typename TX, typename TD, int V>
+int run_bn(const b200jt_tensor* x, const b200jt_tensor* dy, float* sums, const b200jt_tensor* dx, const BnArgs& g, cudaStream_t st) {
+    const bool vec = g.HW % V == 0 && ((uintptr_t)x->ptr | (uintptr_t)dy->ptr | (uintptr_t)dx->ptr) % 16 == 0;
+    int rc = vec ? launch_bn_held<TX, TD, V>(x, dy, sums, dx, g, st) : launch_bn_held<TX, TD, 1>(x, dy, sums, dx, g, st);
+    if (rc != 1) return rc;
+    rc = run_bn_sums<TX, TD, V>(x, dy, sums, g, st);
+    return rc ? rc : run_bn_dx<TX, TD, V>(x, dy, sums, dx, g, st);
 }
 
 inline bool f32_or_bf16(int dt) { return dt == B200JT_FLOAT32 || dt == B200JT_BFLOAT16; }
@@ -515,4 +694,16 @@ extern "C" int b200jt_bn_backward_dx(const b200jt_tensor* x, const b200jt_tensor
     using B = __nv_bfloat16;
     if (x->dtype == B200JT_FLOAT32) return dy->dtype == B200JT_FLOAT32 ? run_bn_dx<float, float, 4>(x, dy, sums, dx, g, st) : run_bn_dx<float, B, 8>(x, dy, sums, dx, g, st);
     return dy->dtype == B200JT_FLOAT32 ? run_bn_dx<B, float, 8>(x, dy, sums, dx, g, st) : run_bn_dx<B, B, 8>(x, dy, sums, dx, g, st);
+}
+
+extern "C" int b200jt_bn_backward(const b200jt_tensor* x, const b200jt_tensor* dy, const float* stats, double count, const float* gamma,
+                                  const float* beta, double eps, int relu, float* sums, const b200jt_tensor* dx, void* stream) {
+    BnArgs g;
+    int rc = bn_args(x, dy, stats, count, gamma, beta, eps, relu, &g);
+    if (rc) return rc;
+    B200JT_CHECK_ARG(sums && numel(x) > 0 && valid_tensor(dx) && dx->dtype == x->dtype && numel(dx) == numel(x), "sums is NULL, x is empty or dx has not x's dtype and size");
+    cudaStream_t st = (cudaStream_t)stream;
+    using B = __nv_bfloat16;
+    if (x->dtype == B200JT_FLOAT32) return dy->dtype == B200JT_FLOAT32 ? run_bn<float, float, 4>(x, dy, sums, dx, g, st) : run_bn<float, B, 8>(x, dy, sums, dx, g, st);
+    return dy->dtype == B200JT_FLOAT32 ? run_bn<B, float, 8>(x, dy, sums, dx, g, st) : run_bn<B, B, 8>(x, dy, sums, dx, g, st);
 }

@@ -375,14 +375,21 @@ def _plan_bn_sums(v, r):
 
 
 def _plan_bn_dx(v, r):
+    """The gradient of x; sums that are still to be computed come out of the same call."""
     leaves, args = _bn_operands(r)
     sums = r[8]
 
     def run():
+        a = args()
         dx = C.alloc(list(v.shape), C.TORCH_DTYPES[v.dtype])
-        C.call("b200jt_bn_backward_dx", *args(), sums._data.data_ptr(), C.desc(dx), what="bn_backward_dx")
+        if sums._data is not None:
+            C.call("b200jt_bn_backward_dx", *a, sums._data.data_ptr(), C.desc(dx), what="bn_backward_dx")
+            return dx
+        both = C.alloc(list(sums.shape), torch.float32)
+        C.call("b200jt_bn_backward", *a, both.data_ptr(), C.desc(dx), what="bn_backward")
+        sums._data = both
         return dx
-    return _plan(leaves + [sums], run)
+    return _plan(leaves, run)
 
 
 _PLANS = {"matmul": _plan_matmul, "conv2d": _plan_conv, "conv2d_transpose": _plan_conv, "conv2d_dx": _plan_conv_dx, "conv2d_dw": _plan_conv_dw,

@@ -224,3 +224,36 @@ def test_ragged_rows(rows, cols, offset, dtype):
         # two columns: the gradient is what is left of a cancellation, and E[x^2] - E[x]^2 loses digits with it
         assert (dx.double() - wx).norm() <= (tol if cols > 8 else 10 * tol) * (wx.norm() + 1e-2 * dy.double().norm()) and kept()
         assert near(params[:cols], (xh * dy.double()).sum(0)) and near(params[cols:], dy.double().sum(0))
+
+
+# ---- BatchNorm's gradient in one launch (csrc/norm_bwd.cu): planes that do not divide the cluster, single elements, what shared
+# memory just holds and what it does not; against float64, and the rounded forms against the two kernels
+@pytest.mark.parametrize("form", [0, 1, 3, 5])
+@pytest.mark.parametrize("xt,dt", [(torch.float32, torch.float32), (torch.bfloat16, torch.bfloat16), (torch.float32, torch.bfloat16), (torch.bfloat16, torch.float32)])
+@pytest.mark.parametrize("shape", [(1, 2, 3, 3), (3, 5, 7, 7), (13, 3, 8, 8), (64, 128, 28, 28), (9, 40, 33, 31), (256, 512, 7, 7), (8, 2, 112, 128), (8, 2, 112, 136), (2, 1, 200, 200)])
+def test_batch_norm_backward_in_one_launch(shape, xt, dt, form):
+    cn, count = shape[1], shape[0] * shape[2] * shape[3]
+    x, dy = (torch.randn(shape, device="cuda") + 0.3).to(xt), torch.randn(shape, device="cuda").to(dt)
+    gamma, beta = torch.rand(cn, device="cuda") + 0.5, torch.randn(cn, device="cuda") * 0.1
+    xd, per = x.double(), lambda t: t.double()[None, :, None, None]
+    stats = torch.cat([xd.sum((0, 2, 3)), (xd * xd).sum((0, 2, 3))]).float()
+    mean = per(stats[:cn].double() / count)
+    rstd = (per(stats[cn:].double() / count) - mean ** 2 + 1e-5).rsqrt()
+    xh = (xd - mean) * rstd
+    act = xh * per(gamma) + per(beta)
+    dy[act.abs() < 1e-4] = 0                               # within rounding of the ReLU's edge: either side of it is right
+    dd = dy.double()
+    head = (C.desc(x), C.desc(dy), stats.data_ptr(), float(count), gamma.data_ptr(), beta.data_ptr(), 1e-5, form)
+    sums, dx = torch.full((4 * cn,), float("nan"), device="cuda"), torch.full(shape, float("nan"), device="cuda", dtype=xt)
+    C.call("b200jt_bn_backward", *head, sums.data_ptr(), C.desc(dx))
+    if form > 1:                                           # 16-bit steps: another order of the sums may turn one of them
+        s2, d2 = torch.empty_like(sums), torch.empty_like(dx)
+        C.call("b200jt_bn_backward_sums", *head, s2.data_ptr())
+        C.call("b200jt_bn_backward_dx", *head, s2.data_ptr(), C.desc(d2))
+        assert (sums - s2)[: 3 * cn].norm() <= 2.0 ** -7 * s2[: 3 * cn].norm() + 1e-5 * count ** 0.5 and (dx.double() - d2.double()).norm() <= 2.0 ** -7 * d2.double().norm()
+        return
+    d = torch.where(act > 0, dd, 0.0) if form else dd
+    s0, s1 = d.sum((0, 2, 3)), (d * xh).sum((0, 2, 3))
+    want = per(gamma) * rstd * (d - (per(s0) + xh * per(s1)) / count)
+    assert (sums[:cn].double() - s0).norm() <= 1e-5 * count ** 0.5 * cn ** 0.5 and (sums[cn:2 * cn].double() - s1).norm() <= 1e-5 * count ** 0.5 * cn ** 0.5
+    assert (dx.double() - want).norm() <= (2.0 ** -8 if xt == torch.bfloat16 else 1e-4) * want.norm() + 1e-6
