@@ -480,7 +480,8 @@ static int launch_rows(const T* x, T* y, const float* gamma, const float* beta, 
         if (cols <= 32 * 8) B200JT_ROW(32, 8);
         else if (cols <= 32 * 16) B200JT_ROW(32, 16);
         else if (cols <= 128 * 8) B200JT_ROW(128, 8);
-        else if (cols <= 128 * 16) B200JT_ROW(128, 16);
+        else if (cols <= 128 * 16 && sizeof(T) == 4) B200JT_ROW(128, 16);       // [32736, 1025] LayerNorm: float32 1.25x, bfloat16 0.86x
+        else if (cols <= 256 * 8) B200JT_ROW(256, 8);
         else if (cols <= 256 * 16) B200JT_ROW(256, 16);
         else B200JT_ROW(256, 32);
         B200JT_LAUNCH_CHECK();
@@ -519,8 +520,9 @@ static int launch_rows(const T* x, T* y, const float* gamma, const float* beta, 
 // the two reductions of the reference's hand-written backward (python/jittor/other/code_softmax.py:109-147). The row of y
 // and of dy live in registers: one read of each, one write of dx.
 // bfloat16: the next row's vectors are loaded, as they lie in memory, before this row's sum goes round the CTA, so that the loads do
-// not wait for the barrier and the stores: [32768, 4096] 147 -> 121 us, [65536, 1024] 105 -> 63. Rows of 8193 to 16384 columns take a CTA of 1024
-// threads ([8192, 16384] bfloat16: 270 us in two sweeps).
+// not wait for the barrier and the stores: [32768, 4096] 147 -> 121 us, [65536, 1024] 105 -> 63. Rows of vectors and 8193 to 16384 columns
+// take a CTA of 1024 threads ([8192, 16384] bfloat16: 126 us, 270 in two sweeps); single elements do not ([4095, 8193] bfloat16 94
+// and 63: the second sweep reads what the first left in the cache).
 template <typename T, typename V, int GROUP, int VPT, bool LOG>
 __global__ void __launch_bounds__(cta_of(GROUP))
 softmax_bwd_reg_kernel(const T* __restrict__ y, const T* __restrict__ dy, T* __restrict__ dx, int64_t rows, int cols) {
@@ -530,8 +532,15 @@ softmax_bwd_reg_kernel(const T* __restrict__ y, const T* __restrict__ dy, T* __r
     const int g = threadIdx.x / GROUP, t = threadIdx.x % GROUP;
     const int nvec = cols / N;
     const int64_t step = (int64_t)gridDim.x * ROWS_PER_CTA;
-    // float32 rows have as many bytes in flight without, and one vector to a lane leaves room for more rows instead
-    constexpr bool AHEAD = sizeof(T) == 2 && N > 1 && (GROUP > 32 || VPT > 1) && VPT <= (GROUP > 512 ? 2 : 4);
+    // float32 rows have as many bytes in flight without, and one vector to a thread leaves room for more rows instead ([4096, 2048]
+    // 6.5 us, 7.1 with)
+    constexpr bool AHEAD = sizeof(T) == 2 && N > 1 && VPT > 1 && VPT <= (GROUP > 512 ? 2 : 4);
+    // Single elements: all loads of the row before its sum, where the compiler would else wait for some of them on the way. [6709, 5001]
+    // bfloat16 190 -> 89 us, [16768, 2001] 68 -> 48, log 127 -> 70, [120000, 255] float32 72 -> 57; not where it measured slower: few
+    // elements to a thread, or 16 of them ([2795, 3001] bfloat16 0.83x, but log 1.13x), wide float32 rows ([11181, 3001] 0.82x)
+    constexpr bool FIRST = (N == 4 && VPT >= 4) ||          // float32 vectors: log of [16384, 512] 12.5 us, 13.6 without
+                           (N == 1 && ((GROUP == 32 && VPT == 8) || GROUP == 64 ||
+                                       (sizeof(T) == 2 && (VPT == 8 || VPT == 32 || (VPT == 16 && LOG)))));
     // the CTA-wide reduction has a barrier inside: rows are taken in rounds the whole CTA goes through together
     if constexpr (AHEAD) {
         typename V::Raw a[VPT], b[VPT];
@@ -586,10 +595,18 @@ softmax_bwd_reg_kernel(const T* __restrict__ y, const T* __restrict__ dy, T* __r
                 if (live && vi < nvec) {
                     V::load(y + row * cols + (int64_t)vi * N, a[k]);
                     V::load(dy + row * cols + (int64_t)vi * N, b[k]);
+                    if (!FIRST)
+#pragma unroll
+                        for (int e = 0; e < N; e++) s += LOG ? b[k][e] : a[k][e] * b[k][e];
+                } else if (FIRST)
+#pragma unroll
+                    for (int e = 0; e < N; e++) a[k][e] = b[k][e] = 0.f;
+            }
+            if (FIRST)
+#pragma unroll
+                for (int k = 0; k < VPT; k++)
 #pragma unroll
                     for (int e = 0; e < N; e++) s += LOG ? b[k][e] : a[k][e] * b[k][e];
-                }
-            }
             s = group_reduce<GROUP, false>(s, sm);
 #pragma unroll
             for (int k = 0; k < VPT; k++) {
@@ -629,17 +646,16 @@ static int launch_softmax_bwd(const T* y, const T* dy, T* dx, int64_t rows, int6
     const int64_t nvec = cols / N;
 #define B200JT_SB(GROUP, VPT)                                                                       \
     softmax_bwd_reg_kernel<T, V, GROUP, VPT, LOG><<<row_grid(rows, GROUP), cta_of(GROUP), 0, st>>>(y, dy, dx, rows, (int)cols)
-    if (!vec_ok && cols <= 1024 * 16) {
+    if (!vec_ok && cols <= 256 * 32) {
         using V = Single<T>;
-        // [60000, 301] float32: 66 us with 256 threads to the row, 40 with 64; [20000, 777] bfloat16 26 and 22 with 128
-        if (cols <= 32 * 8) B200JT_SB(32, 8);
+        // [60000, 301] float32: 66 us with 256 threads to the row, 40 with 64; [43000, 777] bfloat16 56 and, with 128, 72
+        if (cols <= 32 * 4) B200JT_SB(32, 4);
+        else if (cols <= 32 * 8) B200JT_SB(32, 8);
         else if (cols <= 64 * 8) B200JT_SB(64, 8);
-        else if (cols <= 128 * 8 && sizeof(T) == 2) B200JT_SB(128, 8);
         else if (cols <= 256 * 4) B200JT_SB(256, 4);
         else if (cols <= 256 * 8) B200JT_SB(256, 8);
         else if (cols <= 256 * 16) B200JT_SB(256, 16);
-        else if (cols <= 256 * 32) B200JT_SB(256, 32);
-        else B200JT_SB(1024, 16);
+        else B200JT_SB(256, 32);
         B200JT_LAUNCH_CHECK();
         return 0;
     }

@@ -140,7 +140,7 @@ def test_few_bins_fold(dtype, bins, reserve):
 # ---- softmax backward: rows in registers with the next one on its way, and rows of up to 16384 columns
 @pytest.mark.parametrize("log", [0, 1])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("rows,cols", [(5, 8), (9500, 40), (2369, 2048), (4740, 1001), (3, 8192), (3, 8193), (150, 8200), (2, 12001), (2400, 16384), (2, 16383), (2, 16400)])
+@pytest.mark.parametrize("rows,cols", [(7, 127), (6, 129), (5, 511), (4, 2047), (3, 2049), (3, 4097), (2, 8191), (5, 8), (9500, 40), (2369, 2048), (4740, 1001), (3, 8192), (3, 8193), (150, 8200), (2, 12001), (2400, 16384), (2, 16383), (2, 16400)])
 def test_softmax_backward(rows, cols, dtype, log):
     x = torch.randn(rows, cols, device="cuda")
     y = (torch.log_softmax(x, 1) if log else torch.softmax(x, 1)).to(dtype)
