@@ -50,6 +50,8 @@ template <> struct Vec<__nv_bfloat16, 8> {
     }
 };
 
+template <typename T, int N> struct alignas(N * sizeof(T) < 16 ? N * sizeof(T) : 16) Raw { T v[N]; };      // a vector as it lies in memory
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
@@ -91,17 +93,36 @@ layer_norm_bwd_kernel(const T* __restrict__ x, const T* __restrict__ dy, const f
     const int nvec = cols / N;
     const float rc = 1.f / (float)cols;
     float ag[PARAMS ? VPT : 1][N] = {}, ab[PARAMS ? VPT : 1][N] = {};
+    // The next row is on its way through this one's reductions where the registers for it cost no resident CTA: [43690, 768] float32
+    // 114 -> 89 us, [8192, 4096] bfloat16 91 -> 70; elsewhere it cost more than it gave ([120000, 128] float32 48 and, with it, 76).
+    constexpr bool AHEAD = DX && PARAMS && N > 1 && (sizeof(T) == 4 ? GROUP == 128 : GROUP == 256 && E == 16);
+    Raw<T, N> na[AHEAD ? VPT : 1], nb[AHEAD ? VPT : 1];
+    // columns beyond the row read its last vector and count as zeros, rows beyond the last read that one: no branch between the loads
+    auto fetch = [&](int64_t row) {
+        row = row < rows ? row : rows - 1;
+#pragma unroll
+        for (int k = 0; k < VPT; k++) {
+            const int64_t at = row * cols + (int64_t)min(t + k * GROUP, nvec - 1) * N;
+            na[k] = *(const Raw<T, N>*)(x + at);
+            nb[k] = *(const Raw<T, N>*)(dy + at);
+        }
+    };
+    if constexpr (AHEAD) fetch((int64_t)blockIdx.x * RPC + g);
     for (int64_t row0 = (int64_t)blockIdx.x * RPC; row0 < rows; row0 += (int64_t)gridDim.x * RPC) {
         const int64_t row = row0 + g;
         if (GROUP == 32 && row >= rows) break;                  // warps leave on their own; a CTA per row leaves as one
-        // columns beyond the row read its last vector and count as zeros: no branch between the loads
         float a[VPT][N], b[VPT][N];
         float s[2] = {0.f, 0.f};
 #pragma unroll
         for (int k = 0; k < VPT; k++) {
-            const int64_t at = row * cols + (int64_t)min(t + k * GROUP, nvec - 1) * N;
-            Vec<T, N>::ld(x + at, a[k]);
-            Vec<T, N>::ld(dy + at, b[k]);
+            if constexpr (AHEAD) {
+                Vec<T, N>::ld(na[k].v, a[k]);
+                Vec<T, N>::ld(nb[k].v, b[k]);
+            } else {
+                const int64_t at = row * cols + (int64_t)min(t + k * GROUP, nvec - 1) * N;
+                Vec<T, N>::ld(x + at, a[k]);
+                Vec<T, N>::ld(dy + at, b[k]);
+            }
         }
 #pragma unroll
         for (int k = 0; k < VPT; k++)
@@ -110,6 +131,7 @@ layer_norm_bwd_kernel(const T* __restrict__ x, const T* __restrict__ dy, const f
                 if (t + k * GROUP >= nvec) a[k][e] = b[k][e] = 0.f;
                 s[0] += a[k][e]; s[1] += a[k][e] * a[k][e];
             }
+        if constexpr (AHEAD) fetch(row + (int64_t)gridDim.x * RPC);
         row_sum<GROUP, 2>(s, sm);
         const float mean = s[0] * rc, var = fmaxf(s[1] * rc - mean * mean, 0.f), rstd = 1.f / sqrtf(var + eps);
         float c[2] = {0.f, 0.f};
@@ -504,11 +526,15 @@ bn_bwd_held_kernel(const TX* __restrict__ x, const TD* __restrict__ dy, float* _
 
 // Rows stay in registers up to 8192 columns (32 elements a thread); the host keeps the op-by-op graph for longer ones.
 constexpr int kMaxCols = 8192;
-// Persistent CTAs: enough rows in flight to cover the latency of a row's reductions, few enough partial rows to fold.
+// Persistent CTAs: enough rows in flight to cover the latency of a row's reductions, few enough partial rows to fold: no more than
+// are resident (two per SM with 16 elements a thread), and beyond one per SM at least four rows for each. [640, 4096] bfloat16 33 ->
+// 19 us, [5000, 4096] 67 -> 42, float32 67 -> 59, [16384, 512] 33 -> 23.5.
 constexpr int kMostCtas = 8;                                   // per SM, over all forms below
-inline int ln_ctas(int64_t rows, int rpc, int per_sm) {
-    const int64_t need = (rows + rpc - 1) / rpc;
-    return (int)std::max<int64_t>(1, std::min<int64_t>(need, (int64_t)(kNumSMs - sm_reserve()) * per_sm));
+inline int ln_ctas(int64_t rows, int rpc, int per_sm, bool params) {
+    const int64_t sms = kNumSMs - sm_reserve();
+    int64_t need = (rows + rpc - 1) / rpc;
+    if (params) need = std::min(need, std::max(sms, rows / 4));
+    return (int)std::max<int64_t>(1, std::min<int64_t>(need, sms * per_sm));
 }
 
 template <typename T, int N, int GROUP, int E>
@@ -533,13 +559,13 @@ template <typename T, int V>
 int run_ln(const T* x, const T* dy, const float* gamma, T* dx, float* params, float* partial, int64_t rows, int cols, float eps, cudaStream_t st) {
     const bool vec = cols % V == 0 && (uintptr_t)x % 16 == 0 && (uintptr_t)dy % 16 == 0 && (uintptr_t)dx % 16 == 0 && (uintptr_t)gamma % 16 == 0;
 #define B200JT_LN(GROUP, E)                                                                                                      \
-    do { const int ctas = ln_ctas(rows, cta_of(GROUP) / GROUP, GROUP != 32 && GROUP < 256 ? kMostCtas : E > 16 ? 2 : 4);         \
+    do { const int ctas = ln_ctas(rows, cta_of(GROUP) / GROUP, GROUP != 32 && GROUP < 256 ? kMostCtas : E > (params ? 8 : 16) ? 2 : 4, params); \
          return vec ? launch_ln<T, V, GROUP, E>(x, dy, gamma, dx, params, partial, rows, cols, eps, ctas, st)                    \
                     : launch_ln<T, 1, GROUP, E>(x, dy, gamma, dx, params, partial, rows, cols, eps, ctas, st); } while (0)
     if (cols <= 256) B200JT_LN(32, 8);
     if (cols <= 512) { if (vec || rows >= 8192) B200JT_LN(32, 16); B200JT_LN(64, 8); }
     if (cols <= 1024 && vec) B200JT_LN(128, 8);
-    if (cols <= 1024) return launch_ln<T, 1, 256, 4>(x, dy, gamma, dx, params, partial, rows, cols, eps, ln_ctas(rows, 1, 4), st);
+    if (cols <= 1024) return launch_ln<T, 1, 256, 4>(x, dy, gamma, dx, params, partial, rows, cols, eps, ln_ctas(rows, 1, 4, params), st);
     if (cols <= 2048) B200JT_LN(256, 8);
     if (cols <= 4096) B200JT_LN(256, 16);
     B200JT_LN(256, 32);
@@ -649,7 +675,7 @@ extern "C" size_t b200jt_layer_norm_backward_workspace(const b200jt_tensor* x, i
     if (!valid_tensor(x) || !want_params) return 0;
     const int64_t cols = x->shape[x->ndim - 1], rows = cols ? numel(x) / cols : 0;
     if (cols < 1 || cols > kMaxCols || rows < 1) return 0;
-    return sizeof(float) * 2 * cols * (size_t)ln_ctas(rows, 1, kMostCtas);
+    return sizeof(float) * 2 * cols * (size_t)ln_ctas(rows, 1, kMostCtas, false);
 }
 
 extern "C" int b200jt_layer_norm_backward(const b200jt_tensor* x, const b200jt_tensor* gamma, const b200jt_tensor* dy, const b200jt_tensor* dx,
