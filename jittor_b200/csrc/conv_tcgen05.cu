@@ -607,7 +607,6 @@ wgrad_bf16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = *tmem_slot;
     asm volatile("griddepcontrol.wait;" ::: "memory");          // for the layout pass
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");      // the fold's CTAs may take their places; they wait for this grid
 
     if (warp == 0) {
         // The whole warp walks the blocks; lane 0 waits for the slot and announces the bytes, then every lane that owns a box
@@ -674,6 +673,7 @@ wgrad_bf16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         const int quad = warp & 3;
         bool ok = mbar_wait(acc_full, 0, abort_flag, 23);
         ok = __all_sync(0xffffffffu, ok);
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");      // the fold's CTAs may take their places; they wait for this grid
         if (ok) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const int c = tm * BM + quad * 32 + lane;                        // TMEM lane = input channel
@@ -824,13 +824,16 @@ int conv2d_wgrad_tc(const void* x, const void* dy, void* dw, const ConvShape& s,
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute early;
     early.id = cudaLaunchAttributeProgrammaticStreamSerialization; early.val.programmaticStreamSerializationAllowed = 1;
-    cfg.gridDim = dim3(grid); cfg.blockDim = dim3(THREADS); cfg.stream = st; cfg.attrs = &early; cfg.numAttrs = 1;
+    cfg.gridDim = dim3(grid); cfg.blockDim = dim3(THREADS); cfg.stream = st; cfg.attrs = &early;
+    // An early start saves some 3 us; but the CTAs then stand on the SMs in the order the layout pass left them, and the taps that
+    // share x and dy through L2 lie further apart: 256 x 256 x 56 x 56 0.93 -> 0.95 ms. Hence for kernels of up to some 150 us.
+    cfg.numAttrs = 2.0 * taps * s.C * s.Co * s.N * OHW < 2e11 ? 1 : 0;
     cfg.dynamicSmemBytes = p.taps_per_cta == 2 ? Ring<2>::SMEM_BYTES : Ring<1>::SMEM_BYTES;
     const auto kernel = p.taps_per_cta == 2 ? (p.bn == 256 ? wgrad_bf16_kernel<256, 2> : wgrad_bf16_kernel<128, 2>)
                                             : (p.bn == 256 ? wgrad_bf16_kernel<256, 1> : wgrad_bf16_kernel<128, 1>);
     B200JT_CUDA(cudaLaunchKernelEx(&cfg, kernel, mx, mdy, part, A));
     const int64_t n = (int64_t)taps * s.C * s.Co;
-    cfg.gridDim = dim3(grid_for(n, 256)); cfg.blockDim = dim3(256); cfg.dynamicSmemBytes = 0;
+    cfg.gridDim = dim3(grid_for(n, 256)); cfg.blockDim = dim3(256); cfg.dynamicSmemBytes = 0; cfg.numAttrs = 1;
     B200JT_CUDA(cudaLaunchKernelEx(&cfg, wgrad_fold_kernel, (const float*)part, (__nv_bfloat16*)dw, p.splits, taps, s.C, s.Co, lay.w_ohwi ? 1 : 0));
     return 0;
 }
