@@ -1,7 +1,8 @@
 // Gradients of LayerNorm and training BatchNorm (with the ReLU that follows it) as the kernels read them, instead of the
 // op-by-op graph of the reverse rules: that graph is nine row or column reduces and a dozen full-size passes per layer
 // (LayerNorm [5000,1001] float32: 7 launches, 106 us; BatchNorm + ReLU [64,128,28,28] bfloat16: 23 launches, 190 us). Both are
-// bound by memory: x and dy are read once (LayerNorm, BatchNorm of layers that shared memory holds) or twice, dx is written once, and everything per channel or column is folded in a fixed order.
+// bound by memory: x and dy are read once (LayerNorm, BatchNorm of layers that shared memory holds) or twice, dx is written
+// once, and everything per channel or column is folded in a fixed order.
 //
 //   LayerNorm   xh = (x - mean) * rstd, g = dy * gamma:  dx = rstd * (g - mean(g) - xh * mean(g * xh)),
 //               dgamma = sum over rows of dy * xh, dbeta = sum of dy
