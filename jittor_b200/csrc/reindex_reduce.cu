@@ -538,8 +538,8 @@ rr_privatised_kernel(const T* __restrict__ y, const E* __restrict__ idx, T* __re
         int hb[kHot];
 #pragma unroll
         for (int k = 0; k < kHot; k++) hb[k] = use_hot ? hot_bin[k] : -2;
-        for_each_pair<T, E, VEC, 2, true>(y, idx, n, [&](int64_t b, T v, bool valid) {
-            const int bi = (int)b;
+        for_each_pair<T, E, VEC, 2, true>(y, idx, n, [&](int64_t b, T v, bool) {
+            const int bi = b >= 0 && b < bins ? (int)b : -1;    // 32 bits of an index only where it is a bin's number (lanes past the end bring -1)
             bool hit = false;
 #pragma unroll
             for (int k = 0; k < kHot; k++) {
@@ -547,7 +547,7 @@ rr_privatised_kernel(const T* __restrict__ y, const E* __restrict__ idx, T* __re
                 hacc[k] += m ? (float)v : 0.f;
                 hit |= m;
             }
-            if (!hit && valid && b >= 0 && b < bins) atomic_apply<T>(mine + b, v, op);
+            if (!hit && bi >= 0) atomic_apply<T>(mine + bi, v, op);
         });
         if (use_hot) {
 #pragma unroll

@@ -110,6 +110,24 @@ def test_few_bins(n, dtype, idx, op):
     assert torch.equal(got.double(), want)
 
 
+# skewed indices: bins above 1 % of a CTA's sample are summed in registers. Enough elements for that path, a ragged tail, indices that
+# name no bin: negative ones, and 64-bit ones whose lower half is a hot bin's number
+@pytest.mark.parametrize("idx", [torch.int32, torch.int64])
+@pytest.mark.parametrize("hot", [1, 3, 6])
+def test_few_bins_hot(hot, idx):
+    import jittor_b200 as jt
+    n, bins = 6_000_003, 997
+    v = torch.randint(-9, 10, (n,), device="cuda").float()                             # whole numbers, sums below 2^24: exact in every order
+    i = torch.randint(-3, bins + 3, (n,), device="cuda")
+    spot = torch.randint(0, 2 * hot, (n,), device="cuda")
+    i = torch.where(spot < hot, 7 + 150 * spot, i)
+    if idx == torch.int64:
+        i = torch.where(torch.rand(n, device="cuda") < 0.1, i + (1 << 32), i)
+    got = jt.array(v).reindex_reduce("add", [bins], ["@e0(i0)"], extras=[jt.array(i.to(idx))]).torch()
+    ok = (i >= 0) & (i < bins)
+    assert torch.equal(got.double(), torch.zeros(bins, device="cuda", dtype=torch.float64).index_add_(0, i[ok], v[ok].double()))
+
+
 # the fold behind the grid barrier: part of 32 bins, more bins than one pass of the grid takes, fewer CTAs; also from a graph
 @pytest.mark.parametrize("reserve", [0, 64])
 @pytest.mark.parametrize("dtype,bins", [(torch.float32, 1), (torch.float32, 33), (torch.int32, 4737), (torch.float32, 20011), (torch.float64, 9500)])
