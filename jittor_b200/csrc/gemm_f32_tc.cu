@@ -16,8 +16,10 @@
 //
 // The operands are scaled by 2^24 on their way and the result by 2^-48: the tensor core takes subnormal parts for zero, and that way
 // every part of every float32, subnormal ones among them, is a normal bfloat16.
-// An element that comes out infinite or NaN is computed again from the float32 operands: an infinity would meet the zeros
-// of the other operand's smaller parts, and values from 2^104, or sums from 2^80 on, leave the scaled range.
+// Infinities (they meet the zeros of the other operand's smaller parts), values from 2^104 and sums from 2^80 on leave the scaled range:
+// there an element that came out infinite or NaN is computed again by float32 FMAs. The split pass notes each operand's largest
+// magnitude, so that a NaN that stems from a NaN in an operand is left as it is. A CTA does this for its own tiles when its pipeline
+// has run empty (a part of K each where a cluster shares a tile): no wait of the ring depends on it.
 #include "gemm_simt.cuh"
 #include "tc_common.cuh"
 
@@ -44,9 +46,11 @@ constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256 + 8 * 32 * TURN_PIT
 constexpr int MAX_SPLIT = 8;
 
 struct Args {
-    const float *a, *b;            // for elements that are computed again
+    const float *a, *b;            // for elements that are computed again, their steps along M, K and N below
     int64_t a_sm, a_sk, b_sk, b_sn;
     int M, N, K, tiles_m, tiles_n, bn, k_blocks, units, group, splits;
+    const float* peaks;            // largest magnitude that each block of the split pass met, a's blocks first
+    int peaks_a, peaks_b;
 };
 
 // rows of 64 bytes, 64-byte swizzle: 8-row groups 512 bytes apart
@@ -54,16 +58,185 @@ __device__ __forceinline__ uint64_t desc_k64(uint32_t saddr) {
     return (uint64_t)((saddr & 0x3FFFF) >> 4) | (uint64_t)1 << 16 | (uint64_t)(512 >> 4) << 32 | (uint64_t)1 << 46 | (uint64_t)4 << 61;
 }
 
-__device__ __noinline__ float dot_again(const Args& A, int m, int n) {
-    const float *a = A.a + m * A.a_sm, *b = A.b + n * A.b_sn;
-    float s[8] = {};                                    // chains as short as the FMA kernel's
-    for (int k = 0; k < A.K; k += 8)
+__device__ __forceinline__ bool finite(float v) { return (__float_as_uint(v) & 0x7f800000u) != 0x7f800000u; }
+
+// Whether anything but a NaN of an operand can have made an element infinite or NaN: by the operands' largest magnitudes, infinities
+// among them and NaN not. All threads of the CTA; `sm` holds two words for each warp.
+__device__ __noinline__ bool left_range(const Args& A, float* sm) {
+    float a = 0.f, b = 0.f;
+    for (int i = threadIdx.x; i < A.peaks_a; i += THREADS) a = fmaxf(a, A.peaks[i]);
+    for (int i = threadIdx.x; i < A.peaks_b; i += THREADS) b = fmaxf(b, A.peaks[A.peaks_a + i]);
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) { a = fmaxf(a, __shfl_xor_sync(0xffffffffu, a, d)); b = fmaxf(b, __shfl_xor_sync(0xffffffffu, b, d)); }
+    if ((threadIdx.x & 31) == 0) { sm[threadIdx.x >> 5] = a; sm[THREADS / 32 + (threadIdx.x >> 5)] = b; }
+    __syncthreads();
+    for (int w = 0; w < THREADS / 32; w++) { a = fmaxf(a, sm[w]); b = fmaxf(b, sm[THREADS / 32 + w]); }
+    __syncthreads();
+    return a >= 0x1p103f || b >= 0x1p103f || (double)a * b * A.K >= 0x1p79;
+}
+
+// 128 x 64 elements of the product from row m0 and column n0 on over k0 <= k < k1, as float32 FMAs, to `out` (rows x cols of them, or
+// only those that are infinite or NaN there). 16 of K at a time go through shared memory, the next ones on their way meanwhile; 256
+// threads hold 8 x 4 elements each and add 256 of K to a sum at a time. All threads of the CTA; bound by the latency of two computing
+// warps a scheduler (FMA pipe 0.4 busy). 4096 x 2048 x 4096 with every element infinite: 4.1 ms, the FMA kernel 1.5; one infinity 1.4.
+constexpr int AGAIN_K = 16, AGAIN_PA = BM + 4, AGAIN_PB = 64 + 4;
+__device__ __noinline__ void fma_again(const Args& A, int m0, int n0, int k0, int k1, float* stage, float* out, int64_t pitch, int rows, int cols, bool only_odd) {
+    constexpr int NA = (BM * AGAIN_K + THREADS - 1) / THREADS, NB = (64 * AGAIN_K + THREADS - 1) / THREADS, SIZE = AGAIN_K * (AGAIN_PA + AGAIN_PB);
+    const bool ak = A.a_sk == 1, bk = A.b_sk == 1;              // neighbouring threads read along the axis that lies in memory
+    // element e of an operand's 16 x `extent` part: where it goes among the 16 of K and along the operand's own axis
+    const auto k_of = [](int e, int extent, bool kc) { return kc ? e % AGAIN_K : e / extent; };
+    const auto own_of = [](int e, int extent, bool kc) { return kc ? e / AGAIN_K : e % extent; };
+    const float *pa[NA], *pb[NB];                               // null where nothing is read
+    float va[NA], vb[NB];
+#pragma unroll
+    for (int i = 0; i < NA; i++) {
+        const int e = threadIdx.x + i * THREADS, r = m0 + own_of(e, BM, ak);
+        pa[i] = e < BM * AGAIN_K && r < A.M ? A.a + r * A.a_sm + (k0 + k_of(e, BM, ak)) * A.a_sk : nullptr;
+    }
+#pragma unroll
+    for (int i = 0; i < NB; i++) {
+        const int e = threadIdx.x + i * THREADS, r = n0 + own_of(e, 64, bk);
+        pb[i] = e < 64 * AGAIN_K && r < A.N ? A.b + r * A.b_sn + (k0 + k_of(e, 64, bk)) * A.b_sk : nullptr;
+    }
+    auto fetch = [&](int k) {
+#pragma unroll
+        for (int i = 0; i < NA; i++) {
+            va[i] = pa[i] && k + k_of(threadIdx.x + i * THREADS, BM, ak) < k1 ? *pa[i] : 0.f;
+            if (pa[i]) pa[i] += AGAIN_K * A.a_sk;
+        }
+#pragma unroll
+        for (int i = 0; i < NB; i++) {
+            vb[i] = pb[i] && k + k_of(threadIdx.x + i * THREADS, 64, bk) < k1 ? *pb[i] : 0.f;
+            if (pb[i]) pb[i] += AGAIN_K * A.b_sk;
+        }
+    };
+    auto put = [&](float* s) {
+#pragma unroll
+        for (int i = 0; i < NA; i++) {
+            const int e = threadIdx.x + i * THREADS;
+            if (e < BM * AGAIN_K) s[k_of(e, BM, ak) * AGAIN_PA + own_of(e, BM, ak)] = va[i];
+        }
+#pragma unroll
+        for (int i = 0; i < NB; i++) {
+            const int e = threadIdx.x + i * THREADS;
+            if (e < 64 * AGAIN_K) s[AGAIN_K * AGAIN_PA + k_of(e, 64, bk) * AGAIN_PB + own_of(e, 64, bk)] = vb[i];
+        }
+    };
+    const int ty = threadIdx.x / 16 * 8, tx = threadIdx.x % 16 * 4;
+    unsigned long long sum[8][2] = {}, acc[8][2] = {};         // pairs of columns
+    fetch(k0);
+    put(stage);
+    __syncthreads();
+    for (int k = k0, it = 0; k < k1; k += AGAIN_K, it++) {
+        const float* s = stage + (it & 1) * SIZE;
+        if (k + AGAIN_K < k1) fetch(k + AGAIN_K);
+        if (threadIdx.x < 256) {
+#pragma unroll
+            for (int q = 0; q < AGAIN_K; q++) {
+                const float4 lo = *(const float4*)(s + q * AGAIN_PA + ty), hi = *(const float4*)(s + q * AGAIN_PA + ty + 4);
+                const ulonglong2 y = *(const ulonglong2*)(s + AGAIN_K * AGAIN_PA + q * AGAIN_PB + tx);
+                const float x[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+#pragma unroll
+                for (int i = 0; i < 8; i++) {
+                    unsigned long long xx;
+                    asm("mov.b64 %0, {%1, %1};" : "=l"(xx) : "f"(x[i]));
+                    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[i][0]) : "l"(xx), "l"(y.x));
+                    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[i][1]) : "l"(xx), "l"(y.y));
+                }
+            }
+            if (it % (256 / AGAIN_K) == 256 / AGAIN_K - 1)
+#pragma unroll
+                for (int i = 0; i < 8; i++)
+#pragma unroll
+                    for (int j = 0; j < 2; j++) { asm("add.rn.f32x2 %0, %0, %1;" : "+l"(sum[i][j]) : "l"(acc[i][j])); acc[i][j] = 0; }
+        }
+        if (k + AGAIN_K < k1) put(stage + (~it & 1) * SIZE);
+        __syncthreads();
+    }
+    if (threadIdx.x < 256)
 #pragma unroll
         for (int i = 0; i < 8; i++)
-            if (k + i < A.K) s[i] = fmaf(a[(k + i) * A.a_sk], b[(k + i) * A.b_sk], s[i]);
-    return ((s[0] + s[1]) + (s[2] + s[3])) + ((s[4] + s[5]) + (s[6] + s[7]));
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+                if (ty + i < rows && tx + j < cols) {
+                    const auto half = [&](unsigned long long v) { return __uint_as_float((uint32_t)(j & 1 ? v >> 32 : v)); };
+                    float* at = out + (ty + i) * pitch + tx + j;
+                    if (!only_odd || !finite(*at)) *at = half(sum[i][j / 2]) + half(acc[i][j / 2]);
+                }
+    __syncthreads();
 }
-__device__ __forceinline__ bool finite(float v) { return (__float_as_uint(v) & 0x7f800000u) != 0x7f800000u; }
+__device__ __forceinline__ void tile_at(const Args& A, int u, int& tm, int& tn) {      // groups of tile-rows are walked together: B tiles stay in L2
+    const int per_group = A.group * A.tiles_n, g = u / per_group, r = u - g * per_group;
+    const int rows = min(A.group, A.tiles_m - g * A.group);
+    tm = g * A.group + r % rows; tn = r / rows;
+}
+
+// The cluster's parts of a tile, each in its CTA's `mine`, are added up in rank order; a CTA stores 1 / splits of the rows. Returns
+// whether one of this thread's elements came out infinite or NaN. AGAIN: only those that did are stored, by the thread that met them.
+template <bool AGAIN>
+__device__ __forceinline__ bool fold_parts(const Args& A, float* c, float* mine, int m0, int n0, int rank) {
+    cg::cluster_group cluster = cg::this_cluster();
+    const int splits = A.splits, rows = BM / splits, quads = A.bn / 4, pitch = A.bn + 4;
+    const bool vec = (A.N & 3) == 0 && ((uintptr_t)c & 15) == 0;
+    bool odd = false;
+    cluster.sync();
+    for (int e = threadIdx.x; e < rows * quads; e += THREADS) {
+        const int r = rank * rows + e / quads, q = (e % quads) * 4;
+        const int m = m0 + r, n = n0 + q;
+        if (m >= A.M || n >= A.N) continue;
+        float4 w[MAX_SPLIT], v = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int p = 0; p < MAX_SPLIT; p++) if (p < splits) w[p] = *(const float4*)(cluster.map_shared_rank(mine, p) + r * pitch + q);
+#pragma unroll
+        for (int p = 0; p < MAX_SPLIT; p++) if (p < splits) { v.x += w[p].x; v.y += w[p].y; v.z += w[p].z; v.w += w[p].w; }
+        const float scale = AGAIN ? 1.f : UNSCALE, o[4] = {v.x * scale, v.y * scale, v.z * scale, v.w * scale};
+        float* out = c + (int64_t)m * A.N + n;
+        if constexpr (AGAIN) {
+#pragma unroll
+            for (int i = 0; i < 4; i++) if (n + i < A.N && !finite(out[i])) out[i] = o[i];
+        } else {
+#pragma unroll
+            for (int i = 0; i < 4; i++) odd |= !finite(o[i]);
+            if (vec) *(float4*)out = make_float4(o[0], o[1], o[2], o[3]);
+            else
+#pragma unroll
+                for (int i = 0; i < 4; i++) if (n + i < A.N) out[i] = o[i];
+        }
+    }
+    return odd;
+}
+
+// What a CTA (or the cluster of one tile) does when an element of its tiles came out infinite or NaN.
+template <bool PAIR>
+__device__ __noinline__ void compute_again(const Args& A, float* c, unsigned char* smem, float* sm) {
+    constexpr int CTAS = PAIR ? 2 : 1;
+    const int splits = PAIR ? 1 : A.splits, rank = PAIR || splits > 1 ? (int)cluster_rank() : 0;
+    const int first = blockIdx.x / (CTAS * splits), step = gridDim.x / (CTAS * splits);
+    if (!left_range(A, sm)) return;
+    int tm, tn;
+    if (!PAIR && splits > 1) {
+        const int pitch = A.bn + 4;
+        float* mine = (float*)smem;
+        tile_at(A, first, tm, tn);
+        for (int n = 0; n < A.bn; n += 64)
+            fma_again(A, tm * BM, tn * A.bn + n, A.k_blocks * rank / splits * BK, min(A.K, A.k_blocks * (rank + 1) / splits * BK), mine + BM * pitch, mine + n, pitch,
+                      BM, min(64, A.bn - n), false);
+        fold_parts<true>(A, c, mine, tm * BM, tn * A.bn, rank);
+        cg::this_cluster().sync();     // no CTA leaves while its tile is read
+        return;
+    }
+    for (int u = first; u < A.units; u += step) {
+        tile_at(A, u, tm, tn);
+        const int m0 = (tm * CTAS + (PAIR ? rank : 0)) * BM, rows = min(BM, A.M - m0), end = min(A.N, (tn + 1) * A.bn);
+        for (int n0 = tn * A.bn; n0 < end; n0 += 64) {
+            const int cols = min(64, end - n0);
+            float* out = c + (int64_t)m0 * A.N + n0;
+            bool odd = false;
+            for (int e = threadIdx.x; e < rows * 64; e += THREADS) odd |= e % 64 < cols && !finite(out[(int64_t)(e / 64) * A.N + e % 64]);
+            if (__syncthreads_or(odd)) fma_again(A, m0, n0, 0, A.K, (float*)smem, out, A.N, rows, cols, true);
+        }
+    }
+}
 
 // PAIR: two CTAs share one tile of 256 rows, each with its own rows of A and half of the columns of B.
 // AMN / BMN: the operand's own axis (M / N) is the contiguous one in memory.
@@ -81,6 +254,7 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     uint64_t* acc_empty = bars + 2 * STAGES + 2;
     uint32_t* tmem_slot = (uint32_t*)(bars + 2 * STAGES + 4);
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
+    volatile int* odd_flag = abort_flag + 1;                           // an element of this CTA's (or of its cluster's) came out infinite or NaN
     float* turn = (float*)(smem + STAGES * STAGE_BYTES + 256);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -89,16 +263,10 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     const int side = PAIR ? rank : 0, split = PAIR ? 0 : rank;
     const int first = blockIdx.x / (CTAS * splits), step = gridDim.x / (CTAS * splits);
     const int kb0 = A.k_blocks * split / splits, kb1 = A.k_blocks * (split + 1) / splits;
-    auto tile_at = [&](int u, int& tm, int& tn) {                      // groups of tile-rows are walked together: B tiles stay in L2
-        const int per_group = A.group * A.tiles_n, g = u / per_group, r = u - g * per_group;
-        const int rows = min(A.group, A.tiles_m - g * A.group);
-        tm = g * A.group + r % rows; tn = r / rows;
-    };
-
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; s++) { mbar_init(full + s, 1); mbar_init(empty + s, 1); }
         for (int b = 0; b < 2; b++) { mbar_init(acc_full + b, 1); mbar_init(acc_empty + b, 8 * CTAS); }
-        *abort_flag = 0;
+        *abort_flag = *odd_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) tmem_alloc<CTAS>(tmem_slot);
@@ -118,7 +286,7 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
             bool ok = true;
             for (int u = first; u < A.units && ok; u += step) {
                 int tm, tn;
-                tile_at(u, tm, tn);
+                tile_at(A, u, tm, tn);
                 const int row0 = (tm * CTAS + side) * BM, col0 = tn * A.bn + side * half;
                 for (int kb = kb0; kb < kb1; kb++) {
                     if (!(ok = mbar_wait(empty + stage, phase ^ 1, abort_flag, 31))) break;
@@ -193,7 +361,7 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         bool ok = true;
         for (int u = first; u < A.units && ok; u += step) {
             int tm, tn;
-            tile_at(u, tm, tn);
+            tile_at(A, u, tm, tn);
             float acc[CHUNKS][32];
 #pragma unroll
             for (int i = 0; i < CHUNKS; i++)
@@ -239,63 +407,37 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
                 bool odd = false;
 #pragma unroll
                 for (int e = 0; e < 32; e++) odd |= !finite(acc[i][e]);
-                odd = __any_sync(0xffffffffu, odd);
+                if (odd) *odd_flag = 1;
                 __syncwarp();
 #pragma unroll
                 for (int e = 0; e < 32; e++) square[lane * TURN_PITCH + e] = acc[i][e];
                 __syncwarp();
                 float* out = c + (int64_t)row0 * A.N + col0 + lane;
                 const int rows = min(32, A.M - row0);
-                if (col0 + lane < A.N) {
-                    if (!odd) {
+                if (col0 + lane < A.N)
 #pragma unroll 8
-                        for (int r = 0; r < rows; r++) out[(int64_t)r * A.N] = square[r * TURN_PITCH + lane] * UNSCALE;
-                    } else {
-                        for (int r = 0; r < rows; r++) {
-                            float v = square[r * TURN_PITCH + lane] * UNSCALE;
-                            if (!finite(v)) v = dot_again(A, row0 + r, col0 + lane);
-                            out[(int64_t)r * A.N] = v;
-                        }
-                    }
-                }
+                    for (int r = 0; r < rows; r++) out[(int64_t)r * A.N] = square[r * TURN_PITCH + lane] * UNSCALE;
             }
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (PAIR) cluster_sync();          // neither CTA leaves while the other may still signal it or read its tiles
-    if (!PAIR && splits > 1) {
-        cg::cluster_group cluster = cg::this_cluster();
-        cluster.sync();
-        int tm, tn;
-        tile_at(first, tm, tn);        // one tile to a cluster
-        const int rows = BM / splits, quads = A.bn / 4, pitch = A.bn + 4;
-        const bool vec = (A.N & 3) == 0 && ((uintptr_t)c & 15) == 0;
-        for (int e = threadIdx.x; e < rows * quads; e += THREADS) {
-            const int r = rank * rows + e / quads, q = (e % quads) * 4;
-            const int m = tm * BM + r, n = tn * A.bn + q;
-            if (m >= A.M || n >= A.N) continue;
-            float4 w[MAX_SPLIT], v = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-            for (int p = 0; p < MAX_SPLIT; p++) if (p < splits) w[p] = *(const float4*)(cluster.map_shared_rank((float*)smem, p) + r * pitch + q);
-#pragma unroll
-            for (int p = 0; p < MAX_SPLIT; p++) if (p < splits) { v.x += w[p].x; v.y += w[p].y; v.z += w[p].z; v.w += w[p].w; }
-            float o[4] = {v.x * UNSCALE, v.y * UNSCALE, v.z * UNSCALE, v.w * UNSCALE};
-#pragma unroll
-            for (int i = 0; i < 4; i++)
-                if (!finite(o[i]) && n + i < A.N) o[i] = dot_again(A, m, n + i);
-            float* out = c + (int64_t)m * A.N + n;
-            if (vec) *(float4*)out = make_float4(o[0], o[1], o[2], o[3]);
-            else
-#pragma unroll
-                for (int i = 0; i < 4; i++) if (n + i < A.N) out[i] = o[i];
-        }
-        cluster.sync();                // no CTA leaves while its tile is read
-    }
     if (warp == 1) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         tmem_dealloc<CTAS>(tmem_base);
     }
+    bool odd = *odd_flag;
+    if (!PAIR && splits > 1) {
+        int tm, tn;
+        tile_at(A, first, tm, tn);     // one tile to a cluster
+        cg::cluster_group cluster = cg::this_cluster();
+        if (fold_parts<false>(A, c, (float*)smem, tm * BM, tn * A.bn, rank))
+            for (int p = 0; p < splits; p++) *cluster.map_shared_rank((int*)odd_flag, p) = 1;
+        cluster.sync();                // no CTA leaves while its tile is read
+        odd = *odd_flag;
+    }
+    if (odd) compute_again<PAIR>(A, c, smem, turn);
 }
 
 // rows of float32 -> three planes of bfloat16 rows (pitch a multiple of 8; what lies past a row's end is never loaded), eight
@@ -312,8 +454,10 @@ __device__ __forceinline__ void split_pair(float x, float y, uint32_t* p) {
     }
 }
 __global__ void __launch_bounds__(256)
-split_rows_kernel(const __grid_constant__ SplitJob a, const __grid_constant__ SplitJob b, int blocks_a) {
+split_rows_kernel(const __grid_constant__ SplitJob a, const __grid_constant__ SplitJob b, int blocks_a, float* __restrict__ peaks) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    __shared__ unsigned most[8];
+    float peak = 0.f;
     const bool second = (int)blockIdx.x >= blocks_a;
     const SplitJob& job = second ? b : a;
     const int64_t n = job.rows * job.chunks, stride = (int64_t)(second ? gridDim.x - blocks_a : blocks_a) * 256;
@@ -329,12 +473,22 @@ split_rows_kernel(const __grid_constant__ SplitJob a, const __grid_constant__ Sp
 #pragma unroll
             for (int e = 0; e < 8; e++) v[e] = c0 + e < job.cols ? p[e] : 0.f;
         }
+#pragma unroll
+        for (int e = 0; e < 8; e++) peak = fmaxf(peak, fabsf(v[e]));         // of a number and NaN the number
         uint32_t q[4][PLANES];
 #pragma unroll
         for (int e = 0; e < 4; e++) split_pair(v[2 * e], v[2 * e + 1], q[e]);
 #pragma unroll
         for (int s = 0; s < PLANES; s++)
             *reinterpret_cast<uint4*>(job.out + s * job.plane + i * 8) = make_uint4(q[0][s], q[1][s], q[2][s], q[3][s]);
+    }
+    const unsigned top = __reduce_max_sync(0xffffffffu, __float_as_uint(peak));         // of floats from 0 up, as of their bits
+    if ((threadIdx.x & 31) == 0) most[threadIdx.x >> 5] = top;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        unsigned t = 0;
+        for (int w = 0; w < 8; w++) t = max(t, most[w]);
+        peaks[blockIdx.x] = __uint_as_float(t);
     }
 }
 
@@ -431,6 +585,7 @@ static Plan plan_for(int64_t M, int64_t N, int64_t K) {
 
 inline int64_t pitch8(int64_t n) { return (n + 7) / 8 * 8; }
 inline size_t plane_elems(int64_t rows, int64_t cols) { return (size_t)rows * pitch8(cols); }
+constexpr size_t PEAK_BYTES = 2 * 8 * kNumSMs * sizeof(float);          // a word for every block of the split pass
 inline size_t planes_bytes(int64_t rows, int64_t cols) { return (plane_elems(rows, cols) * PLANES * 2 + 255) & ~(size_t)255; }
 
 }  // namespace tcf32
@@ -441,7 +596,7 @@ bool matmul_f32_tc_wanted(int64_t M, int64_t N, int64_t K) {
 }
 size_t matmul_f32_tc_workspace(int64_t M, int64_t N, int64_t K, bool trans_a, bool trans_b) {
     using namespace tcf32;
-    return (trans_a ? planes_bytes(K, M) : planes_bytes(M, K)) + (trans_b ? planes_bytes(N, K) : planes_bytes(K, N)) + 256;
+    return (trans_a ? planes_bytes(K, M) : planes_bytes(M, K)) + (trans_b ? planes_bytes(N, K) : planes_bytes(K, N)) + PEAK_BYTES + 256;
 }
 int matmul_f32_tc(const void* a, const void* b, void* c, int64_t M, int64_t N, int64_t K, bool trans_a, bool trans_b, void* workspace, cudaStream_t st) {
     using namespace tcf32;
@@ -450,13 +605,15 @@ int matmul_f32_tc(const void* a, const void* b, void* c, int64_t M, int64_t N, i
     __nv_bfloat16* pa = (__nv_bfloat16*)(((uintptr_t)workspace + 255) & ~(uintptr_t)255);
     const int64_t ra = amn ? K : M, ca = amn ? M : K, rb = bmn ? K : N, cb = bmn ? N : K;
     __nv_bfloat16* pb = (__nv_bfloat16*)((unsigned char*)pa + planes_bytes(ra, ca));
+    float* peaks = (float*)((unsigned char*)pb + planes_bytes(rb, cb));
+    unsigned ga, gb;
     {
         const auto job = [](const void* in, __nv_bfloat16* out, int64_t rows, int64_t cols) {
             return SplitJob{(const float*)in, out, rows, pitch8(cols) / 8, (int64_t)plane_elems(rows, cols), (int)cols, cols % 4 == 0 && (uintptr_t)in % 16 == 0};
         };
         const SplitJob ja = job(a, pa, ra, ca), jb = job(b, pb, rb, cb);
-        const unsigned ga = grid_for(ja.rows * ja.chunks, 256), gb = grid_for(jb.rows * jb.chunks, 256);
-        split_rows_kernel<<<ga + gb, 256, 0, st>>>(ja, jb, (int)ga);
+        ga = grid_for(ja.rows * ja.chunks, 256); gb = grid_for(jb.rows * jb.chunks, 256);
+        split_rows_kernel<<<ga + gb, 256, 0, st>>>(ja, jb, (int)ga, peaks);
         B200JT_LAUNCH_CHECK();
     }
     const int ctas = p.pair ? 2 : 1;
@@ -470,6 +627,7 @@ int matmul_f32_tc(const void* a, const void* b, void* c, int64_t M, int64_t N, i
     A.M = (int)M; A.N = (int)N; A.K = (int)K; A.bn = p.bn; A.k_blocks = (int)((K + BK - 1) / BK); A.splits = p.splits;
     A.tiles_m = (int)((M + BM * ctas - 1) / (BM * ctas)); A.tiles_n = (int)((N + p.bn - 1) / p.bn);
     A.group = std::max(1, 1024 / (BM * ctas));
+    A.peaks = peaks; A.peaks_a = (int)ga; A.peaks_b = (int)gb;
     const int64_t units = (int64_t)A.tiles_m * A.tiles_n;
     if (units * p.splits >= (1LL << 30)) return fail(-1, "matmul: too many tiles");
     A.units = (int)units;

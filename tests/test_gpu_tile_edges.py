@@ -71,6 +71,36 @@ def test_f32_tensor_core_matmul_range():
         assert not torch.isfinite(got[50, 60])
 
 
+# Everything out of the scaled range, and single infinities and NaN, with several tiles to a CTA, tiles split over clusters, pairs,
+# and a K whose recomputation takes longer than the ring's waits last: equal to float64 but for rounding wherever that is finite
+@pytest.mark.parametrize("ta,tb", [(0, 0), (0, 1), (1, 0), (1, 1)])
+@pytest.mark.parametrize("pair,bn,splits,m,k,n", [(0, 128, 8, 130, 1000, 200), (0, 32, 1, 2500, 40, 1027), (0, 96, 1, 2561, 33, 1537), (1, 256, 1, 5000, 40, 4099), (1, 192, 1, 300, 513, 260),
+                                                  (0, 128, 8, 200, 1 << 16, 129), (1, 256, 1, 5200, 1 << 13, 1030)])
+def test_f32_tensor_core_matmul_beyond_the_scaled_range(m, k, n, pair, bn, splits, ta, tb):
+    a, b = torch.randn(*((k, m) if ta else (m, k)), device="cuda"), torch.randn(*((n, k) if tb else (k, n)), device="cuda")
+    av, bv = a.t() if ta else a, b.t() if tb else b                                   # as M x K and K x N
+
+    def run():
+        with forced(F32TC=1, F32TC_PAIR=pair, F32TC_BN=bn, F32TC_SPLITS=splits):
+            c = matmul(a, b, ta, tb).double()
+        assert C.lib.b200jt_device_status() == 0
+        return c, av.double() @ bv.double(), (av.double().abs() @ bv.double().abs())
+
+    a *= 1e33                                                                          # all operands of one side beyond 2^104
+    c, want, size = run()
+    # parts of at most 256 of k by fused multiply-adds, added up one after the other; where K is split, up to eight more additions
+    assert (c - want).norm() <= (256 / 8 + k / 256 + 8) * 2.0 ** -24 * size.norm()
+    a /= 1e33
+    av[m // 2, k // 3], bv[k // 2, n - 1], bv[k // 5, 0] = float("inf"), float("nan"), -float("inf")
+    c, want, size = run()
+    assert torch.equal(torch.isnan(c), torch.isnan(want)) and torch.equal(torch.isinf(c), torch.isinf(want))
+    assert torch.equal(c[torch.isinf(c)], want[torch.isinf(want)])
+    ok = torch.isfinite(want)
+    assert (c[ok] - want[ok]).norm() <= (4 + k / 128) * 2.0 ** -23 * size[ok].norm()
+    a.fill_(float("nan"))
+    assert bool(torch.isnan(run()[0]).all())
+
+
 def test_f32_matmul_without_scratch_stays_on_the_fma_pipe():
     a, b = torch.randn(600, 300, device="cuda"), torch.randn(300, 700, device="cuda")
     with forced(F32TC=0):
