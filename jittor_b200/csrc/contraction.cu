@@ -160,10 +160,10 @@ extern "C" int b200jt_conv2d_formats(const b200jt_tensor* x, const b200jt_tensor
                         "multiple of 8 and >= 64, out channels >= 64, at least 1024 output pixels, 16-byte aligned tensors)");
     const size_t need = conv2d_tc_workspace(s);
     B200JT_CHECK_ARG(workspace_bytes >= need && workspace, "workspace too small: need " + std::to_string(need) + " bytes");
-    rc = conv2d_tc(x->ptr, w->ptr, y->ptr, stats, s, workspace, (cudaStream_t)stream, lay);
-    if (rc == 1) return 0;             // statistics came out of the conv epilogue
+    bool filled = false;
+    rc = conv2d_tc(x->ptr, w->ptr, y->ptr, stats, s, workspace, (cudaStream_t)stream, lay, &filled);
     if (rc) return rc;
-    if (stats) {
+    if (stats && !filled) {
         // wider than the epilogue keeps per CTA: statistics of the stored values by a separate pass are only built for NCHW
         return fail(-5, "b200jt_conv2d_formats: fused statistics need out channels <= 512 with an acdb output");
     }
@@ -222,9 +222,9 @@ extern "C" int b200jt_conv2d(const b200jt_tensor* x, const b200jt_tensor* w, con
         if (groups == 1 && x->dtype == B200JT_BFLOAT16 && conv2d_tc_supported(s, x->ptr, w->ptr, y->ptr)) {
             const size_t need = conv2d_tc_workspace(s);
             B200JT_CHECK_ARG(workspace_bytes >= need && workspace, "workspace too small: need " + std::to_string(need) + " bytes");
-            rc = conv2d_tc(x->ptr, w->ptr, y->ptr, stats, s, workspace, st);
-            if (rc == 1) return 0;             // statistics came out of the conv epilogue
-            if (rc) return rc;
+            bool filled = false;
+            rc = conv2d_tc(x->ptr, w->ptr, y->ptr, stats, s, workspace, st, ConvLayout(), &filled);
+            if (rc || filled) return rc;       // statistics come out of the conv epilogue
         } else {
             rc = x->dtype == B200JT_FLOAT32 && conv2d_f32_supported(s) ? conv2d_f32(x->ptr, w->ptr, y->ptr, s, st)
                                                                        : conv2d_simt(x->ptr, w->ptr, y->ptr, x->dtype, s, st);
@@ -328,8 +328,8 @@ extern "C" int b200jt_conv2d_backward_x(const b200jt_tensor* dy, const b200jt_te
     }
     ConvLayout lay;
     lay.w_grad = true;
-    const int rc = conv2d_tc(src, w->ptr, dx->ptr, nullptr, s, (char*)workspace + spread, st, lay);
-    return rc == 1 ? 0 : rc;
+    bool filled;
+    return conv2d_tc(src, w->ptr, dx->ptr, nullptr, s, (char*)workspace + spread, st, lay, &filled);
 }
 
 extern "C" int b200jt_conv2d_backward_w(const b200jt_tensor* x, const b200jt_tensor* dy, const b200jt_tensor* dw,

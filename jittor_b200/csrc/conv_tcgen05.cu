@@ -464,7 +464,7 @@ size_t conv2d_tc_workspace(const ConvShape& s) {
 }
 
 int conv2d_tc(const void* x, const void* w, void* y, float* stats, const ConvShape& s, void* workspace, cudaStream_t st,
-              const ConvLayout& lay) {
+              const ConvLayout& lay, bool* stats_filled) {
     using namespace tcconv;
     unsigned char* ws = (unsigned char*)(((uintptr_t)workspace + 1023) & ~(uintptr_t)1023);
     // NHWC ("acdb") activations are what the kernel reads: no staging pass for x then
@@ -530,7 +530,8 @@ int conv2d_tc(const void* x, const void* w, void* y, float* stats, const ConvSha
     cfg.blockDim = dim3(THREADS); cfg.dynamicSmemBytes = SMEM_BYTES; cfg.stream = st; cfg.attrs = at; cfg.numAttrs = pair ? 2 : 1;
     void* args[] = {&mx, &mw, &y, &fused, &A};
     B200JT_CUDA(cudaLaunchKernelExC(&cfg, kernel_of(lay.y_nhwc, bn, pair), args));
-    return fused ? 1 : 0;      // 1: statistics were produced by the epilogue
+    *stats_filled = fused != nullptr;
+    return 0;
 }
 
 // ---- weight gradient ---------------------------------------------------------------------------------------

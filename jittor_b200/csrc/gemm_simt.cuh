@@ -30,9 +30,9 @@ bool conv2d_tc_supported(const ConvShape& s, const void* x, const void* w, const
 bool conv2d_tc_layout_supported(const ConvShape& s);
 bool conv2d_wgrad_tc_layout_supported(const ConvShape& s);
 size_t conv2d_tc_workspace(const ConvShape& s);
-// returns < 0 / > 1 on error, 0 on success, 1 on success with `stats` filled by the epilogue
+// `stats_filled`: whether the epilogue fills `stats` (the return value, as everywhere, is 0 or an error, which may be any number)
 int conv2d_tc(const void* x, const void* w, void* y, float* stats, const ConvShape& s, void* workspace, cudaStream_t st,
-              const ConvLayout& lay = ConvLayout());
+              const ConvLayout& lay, bool* stats_filled);
 // weight gradient on tcgen05 (bf16, groups == 1): K = N*OH*OW pixels, split over CTAs, fp32 partial sums folded in a fixed order
 bool conv2d_wgrad_tc_supported(const ConvShape& s, const void* x, const void* dy, const void* dw);
 size_t conv2d_wgrad_tc_workspace(const ConvShape& s);

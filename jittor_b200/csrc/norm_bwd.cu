@@ -622,14 +622,15 @@ int run_bn_dx(const b200jt_tensor* x, const b200jt_tensor* dy, const float* sums
     return 0;
 }
 
-// 0: done; 1: the layer is not held (b200jt_bn_backward then runs the two kernels)
+// `held`: whether shared memory holds the layer; if not, nothing was launched (the return value is 0 or a CUDA error, which may be 1)
 template <typename TX, typename TD, int N>
-int launch_bn_held(const b200jt_tensor* x, const b200jt_tensor* dy, float* sums, const b200jt_tensor* dx, const BnArgs& g, cudaStream_t st) {
+int launch_bn_held(const b200jt_tensor* x, const b200jt_tensor* dy, float* sums, const b200jt_tensor* dx, const BnArgs& g, cudaStream_t st, bool* held) {
     const int64_t plane = g.HW * (int64_t)(sizeof(TX) + sizeof(TD));
     int size = bn_cluster(g, N);
     while (size < 8 && size * 2 <= g.N_ && (g.N_ + size - 1) / size * plane > kHeldWanted) size *= 2;
     const int64_t smem = (g.N_ + size - 1) / size * plane + 16;
-    if (smem > kHeldMost) return 1;
+    *held = smem <= kHeldMost;
+    if (!*held) return 0;
     const auto kernel = half_steps<TX, TD, N>(g) ? bn_bwd_held_kernel<TX, TD, N, can_half<TX, TD, N>> : bn_bwd_held_kernel<TX, TD, N, false>;
     static const cudaError_t attr = [] {
         const cudaError_t e = cudaFuncSetAttribute(bn_bwd_held_kernel<TX, TD, N, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kHeldMost);
@@ -647,8 +648,9 @@ int launch_bn_held(const b200jt_tensor* x, const b200jt_tensor* dy, float* sums,
 template <typename TX, typename TD, int V>
 int run_bn(const b200jt_tensor* x, const b200jt_tensor* dy, float* sums, const b200jt_tensor* dx, const BnArgs& g, cudaStream_t st) {
     const bool vec = g.HW % V == 0 && ((uintptr_t)x->ptr | (uintptr_t)dy->ptr | (uintptr_t)dx->ptr) % 16 == 0;
-    int rc = vec ? launch_bn_held<TX, TD, V>(x, dy, sums, dx, g, st) : launch_bn_held<TX, TD, 1>(x, dy, sums, dx, g, st);
-    if (rc != 1) return rc;
+    bool held;
+    int rc = vec ? launch_bn_held<TX, TD, V>(x, dy, sums, dx, g, st, &held) : launch_bn_held<TX, TD, 1>(x, dy, sums, dx, g, st, &held);
+    if (rc || held) return rc;
     rc = run_bn_sums<TX, TD, V>(x, dy, sums, g, st);
     return rc ? rc : run_bn_dx<TX, TD, V>(x, dy, sums, dx, g, st);
 }
