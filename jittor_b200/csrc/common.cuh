@@ -23,8 +23,9 @@ int  fail(int code, const std::string& msg);
     do { if (!(cond)) return ::b200jt::fail(-1, std::string(__func__) + ": " + (msg)); } while (0)
 
 #define B200JT_CUDA(expr)                                                        \
-    do { cudaError_t e_ = (expr); if (e_ != cudaSuccess)                         \
-        return ::b200jt::fail((int)e_, std::string(__func__) + ": " #expr ": " + cudaGetErrorString(e_)); } while (0)
+    do { cudaError_t e_ = (expr); if (e_ != cudaSuccess) {                       \
+        cudaGetLastError();     /* reported here: not once more by the next launch */ \
+        return ::b200jt::fail((int)e_, std::string(__func__) + ": " #expr ": " + cudaGetErrorString(e_)); } } while (0)
 
 #define B200JT_LAUNCH_CHECK()  B200JT_CUDA(cudaGetLastError())
 

@@ -9,15 +9,15 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 # what the entry points below call of the runtime; cudaLaunchKernelExC answers what it was told to
 FAKE = r"""
-static int made, answer;
+static int made, answer, last;
 static int encode(void) { return 0; }
 int cudaFuncSetAttribute(const void* f, int a, int v) { return 0; }
 int cudaOccupancyMaxActiveClusters(int* n, const void* f, const void* c) { *n = 74; return 0; }
 int cudaGetDriverEntryPointByVersion(const char* s, void** p, unsigned v, unsigned long long f, int* q) { *p = (void*)encode; if (q) *q = 0; return 0; }
 int cudaGetDriverEntryPoint(const char* s, void** p, unsigned long long f, int* q) { *p = (void*)encode; if (q) *q = 0; return 0; }
 int cudaLaunchKernel(const void* f, ...) { return 0; }
-int cudaGetLastError(void) { return 0; }
-int cudaLaunchKernelExC(const void* c, const void* f, void** a) { made++; return answer; }
+int cudaGetLastError(void) { int e = last; last = 0; return e; }
+int cudaLaunchKernelExC(const void* c, const void* f, void** a) { made++; return last = answer; }
 void fake_answer(int e) { answer = e; made = 0; }
 int fake_launches(void) { return made; }
 """
@@ -46,7 +46,7 @@ fake = ctypes.CDLL(None)
 for name, call in calls.items():
     for error in (0, 1, 9):
         fake.fake_answer(error)
-        print(name, error, call(), fake.fake_launches())
+        print(name, error, call(), fake.fake_launches(), fake.cudaGetLastError())
 """
 
 
@@ -57,5 +57,5 @@ def test_a_failed_launch_is_reported(tmp_path):
     env = dict(os.environ, LD_PRELOAD=str(so), CUDA_VISIBLE_DEVICES="")
     out = subprocess.run([sys.executable, "-c", CALLS], cwd=ROOT, env=env, capture_output=True, text=True, timeout=300)
     assert out.returncode == 0, out.stderr
-    want = [f"{name} {error} {error} 1" for name in ("bn_backward", "conv2d", "conv2d_formats", "conv2d_backward_x") for error in (0, 1, 9)]
-    assert out.stdout.splitlines() == want               # the error itself, after the one launch that failed
+    want = [f"{name} {error} {error} 1 0" for name in ("bn_backward", "conv2d", "conv2d_formats", "conv2d_backward_x") for error in (0, 1, 9)]
+    assert out.stdout.splitlines() == want               # the error itself, after the one launch that failed; none is left for the next call
