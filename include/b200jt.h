@@ -238,6 +238,8 @@ int b200jt_optim_step(const char* kind, int count, const int64_t* sizes, const f
  * chosen by MatmulTuner for reduce.add(multiply(broadcast_to(a), broadcast_to(b))), python/jittor/src/opt/tuner/matmul_tuner.cc:21-102.
  * a, b, c: float32 or bfloat16, same dtype. */
 size_t b200jt_matmul_workspace(const b200jt_tensor* a, const b200jt_tensor* b, const b200jt_tensor* c, int trans_a, int trans_b);
+/* What b200jt_matmul cannot do without; with less than b200jt_matmul_workspace bytes it takes longer. */
+size_t b200jt_matmul_least_workspace(const b200jt_tensor* a, const b200jt_tensor* b, const b200jt_tensor* c, int trans_a, int trans_b);
 int b200jt_matmul(const b200jt_tensor* a, const b200jt_tensor* b, const b200jt_tensor* c,
                   int trans_a, int trans_b, void* workspace, size_t workspace_bytes, void* stream);
 

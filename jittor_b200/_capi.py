@@ -92,6 +92,7 @@ SIGNATURES = [
     ("b200jt_optim_step", _i, [ctypes.c_char_p, _i, ctypes.POINTER(ctypes.c_int64)] + [ctypes.POINTER(_vp)] * 7
      + [ctypes.POINTER(_d), _i, _i, _vp]),
     ("b200jt_matmul_workspace", _sz, [_TP, _TP, _TP, _i, _i]),
+    ("b200jt_matmul_least_workspace", _sz, [_TP, _TP, _TP, _i, _i]),
     ("b200jt_matmul", _i, [_TP, _TP, _TP, _i, _i, _vp, _sz, _vp]),
     ("b200jt_batched_matmul", _i, [_TP, _TP, _TP, _i, _i, _vp]),
     ("b200jt_device_status", _i, []),
@@ -317,12 +318,26 @@ def full(shape, value, dtype):
     return t
 
 
+# entry points that also run, if slower, with less scratch memory than they ask for -> what they cannot do without (host.cpp knows it too)
+LEAST = {"b200jt_matmul_workspace": "b200jt_matmul_least_workspace"}
+
+
 def workspace(name, *args):
-    """(bytes, pointer, tensor that owns it) of the scratch memory `name` asks for."""
+    """(bytes, pointer, tensor that owns it) of the scratch memory `name` asks for, or that it runs with where there is no room."""
     n = getattr(lib, name)(*args)
     if n == 0:
         return 0, None, None
-    t = torch.empty(int(n), dtype=torch.uint8, device="cuda")
+    try:
+        t = torch.empty(int(n), dtype=torch.uint8, device="cuda")
+    except torch.OutOfMemoryError:
+        if name not in LEAST:
+            raise
+        if recording():
+            recorder.ok = False               # not the steps of the next run, which may find room
+        n = getattr(lib, LEAST[name])(*args)
+        if n == 0:
+            return 0, None, None
+        t = torch.empty(int(n), dtype=torch.uint8, device="cuda")
     if recording():
         recorder.workspace(name, args, t)
     return n, t.data_ptr(), t

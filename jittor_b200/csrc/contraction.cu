@@ -16,10 +16,16 @@ extern "C" size_t b200jt_matmul_workspace(const b200jt_tensor* a, const b200jt_t
     int64_t M, N, K;
     if (!matmul_dims(a, b, trans_a, trans_b, &M, &N, &K) || !valid_tensor(c)) return 0;
     if (a->dtype == B200JT_BFLOAT16 && matmul_tc_supported(M, N, K, a->ptr, b->ptr, c->ptr))
-        return matmul_tc_workspace(M, N, K, trans_a != 0, trans_b != 0);
+        return matmul_tc_workspace(M, N, K, trans_a != 0, trans_b != 0, true);
     if (a->dtype == B200JT_FLOAT32)
         return matmul_f32_tc_wanted(M, N, K) ? matmul_f32_tc_workspace(M, N, K, trans_a != 0, trans_b != 0) : matmul_f32_workspace(M, N, K);
     return 0;
+}
+
+extern "C" size_t b200jt_matmul_least_workspace(const b200jt_tensor* a, const b200jt_tensor* b, const b200jt_tensor* c, int trans_a, int trans_b) {
+    int64_t M, N, K;
+    if (!matmul_dims(a, b, trans_a, trans_b, &M, &N, &K) || !valid_tensor(c)) return 0;
+    return a->dtype == B200JT_BFLOAT16 && matmul_tc_supported(M, N, K, a->ptr, b->ptr, c->ptr) ? matmul_tc_workspace(M, N, K, trans_a != 0, trans_b != 0, false) : 0;
 }
 
 /* Status word of the tensor-core kernels: 0, or the code of the first bounded wait that expired since the last call
@@ -44,9 +50,11 @@ extern "C" int b200jt_matmul(const b200jt_tensor* a, const b200jt_tensor* b, con
     if (M == 0 || N == 0) return 0;
     cudaStream_t st = (cudaStream_t)stream;
     if (a->dtype == B200JT_BFLOAT16 && matmul_tc_supported(M, N, K, a->ptr, b->ptr, c->ptr)) {
-        const size_t need = matmul_tc_workspace(M, N, K, trans_a != 0, trans_b != 0);
-        B200JT_CHECK_ARG(workspace_bytes >= need && (need == 0 || workspace), "workspace too small: need " + std::to_string(need) + " bytes");
-        return matmul_tc(a->ptr, b->ptr, c->ptr, M, N, K, trans_a != 0, trans_b != 0, workspace, st);
+        const auto fits = [&](size_t need) { return workspace_bytes >= need && (need == 0 || workspace); };
+        const bool split = fits(matmul_tc_workspace(M, N, K, trans_a != 0, trans_b != 0, true));         // K may be split over partial sums
+        const size_t need = split ? 0 : matmul_tc_workspace(M, N, K, trans_a != 0, trans_b != 0, false);
+        B200JT_CHECK_ARG(split || fits(need), "workspace too small: need " + std::to_string(need) + " bytes");
+        return matmul_tc(a->ptr, b->ptr, c->ptr, M, N, K, trans_a != 0, trans_b != 0, workspace, split, st);
     }
     if (a->dtype == B200JT_FLOAT32 && matmul_f32_tc_wanted(M, N, K) && workspace &&
         workspace_bytes >= matmul_f32_tc_workspace(M, N, K, trans_a != 0, trans_b != 0))

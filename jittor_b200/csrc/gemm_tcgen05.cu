@@ -496,12 +496,13 @@ bool matmul_tc_supported(int64_t M, int64_t N, int64_t K, const void* a, const v
            ((uintptr_t)a % 16 == 0) && ((uintptr_t)b % 16 == 0) && ((uintptr_t)c % 2 == 0) && tc::encode_fn() != nullptr;
 }
 
-size_t matmul_tc_workspace(int64_t M, int64_t N, int64_t K, bool trans_a, bool trans_b) {
+size_t matmul_tc_workspace(int64_t M, int64_t N, int64_t K, bool trans_a, bool trans_b, bool may_split) {
     using namespace tc;
     const int64_t ca = trans_a ? M : K, cb = trans_b ? K : N;
     size_t bytes = 0;
     if (ca % 8) bytes += round256((size_t)(trans_a ? K : M) * pitch8(ca) * 2);
     if (cb % 8) bytes += round256((size_t)(trans_b ? N : K) * pitch8(cb) * 2);
+    if (!may_split) return bytes;
     const Plan p = plan_for(1, M, N, K, !trans_b, true);
     if (p.splits > 1) {
         const int64_t tile_m = BM * p.mt * (1 + p.pair);
@@ -511,10 +512,10 @@ size_t matmul_tc_workspace(int64_t M, int64_t N, int64_t K, bool trans_a, bool t
 }
 
 int matmul_tc(const void* a, const void* b, void* c, int64_t M, int64_t N, int64_t K, bool trans_a, bool trans_b,
-              void* workspace, cudaStream_t st) {
+              void* workspace, bool may_split, cudaStream_t st) {
     using namespace tc;
     unsigned char* ws = (unsigned char*)workspace;
-    const Plan p = plan_for(1, M, N, K, !trans_b, true);
+    const Plan p = plan_for(1, M, N, K, !trans_b, may_split);
     auto padded = [&](const void*& q, int64_t rows, int64_t cols) {
         if (cols % 8 == 0) return cols;
         const int64_t pitch = pitch8(cols);

@@ -415,7 +415,7 @@ struct Entry { const char* name; Invoke invoke; void* fn; };
 Entry g_entries[] = {
     E(b200jt_reindex), E(b200jt_reindex_reduce_workspace), E(b200jt_reindex_reduce), E(b200jt_setitem), E(b200jt_broadcast_to),
     E(b200jt_reduce_workspace), E(b200jt_reduce), E(b200jt_binary), E(b200jt_unary), E(b200jt_ternary), E(b200jt_fused_chain),
-    E(b200jt_softmax), E(b200jt_softmax_backward), E(b200jt_layer_norm), E(b200jt_matmul_workspace), E(b200jt_matmul),
+    E(b200jt_softmax), E(b200jt_softmax_backward), E(b200jt_layer_norm), E(b200jt_matmul_workspace), E(b200jt_matmul_least_workspace), E(b200jt_matmul),
     E(b200jt_batched_matmul), E(b200jt_conv2d_workspace), E(b200jt_conv2d), E(b200jt_conv2d_formats_workspace), E(b200jt_conv2d_formats),
     E(b200jt_conv2d_transpose), E(b200jt_conv2d_backward_w), E(b200jt_conv2d_backward_w_workspace), E(b200jt_conv2d_backward_w_tc),
     E(b200jt_conv2d_backward_w_formats_workspace), E(b200jt_conv2d_backward_w_formats), E(b200jt_bn_stats), E(b200jt_bn_apply),
@@ -437,6 +437,7 @@ struct Step {
     at::ScalarType type = at::kByte;       // ALLOC
     double value = 0;                      // FILL
     Entry* entry = nullptr;                // CALL, WORKSPACE
+    Entry* least = nullptr;                // WORKSPACE: what the call cannot do without, where it takes less than it asks for
     std::vector<Slot> slots;
     std::vector<Patch> patches;
     std::vector<std::pair<int, int>> nbytes;   // (slot, buffer): the size of a workspace passed beside its pointer
@@ -589,6 +590,7 @@ std::shared_ptr<Tape> build_tape(PyObject* spec, int n_leaves) {
             st.buf = (int)PyLong_AsLong(PyTuple_GET_ITEM(s, 1));
             const char* name = PyUnicode_AsUTF8(PyTuple_GET_ITEM(s, 2));
             if (!name || !(st.entry = entry_of(name))) return nullptr;
+            if (!std::strcmp(name, "b200jt_matmul_workspace")) st.least = entry_of("b200jt_matmul_least_workspace");
             PyObject* args = PyTuple_GET_ITEM(s, 3);
             st.slots.reserve((size_t)PyList_GET_SIZE(args));
             for (Py_ssize_t k = 0; k < PyList_GET_SIZE(args); k++) if (!add_arg(*t, st, PyList_GET_ITEM(args, k))) return nullptr;
@@ -688,9 +690,15 @@ bool replay(Tape& t, const Walk& w) {
             }
             for (auto& n : st.nbytes) st.slots[n.first].i = bufs[n.second].defined() ? bufs[n.second].numel() : 0;
             if (st.stream >= 0) st.slots[st.stream].p = stream;
-            const int64_t rc = st.entry->invoke(st.entry->fn, st.slots.data());
+            int64_t rc = st.entry->invoke(st.entry->fn, st.slots.data());
             if (st.kind == Step::WORKSPACE) {
-                if (rc > 0) bufs[st.buf] = at::Tensor(at::detail::empty_cuda({rc}, at::kByte, device, std::nullopt));
+                auto get = [&] { if (rc > 0) bufs[st.buf] = at::Tensor(at::detail::empty_cuda({rc}, at::kByte, device, std::nullopt)); };
+                if (!st.least) get();
+                else {
+                    bool room = true;
+                    try { get(); } catch (const c10::OutOfMemoryError&) { room = false; }
+                    if (!room) { rc = st.least->invoke(st.least->fn, st.slots.data()); get(); }
+                }
             } else if (rc != 0) {
                 const std::string why = g_last_error ? g_last_error() : "";
                 if (hand_out(at)) PyErr_Format(h_error, "%s: %s (status %d)", st.what.c_str(), why.c_str(), (int)rc);

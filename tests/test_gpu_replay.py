@@ -186,6 +186,26 @@ def test_running_out_of_memory_is_the_same_error_from_planner_and_replay():
     assert torch.equal(graph().torch(), want)
 
 
+# float32: operands split into parts; bfloat16: partial sums of a split K; an odd K needs room for operands at TMA's pitch besides
+@pytest.mark.parametrize("m,k,n,dtype,spare", [(2048, 2048, 2048, torch.float32, 20 << 20), (512, 16384, 512, torch.bfloat16, 4 << 20), (512, 16383, 512, torch.bfloat16, 22 << 20)])
+def test_a_product_runs_where_there_is_no_room_for_all_its_scratch(m, k, n, dtype, spare):
+    x, w = data(1, m, k, dtype=dtype), data(2, k, n, dtype=dtype)
+    out = torch.empty(m, n, dtype=dtype, device="cuda")
+    args = (C.desc(x.torch()), C.desc(w.torch()), C.desc(out), 0, 0)
+    assert C.lib.b200jt_matmul_least_workspace(*args) < spare < C.lib.b200jt_matmul_workspace(*args) + out.numel() * out.element_size()
+    want = x.torch().double() @ w.torch().double()
+    del out
+    for prepared in (False, True):
+        C.host.clear()
+        if prepared:
+            nn.matmul(x, w).sync()                            # recorded
+        with limited_memory(spare):
+            y = nn.matmul(x, w).sync()
+        assert (y.torch().double() - want).norm() <= (1e-5 if dtype == torch.float32 else 2.0 ** -8) * want.norm()
+        for _ in range(2):                                    # and with its scratch once there is room
+            assert (nn.matmul(x, w).torch().double() - want).norm() <= (1e-5 if dtype == torch.float32 else 2.0 ** -8) * want.norm()
+
+
 @pytest.mark.parametrize("prepared", [False, True])
 def test_running_statistics_move_once_when_a_later_step_fails(prepared):
     x = torch.randn(4, 16, 8, 8, device="cuda") + 0.3
