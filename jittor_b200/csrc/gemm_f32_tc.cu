@@ -545,10 +545,12 @@ struct Plan { bool tc, pair; int bn, splits; };
 // and the estimates are within a fifth of the times measured for 28 shapes; 500 x 777 x 1000: 29 and 18 us, 1024 x 1024 x 1024: 61
 // and 28, 4096 x 2048 x 4096: 1410 and 349. 3 us in hand: of 54 products drawn from 16 to 9472 a side none was then slower than
 // the FMA kernel by more than the timer shows (with 1 us in hand, and half of what the stores take: 4588 x 72 x 3272, 64 and 69).
-static Plan estimate(int64_t M, int64_t N, int64_t K) {
+// `force`: B200JT_F32TC, with which tests force each path in turn; the switches of its tiles count only beside it.
+static Plan estimate(int64_t M, int64_t N, int64_t K, const char* force) {
     Plan best{false, false, 128, 1};
     double best_ns = 1e30;
-    const char* fp = getenv("B200JT_F32TC_PAIR"); const char* fb = getenv("B200JT_F32TC_BN"); const char* fs = getenv("B200JT_F32TC_SPLITS");
+    const auto set = [&](const char* name) { return force ? getenv(name) : nullptr; };
+    const char* fp = set("B200JT_F32TC_PAIR"); const char* fb = set("B200JT_F32TC_BN"); const char* fs = set("B200JT_F32TC_SPLITS");
     const int64_t kb = (K + BK - 1) / BK;
     for (int pair = 0; pair < 2; pair++) {
         if ((fp && atoi(fp) != pair) || (pair && !slots().pair)) continue;
@@ -566,20 +568,19 @@ static Plan estimate(int64_t M, int64_t N, int64_t K) {
             }
         }
     }
-    const char* f = getenv("B200JT_F32TC");                 // read on every call: tests force each path in turn
-    best.tc = best_ns < 1e30 && (f ? atoi(f) != 0 : best_ns + 3000 < matmul_f32_ns(M, N, K));
+    best.tc = best_ns < 1e30 && (force ? atoi(force) != 0 : best_ns + 3000 < matmul_f32_ns(M, N, K));
     return best;
 }
 
 // Some 400 candidates of both paths, a few us: each thread keeps its last 64 plans.
 static Plan plan_for(int64_t M, int64_t N, int64_t K) {
-    if (getenv("B200JT_F32TC")) return estimate(M, N, K);
+    if (const char* force = getenv("B200JT_F32TC")) return estimate(M, N, K, force);
     struct Entry { int64_t M = -1, N = 0, K = 0; Plan p; };
     static thread_local Entry kept[64];
     uint64_t h = 0;
     for (int64_t k : {M, N, K}) h = (h ^ (uint64_t)k) * 0x9E3779B97F4A7C15ull;
     Entry& e = kept[h >> 58];
-    if (e.M != M || e.N != N || e.K != K) e = {M, N, K, estimate(M, N, K)};
+    if (e.M != M || e.N != N || e.K != K) e = {M, N, K, estimate(M, N, K, nullptr)};
     return e.p;
 }
 

@@ -109,6 +109,22 @@ def test_f32_matmul_without_scratch_stays_on_the_fma_pipe():
         assert torch.equal(matmul(a, b, 0, 0, scratch=False), want)
 
 
+def test_f32_tile_switches_do_not_outlast_or_precede_a_plan():
+    """Switches of the tiles without that of the path: a thread that plans a size under them goes as one that does not."""
+    import threading
+    a, b, seen = torch.randn(500, 777, device="cuda"), torch.randn(777, 1000, device="cuda"), []
+
+    def run():                                                                         # each thread plans for itself
+        for _ in range(2):
+            with forced(F32TC_SPLITS=1, F32TC_PAIR=0) if len(seen) == 2 else forced():
+                seen.append(matmul(a, b, 0, 0))
+    for _ in range(2):
+        t = threading.Thread(target=run)
+        t.start()
+        t.join()
+    assert len(seen) == 4 and all(torch.equal(seen[0], s) for s in seen[1:])
+
+
 # ---- bfloat16 products whose last round alone is split (csrc/gemm_tcgen05.cu)
 @pytest.mark.parametrize("ta,tb", [(0, 0), (1, 0), (0, 1)])
 @pytest.mark.parametrize("pair,mt,bn,splits,m,k,n", [(0, 1, 64, 2, 1300, 300, 1000), (0, 1, 32, 3, 1283, 200, 500), (1, 1, 64, 4, 2570, 260, 600),
