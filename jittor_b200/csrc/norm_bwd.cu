@@ -560,12 +560,13 @@ template <typename T, int V>
 int run_ln(const T* x, const T* dy, const float* gamma, T* dx, float* params, float* partial, int64_t rows, int cols, float eps, cudaStream_t st) {
     const bool vec = cols % V == 0 && (uintptr_t)x % 16 == 0 && (uintptr_t)dy % 16 == 0 && (uintptr_t)dx % 16 == 0 && (uintptr_t)gamma % 16 == 0;
 #define B200JT_LN(GROUP, E)                                                                                                      \
-    do { const int ctas = ln_ctas(rows, cta_of(GROUP) / GROUP, GROUP != 32 && GROUP < 256 ? kMostCtas : E > (params ? 8 : 16) ? 2 : 4, params); \
+    do { const int ctas = ln_ctas(rows, cta_of(GROUP) / GROUP, E > (params ? 8 : 16) ? 2 : 4, params);                           \
          return vec ? launch_ln<T, V, GROUP, E>(x, dy, gamma, dx, params, partial, rows, cols, eps, ctas, st)                    \
                     : launch_ln<T, 1, GROUP, E>(x, dy, gamma, dx, params, partial, rows, cols, eps, ctas, st); } while (0)
     if (cols <= 256) B200JT_LN(32, 8);
-    if (cols <= 512) { if (vec || rows >= 8192) B200JT_LN(32, 16); B200JT_LN(64, 8); }
-    if (cols <= 1024 && vec) B200JT_LN(128, 8);
+    if (cols <= 512 && (vec || rows >= 8192)) B200JT_LN(32, 16);
+    if (cols <= 512) return launch_ln<T, 1, 64, 8>(x, dy, gamma, dx, params, partial, rows, cols, eps, ln_ctas(rows, 1, kMostCtas, params), st);
+    if (cols <= 1024 && vec) return launch_ln<T, V, 128, 8>(x, dy, gamma, dx, params, partial, rows, cols, eps, ln_ctas(rows, 1, kMostCtas, params), st);
     if (cols <= 1024) return launch_ln<T, 1, 256, 4>(x, dy, gamma, dx, params, partial, rows, cols, eps, ln_ctas(rows, 1, 4, params), st);
     if (cols <= 2048) B200JT_LN(256, 8);
     if (cols <= 4096) B200JT_LN(256, 16);
