@@ -530,7 +530,7 @@ constexpr int kMaxCols = 8192;
 // Persistent CTAs: enough rows in flight to cover the latency of a row's reductions, few enough partial rows to fold: no more than
 // are resident (two per SM with 16 elements a thread), and beyond one per SM at least four rows for each. [640, 4096] bfloat16 33 ->
 // 19 us, [5000, 4096] 67 -> 42, float32 67 -> 59, [16384, 512] 33 -> 23.5.
-constexpr int kMostCtas = 8;                                   // per SM, over all forms below
+constexpr int kMostCtas = 8;                                   // per SM, of the forms for up to 1024 columns; four of those beyond
 inline int ln_ctas(int64_t rows, int rpc, int per_sm, bool params) {
     const int64_t sms = kNumSMs - sm_reserve();
     int64_t need = (rows + rpc - 1) / rpc;
@@ -679,7 +679,7 @@ extern "C" size_t b200jt_layer_norm_backward_workspace(const b200jt_tensor* x, i
     if (!valid_tensor(x) || !want_params) return 0;
     const int64_t cols = x->shape[x->ndim - 1], rows = cols ? numel(x) / cols : 0;
     if (cols < 1 || cols > kMaxCols || rows < 1) return 0;
-    return sizeof(float) * 2 * cols * (size_t)ln_ctas(rows, 1, kMostCtas, false);
+    return sizeof(float) * 2 * cols * (size_t)ln_ctas(rows, 1, cols <= 1024 ? kMostCtas : 4, true);
 }
 
 extern "C" int b200jt_layer_norm_backward(const b200jt_tensor* x, const b200jt_tensor* gamma, const b200jt_tensor* dy, const b200jt_tensor* dx,

@@ -25,6 +25,14 @@ def test_library_exports_every_declared_symbol():
     assert _capi.lib.b200jt_version() >= 100
 
 
+@pytest.mark.parametrize("rows,cols,ctas", [(5, 4096, 5), (640, 4096, 160), (5000, 8192, 592), (100000, 1025, 592), (100000, 1024, 1184), (100000, 300, 1184)])
+def test_layer_norm_backward_asks_for_the_partial_rows_it_writes(rows, cols, ctas):
+    d = _capi.Tensor()
+    d.ptr, d.dtype, d.ndim = 4096, _capi.DTYPE_CODES["float32"], 2
+    d.shape[0], d.shape[1] = rows, cols
+    assert _capi.lib.b200jt_layer_norm_backward_workspace(d, 1) == 2 * cols * 4 * ctas
+
+
 def test_no_cuda_means_loud_failure():
     import torch
     if torch.cuda.is_available():
