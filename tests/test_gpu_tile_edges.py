@@ -52,6 +52,37 @@ def test_f32_tensor_core_matmul(m, k, n, pair, bn, splits, ta, tb):
     assert C.lib.b200jt_device_status() == 0
 
 
+# Relative to the result, operands of both signs and of one. Truncation loses at most 2^-23 of the sum so far at each of the last four
+# additions of a group, 1.25 * 2^-23 of its sum on average where all have one sign; the group sums, up to 64 of them, are rounded to
+# nearest, 2^-24 each, in random directions. Without the products of the third parts (2^-18 of an operand) or of the two second
+# parts it would be some ten times the bound.
+@pytest.mark.parametrize("pair,bn,splits", [(0, 128, 1), (0, 64, 8), (1, 256, 1)])
+@pytest.mark.parametrize("k", [64, 257, 1024, 4096])
+@pytest.mark.parametrize("sign", ["both", "one"])
+def test_f32_tensor_core_matmul_accuracy(sign, k, pair, bn, splits):
+    a, b = torch.randn(256, k, device="cuda"), torch.randn(k, 384, device="cuda")
+    if sign == "one":
+        a, b = a.abs(), b.abs()
+    with forced(F32TC=1, F32TC_PAIR=pair, F32TC_BN=bn, F32TC_SPLITS=min(splits, k // 32)):
+        c = matmul(a, b, 0, 0)
+    want = product(a, b, 0, 0)
+    assert (c.double() - want).norm() <= 2.5 * 2.0 ** -23 * want.norm()
+
+
+@pytest.mark.parametrize("pair,bn,splits", [(0, 96, 1), (0, 128, 4), (1, 256, 1)])
+def test_f32_tensor_core_matmul_keeps_all_bits(pair, bn, splits):
+    """24 significant bits times powers of two, one to a row or column: nothing is rounded, so nothing may be lost."""
+    m, k = 270, 300
+    pick = torch.randperm(k, device="cuda")
+    scale = torch.ldexp(torch.ones(k, device="cuda"), torch.randint(-20, 20, (k,), device="cuda")) * torch.randint(0, 2, (k,), device="cuda").sub(0.5).sign()
+    p = torch.zeros(k, k, device="cuda")
+    p[pick, torch.arange(k, device="cuda")] = scale
+    v = torch.randn(m, k, device="cuda")
+    with forced(F32TC=1, F32TC_PAIR=pair, F32TC_BN=bn, F32TC_SPLITS=splits):
+        assert torch.equal(matmul(v, p, 0, 0), v[:, pick] * scale)
+        assert torch.equal(matmul(p, v, 1, 1), (v[:, pick] * scale).t())
+
+
 def test_f32_tensor_core_matmul_range():
     """Subnormal and huge operands, overflow, infinities and NaN come out as from float32 arithmetic."""
     m, k, n = 130, 200, 140
@@ -136,6 +167,70 @@ def test_bf16_matmul_split_last_round(pair, mt, bn, splits, m, k, n, ta, tb):
     want = product(a, b, ta, tb)
     assert (c.double() - want).abs().max() <= 2.0 ** -8 * want.abs().max()             # one rounding to bfloat16 of a float32 sum
     assert C.lib.b200jt_device_status() == 0
+
+
+# ---- kernels that start while the pass before them drains: one after the other on one scratch buffer, with other inputs each time, give
+# what each gives alone; also from a graph whose inputs change
+def early_product(dtype, m, k, n, ta, tb):
+    a, b = torch.randn(*((k, m) if ta else (m, k)), device="cuda").to(dtype), torch.randn(*((n, k) if tb else (k, n)), device="cuda").to(dtype)
+    c = torch.empty(m, n, dtype=dtype, device="cuda")
+    args = (C.desc(a), C.desc(b), C.desc(c), ta, tb)
+    return [a, b], [c], int(C.lib.b200jt_matmul_workspace(*args)), lambda p, size: C.call("b200jt_matmul", *args, p, size)
+
+
+def early_conv(kind, last):
+    n, ci, co, side = 8, 64, 128, 28
+    shape = lambda c: (n, side, side, c) if last else (n, c, side, side)
+    x, y, w = torch.randn(shape(ci), device="cuda").bfloat16(), torch.randn(shape(co), device="cuda").bfloat16(), torch.randn(co, ci, 3, 3, device="cuda").bfloat16()
+    fmt = (b"acdb", b"oihw", b"acdb") if last else (b"abcd", b"oihw", b"abcd")
+    args = (C.desc(x), C.desc(w), C.desc(y), 1, 1, 1, 1, 1, 1, *fmt)
+    if kind == "forward":
+        stats = torch.empty(2 * co, device="cuda")
+        return [x, w], [y, stats], int(C.lib.b200jt_conv2d_formats_workspace(*args)), lambda p, size: C.call("b200jt_conv2d_formats", *args, stats.data_ptr(), p, size)
+    args = (C.desc(x), C.desc(y), C.desc(w), 1, 1, 1, 1, 1, 1, *fmt)
+    return [x, y], [w], int(C.lib.b200jt_conv2d_backward_w_formats_workspace(*args)), lambda p, size: C.call("b200jt_conv2d_backward_w_formats", *args, p, size)
+
+
+@pytest.mark.parametrize("make,args", [(early_product, (torch.float32, 500, 777, 1000, 0, 0)), (early_product, (torch.float32, 500, 777, 1000, 1, 1)),
+                                       (early_product, (torch.bfloat16, 500, 777, 1000, 0, 0)), (early_conv, ("forward", 0)), (early_conv, ("forward", 1)),
+                                       (early_conv, ("weights", 0)), (early_conv, ("weights", 1))])
+def test_early_starts(make, args):
+    calls = [make(*args) for _ in range(5)]
+    size = calls[0][2]
+    ws = torch.empty(size, dtype=torch.uint8, device="cuda")
+    run = lambda i: calls[i][3](ctypes.c_void_p(ws.data_ptr()), size)
+
+    def alone():
+        out = []
+        for i in range(len(calls)):
+            ws.fill_(0xff)                                                             # NaN, had anything read it too early
+            torch.cuda.synchronize()
+            run(i)
+            torch.cuda.synchronize()
+            out.append([t.clone() for t in calls[i][1]])
+        return out
+
+    def same(want):
+        for i, w in enumerate(want):
+            assert torch.equal(calls[i][1][0], w[0])
+            for t, s in zip(calls[i][1][1:], w[1:]):                                   # channel sums: added up in the order of arrival
+                assert (t - s).norm() <= 1e-5 * s.norm()
+    want = alone()
+    for _ in range(8):
+        for i in range(len(calls)):
+            run(i)
+    same(want)
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        for i in range(len(calls)):
+            run(i)
+    for c in calls:
+        for t in c[0]:
+            t.copy_(torch.randn(t.shape, device="cuda"))
+    want = alone()
+    g.replay()
+    g.replay()
+    same(want)
 
 
 # ---- few bins (csrc/reindex_reduce.cu): whole, part and no batches of a thread's two vectors
@@ -321,3 +416,40 @@ def test_batch_norm_backward_in_one_launch(shape, xt, dt, form):
     want = per(gamma) * rstd * (d - (per(s0) + xh * per(s1)) / count)
     assert (sums[:cn].double() - s0).norm() <= 1e-5 * count ** 0.5 * cn ** 0.5 and (sums[cn:2 * cn].double() - s1).norm() <= 1e-5 * count ** 0.5 * cn ** 0.5
     assert (dx.double() - want).norm() <= (2.0 ** -8 if xt == torch.bfloat16 else 1e-4) * want.norm() + 1e-6
+
+
+@pytest.mark.parametrize("xt,dt", [(torch.bfloat16, torch.bfloat16), (torch.bfloat16, torch.float32)])
+@pytest.mark.parametrize("form", [2, 3, 4, 5])
+@pytest.mark.parametrize("shape", [(3, 5, 7, 7), (13, 3, 8, 8), (64, 128, 28, 28), (256, 512, 7, 7), (2, 1, 200, 200)])
+def test_batch_norm_backward_rounded_steps(shape, form, xt, dt):
+    """The forms that round as a 16-bit graph does, step by step in torch: 2 and 3 with a float32 activation, 4 and 5 with every step to
+    bfloat16, odd ones with a ReLU."""
+    n, cn, hw = shape[0], shape[1], shape[2] * shape[3]
+    count = float(n * hw)
+    x, dy = (torch.randn(shape, device="cuda") + 0.3).to(xt), torch.randn(shape, device="cuda").to(dt)
+    gamma, beta = torch.rand(cn, device="cuda") + 0.5, torch.randn(cn, device="cuda") * 0.1
+    bf = lambda t: t.bfloat16().float()
+    at = bf if form >= 4 else lambda t: t                                              # steps that only the second pair rounds
+    per = lambda t: t[None, :, None, None]
+    total = lambda t: t.double().sum((0, 2, 3)).float()
+    xf, df, rc = x.float(), dy.float(), torch.tensor(1.0 / count, device="cuda")
+    stats = torch.cat([total(xf), total(xf * xf)])
+    mean, square = bf(stats[:cn] * rc), total(bf(xf * xf)) * rc
+    sd = bf(bf(bf(bf(square) - bf(mean * mean)).clamp(min=0) + 1e-5).sqrt())
+    w = at(gamma / sd)
+    b = at(beta - at(mean * w))
+    u = torch.where(at(xf * per(w)) + per(b) > 0, df, 0.0) if form % 2 else df
+    s0, s1 = at(total(u)), at(total(at(xf * u)))
+    dw = at(s1 + at(mean * -s0))
+    dvar = bf(bf(at(-dw * gamma) / bf(sd * sd)) / bf(sd * 2))
+    t = bf(mean * -dvar)
+    p, q = bf(dvar * rc), bf(bf(bf(bf(w * -s0) + t) + t) * rc)
+    step = bf(xf * per(p))
+    want = bf(bf(bf(per(w) * u) + step) + step) + per(q)
+    sums, dx = torch.full((4 * cn,), float("nan"), device="cuda"), torch.full(shape, float("nan"), device="cuda", dtype=xt)
+    C.call("b200jt_bn_backward", C.desc(x), C.desc(dy), stats.data_ptr(), count, gamma.data_ptr(), beta.data_ptr(), 1e-5, form, sums.data_ptr(), C.desc(dx))
+    # another order of the sums may turn a rounding of a channel's number, 2^-8 of it, and with it the channel's elements
+    near = lambda got, ref, floor: (got.double() - ref.double()).norm() <= 2.0 ** -7 * ref.double().norm() + floor
+    assert near(sums[:cn], s0, 1e-5 * count ** 0.5) and near(sums[2 * cn:3 * cn], square, 0)
+    assert near(sums[3 * cn:], dw, 2.0 ** -7 * float((mean * s0).norm()) + 1e-5 * count ** 0.5)
+    assert near(dx, want, 0)
