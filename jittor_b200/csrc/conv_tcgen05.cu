@@ -493,7 +493,9 @@ int conv2d_tc(const void* x, const void* w, void* y, float* stats, const ConvSha
     // Tile by estimated time: the grid is persistent with a static round-robin, so it takes ceil(tiles / slots) rounds, each of a
     // tile's main loop and the part of its epilogue that the next tile's main loop does not hide (about half). A k-block of 64 channels
     // measured 342, 354, 477 ns with 64, 128, 256 output channels and 347, 380, 445 ns on a pair: most of it is the feed of the
-    // x boxes (their 128 rows of 128 bytes), so narrow tiles feed the MMAs worse but leave less of the last round idle.
+    // x boxes (their 128 rows of 128 bytes), so narrow tiles feed the MMAs worse but leave less of the last round idle. The epilogue costs
+    // 12.5 ns a channel, with statistics too since they come from the square: over 24 layers with statistics, each forced through the six
+    // variants, the choice is 0.9 % from the best on average and 5 % at most (with 23 ns, what the shuffles took, 1.4 and 10 %).
     const int slots = pair_slots();
     const char* bn_env = getenv("B200JT_CONV_BN");          // read on every call: tests force each variant in turn
     const char* pair_env = getenv("B200JT_CONV_PAIR");
@@ -506,7 +508,7 @@ int conv2d_tc(const void* x, const void* w, void* y, float* stats, const ConvSha
             if ((forced_bn == 64 || forced_bn == 128 || forced_bn == 256) && forced_bn != b) continue;
             const int64_t t = (A.pixels + BM * (p + 1) - 1) / (BM * (p + 1)) * ((s.Co + b - 1) / b);
             const double block = 300 + (p ? 0.57 : 0.69) * b;
-            const double epilogue = 600 + b * (stats ? 23.0 : 12.5);
+            const double epilogue = 600 + b * 12.5;
             const int n = p ? slots : kNumSMs;
             const double ns = (double)((t + n - 1) / n) * (k_blocks * block + 0.5 * epilogue + 250 * p) + epilogue;
             if (ns < best) { best = ns; pair = p; bn = b; }
