@@ -828,8 +828,10 @@ int conv2d_wgrad_tc(const void* x, const void* dy, void* dw, const ConvShape& s,
     cudaLaunchAttribute early;
     early.id = cudaLaunchAttributeProgrammaticStreamSerialization; early.val.programmaticStreamSerializationAllowed = 1;
     cfg.gridDim = dim3(grid); cfg.blockDim = dim3(THREADS); cfg.stream = st; cfg.attrs = &early;
-    // An early start saves some 3 us; but the CTAs then stand on the SMs in the order the layout pass left them, and the taps that
-    // share x and dy through L2 lie further apart: 256 x 256 x 56 x 56 0.93 -> 0.95 ms. Hence for kernels of up to some 150 us.
+    // An early start saves 0.4 to 1.4 us from a graph, more of direct launches; but the CTAs then stand on the SMs in the order the
+    // layout pass left them, and the taps that share x and dy through L2 lie further apart. Nine layers of 0.7e10 to 1.2e11 operations are all
+    // faster with it (64 x 64 x 56 x 56 85.6 -> 84.7 us, 128 x 256 x 28 x 28 134.2 -> 133.4); of four with 2.4e11 one is slower
+    // (256 x 256 x 28 x 28 241.7 -> 244.8), the others as they were; from 3.6e11 on the power cap's noise hides it.
     cfg.numAttrs = 2.0 * taps * s.C * s.Co * s.N * OHW < 2e11 ? 1 : 0;
     cfg.dynamicSmemBytes = p.taps_per_cta == 2 ? Ring<2>::SMEM_BYTES : Ring<1>::SMEM_BYTES;
     const auto kernel = p.taps_per_cta == 2 ? (p.bn == 256 ? wgrad_bf16_kernel<256, 2> : wgrad_bf16_kernel<128, 2>)

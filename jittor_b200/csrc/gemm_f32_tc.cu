@@ -1,6 +1,7 @@
 // float32 matmul on the 5th-generation tensor cores: every operand is split into three bfloat16 parts that add up to it
-// (x = x0 + x1 + x2, each part the rest rounded to nearest), and C is the sum of the six products whose weight is above
-// 2^-27: x0 y0 + x0 y1 + x1 y0 + x1 y1 + x0 y2 + x2 y0. The products of bfloat16 parts are exact in float32.
+// (x = x0 + x1 + x2, each part the rest rounded to nearest), and C is the sum of the six largest of the nine products of parts:
+// x0 y0 + x0 y1 + x1 y0 + x1 y1 + x0 y2 + x2 y0. The other three are 2^-24 of a product together at most, and leave an error of 2^-27.4
+// (2-norm, normal operands) by themselves. The products of bfloat16 parts are exact in float32.
 //
 //   split pass   both operands -> three planes of bfloat16 rows at a pitch TMA takes, one launch;
 //   main kernel  the warp-specialised ring of the bfloat16 GEMM with stages of 32 of K that hold all planes of both operands
@@ -9,8 +10,11 @@
 //                the largest into a fresh accumulator, and the epilogue's warps add it to float32 registers while the next
 //                two stages fill the other one. (After every stage, the way of the accumulators out of TMEM is what bounds a
 //                pair: 456 instead of 349 us for 4096 x 2048 x 4096.)
-//   error        relative to a 64-bit product (2-norm, normal operands): 0.8e-7 to 1.3e-7 for K = 64 to 4096, where the kernel
-//                on the FMA pipe, whose chains are longer, has 1.4e-7 to 8.1e-7.
+//   error        relative to a 64-bit product (2-norm): normal operands 0.8e-7 to 1.3e-7 for K = 64 to 4096, where the kernel
+//                on the FMA pipe, whose chains are longer, has 1.3e-7 to 8.1e-7. Operands of one sign (|normal|): 0.8e-7 to 1.3e-7,
+//                of which 0.84e-7 is the truncation, always towards zero; the FMA kernel 0.5e-7 (500 x 4096 x 1000, K in short
+//                chains over many CTAs) to 1.9e-7 (1024 x 777 x 1024). Collecting after every stage where CTAs work alone: one sign
+//                0.66e-7 to 0.9e-7, but both signs up to 1.6e-7 and up to 4 % more time.
 //   few tiles    K is split over a cluster of up to 8 CTAs that fold their tiles through distributed shared memory in rank
 //                order; large products use CTA pairs (tcgen05 cta_group::2, 256 x 256 tiles).
 //

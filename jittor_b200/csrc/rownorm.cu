@@ -475,7 +475,9 @@ static int launch_rows(const T* x, T* y, const float* gamma, const float* beta, 
     row_reg_kernel<T, V, GROUP, VPT, OP><<<row_grid(rows, GROUP), cta_of(GROUP), 0, st>>>(x, y, gamma, beta, rows, (int)cols, eps)
     if (!vec_ok && cols <= 256 * 32) {
         using V = Single<T>;
-        // rows in flight cover the latency of a row's loads and reductions: [60000, 301] float32 softmax 77 us with 256 threads to
+        // The fewest threads whose share of the row stays in registers with enough CTAs beside them: one array of the row here, so 16
+        // elements to a thread; the gradient of softmax holds two and goes to 8, that of LayerNorm keeps the sums of its columns
+        // besides. Rows in flight cover the latency of a row's loads and reductions: [60000, 301] float32 softmax 77 us with 256 threads to
         // the row, 24 with a warp; [20000, 777] bfloat16 29 and 21 with 128
         if (cols <= 32 * 8) B200JT_ROW(32, 8);
         else if (cols <= 32 * 16) B200JT_ROW(32, 16);
@@ -648,7 +650,8 @@ static int launch_softmax_bwd(const T* y, const T* dy, T* dx, int64_t rows, int6
     softmax_bwd_reg_kernel<T, V, GROUP, VPT, LOG><<<row_grid(rows, GROUP), cta_of(GROUP), 0, st>>>(y, dy, dx, rows, (int)cols)
     if (!vec_ok && cols <= 256 * 32) {
         using V = Single<T>;
-        // [60000, 301] float32: 66 us with 256 threads to the row, 40 with 64; [43000, 777] bfloat16 56 and, with 128, 72
+        // up to 8 elements of two arrays to a thread (the forward pass: 16 of one). [60000, 301] float32: 66 us with 256 threads to the row,
+        // 40 with 64; [43000, 777] bfloat16 56 and, with 128, 72
         if (cols <= 32 * 4) B200JT_SB(32, 4);
         else if (cols <= 32 * 8) B200JT_SB(32, 8);
         else if (cols <= 64 * 8) B200JT_SB(64, 8);

@@ -55,7 +55,7 @@ def test_f32_tensor_core_matmul(m, k, n, pair, bn, splits, ta, tb):
 # Relative to the result, operands of both signs and of one. Truncation loses at most 2^-23 of the sum so far at each of the last four
 # additions of a group, 1.25 * 2^-23 of its sum on average where all have one sign; the group sums, up to 64 of them, are rounded to
 # nearest, 2^-24 each, in random directions. Without the products of the third parts (2^-18 of an operand) or of the two second
-# parts it would be some ten times the bound.
+# parts the error for operands of both signs would be 8 to 12 times the bound.
 @pytest.mark.parametrize("pair,bn,splits", [(0, 128, 1), (0, 64, 8), (1, 256, 1)])
 @pytest.mark.parametrize("k", [64, 257, 1024, 4096])
 @pytest.mark.parametrize("sign", ["both", "one"])
